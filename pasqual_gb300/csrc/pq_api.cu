@@ -80,12 +80,11 @@ struct pq_ctx {
     bool have_reads = false;
 
     // per direction
-    DevBuf sa[2], blk[2], sb[2], ri[2], kstart[2], kend[2], pk[2], isa[2];
+    DevBuf sa[2], blk[2], sb[2], ri[2], kstart[2], kend[2], pk[2];
     bool sa_ok[2] = {false, false}, fm_ok[2] = {false, false};
     int fm_k[2] = {0, 0};
     DevBuf sort_tmp, counts;
-    const uint32_t* sorted_keys[2] = {nullptr, nullptr};   // the last sort's keys, inside sort_tmp
-    int kmer_from_sort[2] = {0, 0};                         // k of the k-mer table a chunked sort entered
+    int kmer_from_sort[2] = {0, 0};                         // k of the k-mer table the last sort entered
     const uint8_t* bwt_hint[2] = {nullptr, nullptr};       // the last sort's BWT symbols, inside sort_tmp
     bool pk_ok[2] = {false, false};                        // pk[dir] holds this read set's packed text
     uint64_t sort_chunk = 0;                                // suffixes per sort chunk (0: automatic)
@@ -242,7 +241,6 @@ void pq_destroy(pq_ctx* ctx) {
         ctx->kstart[d].release();
         ctx->kend[d].release();
         ctx->pk[d].release();
-        ctx->isa[d].release();
         ctx->lx_bnd[d].release();
         ctx->lx_base[d].release();
         ctx->lx_par[d].release();
@@ -342,9 +340,8 @@ int pq_get_counts(pq_ctx* ctx, pq_idx C[6], pq_idx suffix_count[4], pq_idx prefi
     return PQ_OK;
 }
 
-// side_outputs: also the BWT symbols of the rows the group refinement places (FM-index work done
-// where the refinement leaves DRAM idle; pq_build_index asks for them), and for a chunked sort the
-// k-mer table from its chunks' keys.  pq_sort itself computes the suffix array only.
+// side_outputs: also every row's BWT symbol and the k-mer table, which the sort has at hand when a
+// bucket is finished (pq_build_index asks for them).  pq_sort itself computes the suffix array only.
 static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
     if (!ctx || (dir != 0 && dir != 1)) return PQ_ERR_ARG;
     if (!ctx->have_reads) return fail(ctx, PQ_ERR_STATE, "pq_set_reads first");
@@ -352,38 +349,23 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
     const size_t n = n_rows(ctx);
     CK(ctx->sa[dir].ensure(n * sizeof(idx_t) + 64));
     CK(ctx->pk[dir].ensure((n / 32 + 4) * sizeof(uint64_t)));
-    // one pass below 2^31 suffixes (32-bit group ranks), else chunks of 6-base buckets
-    const size_t one_pass_max = (size_t(1) << 31) - 1;
-    const bool chunked = n > one_pass_max || (ctx->sort_chunk && n > ctx->sort_chunk);
-    const size_t cap = std::min(ctx->sort_chunk ? size_t(ctx->sort_chunk) : (size_t(1) << 30), one_pass_max);
-    size_t tmp_bytes = chunked ? pq::suffix_sort_chunked_tmp_bytes(n, cap) : pq::suffix_sort_tmp_bytes(n);
+    const size_t cap = size_t(ctx->sort_chunk);
+    const size_t tmp_bytes = pq::suffix_sort_tmp_bytes(n, ctx->num_reads, ctx->L, cap);
     CK(ctx->sort_tmp.ensure(tmp_bytes));
     CK(cudaEventRecord(ctx->ev0, ctx->st));
-    ctx->sorted_keys[0] = ctx->sorted_keys[1] = nullptr;     // the scratch is about to be reused
-    ctx->bwt_hint[0] = ctx->bwt_hint[1] = nullptr;
-    const uint8_t** hint_out = side_outputs ? &ctx->bwt_hint[dir] : nullptr;
-    idx_t* isa_out = nullptr;       // the search needs no inverse suffix array
-    // a chunked index-build sort also enters the k-mer table from its chunks' keys (k >= 6: a
-    // k-mer's rows then lie in one 6-base bucket, so in one chunk)
-    ctx->kmer_from_sort[dir] = 0;
+    ctx->bwt_hint[0] = ctx->bwt_hint[1] = nullptr;           // the scratch is about to be reused
     const int kk = ctx->seed_k;
-    const bool kmer_in_sort = side_outputs && chunked && kk >= 6 && kk <= pq::kSortKeyBases;
-    if (kmer_in_sort) {
+    ctx->kmer_from_sort[dir] = 0;
+    if (side_outputs) {
         const size_t nk = size_t(1) << (2 * kk);
         CK(ctx->kstart[dir].ensure(nk * sizeof(idx_t)));
         CK(ctx->kend[dir].ensure(nk * sizeof(idx_t)));
-        CK(pq::kmer_table_clear(kk, ctx->kstart[dir].as<idx_t>(), ctx->kend[dir].as<idx_t>(), ctx->st));
     }
-    int rc = chunked ? pq::suffix_sort_chunked(ctx->reads.as<uint8_t>(), ctx->num_reads, ctx->L, dir,
-                                               ctx->sa[dir].as<idx_t>(), cap, ctx->sort_tmp.p, tmp_bytes, ctx->st,
-                                               hint_out, ctx->pk[dir].as<uint64_t>(), isa_out,
-                                               idx_t(ctx->L - ctx->t),
-                                               kmer_in_sort ? ctx->kstart[dir].as<idx_t>() : nullptr,
-                                               kmer_in_sort ? ctx->kend[dir].as<idx_t>() : nullptr, kk)
-                     : pq::suffix_sort(ctx->reads.as<uint8_t>(), ctx->num_reads, ctx->L, dir,
-                                       ctx->sa[dir].as<idx_t>(), ctx->sort_tmp.p, tmp_bytes, ctx->st,
-                                       &ctx->sorted_keys[dir], hint_out, ctx->pk[dir].as<uint64_t>(), isa_out,
-                                       idx_t(ctx->L - ctx->t));
+    bool kmer_done = false;
+    const int rc = pq::suffix_sort(ctx->reads.as<uint8_t>(), ctx->num_reads, ctx->L, dir, ctx->sa[dir].as<idx_t>(), cap,
+                                   ctx->sort_tmp.p, tmp_bytes, ctx->st, side_outputs ? &ctx->bwt_hint[dir] : nullptr,
+                                   ctx->pk[dir].as<uint64_t>(), side_outputs ? ctx->kstart[dir].as<idx_t>() : nullptr,
+                                   side_outputs ? ctx->kend[dir].as<idx_t>() : nullptr, kk, &kmer_done);
     ctx->pk_ok[dir] = rc == 0;
     if (rc == int(cudaErrorNotSupported))
         return fail(ctx, PQ_ERR_CAPACITY, "suffix sort: a 6-base bucket holds more suffixes than a sort chunk");
@@ -391,7 +373,7 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
     CK(cudaEventRecord(ctx->ev1, ctx->st));
     CK(cudaEventSynchronize(ctx->ev1));
     cudaEventElapsedTime(&ctx->ms_sort, ctx->ev0, ctx->ev1);
-    if (kmer_in_sort) ctx->kmer_from_sort[dir] = kk;
+    if (kmer_done) ctx->kmer_from_sort[dir] = kk;
     ctx->sa_ok[dir] = true;
     ctx->fm_ok[dir] = false;
     ctx->graph_ok = false;
@@ -414,7 +396,6 @@ int pq_set_sa(pq_ctx* ctx, int dir, const pq_idx* sa, int from_device) {
         CK(cudaMemcpyAsync(ctx->sa[dir].p, sa, n * sizeof(idx_t),
                            from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    ctx->sorted_keys[dir] = nullptr;
     ctx->bwt_hint[dir] = nullptr;
     ctx->kmer_from_sort[dir] = 0;
     ctx->sa_ok[dir] = true;
@@ -518,7 +499,6 @@ int pq_build_fm(pq_ctx* ctx, int dir) {
     CK(ctx->kstart[dir].ensure(nk * sizeof(idx_t)));
     CK(ctx->kend[dir].ensure(nk * sizeof(idx_t)));
     CK(ctx->pk[dir].ensure((n / 32 + 4) * sizeof(uint64_t)));
-    ctx->isa[dir].release();
     CK(cudaEventRecord(ctx->ev0, ctx->st));
     if (!ctx->pk_ok[dir])
         CK(pq::pack_text(ctx->reads.as<uint8_t>(), n, idx_t(ctx->L), dir, ctx->pk[dir].as<uint64_t>(), ctx->st));
@@ -529,7 +509,7 @@ int pq_build_fm(pq_ctx* ctx, int dir) {
     if (ctx->kmer_from_sort[dir] != k)
         CK(pq::build_kmer_table(ctx->sa[dir].as<idx_t>(), ctx->num_reads, idx_t(ctx->L), k,
                                 ctx->kstart[dir].as<idx_t>(), ctx->kend[dir].as<idx_t>(), ctx->st,
-                                ctx->sorted_keys[dir], ctx->pk[dir].as<uint64_t>()));
+                                ctx->pk[dir].as<uint64_t>()));
     ctx->kmer_from_sort[dir] = 0;
     CK(cudaEventRecord(ctx->ev1, ctx->st));
     CK(cudaEventSynchronize(ctx->ev1));
@@ -557,7 +537,6 @@ int pq_build_index(pq_ctx* ctx) {
     // the sort's working memory is not needed by the search: give it back when device
     // memory is short (under a quarter free), else keep it for the next build of the same size
     // (a cudaMalloc and cudaFree of tens of GB per build)
-    ctx->sorted_keys[0] = ctx->sorted_keys[1] = nullptr;
     ctx->bwt_hint[0] = ctx->bwt_hint[1] = nullptr;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < total_b / 4) {

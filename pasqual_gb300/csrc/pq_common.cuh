@@ -76,8 +76,9 @@ struct FmView {
 struct DivL {
     uint64_t m;
     uint32_t L;
+    uint32_t m32;       // floor((2^32 - 1) / L)
 };
-inline DivL make_divl(uint32_t L) { return DivL{~uint64_t(0) / L + 1, L}; }
+inline DivL make_divl(uint32_t L) { return DivL{~uint64_t(0) / L + 1, L, ~uint32_t(0) / L}; }
 __device__ __forceinline__ uint64_t div_l(uint64_t p, const DivL& d) { return __umul64hi(p, d.m); }
 
 namespace pq {

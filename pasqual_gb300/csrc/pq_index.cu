@@ -28,9 +28,9 @@ __device__ __forceinline__ int packed_at(const uint64_t* __restrict__ pk, size_t
 
 // One warp per 64-row block: BWT symbol of each row (`$` for a read-start suffix, else the
 // preceding base), packed into lo/hi/dol masks with ballots; per-block symbol counts go into
-// cnt[] for the superblock pass.  A row's symbol comes from the sort's hints when it left one
-// (hint != 0xff: the rows its group refinement placed), else from the packed text when given (a
-// quarter of the bytes of the text, so more of it stays in L2), else from the text.
+// cnt[] for the superblock pass.  A row's symbol comes from the sort when it left them (hint), else
+// from the packed text when given (a quarter of the bytes of the text, so more of it stays in L2),
+// else from the text.
 __global__ void k_bwt_blocks(const idx_t* __restrict__ sa, const uint8_t* __restrict__ reads,
                              const uint64_t* __restrict__ pk, const uint8_t* __restrict__ hint, idx_t n, idx_t L,
                              int dir, idx_t nblk, OccBlock* __restrict__ blk) {
@@ -300,59 +300,6 @@ __global__ void k_kmer_bounds_pk(const idx_t* __restrict__ sa, const uint64_t* _
     }
 }
 
-// k-mer table straight from the sorted suffix keys (first 14 bases in bits 31..4, min(length, 14)
-// in bits 3..0), read in order: a row's k-mer is the key's top 2k bits when the suffix has k bases
-__device__ __forceinline__ uint32_t key_code(uint32_t key, int k) {
-    return int(key & 15) >= k ? (key >> (32 - 2 * k)) : 0xffffffffu;
-}
-
-// four rows a thread from one 16-byte load (the key array starts 16-byte aligned), plus the
-// neighbours on either side; key[i] is the key of row off + i (the keys of one chunk of a chunked
-// sort: for k >= 6 a k-mer's rows share one 6-base bucket of that sort, so never span two chunks)
-__global__ void k_kmer_bounds_keys(const uint32_t* __restrict__ key, idx_t n, int k, idx_t* __restrict__ kstart,
-                                   idx_t* __restrict__ kend, size_t off) {
-    const size_t stride = size_t(gridDim.x) * blockDim.x;
-    const size_t nn = size_t(n);
-    for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; 4 * q < nn; q += stride) {
-        const size_t r0 = 4 * q;
-        uint32_t c[6];                               // rows r0 - 1 .. r0 + 4
-        if (r0 + 4 <= nn) {
-            const uint4 v = *reinterpret_cast<const uint4*>(key + r0);
-            c[1] = key_code(v.x, k);
-            c[2] = key_code(v.y, k);
-            c[3] = key_code(v.z, k);
-            c[4] = key_code(v.w, k);
-        } else {
-            #pragma unroll
-            for (int u = 0; u < 4; ++u) c[1 + u] = r0 + u < nn ? key_code(key[r0 + u], k) : 0xfffffffeu;
-        }
-        c[0] = r0 > 0 ? key_code(key[r0 - 1], k) : 0xfffffffeu;
-        c[5] = r0 + 4 < nn ? key_code(key[r0 + 4], k) : 0xfffffffeu;
-        #pragma unroll
-        for (int u = 1; u <= 4; ++u) {
-            const size_t r = r0 + u - 1;
-            if (r >= nn || c[u] == 0xffffffffu) continue;
-            if (c[u - 1] != c[u]) kstart[c[u]] = idx_t(off + r);
-            if (c[u + 1] != c[u]) kend[c[u]] = idx_t(off + r);
-        }
-    }
-}
-
-
-// inverse suffix array restricted to read offsets 1..M: isa[read * M + offset - 1] = row of the
-// suffix at that offset (the rows the interval scan looks up: suffixes of length L - M .. L - 1)
-// hint (or null): the sort's BWT symbols; rows with one (!= 0xff) already have their entry
-__global__ void k_isa(const idx_t* __restrict__ sa, size_t n, idx_t L, idx_t M, idx_t* __restrict__ isa,
-                      const uint8_t* __restrict__ hint) {
-    const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += stride) {
-        if (hint && hint[r] != 0xff) continue;
-        const idx_t p = sa[r];
-        const idx_t rd = p / L, off = p - rd * L;
-        if (off >= 1 && off <= M) isa[size_t(rd) * M + (off - 1)] = idx_t(r);
-    }
-}
-
 __global__ void k_fill_idx(idx_t* __restrict__ a, size_t m, idx_t v) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) a[i] = v;
@@ -485,22 +432,12 @@ cudaError_t kmer_table_clear(int k, idx_t* kstart, idx_t* kend, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t kmer_table_from_keys(const uint32_t* keys, size_t m, size_t off, int k, idx_t* kstart, idx_t* kend,
-                                 cudaStream_t st) {
-    if (m) { k_kmer_bounds_keys<<<grid_for((m + 3) / 4, 256), 256, 0, st>>>(keys, idx_t(m), k, kstart, kend, off); note_launch(); }
-    return cudaGetLastError();
-}
-
 cudaError_t build_kmer_table(const idx_t* sa, idx_t num_reads, idx_t L, int k, idx_t* kstart, idx_t* kend,
-                             cudaStream_t st, const uint32_t* sorted_keys, const uint64_t* pk) {
+                             cudaStream_t st, const uint64_t* pk) {
     const size_t n = size_t(num_reads) * L;
     cudaError_t e = kmer_table_clear(k, kstart, kend, st);
     if (e != cudaSuccess) return e;
-    if (n && sorted_keys && k <= kSortKeyBases && reinterpret_cast<uintptr_t>(sorted_keys) % 16 == 0) {
-        return kmer_table_from_keys(sorted_keys, n, 0, k, kstart, kend, st);
-    } else if (n) {
-        { k_kmer_bounds_pk<<<grid_for(n, 256), 256, 0, st>>>(sa, pk, n, L, k, kstart, kend); note_launch(); }
-    }
+    if (n) { k_kmer_bounds_pk<<<grid_for(n, 256), 256, 0, st>>>(sa, pk, n, L, k, kstart, kend); note_launch(); }
     return cudaGetLastError();
 }
 
@@ -508,12 +445,6 @@ cudaError_t read_seeds(const uint8_t* reads, idx_t num_reads, int L, int dir, in
                        const idx_t* kend, idx_t* start, idx_t* size, cudaStream_t st) {
     if (num_reads)
         { k_read_seeds<<<grid_for(num_reads, 256), 256, 0, st>>>(reads, num_reads, L, dir, k, kstart, kend, start, size); note_launch(); }
-    return cudaGetLastError();
-}
-
-cudaError_t build_isa(const idx_t* sa, size_t n, idx_t L, idx_t M, idx_t* isa, cudaStream_t st,
-                      const uint8_t* hint) {
-    if (n && M) { k_isa<<<grid_for(n, 256), 256, 0, st>>>(sa, n, L, M, isa, hint); note_launch(); }
     return cudaGetLastError();
 }
 

@@ -16,19 +16,11 @@ cudaError_t build_occ(const idx_t* sa, const uint8_t* reads, idx_t num_reads, id
 cudaError_t kernel_copy(void* dst, const void* src, size_t n, cudaStream_t st);
 cudaError_t read_counts(const uint8_t* reads, idx_t num_reads, idx_t L, unsigned long long* out13,
                         cudaStream_t st);
-// k-mer table of direction dir: from the sort's keys when sorted_keys is given, else from the
-// suffix array and the packed text pk (each one streaming pass)
+// k-mer table of direction dir from the suffix array and the packed text pk (one streaming pass)
 cudaError_t build_kmer_table(const idx_t* sa, idx_t num_reads, idx_t L, int k, idx_t* kstart, idx_t* kend,
-                             cudaStream_t st, const uint32_t* sorted_keys, const uint64_t* pk);
-// The k-mer table in parts: cleared (every k-mer absent), then entered from runs of sorted keys
-// (rows off .. off + m - 1), as each chunk of a chunked sort finishes.
+                             cudaStream_t st, const uint64_t* pk);
+// the table with every k-mer absent
 cudaError_t kmer_table_clear(int k, idx_t* kstart, idx_t* kend, cudaStream_t st);
-cudaError_t kmer_table_from_keys(const uint32_t* keys, size_t m, size_t off, int k, idx_t* kstart, idx_t* kend,
-                                 cudaStream_t st);
-// rows of the suffixes at read offsets 1..M (isa[read * M + offset - 1]); M = L - t.  hint: the
-// sort's BWT symbols, whose rows (symbol != 0xff) the sort has already entered, or null (all rows)
-cudaError_t build_isa(const idx_t* sa, size_t n, idx_t L, idx_t M, idx_t* isa, cudaStream_t st,
-                      const uint8_t* hint = nullptr);
 // The per-read seed intervals the reference's sort records (index_t.interval_start/end/depth,
 // src/sufsort.c:178-209, 322-334) from a finished suffix array and the packed text of its
 // direction (pq_seeds.cu).  seed_init writes the depth-1 seeds build_idx starts from; sort_seeds

@@ -5,17 +5,21 @@
 // sort on 3-character "triplet" ranks with insertion sort for small buckets; its single-threaded
 // output order is: read-bounded suffix strings, end-of-read lowest, ties by text position.
 //
-// GB300 design: the text is packed 2 bits per base; every suffix gets a 32-bit key made of its
-// first 14 bases (padded with A) and the number of those bases that exist (0..14) -- comparing
-// (padded bases, length) is exactly the end-of-read-lowest order on the first 14 bases.  Four
-// stable radix passes sort the keys; every group of equal keys whose suffixes go on past base 14
-// is then finished where it lies (group refinement, below).  At read coverage c such a group
-// holds about c suffixes of one genome locus whatever the key length, so a short key costs the
-// refinement little and halves the radix passes of a 29-base key.  Every radix pass is stable and
-// the input starts in text order, so equal suffixes stay in text order: the canonical tie-break.
-// Inputs the refinement cannot finish (groups larger than its scratch, reads longer than
-// 268 bases) are sorted by prefix doubling on 29-base 64-bit keys instead: ranks by
-// (rank(p), rank(p+h) or "empty" past the read end) for h = 29, 58, 116, ...
+// GB300 design: the text is packed 2 bits per base.  Every suffix becomes one 64-bit element --
+// its next bases, min(length, head), its position and its BWT symbol, highest first -- made
+// straight from the text by the first of two partition passes on the leading bases (most
+// significant digit first).  Elements are distinct and carry their position, so the partitions
+// need not be stable: a tile reserves its place in every bucket with one atomic per bucket, and
+// there is no per-tile count matrix, no scan of one and no second sweep.  The buckets (about a
+// thousand suffixes) are then finished one per CTA in shared memory: split once more by their
+// next differing bits, every sub-bucket of up to 32 suffixes sorted by one warp on the rest of its
+// bases, and the finished rows streamed out with their BWT symbols and k-mer table entries.
+// Suffixes of a few bases, of which every string has nr / 4^m equal copies, are sorted apart by a
+// stable radix sort.  Buckets too large for shared memory (low-complexity sequence) are split
+// further by the host, by the highest bits in which their elements differ; groups of more than a
+// thousand suffixes equal in all bases of their elements get new elements of their next bases.
+// Reads longer than the shared-memory network's words are sorted by prefix doubling on 29-base
+// 64-bit keys: ranks by (rank(p), rank(p+h) or "empty" past the read end) for h = 29, 58, 116, ...
 #include "pq_sort.cuh"
 #include "pq_index.cuh"
 
@@ -24,25 +28,7 @@
 
 namespace pq {
 
-constexpr int kHead = kSortKeyBases;     // bases per 32-bit head key (4 radix passes)
-constexpr int kWide = 29;                 // bases per 64-bit key (big groups, prefix doubling)
-
-// Key layouts: the bases (padded with A, first base highest) above the number of them that exist.
-//   uint32_t: 14 bases in bits 31..4, length 0..14 in bits 3..0
-//   uint64_t: 29 bases in bits 63..6, length 0..29 in bits 5..0
-template <class K> struct KeyFmt;
-template <> struct KeyFmt<uint32_t> {
-    static constexpr int bases = kHead, len_bits = 4;
-};
-template <> struct KeyFmt<uint64_t> {
-    static constexpr int bases = kWide, len_bits = 6;
-};
-template <class K>
-__device__ __forceinline__ int key_len(K k) { return int(k & K((1u << KeyFmt<K>::len_bits) - 1)); }
-constexpr int RS_THREADS = 256;
-constexpr int RS_IPT = 8;
-constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_MAX_CTAS = 152 * 4;
+constexpr int kWide = 29;                 // bases per 64-bit key of the prefix doubling
 
 __host__ __device__ __forceinline__ size_t zmin(size_t a, size_t b) { return a < b ? a : b; }
 
@@ -50,6 +36,13 @@ static inline unsigned grid_for(size_t work, int threads, int per_sm = 8) {
     size_t g = (work + threads - 1) / threads;
     size_t cap = size_t(152) * per_sm * 4;
     return unsigned(std::max<size_t>(1, std::min(g, cap)));
+}
+
+static int device_sms() {
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
 }
 
 // ------------------------------------------------------------------------------ packed text
@@ -99,66 +92,29 @@ __device__ __forceinline__ uint64_t window(const uint64_t* __restrict__ pk, size
     return s ? ((a << s) | (b >> (64 - s))) : a;
 }
 
-// the key of a suffix whose bases start the 64-bit window x and of which m exist (m >= 0)
-template <class K>
-__device__ __forceinline__ K make_key(uint64_t x, int m) {
-    constexpr int B = KeyFmt<K>::bases;
-    const int w = m < B ? m : B;
-    if (w <= 0) return K(0);
-    const uint64_t top = x & (~uint64_t(0) << (64 - 2 * w));
-    return K(K(top >> (64 - 8 * int(sizeof(K)))) | K(w));
+// the 64-bit key of a suffix whose bases start the window x and of which m exist (m >= 0): 29 bases
+// (padded with A, first base highest) in bits 63..6, how many of them exist (0..29) in bits 5..0
+__device__ __forceinline__ uint64_t make_wide_key(uint64_t x, int m) {
+    const int w = m < kWide ? m : kWide;
+    if (w <= 0) return 0;
+    return (x & (~uint64_t(0) << (64 - 2 * w))) | uint64_t(w);
 }
 
-template <class K>
-__global__ void k_init_keys(const uint64_t* __restrict__ pk, size_t n, idx_t L, K* __restrict__ key,
+__global__ void k_init_keys(const uint64_t* __restrict__ pk, size_t n, idx_t L, uint64_t* __restrict__ key,
                             idx_t* __restrict__ val) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     for (size_t p = size_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n; p += stride) {
-        key[p] = make_key<K>(window(pk, p), int(L - idx_t(p % L)));
+        key[p] = make_wide_key(window(pk, p), int(L - idx_t(p % L)));
         val[p] = idx_t(p);
     }
 }
 
-// The 32-bit head keys four positions a thread: one division for the first position's read
-// offset, the windows of all four from the same two packed-text words, and 16-byte stores of the
-// keys (and of the values when they are 32-bit); the key and value arrays start 16-byte aligned.
-__global__ void k_init_keys4(const uint64_t* __restrict__ pk, size_t n, idx_t L, uint32_t* __restrict__ key,
-                             idx_t* __restrict__ val) {
-    const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; 4 * q < n; q += stride) {
-        const size_t p0 = 4 * q;
-        int off = int(p0 % size_t(L));
-        const size_t w = p0 >> 5;
-        const uint64_t a = pk[w], b = pk[w + 1];
-        uint32_t kk[4];
-        idx_t vv[4];
-        #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int s = int((p0 + u) & 31) * 2;
-            const uint64_t x = s ? ((a << s) | (b >> (64 - s))) : a;
-            kk[u] = make_key<uint32_t>(x, int(L) - off);
-            vv[u] = idx_t(p0 + u);
-            if (++off == int(L)) off = 0;
-        }
-        if (p0 + 4 <= n) {
-            *reinterpret_cast<uint4*>(key + p0) = make_uint4(kk[0], kk[1], kk[2], kk[3]);
-            if (sizeof(idx_t) == 4) {
-                *reinterpret_cast<uint4*>(val + p0) = make_uint4(uint32_t(vv[0]), uint32_t(vv[1]), uint32_t(vv[2]),
-                                                                 uint32_t(vv[3]));
-            } else {
-                #pragma unroll
-                for (int u = 0; u < 4; ++u) val[p0 + u] = vv[u];
-            }
-        } else {
-            for (int u = 0; p0 + u < n; ++u) {
-                key[p0 + u] = kk[u];
-                val[p0 + u] = vv[u];
-            }
-        }
-    }
-}
-
 // ------------------------------------------------------------------------------ radix sort
+
+constexpr int RS_THREADS = 256;
+constexpr int RS_IPT = 8;
+constexpr int RS_WARPS = RS_THREADS / 32;
+constexpr int RS_MAX_CTAS = 152 * 4;
 
 // Digit histograms of all byte positions over the whole key array (order independent): a pass
 // whose digit is constant over all keys is the identity and is skipped.
@@ -199,39 +155,35 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const K* __restrict__
     }
 }
 
-// single-CTA exclusive scan of m 64-bit counts, in place: each of the 1024 threads sums one
-// contiguous segment, the segment totals are scanned once, and each thread rewrites its segment
-__global__ void k_scan_small(unsigned long long* __restrict__ a, size_t m) {
-    __shared__ unsigned long long wsum[32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const size_t seg = (m + 1023) / 1024;
-    const size_t b = zmin(m, size_t(threadIdx.x) * seg), e = zmin(m, b + seg);
-    unsigned long long mine = 0;
-    for (size_t i = b; i < e; ++i) mine += a[i];
-    unsigned long long x = mine;
-    #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        unsigned long long w = wsum[lane], z = w;
+// one CTA per digit: exclusive scan of the digit's counts over the parts, in place, and their total
+__global__ void __launch_bounds__(RS_THREADS) k_rs_scan(unsigned long long* __restrict__ cnt, unsigned ctas,
+                                                        unsigned long long* __restrict__ total) {
+    __shared__ unsigned long long wsum[RS_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long* row = cnt + size_t(blockIdx.x) * ctas;
+    unsigned long long carry = 0;
+    for (unsigned b = 0; b < ctas; b += RS_THREADS) {
+        const unsigned i = b + tid;
+        const unsigned long long v = i < ctas ? row[i] : 0ull;
+        unsigned long long x = v;
         #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long y = __shfl_up_sync(0xffffffffu, z, o);
-            if (lane >= o) z += y;
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-        wsum[lane] = z - w;
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        unsigned long long pre = carry, all = 0;
+        #pragma unroll
+        for (int w = 0; w < RS_WARPS; ++w) {
+            pre += w < warp ? wsum[w] : 0ull;
+            all += wsum[w];
+        }
+        if (i < ctas) row[i] = pre + x - v;
+        carry += all;
+        __syncthreads();
     }
-    __syncthreads();
-    unsigned long long run = wsum[wid] + x - mine;
-    for (size_t i = b; i < e; ++i) {
-        unsigned long long v = a[i];
-        a[i] = run;
-        run += v;
-    }
+    if (tid == 0) total[blockIdx.x] = carry;
 }
 
 // 16-byte asynchronous global -> shared copies (bypassing registers and L1)
@@ -262,7 +214,8 @@ constexpr int RS_TILE_MAX = 4096;           // parts are whole multiples of ever
 template <class K, class V>
 __global__ void __launch_bounds__(RsCfg<K, V>::threads, RsCfg<K, V>::min_blocks)
 k_rs_downsweep(const K* __restrict__ kin, const V* __restrict__ vin, K* __restrict__ kout, V* __restrict__ vout,
-               size_t n, int shift, size_t part, const unsigned long long* __restrict__ offs, int staged) {
+               size_t n, int shift, size_t part, const unsigned long long* __restrict__ offs,
+               const unsigned long long* __restrict__ total, int staged) {
     constexpr int T = RsCfg<K, V>::threads;
     constexpr int TILE = RsCfg<K, V>::tile;
     constexpr int NW = T / 32;
@@ -279,7 +232,25 @@ k_rs_downsweep(const K* __restrict__ kin, const V* __restrict__ vin, K* __restri
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt_mask = (1u << lane) - 1;
-    for (int d = tid; d < 256; d += T) base[d] = offs[size_t(d) * gridDim.x + blockIdx.x];
+    {   // a digit's place: the totals of the smaller digits plus the earlier parts' counts
+        __shared__ unsigned long long s_tot[8];
+        unsigned long long v0 = 0, x = 0;
+        if (tid < 256) {
+            v0 = total[tid];
+            x = v0;
+            #pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) s_tot[warp] = x;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            for (int w = 0; w < warp; ++w) x += s_tot[w];
+            base[tid] = x - v0 + offs[size_t(tid) * gridDim.x + blockIdx.x];
+        }
+    }
     const size_t beg = size_t(blockIdx.x) * part;
     const size_t end = zmin(n, beg + part);
     auto prefetch = [&](size_t t) {
@@ -397,7 +368,6 @@ static size_t rs_down_smem() {
     constexpr int T = RsCfg<K, V>::threads, TILE = RsCfg<K, V>::tile;
     return 2 * size_t(TILE) * (sizeof(K) + sizeof(V)) + size_t(T / 32 + 2) * 256 * 4 + 32 * 4 + 256 * 8;
 }
-
 cudaError_t pack_text(const uint8_t* reads, size_t n, idx_t L, int dir, uint64_t* pk, cudaStream_t st) {
     const size_t nwords = n / 32 + 4;
     { k_pack_text<<<grid_for(nwords, 256), 256, 0, st>>>(reads, n, L, dir, nwords, pk); note_launch(); }
@@ -406,7 +376,7 @@ cudaError_t pack_text(const uint8_t* reads, size_t n, idx_t L, int dir, uint64_t
 
 size_t radix_tmp_bytes(size_t n) {
     (void)n;
-    return (size_t(256) * RS_MAX_CTAS + 8 * 256 + 64) * sizeof(unsigned long long);
+    return (size_t(256) * RS_MAX_CTAS + 9 * 256 + 64) * sizeof(unsigned long long);
 }
 
 template <class K, class V>
@@ -418,6 +388,7 @@ int radix_sort_pairs(K** k0, V** v0, K** k1, V** v1, size_t n, int lo_bit, int h
     if (tmp_bytes < radix_tmp_bytes(n)) return int(cudaErrorInvalidValue);
     unsigned long long* cnt = reinterpret_cast<unsigned long long*>(tmp);
     unsigned long long* gh = cnt + size_t(256) * RS_MAX_CTAS;
+    unsigned long long* total = gh + 8 * 256;
     std::vector<unsigned long long> h(size_t(D) * 256, 0);
     if (skip_trivial) {
         cudaMemsetAsync(gh, 0, 8 * 256 * sizeof(unsigned long long), st);
@@ -448,25 +419,21 @@ int radix_sort_pairs(K** k0, V** v0, K** k1, V** v1, size_t n, int lo_bit, int h
             if (h[size_t(d) * 256 + b] == n) trivial = true;
         if (trivial) continue;
         { k_rs_upsweep<K><<<unsigned(ctas), RS_THREADS, 0, st>>>(*k0, n, 8 * d, part, cnt); note_launch(); }
-        { k_scan_small<<<1, 1024, 0, st>>>(cnt, 256 * ctas); note_launch(); }
+        { k_rs_scan<<<256, RS_THREADS, 0, st>>>(cnt, unsigned(ctas), total); note_launch(); }
         // whole tiles are prefetched by 16-byte copies when both inputs are 16-byte aligned
         const int staged = (reinterpret_cast<uintptr_t>(*k0) % 16 == 0 && reinterpret_cast<uintptr_t>(*v0) % 16 == 0);
         { k_rs_downsweep<K, V><<<unsigned(ctas), RsCfg<K, V>::threads, smem, st>>>(*k0, *v0, *k1, *v1, n, 8 * d, part,
-                                                                                   cnt, staged); note_launch(); }
+                                                                                   cnt, total, staged); note_launch(); }
         std::swap(*k0, *k1);
         std::swap(*v0, *v1);
     }
     return int(cudaGetLastError());
 }
 
-template int radix_sort_pairs<uint64_t, uint32_t>(uint64_t**, uint32_t**, uint64_t**, uint32_t**, size_t, int, int,
-                                                  void*, size_t, cudaStream_t, bool);
-template int radix_sort_pairs<uint64_t, uint64_t>(uint64_t**, uint64_t**, uint64_t**, uint64_t**, size_t, int, int,
-                                                  void*, size_t, cudaStream_t, bool);
-template int radix_sort_pairs<uint32_t, uint32_t>(uint32_t**, uint32_t**, uint32_t**, uint32_t**, size_t, int, int,
-                                                  void*, size_t, cudaStream_t, bool);
-template int radix_sort_pairs<uint32_t, uint64_t>(uint32_t**, uint64_t**, uint32_t**, uint64_t**, size_t, int, int,
-                                                  void*, size_t, cudaStream_t, bool);
+template int radix_sort_pairs<uint64_t, idx_t>(uint64_t**, idx_t**, uint64_t**, idx_t**, size_t, int, int, void*, size_t,
+                                               cudaStream_t, bool);
+template int radix_sort_pairs<uint32_t, idx_t>(uint32_t**, idx_t**, uint32_t**, idx_t**, size_t, int, int, void*, size_t,
+                                               cudaStream_t, bool);
 
 // ------------------------------------------------------------------------------ group ranks
 
@@ -597,372 +564,1110 @@ __global__ void k_copy_vals(const V* __restrict__ v, size_t n, idx_t* __restrict
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) sa[i] = idx_t(v[i]);
 }
-
-// ------------------------------------------------------------------------------ group refinement
+// ------------------------------------------------------------------------------ elements and plan
 //
-// After the sort on 14-base keys, every group of equal keys whose suffixes all go on past base 14
-// still has to be ordered.  At read coverage c such groups hold about c suffixes, so instead of
-// more whole-array passes each group is finished where it lies: every suffix loads the rest of
-// its bases as W 64-bit words (bases past its end read as A) and the group is sorted by
-// (words, suffix length, position) -- the end-of-read-lowest order, ties by position.  Groups of
-// up to 32 and up to 128 suffixes are sorted by one warp in registers (1 or 4 per lane, several
-// groups packed per warp), up to 1024 by one CTA in shared memory, all with bitonic networks;
-// larger ones by a radix sort of their range on the next 29 bases.
+// An element, highest bits first: kbits of the suffix's text (after the first d1 bits, padded with
+// A past its end), min(length, head) in 5 bits, the position, the BWT symbol in 3 bits (0 = `$`,
+// else the preceding base).  Comparing two elements of one first-level bucket as integers compares
+// the suffixes' first `head` bases, end-of-read lowest, then the positions.
 
-constexpr int kRefineMaxWords = 8;          // suffixes up to 14 + 30 + 224 bases
-constexpr int kGroupWarp4 = 128;            // largest group sorted by one warp, 4 per lane
-constexpr int kGroupCta = 1024;             // largest group sorted in shared memory
+constexpr int kLenBits = 5, kSymBits = 3;
+constexpr int kLocalSmall = 2560;           // buckets finished by a CTA of 128 threads
+constexpr int kLocalLarge = 8192;           // ... of 256 threads; larger ones are split further
+constexpr int kSplitTile = 8192;            // elements per tile of the partition passes
+constexpr int kSplitThreads = 512;
+constexpr int kMaxDigit = 11;               // bits of one partition pass
+constexpr int kMaxWords = 9;                // 64-bit words of a suffix the networks compare
+constexpr int kChunkMaxLen = 268;           // longest reads sorted in chunks
+#ifdef PQ_IDX64
+using kmer_int = unsigned long long;
+#else
+using kmer_int = unsigned;
+#endif
+constexpr int kMoreBits = 10;               // bits of one further split
 
-// Group classes: 0 = 2..32 suffixes, 1 = 33..128, 2 = 129..1024 (entries (start << 24) | size),
-// 3 = larger (start, size pairs).
-struct GroupLists {
-    unsigned long long* list[4];
-    unsigned long long* counts;             // [4]
-    size_t cap[4];                          // entries (pairs for class 3)
-    uint8_t* bwt;                           // BWT symbols of the rows the refinement places, or null
-    idx_t* isa;                             // their inverse-SA entries (offsets 1..M), or null
-    idx_t isa_m;                            // M
-    size_t row_base;                        // suffix-array row of val[0]
+struct MsdPlan {
+    size_t n;
+    DivL dl;
+    int P;                  // position bits
+    int d1, d2;             // bits of the two partition passes (d2 = 0: one pass)
+    int kbits, head;        // text bits of an element's key; bases it and the first pass tell apart
+    int S;                  // suffixes of at most S bases are sorted apart (0: none)
+    int len_shift, key_shift;
 };
 
-// side outputs of a row the refinement has placed: its BWT symbol and, for read offsets 1..M,
-// its inverse-SA entry isa[read * M + offset - 1] = row (written here, where the refinement's
-// ALU-bound networks leave DRAM idle, instead of by a separate scatter over every row)
-__device__ __forceinline__ void row_outputs(uint8_t* __restrict__ bwt, idx_t* __restrict__ isa, idx_t M,
-                                            size_t row, idx_t pos, idx_t L, uint8_t sym) {
-    if (bwt) bwt[row] = sym;
-    if (isa) {
-        const idx_t rd = pos / L, off = pos - rd * L;
-        if (off >= 1 && off <= M) isa[size_t(rd) * M + (off - 1)] = idx_t(row);
+// d1 and d2 by the bucket size aimed at: 600 to 1200 suffixes where there are enough of them to fill
+// the chip (smaller: more counters and barriers per suffix; larger: buckets beyond the small
+// kernel's 2560 under a skewed base composition), 400 at most for inputs of under 4 M suffixes,
+// whose few buckets would otherwise leave most SMs idle.  One pass covers 2^11 buckets (its counters, and 4 elements
+// a bucket and tile, the least that fills a sector).
+static MsdPlan make_plan(size_t n, size_t nr, idx_t L, bool shorts) {
+    MsdPlan p{};
+    p.n = n;
+    p.dl = make_divl(uint32_t(L));
+    p.P = 1;
+    while ((size_t(1) << p.P) < n) ++p.P;
+    const size_t target = n < (size_t(1) << 22) ? 400 : 1200;
+    int bt = 2;
+    while (bt < 2 * kMaxDigit && (n >> bt) > target) ++bt;
+    if (n < (size_t(1) << 22)) bt = std::min(bt, kMaxDigit);
+    p.d1 = bt <= kMaxDigit ? bt : (bt + 1) / 2;
+    p.d2 = bt - p.d1;
+    p.kbits = std::min(64 - kLenBits - kSymBits - p.P, 62 - p.d1);
+    if ((p.d1 + p.kbits) & 1) --p.kbits;
+    p.head = (p.d1 + p.kbits) / 2;
+    p.len_shift = kSymBits + p.P;
+    p.key_shift = p.len_shift + kLenBits;
+    // a string of m bases has about nr / 4^m equal suffixes of that length: those of more than 512
+    // (a quarter of the suffixes at most, which bounds the memory they take)
+    if (shorts)
+        while (p.S < 7 && 4 * (p.S + 1) <= int(L) && 2 * p.S + 2 <= bt && (nr >> (2 * p.S + 2)) > 512) ++p.S;
+    return p;
+}
+
+// words of the networks: bases from the partition's own on, 29 in the first word, 32 in the others
+static int plan_words(const MsdPlan& p) {
+    const int rest = int(p.dl.L) - (p.d1 + p.d2) / 2 - 29;
+    return 1 + (rest > 0 ? (rest + 31) / 32 : 0);
+}
+
+// bases from text position p to the end of its read; positions of a 32-bit index take one 32-bit
+// multiply-high by floor(2^32 / L): the quotient is short by at most one below 2^32
+__device__ __forceinline__ int suffix_bases(size_t p, const DivL& dl) {
+#ifdef PQ_IDX64
+    return int(dl.L - uint32_t(p - div_l(p, dl) * dl.L));
+#else
+    const uint32_t x = uint32_t(p), q = __umulhi(x, dl.m32), r = x - q * dl.L;
+    return int((r >= dl.L ? 2 * dl.L : dl.L) - r);
+#endif
+}
+
+// the element of the suffix at p (m bases, whose text starts the window x, preceded by the base
+// `prev`) and its first-level digit
+__device__ __forceinline__ uint64_t make_element(const MsdPlan& a, size_t p, int m, uint64_t x, int prev, bool dollar,
+                                                 unsigned& digit) {
+    const uint64_t xm = m < 32 ? x & (~uint64_t(0) << (64 - 2 * m)) : x;
+    digit = unsigned(xm >> (64 - a.d1));
+    const uint64_t key = (xm << a.d1) >> (64 - a.kbits);
+    const int w = m < a.head ? m : a.head;
+    return (key << a.key_shift) | (uint64_t(w) << a.len_shift) | (uint64_t(p) << kSymBits) |
+           uint64_t(dollar ? 0 : prev + 1);
+}
+
+// A thread's 16 consecutive text positions from two words of the packed text: f(position, window,
+// bases to the end of the read, preceding base, first of its read)
+template <class F>
+__device__ __forceinline__ void for_positions(const uint64_t* __restrict__ pk, size_t p0, size_t n, const DivL& dl, F f) {
+    if (p0 >= n) return;
+    const size_t w = p0 >> 5;
+    const uint64_t a = pk[w], b = pk[w + 1];
+    const int s0 = int(p0 & 31);                // 0 or 16
+    int prev = s0 ? int(a >> (64 - 2 * s0)) & 3 : (w ? int(pk[w - 1]) & 3 : 0);
+    int m = suffix_bases(p0, dl);
+    #pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const int sh = 2 * (s0 + j);
+        const uint64_t x = sh ? ((a << sh) | (b >> (64 - sh))) : a;
+        if (p0 + size_t(j) < n) f(j, p0 + size_t(j), x, m, prev, m == int(dl.L));
+        prev = int(x >> 62);
+        m = m == 1 ? int(dl.L) : m - 1;
     }
 }
 
-// BWT symbol of the suffix at p: 0 (`$`) at a read start, else the preceding base (1..4)
-__device__ __forceinline__ uint8_t bwt_symbol(const uint64_t* __restrict__ pk, size_t p, idx_t L) {
-    if (p % size_t(L) == 0) return 0;
-    const size_t q = p - 1;
-    return uint8_t(((pk[q >> 5] >> (62 - 2 * int(q & 31))) & 3) + 1);
-}
-
-__device__ __forceinline__ int group_class(size_t m) {
-    if (m < 2) return -1;
-    if (m <= 32) return 0;
-    if (m <= size_t(kGroupWarp4)) return 1;
-    return m <= size_t(kGroupCta) ? 2 : 3;
-}
-
-// One CTA per tile of 4096 sorted keys.  Two bit masks per tile, by ballots: group heads, and
-// keys whose suffix is longer than the key's bases.  Then one thread per mask word walks the set
-// bits of (head & long) only: a group ends at the next head bit (in the mask; a group running past
-// the tile end is followed in global memory by a galloping search), and the groups are listed by
-// size class.  List slots are taken with one atomic per list per tile, after a block-wide prefix
-// of the per-thread counts; the walk runs twice (count, then write).
-constexpr int kGlTile = 4096;
-constexpr int kGlThreads = 256;
-constexpr int kGlPer = kGlTile / kGlThreads;      // positions per thread (j = tid + 256 i)
-constexpr int kGlWords = kGlTile / 32;
-
-__device__ __forceinline__ void block_scan4(unsigned (&c)[4], unsigned (&excl)[4], unsigned (*wsum)[4],
-                                            unsigned* tot) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned x[4] = {c[0], c[1], c[2], c[3]};
+// exclusive scan of cnt[0, bins) into start[0, bins) by the whole CTA of T threads (bins a power of
+// two; the caller synchronises before reading start); returns the total to every thread
+template <int T>
+__device__ __forceinline__ unsigned bins_exclusive(const unsigned* cnt, unsigned* start, int bins, unsigned* wsum) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int per = bins > T ? bins / T : 1;
+    const int b0 = tid * per;
+    unsigned mine = 0;
+    if (b0 < bins)
+        for (int i = 0; i < per; ++i) mine += cnt[b0 + i];
+    unsigned x = mine;
     #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, x[q], o);
-            if (lane >= o) x[q] += y;
-        }
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
-    if (lane == 31) {
-        #pragma unroll
-        for (int q = 0; q < 4; ++q) wsum[warp][q] = x[q];
-    }
+    if (lane == 31) wsum[warp] = x;
     __syncthreads();
+    unsigned pre = 0, all = 0;
     #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        unsigned before = 0, all = 0;
-        for (int w = 0; w < kGlThreads / 32; ++w) {
-            before += w < warp ? wsum[w][q] : 0u;
-            all += wsum[w][q];
+    for (int w = 0; w < T / 32; ++w) {
+        pre += w < warp ? wsum[w] : 0u;
+        all += wsum[w];
+    }
+    unsigned run = pre + x - mine;
+    if (b0 < bins)
+        for (int i = 0; i < per; ++i) {
+            const unsigned c = cnt[b0 + i];
+            start[b0 + i] = run;
+            run += c;
         }
-        excl[q] = before + x[q] - c[q];
-        tot[q] = all;
+    return all;
+}
+
+// ------------------------------------------------------------------------------ partition passes
+
+// how many suffixes start with each d1-bit prefix (padded with A)
+__global__ void __launch_bounds__(kSplitThreads) k_msd_hist(const uint64_t* __restrict__ pk, MsdPlan a,
+                                                            unsigned long long* __restrict__ cnt) {
+    __shared__ unsigned h[1 << kMaxDigit];
+    const int bins = 1 << a.d1;
+    for (int i = threadIdx.x; i < bins; i += kSplitThreads) h[i] = 0;
+    __syncthreads();
+    const size_t stride = size_t(gridDim.x) * kSplitThreads * 16;
+    for (size_t p0 = (size_t(blockIdx.x) * kSplitThreads + threadIdx.x) * 16; p0 < a.n; p0 += stride)
+        for_positions(pk, p0, a.n, a.dl, [&](int, size_t, uint64_t x, int m, int, bool) {
+            const uint64_t xm = m < 32 ? x & (~uint64_t(0) << (64 - 2 * m)) : x;
+            atomicAdd(&h[xm >> (64 - a.d1)], 1u);
+        });
+    __syncthreads();
+    for (int i = threadIdx.x; i < bins; i += kSplitThreads)
+        if (h[i]) atomicAdd(&cnt[i], (unsigned long long)h[i]);
+}
+
+// A chunk's bucket numbers: the first 6 bases (padded with A) above min(length, 6), in suffix order
+constexpr int kBucketBases = 6;
+constexpr int kBuckets = (1 << (2 * kBucketBases)) * 8;
+__device__ __forceinline__ uint32_t bucket6(uint64_t x, int m) {
+    const int w = m < kBucketBases ? m : kBucketBases;
+    const uint32_t pre = uint32_t(x >> (64 - 2 * kBucketBases)) & (~0u << (2 * (kBucketBases - w)));
+    return (pre << 3) | uint32_t(w);
+}
+
+// First pass: every suffix of more than S bases (of a chunk: whose 6-base bucket lies in
+// [c0, c1)) as an element into its d1-bit bucket.  Bound by the 8 bytes written per suffix (the
+// text is a quarter byte): a tile of 8192 positions is ranked with one shared-memory atomic a
+// suffix, takes its place in every bucket with one global atomic a bucket, and leaves through
+// shared memory in runs.
+struct MsdSmem {            // dynamic shared memory of the partition passes
+    static constexpr size_t bins = size_t(1) << kMaxDigit;
+    static constexpr size_t elems = size_t(kSplitTile) * 8;
+    static constexpr size_t bytes(int bits, bool digits) {
+        return elems + (size_t(1) << bits) * (8 + 4 + 4) + (digits ? size_t(kSplitTile) * 2 : 0);
+    }
+};
+
+__global__ void __launch_bounds__(kSplitThreads, 2) k_msd_text(const uint64_t* __restrict__ pk, MsdPlan a,
+                                                               unsigned long long* __restrict__ cursor,
+                                                               uint64_t* __restrict__ out, uint32_t c0, uint32_t c1) {
+    extern __shared__ __align__(16) unsigned char msd_smem[];
+    __shared__ unsigned wsum[kSplitThreads / 32];
+    const int bins = 1 << a.d1, tid = threadIdx.x;
+    uint64_t* se = reinterpret_cast<uint64_t*>(msd_smem);
+    unsigned long long* gb = reinterpret_cast<unsigned long long*>(se + kSplitTile);
+    unsigned* cnt = reinterpret_cast<unsigned*>(gb + bins);
+    unsigned* start = cnt + bins;
+    uint16_t* sd = reinterpret_cast<uint16_t*>(start + bins);
+    const bool chunk = c1 < uint32_t(kBuckets) || c0 > 0;
+    const size_t tiles = (a.n + kSplitTile - 1) / kSplitTile;
+    for (size_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        for (int i = tid; i < bins; i += kSplitThreads) cnt[i] = 0;
+        __syncthreads();
+        uint64_t v[16];
+        unsigned dr[16];                        // digit << 16 | rank within the tile's bucket
+        #pragma unroll
+        for (int j = 0; j < 16; ++j) dr[j] = ~0u;
+        for_positions(pk, t * kSplitTile + size_t(tid) * 16, a.n, a.dl,
+                      [&](int j, size_t p, uint64_t x, int m, int prev, bool dollar) {
+            if (m <= a.S) return;
+            if (chunk) {
+                const uint32_t c = bucket6(x, m);
+                if (c < c0 || c >= c1) return;
+            }
+            unsigned d;
+            v[j] = make_element(a, p, m, x, prev, dollar, d);
+            dr[j] = (d << 16) | atomicAdd(&cnt[d], 1u);
+        });
+        __syncthreads();
+        const unsigned total = bins_exclusive<kSplitThreads>(cnt, start, bins, wsum);
+        __syncthreads();
+        for (int d = tid; d < bins; d += kSplitThreads) {
+            const unsigned c = cnt[d];
+            if (c) gb[d] = atomicAdd(&cursor[d], (unsigned long long)c) - start[d];
+        }
+        #pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (dr[j] != ~0u) {
+                const unsigned q = start[dr[j] >> 16] + (dr[j] & 0xffffu);
+                se[q] = v[j];
+                sd[q] = uint16_t(dr[j] >> 16);
+            }
+        __syncthreads();
+        for (unsigned j = tid; j < total; j += kSplitThreads) out[gb[sd[j]] + j] = se[j];
+        __syncthreads();
     }
 }
 
-// first index >= e0 whose key differs from k (keys sorted; key[e0 - 1] == k), or n
-template <class K>
-__device__ size_t run_end(const K* __restrict__ key, size_t n, size_t e0, K k) {
-    size_t lo = e0, step = 32;                      // key[lo - 1] == k
-    size_t hi = lo;
-    while (true) {                                  // gallop: hi = first probe that differs (or n)
-        hi = lo + step < n ? lo + step : n;
-        if (hi == n || key[hi] != k) break;
-        lo = hi + 1;
-        step *= 2;
-    }
-    // the answer lies in [lo, hi]: the first index there with key != k (hi qualifies)
+// Ranges [start, end) of elements to split by one digit each, in tiles of kSplitTile: tile0 is the
+// exclusive scan of their tile counts (count + 1 entries).
+struct MsdRanges {
+    const unsigned long long* start;
+    const unsigned long long* end;
+    const unsigned* tile0;
+    const int* shift;                   // a range's digit is (element >> shift) & (2^bits - 1),
+    int ushift;                         // with one shift for all when `shift` is null
+    int count, bits;
+};
+__device__ __forceinline__ int range_of(const MsdRanges& r, unsigned tile) {
+    int lo = 0, hi = r.count - 1;
     while (lo < hi) {
-        const size_t mid = lo + (hi - lo) / 2;
-        if (key[mid] != k) hi = mid;
-        else lo = mid + 1;
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(r.tile0 + mid) <= tile) lo = mid;
+        else hi = mid - 1;
     }
     return lo;
 }
 
-template <class K>
-__global__ void __launch_bounds__(kGlThreads, 5) k_group_lists(const K* __restrict__ key, size_t n, GroupLists G,
-                                                           size_t base) {
-    __shared__ uint32_t hm[kGlWords + 1];               // heads; sentinel word at the end
-    __shared__ uint32_t lm[kGlWords];                   // long suffixes
-    __shared__ unsigned wsum[kGlThreads / 32][4];
-    __shared__ unsigned long long sbase[4];
-    __shared__ K last[kGlPer][kGlThreads / 32];         // each warp's lane-31 key, per round
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (size_t t0 = size_t(blockIdx.x) * kGlTile; t0 < n; t0 += size_t(gridDim.x) * kGlTile) {
-        // all of the thread's keys in flight at once; a key's predecessor comes from the lane
-        // before, or for lane 0 from the warp before (or the round before) through shared memory
-        K kk[kGlPer];
-        #pragma unroll
-        for (int q = 0; q < kGlPer; ++q) {
-            const size_t i = t0 + threadIdx.x + size_t(kGlThreads) * q;
-            kk[q] = i < n ? key[i] : K(0);
-        }
-        const K before_tile = (t0 > 0 && threadIdx.x == 0) ? key[t0 - 1] : K(0);
-        if (lane == 31) {
-            #pragma unroll
-            for (int q = 0; q < kGlPer; ++q) last[q][warp] = kk[q];
-        }
-        __syncthreads();
-        #pragma unroll
-        for (int q = 0; q < kGlPer; ++q) {
-            const int j = threadIdx.x + kGlThreads * q;
-            const size_t i = t0 + j;
-            K prev = __shfl_up_sync(0xffffffffu, kk[q], 1);
-            if (lane == 0) prev = warp ? last[q][warp - 1] : (q ? last[q - 1][kGlThreads / 32 - 1] : before_tile);
-            const bool head = i < n && (i == 0 || kk[q] != prev);
-            const uint32_t hb = __ballot_sync(0xffffffffu, head);
-            const uint32_t lb = __ballot_sync(0xffffffffu, i < n && key_len<K>(kk[q]) == KeyFmt<K>::bases);
-            if (lane == 0) {
-                hm[j >> 5] = hb;
-                lm[j >> 5] = lb;
-            }
-        }
-        if (threadIdx.x == 0) hm[kGlWords] = 1u;        // sentinel: the tile end
-        __syncthreads();
-        // walk: thread t < kGlWords owns mask word t
-        auto group_size = [&](int j) -> size_t {
-            int w = (j + 1) >> 5;
-            uint32_t bits = (j + 1 < kGlTile) ? hm[w] & (~0u << ((j + 1) & 31)) : hm[w];
-            while (!bits) bits = hm[++w];               // ends at the sentinel word at the latest
-            const int nxt = 32 * w + __ffs(bits) - 1;
-            const size_t i = t0 + size_t(j);
-            size_t e = t0 + size_t(nxt);
-            if (nxt >= kGlTile) e = t0 + kGlTile < n ? run_end<K>(key, n, t0 + kGlTile, key[i]) : n;
-            if (e > n) e = n;
-            return e - i;
-        };
-        const int tw = threadIdx.x;
-        const uint32_t mine = tw < kGlWords ? (hm[tw] & lm[tw]) : 0u;
-        unsigned c[4] = {0, 0, 0, 0};
-        for (uint32_t bits = mine; bits; bits &= bits - 1) {
-            const int cl = group_class(group_size(32 * tw + __ffs(bits) - 1));
-            #pragma unroll
-            for (int z = 0; z < 4; ++z) c[z] += cl == z ? 1u : 0u;
-        }
-        unsigned excl[4], tot[4];
-        block_scan4(c, excl, wsum, tot);
-        if (threadIdx.x == 0) {
-            #pragma unroll
-            for (int q = 0; q < 4; ++q) sbase[q] = tot[q] ? atomicAdd(&G.counts[q], (unsigned long long)tot[q]) : 0ull;
-        }
-        __syncthreads();
-        unsigned long long at[4] = {sbase[0] + excl[0], sbase[1] + excl[1], sbase[2] + excl[2], sbase[3] + excl[3]};
-        for (uint32_t bits = mine; bits; bits &= bits - 1) {
-            const int j = 32 * tw + __ffs(bits) - 1;
-            const size_t m = group_size(j);
-            const int cl = group_class(m);
-            const size_t i = base + t0 + size_t(j);
-            if (cl == 3) {
-                if (at[3] < G.cap[3]) {
-                    G.list[3][2 * at[3]] = i;
-                    G.list[3][2 * at[3] + 1] = m;
+__global__ void __launch_bounds__(1024) k_msd_tiles(const unsigned long long* __restrict__ start,
+                                                    const unsigned long long* __restrict__ end, int count,
+                                                    unsigned* __restrict__ tile0) {
+    __shared__ unsigned cnt[1 << kMaxDigit], ex[1 << kMaxDigit], wsum[32];
+    for (int i = threadIdx.x; i < count; i += 1024)
+        cnt[i] = unsigned((end[i] - start[i] + kSplitTile - 1) / kSplitTile);
+    __syncthreads();
+    const unsigned total = bins_exclusive<1024>(cnt, ex, count, wsum);
+    __syncthreads();
+    for (int i = threadIdx.x; i < count; i += 1024) tile0[i] = ex[i];
+    if (threadIdx.x == 0) tile0[count] = total;
+}
+
+// digit counts of every range, cnt[range << bits | digit]: a CTA takes consecutive tiles and adds
+// its counts when the range changes
+__global__ void __launch_bounds__(kSplitThreads) k_msd_count(const uint64_t* __restrict__ in, MsdRanges r,
+                                                             unsigned long long* __restrict__ cnt) {
+    __shared__ unsigned h[1 << kMaxDigit];
+    const int bins = 1 << r.bits, tid = threadIdx.x;
+    const unsigned tiles = r.tile0[r.count];
+    const unsigned per = (tiles + gridDim.x - 1) / gridDim.x;
+    const unsigned t0 = min(tiles, blockIdx.x * per), t1 = min(tiles, t0 + per);
+    if (t0 >= t1) return;
+    for (int i = tid; i < bins; i += kSplitThreads) h[i] = 0;
+    __syncthreads();
+    int q = range_of(r, t0);
+    for (unsigned t = t0; t < t1; ++t) {
+        if (t >= __ldg(r.tile0 + q + 1)) {
+            __syncthreads();
+            for (int i = tid; i < bins; i += kSplitThreads)
+                if (h[i]) {
+                    atomicAdd(&cnt[(size_t(q) << r.bits) + i], (unsigned long long)h[i]);
+                    h[i] = 0;
                 }
-                ++at[3];
-            } else if (cl >= 0) {
-                if (at[cl] < G.cap[cl]) G.list[cl][at[cl]] = (uint64_t(i) << 24) | m;
-                ++at[cl];
-            }
+            q = range_of(r, t);
+            __syncthreads();
+        }
+        const int shift = r.shift ? r.shift[q] : r.ushift;
+        const size_t b = r.start[q] + size_t(t - r.tile0[q]) * kSplitTile;
+        const size_t e = zmin(r.end[q], b + kSplitTile);
+        #pragma unroll 4
+        for (size_t i = b + tid; i < e; i += kSplitThreads) atomicAdd(&h[(in[i] >> shift) & (bins - 1)], 1u);
+    }
+    __syncthreads();
+    for (int i = tid; i < bins; i += kSplitThreads)
+        if (h[i]) atomicAdd(&cnt[(size_t(q) << r.bits) + i], (unsigned long long)h[i]);
+}
+
+// Second pass: the elements of every range into its children (cursor[range << bits | digit] is
+// their next place in `out`), a tile at a time as in the first pass; 8 bytes read and written per
+// suffix.
+__global__ void __launch_bounds__(kSplitThreads, 2) k_msd_split(const uint64_t* __restrict__ in, MsdRanges r,
+                                                                unsigned long long* __restrict__ cursor,
+                                                                uint64_t* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char msd_smem[];
+    __shared__ unsigned wsum[kSplitThreads / 32];
+    const int bins = 1 << r.bits, tid = threadIdx.x;
+    uint64_t* se = reinterpret_cast<uint64_t*>(msd_smem);
+    unsigned long long* gb = reinterpret_cast<unsigned long long*>(se + kSplitTile);
+    unsigned* cnt = reinterpret_cast<unsigned*>(gb + bins);
+    unsigned* start = cnt + bins;
+    const unsigned tiles = r.tile0[r.count];
+    constexpr int kPer = kSplitTile / kSplitThreads;
+    for (unsigned t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int q = range_of(r, t);
+        const int shift = r.shift ? r.shift[q] : r.ushift;
+        const size_t b = r.start[q] + size_t(t - __ldg(r.tile0 + q)) * kSplitTile;
+        const int m = int(zmin(size_t(kSplitTile), r.end[q] - b));
+        uint64_t v[kPer];
+        #pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = tid + j * kSplitThreads;
+            v[j] = i < m ? in[b + i] : 0;
+        }
+        for (int i = tid; i < bins; i += kSplitThreads) cnt[i] = 0;
+        __syncthreads();
+        unsigned rk[kPer];
+        #pragma unroll
+        for (int j = 0; j < kPer; ++j)
+            if (tid + j * kSplitThreads < m) rk[j] = atomicAdd(&cnt[unsigned(v[j] >> shift) & (bins - 1)], 1u);
+        __syncthreads();
+        bins_exclusive<kSplitThreads>(cnt, start, bins, wsum);
+        __syncthreads();
+        for (int d = tid; d < bins; d += kSplitThreads) {
+            const unsigned c = cnt[d];
+            if (c) gb[d] = atomicAdd(&cursor[(size_t(q) << r.bits) + d], (unsigned long long)c) - start[d];
+        }
+        #pragma unroll
+        for (int j = 0; j < kPer; ++j)
+            if (tid + j * kSplitThreads < m) se[start[unsigned(v[j] >> shift) & (bins - 1)] + rk[j]] = v[j];
+        __syncthreads();
+        for (int j = tid; j < m; j += kSplitThreads) {
+            const uint64_t e = se[j];
+            out[gb[unsigned(e >> shift) & (bins - 1)] + j] = e;
         }
         __syncthreads();
     }
 }
 
-// the W words of bases off, off+32, ... of the suffix at p (length m_len), zero past its end
-template <int W>
-__device__ __forceinline__ void suffix_words(const uint64_t* __restrict__ pk, size_t p, int m_len, int off,
-                                             uint64_t w[W]) {
-    #pragma unroll
-    for (int j = 0; j < W; ++j) {
-        const int rem = m_len - off - 32 * j;
-        uint64_t x = 0;
-        if (rem > 0) {
-            x = window(pk, p + off + 32 * size_t(j));
-            if (rem < 32) x &= ~uint64_t(0) << (64 - 2 * rem);
-        }
-        w[j] = x;
-    }
-}
+// ------------------------------------------------------------------------------ buckets
 
-template <int W>
-__device__ __forceinline__ bool tuple_less(const uint64_t a[W], uint64_t alen, uint64_t apos, const uint64_t b[W],
-                                           uint64_t blen, uint64_t bpos) {
-    #pragma unroll
-    for (int j = 0; j < W; ++j)
-        if (a[j] != b[j]) return a[j] < b[j];
-    if (alen != blen) return alen < blen;
-    return apos < bpos;
-}
+// A bucket to finish: elements [start, start + size), whose suffixes share their first `off` bases;
+// id (off = 0 only) is its d1 + d2-bit prefix.
+struct __align__(16) MsdBucket {
+    unsigned long long start;
+    unsigned size;
+    unsigned id_off;                    // off << 22 | id
+};
+constexpr int kIdBits = 22;
 
-// Groups of 2..32E suffixes, several per warp: a warp takes 8 list entries at a time and packs
-// consecutive ones into its 32E slots (slot e * 32 + lane is register set e of that lane) while
-// they fit; one bitonic network over the 32E slots on (segment, bases from `from` on, length,
-// slot) then sorts every packed group in place (each segment keeps its slots, since segments are
-// numbered in slot order and empty slots sort last).  The segment number (3 bits) rides in the top
-// of the first word, which holds the next 30 bases; the other words hold 32 each.  A group's
-// members arrive in ascending position (every radix pass is stable from text order), so the
-// original slot breaks ties exactly as the position does; the positions wait in shared memory
-// and are gathered by slot at the end.  Distances below 32 exchange by shuffle, larger ones swap
-// registers within a lane.
-template <int W>
-struct RefineItem {
-    uint64_t w[W];                              // w[0] = segment (3 bits) | 30 bases | 0
-    uint32_t tail;                              // (length << 8) | original slot
+// Device counters of one sort
+struct MsdCounters {
+    unsigned long long small, large, more, mid, big, huge;      // list lengths (see MsdLists)
+    unsigned long long next_small, next_large;                  // next bucket to take
+};
+// small, large: buckets for the two local kernels; more: buckets larger than both; mid, big, huge:
+// groups of 33..128, 129..1024 and more suffixes equal in all bases of their elements
+struct MsdLists {
+    MsdBucket *small, *large, *more;
+    unsigned long long *mid, *big, *huge;       // start << 24 | bases known equal << 14 | size
+    unsigned long long cap_more, cap_mid, cap_big, cap_huge;
+    MsdCounters* c;
 };
 
-// the words of RefineItem for the suffix at p (length m_len): bases from `off` on, zero past its end
-template <int W>
-__device__ __forceinline__ void refine_words(const uint64_t* __restrict__ pk, size_t p, int m_len, int off, uint32_t seg,
-                                             uint64_t w[W]) {
-    const int rem0 = m_len - off;
-    uint64_t x = 0;
-    if (rem0 > 0) {
-        x = window(pk, p + off) & (~uint64_t(0) << 4);            // 30 bases
-        if (rem0 < 30) x &= ~uint64_t(0) << (64 - 2 * rem0);
-    }
-    w[0] = (uint64_t(seg) << 61) | (x >> 3);
+__device__ __forceinline__ void list_bucket(const MsdLists& G, int cls, const MsdBucket& b) {
+    const int lane = threadIdx.x & 31;
     #pragma unroll
-    for (int j = 1; j < W; ++j) {
-        const int rem = rem0 - 30 - 32 * (j - 1);
-        uint64_t y = 0;
-        if (rem > 0) {
-            y = window(pk, p + off + 30 + 32 * size_t(j - 1));
-            if (rem < 32) y &= ~uint64_t(0) << (64 - 2 * rem);
-        }
-        w[j] = y;
+    for (int z = 0; z < 3; ++z) {
+        const unsigned peers = __ballot_sync(0xffffffffu, cls == z);
+        if (!peers) continue;
+        unsigned long long* c = z == 0 ? &G.c->small : (z == 1 ? &G.c->large : &G.c->more);
+        MsdBucket* l = z == 0 ? G.small : (z == 1 ? G.large : G.more);
+        unsigned long long at = 0;
+        if (lane == __ffs(peers) - 1) at = atomicAdd(c, (unsigned long long)__popc(peers));
+        at = __shfl_sync(0xffffffffu, at, __ffs(peers) - 1) + __popc(peers & ((1u << lane) - 1u));
+        if (cls == z && (z != 2 || at < G.cap_more)) l[at] = b;
     }
 }
+
+// The children of first-level bucket blockIdx.x: from their counts (of long suffixes, or with
+// `incl` of all) and the short suffixes of each (which come first in it), the place of each child's
+// long suffixes (lstart, kept, and cursor, which the next pass advances); with `lists`, the
+// non-empty ones listed by size.
+constexpr int kScanThreads = 256;
+__global__ void __launch_bounds__(kScanThreads) k_msd_children(const unsigned long long* __restrict__ cnt,
+                                                               const unsigned long long* __restrict__ shorts, int bits,
+                                                               int incl, const unsigned long long* __restrict__ base,
+                                                               unsigned long long* __restrict__ lstart,
+                                                               unsigned long long* __restrict__ cursor, int lists,
+                                                               MsdLists G) {
+    __shared__ unsigned long long wsum[kScanThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int bins = 1 << bits;
+    const size_t c0 = size_t(blockIdx.x) << bits;
+    const int per = bins > kScanThreads ? bins / kScanThreads : 1;
+    const int b0 = tid * per;
+    unsigned long long mine = 0;
+    for (int i = 0; i < per; ++i)
+        if (b0 + i < bins) mine += cnt[c0 + b0 + i] + (shorts && !incl ? shorts[c0 + b0 + i] : 0ull);
+    unsigned long long x = mine;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    unsigned long long run = x - mine + (base ? base[blockIdx.x] : 0ull);
+    for (int w = 0; w < warp; ++w) run += wsum[w];
+    for (int i = 0; i < per; ++i) {
+        int cls = -1;
+        MsdBucket b{};
+        if (b0 + i < bins) {
+            const size_t c = c0 + b0 + i;
+            const unsigned long long sh = shorts ? shorts[c] : 0ull;
+            const unsigned long long all = cnt[c] + (incl ? 0ull : sh), longs = all - sh;
+            lstart[c] = run + sh;
+            cursor[c] = run + sh;
+            if (lists && longs) {
+                cls = longs <= kLocalSmall ? 0 : (longs <= kLocalLarge ? 1 : 2);
+                b.start = run + sh;
+                b.size = unsigned(longs < 0xffffffffull ? longs : 0xffffffffull);
+                b.id_off = unsigned(c);
+            }
+            run += all;
+        }
+        if (lists) list_bucket(G, cls, b);
+    }
+}
+
+// ------------------------------------------------------------------------------ short suffixes
+//
+// The suffixes of m <= S bases: every string has about nr / 4^m equal copies, in read order.  Sorted
+// by a stable radix sort (from read order) on the string's preorder number in the trie of S bases,
+// which is suffix order: for bases s_0 .. s_{m-1}, sum_i (1 + s_i T(S - 1 - i)) with T(h) the nodes
+// of a subtree of height h, i.e. (4 v - sum s_i) / 3 + m with v the padded value.
+
+constexpr int kShortSym = 20;           // a short suffix's BWT symbol, above the sorted key bits
+
+__global__ void k_short_keys(const uint64_t* __restrict__ pk, size_t nr, idx_t L, int S, uint32_t* __restrict__ key,
+                             idx_t* __restrict__ val) {
+    const size_t stride = size_t(gridDim.x) * blockDim.x;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nr * size_t(S); i += stride) {
+        const size_t r = i / unsigned(S);
+        const int m = int(i - r * unsigned(S)) + 1;
+        const size_t p = r * size_t(L) + size_t(L) - size_t(m);
+        const uint32_t v = uint32_t((window(pk, p) & (~uint64_t(0) << (64 - 2 * m))) >> (64 - 2 * S));
+        const uint32_t sum = uint32_t(__popc(v & 0x55555555u)) + 2u * uint32_t(__popc(v & 0xaaaaaaaau));
+        const uint32_t code = (4u * v - sum) / 3u + uint32_t(m);
+        const uint32_t sym = m == int(L) ? 0u : (uint32_t(pk[(p - 1) >> 5] >> (62 - 2 * int((p - 1) & 31))) & 3u) + 1u;
+        key[i] = code | (sym << kShortSym);
+        val[i] = idx_t(p);
+    }
+}
+
+// the bucket of a short suffix at p (its bases, padded with A)
+__device__ __forceinline__ size_t short_bucket(const uint64_t* __restrict__ pk, size_t p, const DivL& dl, int bits) {
+    const int m = suffix_bases(p, dl);
+    return size_t((window(pk, p) & (~uint64_t(0) << (64 - 2 * m))) >> (64 - bits));
+}
+
+// per bucket: how many short suffixes it has and the index of the first of them (they are
+// consecutive); every run of equal strings adds its ends
+__global__ void k_short_runs(const uint64_t* __restrict__ pk, const uint32_t* __restrict__ key,
+                             const idx_t* __restrict__ val, size_t m, DivL dl, int bits,
+                             unsigned long long* __restrict__ count, unsigned long long* __restrict__ first) {
+    const size_t stride = size_t(gridDim.x) * blockDim.x;
+    constexpr uint32_t mask = (1u << kShortSym) - 1u;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
+        const uint32_t k = key[i] & mask;
+        const bool head = i == 0 || (key[i - 1] & mask) != k, tail = i + 1 == m || (key[i + 1] & mask) != k;
+        if (!head && !tail) continue;
+        const size_t b = short_bucket(pk, size_t(val[i]), dl, bits);
+        if (head) {
+            atomicMin(&first[b], (unsigned long long)i);
+            atomicAdd(&count[b], 0ull - (unsigned long long)i);
+        }
+        if (tail) atomicAdd(&count[b], (unsigned long long)i + 1ull);
+    }
+}
+
+// the rows of the short suffixes: before their bucket's long ones; those of at least k bases also
+// belong to a k-mer (k <= S only: kstart null otherwise)
+__global__ void k_short_place(const uint64_t* __restrict__ pk, const uint32_t* __restrict__ key,
+                              const idx_t* __restrict__ val, size_t m, DivL dl, int bits,
+                              const unsigned long long* __restrict__ count, const unsigned long long* __restrict__ first,
+                              const unsigned long long* __restrict__ lstart, idx_t* __restrict__ sa,
+                              uint8_t* __restrict__ bwt, idx_t* __restrict__ kstart, idx_t* __restrict__ kend, int k) {
+    const size_t stride = size_t(gridDim.x) * blockDim.x;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
+        const idx_t p = val[i];
+        const size_t b = short_bucket(pk, size_t(p), dl, bits);
+        const size_t row = size_t(lstart[b] - count[b] + (i - first[b]));
+        sa[row] = p;
+        if (bwt) bwt[row] = uint8_t(key[i] >> kShortSym);
+        if (kstart && suffix_bases(size_t(p), dl) >= k) {
+            const size_t c = size_t(window(pk, size_t(p)) >> (64 - 2 * k));
+            atomicMin(reinterpret_cast<kmer_int*>(kstart + c), kmer_int(row));
+            atomicMax(reinterpret_cast<kmer_int*>(kend + c), kmer_int(row));
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------ networks
+//
+// Suffixes are compared by W 64-bit words of their bases (zero past the end: padded with A), then
+// by a tail that holds the length and what breaks ties.
 
 // a < b on (w[0..W-1], tail) as one unsigned multi-word number: the borrow out of the
 // subtraction a - b, least significant word first, in one chain of subtract-with-borrow
 // instructions (no branches; the chain must sit in one asm statement to keep the carry flag).
-#define PQ_SUBC(x, y) "subc.cc.u64 t, %" #x ", %" #y ";\n\t"
-#define PQ_LT_HEAD "{\n\t.reg .u64 t;\n\t.reg .u32 s, z;\n\tmov.u32 z, 0;\n\tsub.cc.u32 s, %1, %2;\n\t"
-#define PQ_LT_TAIL "subc.u32 %0, z, z;\n\t}"
-#define PQ_WORD(j) "l"(a.w[j]), "l"(b.w[j])
-
+template <int W, class Tail>
+struct SortItem {
+    uint64_t w[W];              // w[0] starts with the segment number
+    Tail tail;
+};
 template <int W>
-__device__ __forceinline__ bool item_less(const RefineItem<W>& a, const RefineItem<W>& b);
+__device__ __forceinline__ bool item_less(const SortItem<W, uint32_t>& a, const SortItem<W, uint32_t>& b);
+template <int W>
+__device__ __forceinline__ bool item_less(const SortItem<W, uint64_t>& a, const SortItem<W, uint64_t>& b);
 
-template <>
-__device__ __forceinline__ bool item_less<1>(const RefineItem<1>& a, const RefineItem<1>& b) {
-    unsigned r;
-    asm(PQ_LT_HEAD PQ_SUBC(3, 4) PQ_LT_TAIL
-        : "=r"(r)
-        : "r"(a.tail), "r"(b.tail), PQ_WORD(0));
-    return r != 0;
-}
-
-template <>
-__device__ __forceinline__ bool item_less<2>(const RefineItem<2>& a, const RefineItem<2>& b) {
-    unsigned r;
-    asm(PQ_LT_HEAD PQ_SUBC(3, 4) PQ_SUBC(5, 6) PQ_LT_TAIL
-        : "=r"(r)
-        : "r"(a.tail), "r"(b.tail), PQ_WORD(1), PQ_WORD(0));
-    return r != 0;
-}
-
-template <>
-__device__ __forceinline__ bool item_less<3>(const RefineItem<3>& a, const RefineItem<3>& b) {
-    unsigned r;
-    asm(PQ_LT_HEAD PQ_SUBC(3, 4) PQ_SUBC(5, 6) PQ_SUBC(7, 8) PQ_LT_TAIL
-        : "=r"(r)
-        : "r"(a.tail), "r"(b.tail), PQ_WORD(2), PQ_WORD(1), PQ_WORD(0));
-    return r != 0;
-}
-
-template <>
-__device__ __forceinline__ bool item_less<4>(const RefineItem<4>& a, const RefineItem<4>& b) {
-    unsigned r;
-    asm(PQ_LT_HEAD PQ_SUBC(3, 4) PQ_SUBC(5, 6) PQ_SUBC(7, 8) PQ_SUBC(9, 10) PQ_LT_TAIL
-        : "=r"(r)
-        : "r"(a.tail), "r"(b.tail), PQ_WORD(3), PQ_WORD(2), PQ_WORD(1), PQ_WORD(0));
-    return r != 0;
-}
-
-template <>
-__device__ __forceinline__ bool item_less<5>(const RefineItem<5>& a, const RefineItem<5>& b) {
-    unsigned r;
-    asm(PQ_LT_HEAD PQ_SUBC(3, 4) PQ_SUBC(5, 6) PQ_SUBC(7, 8) PQ_SUBC(9, 10) PQ_SUBC(11, 12) PQ_LT_TAIL
-        : "=r"(r)
-        : "r"(a.tail), "r"(b.tail), PQ_WORD(4), PQ_WORD(3), PQ_WORD(2), PQ_WORD(1), PQ_WORD(0));
-    return r != 0;
-}
-
-template <>
-__device__ __forceinline__ bool item_less<6>(const RefineItem<6>& a, const RefineItem<6>& b) {
-    unsigned r;
-    asm(PQ_LT_HEAD PQ_SUBC(3, 4) PQ_SUBC(5, 6) PQ_SUBC(7, 8) PQ_SUBC(9, 10) PQ_SUBC(11, 12) PQ_SUBC(13, 14) PQ_LT_TAIL
-        : "=r"(r)
-        : "r"(a.tail), "r"(b.tail), PQ_WORD(5), PQ_WORD(4), PQ_WORD(3), PQ_WORD(2), PQ_WORD(1), PQ_WORD(0));
-    return r != 0;
-}
-
-template <>
-__device__ __forceinline__ bool item_less<7>(const RefineItem<7>& a, const RefineItem<7>& b) {
-    unsigned r;
-    asm(PQ_LT_HEAD PQ_SUBC(3, 4) PQ_SUBC(5, 6) PQ_SUBC(7, 8) PQ_SUBC(9, 10) PQ_SUBC(11, 12) PQ_SUBC(13, 14) PQ_SUBC(15, 16) PQ_LT_TAIL
-        : "=r"(r)
-        : "r"(a.tail), "r"(b.tail), PQ_WORD(6), PQ_WORD(5), PQ_WORD(4), PQ_WORD(3), PQ_WORD(2), PQ_WORD(1), PQ_WORD(0));
-    return r != 0;
-}
-
-template <>
-__device__ __forceinline__ bool item_less<8>(const RefineItem<8>& a, const RefineItem<8>& b) {
-    unsigned r;
-    asm(PQ_LT_HEAD PQ_SUBC(3, 4) PQ_SUBC(5, 6) PQ_SUBC(7, 8) PQ_SUBC(9, 10) PQ_SUBC(11, 12) PQ_SUBC(13, 14) PQ_SUBC(15, 16) PQ_SUBC(17, 18) PQ_LT_TAIL
-        : "=r"(r)
-        : "r"(a.tail), "r"(b.tail), PQ_WORD(7), PQ_WORD(6), PQ_WORD(5), PQ_WORD(4), PQ_WORD(3), PQ_WORD(2), PQ_WORD(1), PQ_WORD(0));
-    return r != 0;
-}
-
-#undef PQ_SUBC
-#undef PQ_LT_HEAD
-#undef PQ_LT_TAIL
+#define PQ_S1 "subc.cc.u64 t, %3, %4;\n\t"
+#define PQ_S2 PQ_S1 "subc.cc.u64 t, %5, %6;\n\t"
+#define PQ_S3 PQ_S2 "subc.cc.u64 t, %7, %8;\n\t"
+#define PQ_S4 PQ_S3 "subc.cc.u64 t, %9, %10;\n\t"
+#define PQ_S5 PQ_S4 "subc.cc.u64 t, %11, %12;\n\t"
+#define PQ_S6 PQ_S5 "subc.cc.u64 t, %13, %14;\n\t"
+#define PQ_S7 PQ_S6 "subc.cc.u64 t, %15, %16;\n\t"
+#define PQ_S8 PQ_S7 "subc.cc.u64 t, %17, %18;\n\t"
+#define PQ_S9 PQ_S8 "subc.cc.u64 t, %19, %20;\n\t"
+#define PQ_WORD(j) "l"(a.w[j]), "l"(b.w[j])
+#define PQ_A1 PQ_WORD(0)
+#define PQ_A2 PQ_WORD(1), PQ_A1
+#define PQ_A3 PQ_WORD(2), PQ_A2
+#define PQ_A4 PQ_WORD(3), PQ_A3
+#define PQ_A5 PQ_WORD(4), PQ_A4
+#define PQ_A6 PQ_WORD(5), PQ_A5
+#define PQ_A7 PQ_WORD(6), PQ_A6
+#define PQ_A8 PQ_WORD(7), PQ_A7
+#define PQ_A9 PQ_WORD(8), PQ_A8
+#define PQ_LESS(W)                                                                                                  \
+    template <>                                                                                                     \
+    __device__ __forceinline__ bool item_less<W>(const SortItem<W, uint32_t>& a, const SortItem<W, uint32_t>& b) {  \
+        unsigned r;                                                                                                 \
+        asm("{\n\t.reg .u64 t;\n\t.reg .u32 s, z;\n\tmov.u32 z, 0;\n\tsub.cc.u32 s, %1, %2;\n\t" PQ_S##W            \
+            "subc.u32 %0, z, z;\n\t}"                                                                               \
+            : "=r"(r) : "r"(a.tail), "r"(b.tail), PQ_A##W);                                                         \
+        return r != 0;                                                                                              \
+    }                                                                                                               \
+    template <>                                                                                                     \
+    __device__ __forceinline__ bool item_less<W>(const SortItem<W, uint64_t>& a, const SortItem<W, uint64_t>& b) {  \
+        unsigned r;                                                                                                 \
+        asm("{\n\t.reg .u64 t;\n\t.reg .u32 z;\n\tmov.u32 z, 0;\n\tsub.cc.u64 t, %1, %2;\n\t" PQ_S##W               \
+            "subc.u32 %0, z, z;\n\t}"                                                                               \
+            : "=r"(r) : "l"(a.tail), "l"(b.tail), PQ_A##W);                                                         \
+        return r != 0;                                                                                              \
+    }
+PQ_LESS(1)
+PQ_LESS(2)
+PQ_LESS(3)
+PQ_LESS(4)
+PQ_LESS(5)
+PQ_LESS(6)
+PQ_LESS(7)
+PQ_LESS(8)
+PQ_LESS(9)
+#undef PQ_LESS
 #undef PQ_WORD
+#undef PQ_S1
+#undef PQ_S2
+#undef PQ_S3
+#undef PQ_S4
+#undef PQ_S5
+#undef PQ_S6
+#undef PQ_S7
+#undef PQ_S8
+#undef PQ_S9
+#undef PQ_A1
+#undef PQ_A2
+#undef PQ_A3
+#undef PQ_A4
+#undef PQ_A5
+#undef PQ_A6
+#undef PQ_A7
+#undef PQ_A8
+#undef PQ_A9
+
+// The bases of the suffix at p (m bases to its end) from base `from` on, 16 to a word, first base
+// highest, zero past the end; mask[i] has the bits of word i that are bases of the suffix.  Only
+// words of the text that hold such bases are loaded.
+template <int W>
+__device__ __forceinline__ void suffix_text(const uint64_t* __restrict__ pk, size_t p, int m, int from, uint32_t (&x)[2 * W],
+                                            uint32_t (&mask)[2 * W]) {
+    const int rem = max(m - from, 0);
+    const size_t q = p + size_t(from);
+    const uint64_t* t = pk + (q >> 5);
+    const int s = int(q & 31), held = rem + s;              // bases from the first word's start
+    uint32_t r[2 * W + 2];
+    #pragma unroll
+    for (int j = 0; j <= W; ++j) {
+        uint64_t v = 0;
+        if (rem > 0 && held > 32 * j) v = t[j];
+        r[2 * j] = uint32_t(v >> 32);
+        r[2 * j + 1] = uint32_t(v);
+    }
+    const bool odd = s >= 16;
+    #pragma unroll
+    for (int i = 0; i <= 2 * W; ++i) r[i] = odd ? r[i + 1] : r[i];
+    #pragma unroll
+    for (int i = 0; i < 2 * W; ++i) {
+        const uint32_t v = uint32_t(max(2 * rem - 32 * i, 0));
+        uint32_t past;
+        asm("shr.u32 %0, %1, %2;" : "=r"(past) : "r"(0xffffffffu), "r"(v));     // 0 from 32 on
+        mask[i] = ~past;
+        x[i] = __funnelshift_l(r[i + 1], r[i], 2 * s) & mask[i];
+    }
+}
+
+// The same as W 64-bit words behind a segment number of SEG bits: (64 - SEG) / 2 bases in the first,
+// 32 in each other.
+template <int W, int SEG>
+__device__ __forceinline__ void pack_words(const uint32_t (&x)[2 * W], uint32_t seg, uint64_t (&w)[W]) {
+    constexpr int kFirst = 2 * ((64 - SEG) / 2);            // text bits of the first word
+    uint64_t y[W];
+    #pragma unroll
+    for (int j = 0; j < W; ++j) y[j] = (uint64_t(x[2 * j]) << 32) | x[2 * j + 1];
+    if constexpr (SEG == 0) {
+        #pragma unroll
+        for (int j = 0; j < W; ++j) w[j] = y[j];
+    } else {
+        w[0] = (uint64_t(seg) << (64 - SEG)) | ((y[0] >> (64 - kFirst)) << (64 - SEG - kFirst));
+        #pragma unroll
+        for (int j = 1; j < W; ++j) w[j] = (y[j - 1] << kFirst) | (y[j] >> (64 - kFirst));
+    }
+}
+template <int W, int SEG>
+__device__ __forceinline__ void sort_words(const uint64_t* __restrict__ pk, size_t p, int m, int from, uint32_t seg,
+                                           uint64_t (&w)[W]) {
+    uint32_t x[2 * W], mask[2 * W];
+    suffix_text<W>(pk, p, m, from, x, mask);
+    pack_words<W, SEG>(x, seg, w);
+}
+
+// ascending bitonic sort of one item a lane; lanes from `len` on hold the largest items
+__device__ __forceinline__ bool item_less(uint64_t a, uint64_t b) { return a < b; }
+__device__ __forceinline__ uint64_t item_xor(uint64_t a, int j) { return __shfl_xor_sync(0xffffffffu, a, j); }
+template <int W>
+__device__ __forceinline__ SortItem<W, uint64_t> item_xor(const SortItem<W, uint64_t>& a, int j) {
+    SortItem<W, uint64_t> o;
+    #pragma unroll
+    for (int q = 0; q < W; ++q) o.w[q] = __shfl_xor_sync(0xffffffffu, a.w[q], j);
+    o.tail = __shfl_xor_sync(0xffffffffu, a.tail, j);
+    return o;
+}
+template <class Item>
+__device__ __forceinline__ void warp_sort(Item& it, int len, int lane) {
+    #pragma unroll
+    for (int k = 2; k <= 32; k <<= 1) {
+        if (k > 2 && len <= (k >> 1)) break;
+        #pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const Item o = item_xor(it, j);
+            const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
+            if (keep_min == item_less(o, it)) it = o;
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------ buckets in shared memory
+
+struct MsdLocal {
+    MsdPlan plan;
+    const uint64_t* pk;
+    uint64_t* buf;                      // the buckets' elements
+    const MsdBucket* list;
+    const unsigned long long* count;
+    unsigned long long* next;
+    MsdLists G;
+    idx_t* sa;                          // rows of element 0 on
+    uint8_t* bwt;                       // or null
+    idx_t *kstart, *kend;               // k-mer table, or null
+    int kmer_k;
+    int kmer_spans;                     // a k-mer's rows may lie in several buckets
+    size_t row0;                        // suffix-array row of element 0
+    int more_bits;                      // text bits of a rebuilt element's key (off > 0)
+};
+
+constexpr int kLocalBits = 11, kLocalBins = 1 << kLocalBits;      // two 16-bit counters to a word
+
+// exclusive scan of the packed counters, in place, by the CTA's T threads (the caller synchronises
+// before reading them)
+template <int T>
+__device__ __forceinline__ void packed_exclusive(unsigned* cnt, unsigned* wsum) {
+    constexpr int kPer = kLocalBins / 2 / T;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned v[kPer], mine = 0;
+    #pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        v[i] = cnt[tid * kPer + i];
+        mine += (v[i] & 0xffffu) + (v[i] >> 16);
+    }
+    unsigned x = mine;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    unsigned run = x - mine;
+    #pragma unroll
+    for (int w = 0; w < T / 32; ++w) run += w < warp ? wsum[w] : 0u;
+    #pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const unsigned lo = v[i] & 0xffffu;
+        cnt[tid * kPer + i] = run | ((run + lo) << 16);
+        run += lo + (v[i] >> 16);
+    }
+}
+
+// first set bit of the boundary mask above slot j (there is one at the bucket's end)
+__device__ __forceinline__ int next_boundary(const unsigned* bm, int j) {
+    int w = (j + 1) >> 5;
+    unsigned x = bm[w] & (~0u << ((j + 1) & 31));
+    while (!x) x = bm[++w];
+    return 32 * w + __ffs(x) - 1;
+}
+
+// ascending sort of e[0, m) by the `threads` threads of a warp or a CTA (t: this one's number):
+// the bitonic network whose comparators all point up (a mirrored first step per merge), so that
+// positions past m act as the largest and are skipped
+template <class Sync>
+__device__ __forceinline__ void smem_sort(uint64_t* e, int m, int t, int threads, Sync sync) {
+    auto exchange = [&](int a, int b) {
+        if (b >= m) return;
+        const uint64_t x = e[a], y = e[b];
+        if (y < x) {
+            e[a] = y;
+            e[b] = x;
+        }
+    };
+    for (int k = 2; k < 2 * m; k <<= 1) {
+        const int half = k >> 1, pairs = (m + k - 1) / k * half;
+        for (int i = t; i < pairs; i += threads) {
+            const int q = i / half, o = i - q * half;
+            exchange(q * k + o, q * k + k - 1 - o);
+        }
+        sync();
+        for (int j = half >> 1; j > 0; j >>= 1) {
+            for (int i = t; i < pairs; i += threads) {
+                const int a = ((i & ~(j - 1)) << 1) | (i & (j - 1));
+                exchange(a, a + j);
+            }
+            sync();
+        }
+    }
+}
+
+// One bucket per CTA and turn.  Bound by instruction issue (the networks) and the gather of each
+// suffix's text, about two sectors.  The elements are split by their next 11 bits into
+// sub-buckets (counted and placed with shared-memory atomics; a bit mask marks where each starts),
+// then every warp walks a stretch of sub-buckets: as many consecutive whole ones as fit 32 lanes
+// are sorted by one bitonic network on (sub-bucket, bases, length, position).  Sub-buckets of more
+// than 32 are first sorted by their elements; suffixes equal in all bases of those, if still more
+// than 32, are listed for the kernels of larger groups, in order of position.
+//
+// A sub-bucket mostly holds the suffixes of one genome locus, equal up to their ends but for a few
+// sequencing errors.  So the network does not carry their bases: every suffix is compared with the
+// longest of its sub-bucket, the positions where any in the warp differs from its longest (within
+// its length) are collected with one OR over the warp per word, and only the bases there, in order,
+// enter the key.  Two suffixes of a sub-bucket that differ within both lengths differ at one of
+// those positions, and past the end of the shorter one its bases there read A, so (those bases,
+// length, position) is their order.  One 64-bit key holds 8 or so such positions beside length and
+// position, two hold 27; only beyond that does the network carry all W words.
+//
+// Measured, one direction of 123 M suffixes of 100-base reads (32-bit positions): the whole sort 4.9
+// ms, 3.3 of them here, against 8.0 ms for four radix passes of 14-base keys, group lists and
+// refinement networks of all words; of 1.13 G suffixes (64-bit): 50 ms, 33 here, against 95.
+template <int W, int CAP, int T>
+__global__ void __launch_bounds__(T, T == 128 ? (W <= 4 ? 8 : 6) : 3) k_msd_local(MsdLocal a) {
+    extern __shared__ __align__(16) unsigned char msd_smem[];
+    uint64_t* se = reinterpret_cast<uint64_t*>(msd_smem);
+    unsigned* cnt = reinterpret_cast<unsigned*>(se + CAP);
+    unsigned* bm = cnt + kLocalBins / 2;                    // [CAP / 32 + 2]
+    constexpr int kOver = CAP / 33 + 1;
+    __shared__ unsigned s_over[kOver], wsum[T / 32], s_diff[2], s_item;
+    __shared__ int s_nover, s_nhuge;
+    __shared__ unsigned s_huge[CAP / 1025 + 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NW = T / 32;
+    const MsdPlan& P = a.plan;
+    const uint64_t pos_mask = (uint64_t(1) << P.P) - 1;
+    const int len_bits = 32 - __clz(int(P.dl.L));
+    const unsigned items = unsigned(*a.count);
+    while (true) {
+        if (tid == 0) {
+            s_item = unsigned(atomicAdd(a.next, 1ull));
+            s_diff[0] = s_diff[1] = 0;
+            s_nover = s_nhuge = 0;
+        }
+        __syncthreads();
+        const unsigned item = s_item;
+        if (item >= items) break;
+        const MsdBucket bk = a.list[item];
+        const int m = int(bk.size), off = int(bk.id_off >> kIdBits);
+        uint64_t* const in = a.buf + bk.start;
+        for (int i = tid; i < kLocalBins / 2; i += T) cnt[i] = 0;
+        const int full = off ? a.more_bits / 2 : P.head;        // length field of a suffix that goes on
+        // the lowest bit of the split, and the bases every sub-bucket then shares
+        int shift, from;
+        if (CAP == kLocalSmall) {                   // the bits below the partition's own
+            shift = max(P.key_shift + P.kbits - P.d2 - kLocalBits, P.key_shift);
+            __syncthreads();
+        } else {                                    // the highest differing ones
+            const uint64_t e0 = in[0];
+            uint64_t diff = 0;
+            for (int j = tid; j < m; j += T) diff |= in[j] ^ e0;
+            const unsigned lo = __reduce_or_sync(0xffffffffu, unsigned(diff));
+            const unsigned hi = __reduce_or_sync(0xffffffffu, unsigned(diff >> 32));
+            if (lane == 0) {
+                if (lo) atomicOr(&s_diff[0], lo);
+                if (hi) atomicOr(&s_diff[1], hi);
+            }
+            __syncthreads();
+            diff = (uint64_t(s_diff[1]) << 32) | s_diff[0];
+            const int hb = diff ? 63 - __clzll((long long)diff) : -1;
+            const bool goes_on = int((e0 >> P.len_shift) & 31u) == full;
+            shift = hb - (kLocalBits - 1);
+            if (hb >= P.key_shift) shift = max(shift, P.key_shift);
+            else if (hb >= P.len_shift) shift = P.len_shift;
+            else if (goes_on || hb < 0) shift = 63;             // equal heads: one sub-bucket
+            else shift = max(shift, 0);                         // equal strings: by position
+        }
+        if (shift < P.key_shift || shift == 63) from = off + full;
+        else if (off) from = off + min(a.more_bits, P.key_shift + P.kbits - shift) / 2;
+        else from = (P.d1 + P.key_shift + P.kbits - shift) / 2;
+        auto bin_of = [&](uint64_t e) { return unsigned(e >> shift) & unsigned(kLocalBins - 1); };
+        for (int j = tid; j < m; j += T) {
+            const unsigned q = bin_of(in[j]);
+            atomicAdd(&cnt[q >> 1], q & 1u ? 0x10000u : 1u);
+        }
+        __syncthreads();
+        packed_exclusive<T>(cnt, wsum);
+        __syncthreads();
+        for (int j = tid; j < m; j += T) {
+            const uint64_t e = in[j];
+            const unsigned q = bin_of(e), half = 16 * (q & 1u);
+            se[(atomicAdd(&cnt[q >> 1], 1u << half) >> half) & 0xffffu] = e;
+        }
+        __syncthreads();
+        const int words = m / 32 + 1;
+        for (int w = warp; w < words; w += NW) {
+            const int j = 32 * w + lane;
+            bool b = j == m;
+            if (j < m) b = j == 0 || bin_of(se[j]) != bin_of(se[j - 1]);
+            const unsigned x = __ballot_sync(0xffffffffu, b);
+            if (lane == 0) bm[w] = x;
+        }
+        if (tid == 0) bm[words] = 0;
+        __syncthreads();
+        // sub-buckets of more than 32: only the last one that starts in a mask word can be
+        for (int w = tid; w < words; w += T) {
+            const unsigned x = bm[w];
+            if (!x) continue;
+            const int j = 32 * w + 31 - __clz(x);
+            if (j >= m) continue;
+            const int g = next_boundary(bm, j) - j;
+            if (g > 32) s_over[atomicAdd(&s_nover, 1)] = (unsigned(j) << 16) | unsigned(g);
+        }
+        __syncthreads();
+        const int nover = s_nover;
+        if (nover) {
+            for (int i = warp; i < nover; i += NW) {
+                const int j = int(s_over[i] >> 16), g = int(s_over[i] & 0xffffu);
+                if (g <= 256) smem_sort(se + j, g, lane, 32, [] { __syncwarp(); });
+            }
+            __syncthreads();
+            for (int i = 0; i < nover; ++i) {
+                const int j = int(s_over[i] >> 16), g = int(s_over[i] & 0xffffu);
+                if (g > 256) smem_sort(se + j, g, tid, T, [] { __syncthreads(); });
+            }
+            // their own sub-buckets: suffixes that go on past equal heads; ended ones are in order
+            for (int i = warp; i < nover; i += NW) {
+                const int j = int(s_over[i] >> 16), g = int(s_over[i] & 0xffffu);
+                for (int q = lane; q < g; q += 32) {
+                    const uint64_t e = se[j + q] >> P.len_shift;
+                    if (q == 0 || e != (se[j + q - 1] >> P.len_shift) || int(e & 31u) < full)
+                        atomicOr(&bm[(j + q) >> 5], 1u << ((j + q) & 31));
+                }
+            }
+            __syncthreads();
+            for (int w = tid; w < words; w += T) {
+                const unsigned x = bm[w];
+                if (!x) continue;
+                const int j = 32 * w + 31 - __clz(x);
+                if (j >= m) continue;
+                const int g = next_boundary(bm, j) - j;
+                if (g <= 32) continue;
+                const int cls = g <= 128 ? 0 : (g <= 1024 ? 1 : 2);
+                unsigned long long* c = cls == 0 ? &a.G.c->mid : (cls == 1 ? &a.G.c->big : &a.G.c->huge);
+                unsigned long long* l = cls == 0 ? a.G.mid : (cls == 1 ? a.G.big : a.G.huge);
+                const unsigned long long cap = cls == 0 ? a.G.cap_mid : (cls == 1 ? a.G.cap_big : a.G.cap_huge);
+                const unsigned long long at = atomicAdd(c, 1ull);
+                if (at < cap)
+                    l[at] = ((bk.start + (unsigned long long)j) << 24) | ((unsigned long long)(off + full) << 14) |
+                            (unsigned long long)g;
+                if (cls == 2) s_huge[atomicAdd(&s_nhuge, 1)] = (unsigned(j) << 16) | unsigned(g);
+            }
+            __syncthreads();
+            // groups that come back with new elements leave theirs in place
+            for (int i = 0; i < s_nhuge; ++i) {
+                const int j = int(s_huge[i] >> 16), g = int(s_huge[i] & 0xffffu);
+                for (int q = tid; q < g; q += T) in[j + q] = se[j + q];
+            }
+        }
+        // every warp's stretch of slots: the sub-buckets that start in it, 32 lanes at a time
+        const int stretch = (m + NW - 1) / NW;
+        const int r1 = min(m, (warp + 1) * stretch);
+        int cur = warp * stretch;
+        if (cur < r1 && !((bm[cur >> 5] >> (cur & 31)) & 1u)) cur = next_boundary(bm, cur);
+        while (cur < r1) {
+            // boundaries at slots cur + 1 .. cur + 32 as bits 0 .. 31
+            const int w = (cur + 1) >> 5;
+            unsigned x = __funnelshift_r(bm[w], bm[w + 1], (cur + 1) & 31);
+            const int room = r1 - cur;                          // sub-buckets from slot r1 on are the next warp's
+            if (room <= 32) {
+                const unsigned low = (1u << (room - 1)) - 1u;
+                const unsigned high = x & ~low;
+                x = (x & low) | (high & (0u - high));
+            }
+            if (!x) {                                           // a listed group
+                cur = next_boundary(bm, cur);
+                continue;
+            }
+            const int len = 32 - __clz(x);
+            const bool single = ((x >> lane) & 1u) && (lane == 0 || ((x >> (lane - 1)) & 1u));
+            const bool need = lane < len && !single;
+            if (__any_sync(0xffffffffu, need)) {
+                const uint64_t e = lane < len ? se[cur + lane] : 0;
+                const uint64_t p = (e >> kSymBits) & pos_mask;
+                const int sl = need ? suffix_bases(size_t(p), P.dl) : 0;
+                const uint32_t seg = uint32_t(__popc(x & ((1u << lane) - 1u)));
+                uint32_t tx[2 * W], mask[2 * W];
+                suffix_text<W>(a.pk, size_t(p), sl, from, tx, mask);
+                // the lane of the longest suffix of this lane's sub-bucket
+                const int first = 31 - __clz(((x << 1) | 1u) & (0xffffffffu >> (31 - lane)));
+                const int last = lane < len ? lane + __ffs(x >> lane) - 1 : lane;
+                unsigned longest = (unsigned(sl) << 5) | unsigned(lane);
+                #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned y = __shfl_up_sync(0xffffffffu, longest, o);
+                    if (lane - o >= first) longest = max(longest, y);
+                }
+                const int pivot = int(__shfl_sync(0xffffffffu, longest, last) & 31u);
+                uint32_t where[2 * W];              // a bit per differing base (its lower one)
+                int np = 0;
+                #pragma unroll
+                for (int i = 0; i < 2 * W; ++i) {
+                    const uint32_t y = __shfl_sync(0xffffffffu, tx[i], pivot);
+                    const uint32_t d = __reduce_or_sync(0xffffffffu, (tx[i] ^ y) & mask[i]);
+                    where[i] = (d | (d >> 1)) & 0x55555555u;
+                    np += __popc(where[i]);
+                }
+                const uint64_t low = (((uint64_t(unsigned(sl)) << P.P) | p) << 5) | uint64_t(unsigned(lane));
+                const int low_bits = len_bits + P.P + 5;
+                const int seg_bits = 32 - __clz(__popc(x) - 1);
+                int src;
+                if (np <= 27) {
+                    // the bases there, in order, below the sub-bucket's number
+                    uint32_t k0 = seg, k1 = 0;
+                    #pragma unroll
+                    for (int i = 0; i < 2 * W; ++i) {
+                        for (uint32_t y = where[i]; y;) {
+                            const int z = __clz(y);                     // the base's upper bit is one higher
+                            k1 = __funnelshift_l(k0, k1, 2);
+                            k0 = __funnelshift_l(tx[i] << (z - 1), k0, 2);
+                            y &= 0x7fffffffu >> z;
+                        }
+                    }
+                    const uint64_t k = (uint64_t(k1) << 32) | k0;
+                    if (seg_bits + 2 * np + low_bits <= 64) {
+                        uint64_t key = lane < len ? (k << low_bits) | low : ~uint64_t(0);
+                        warp_sort(key, len, lane);
+                        src = int(key & 31u);
+                    } else {
+                        SortItem<1, uint64_t> it;
+                        it.w[0] = lane < len ? k : ~uint64_t(0);
+                        it.tail = lane < len ? low : ~uint64_t(0);
+                        warp_sort(it, len, lane);
+                        src = int(it.tail & 31u);
+                    }
+                } else {
+                    SortItem<W, uint64_t> it;
+                    pack_words<W, 5>(tx, seg, it.w);
+                    it.tail = low;
+                    if (lane >= len) {
+                        #pragma unroll
+                        for (int j = 0; j < W; ++j) it.w[j] = ~uint64_t(0);
+                        it.tail = ~uint64_t(0);
+                    }
+                    warp_sort(it, len, lane);
+                    src = int(it.tail & 31u);
+                }
+                const uint64_t sorted = __shfl_sync(0xffffffffu, e, src);
+                if (lane < len) se[cur + lane] = sorted;
+                __syncwarp();
+            }
+            cur += len;
+        }
+        __syncthreads();
+        // the finished rows
+        for (int j = tid; j < m; j += T) {
+            const uint64_t e = se[j];
+            a.sa[bk.start + j] = idx_t((e >> kSymBits) & pos_mask);
+            if (a.bwt) a.bwt[bk.start + j] = uint8_t(e & 7u);
+        }
+        if (a.kstart && !off) {
+            // k-mer of a row (k <= head): the bucket's first d1 bits and the key; absent in a
+            // suffix of fewer bases.  Buckets of whole k-mers write each one's two rows; when a
+            // k-mer spans buckets its rows are agreed on by minimum and maximum.
+            const int k = a.kmer_k, top = 2 * k - P.d1;
+            const uint64_t id1 = uint64_t(bk.id_off & ((1u << kIdBits) - 1)) >> P.d2;
+            const int low = max(P.key_shift + P.kbits - top, 0);        // lowest k-mer bit of an element
+            auto has = [&](uint64_t e) { return int((e >> P.len_shift) & 31u) >= k; };
+            const bool spans = a.kmer_spans;
+            for (int j = tid; j < m; j += T) {
+                const uint64_t e = se[j];
+                if (!has(e)) continue;
+                bool begins = j == 0, ends = j + 1 == m;
+                if (!begins) {
+                    const uint64_t y = se[j - 1];
+                    begins = (top > 0 && ((e ^ y) >> low)) || !has(y);
+                }
+                if (!ends) {
+                    const uint64_t y = se[j + 1];
+                    ends = (top > 0 && ((e ^ y) >> low)) || !has(y);
+                }
+                if (!begins && !ends) continue;
+                const uint64_t key = e >> P.key_shift;
+                const unsigned c = unsigned(top >= 0 ? (id1 << top) | (key >> (P.kbits - top)) : id1 >> (-top));
+                const idx_t row = idx_t(a.row0 + bk.start + j);
+                if (begins) {
+                    if (spans) atomicMin(reinterpret_cast<kmer_int*>(a.kstart + c), kmer_int(row));
+                    else a.kstart[c] = row;
+                }
+                if (ends) {
+                    if (spans) atomicMax(reinterpret_cast<kmer_int*>(a.kend + c), kmer_int(row));
+                    else a.kend[c] = row;
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+template <int CAP>
+static constexpr size_t local_smem() { return size_t(CAP) * 8 + (kLocalBins / 2 + CAP / 32 + 2) * sizeof(unsigned); }
+
+// ------------------------------------------------------------------------------ larger groups
+//
+// Suffixes equal in all bases of their elements, listed by position: 33..128 are sorted by one warp
+// (4 slots a lane, several groups packed and told apart by a segment number), 129..1024 by one CTA
+// in shared memory.  A listed group starts at element `start` and is equal up to base `from`.
+
+__device__ __forceinline__ int group_size(unsigned long long g) { return int(g & 0x3fffu); }
+__device__ __forceinline__ int group_from(unsigned long long g) { return int((g >> 14) & 0x3ffu); }
 
 constexpr int kRefineThreads = 256;
 
-template <int W, int E>
-__global__ void __launch_bounds__(kRefineThreads, E == 1 ? (W <= 3 ? 5 : 1) : (W <= 4 ? 3 : 1)) k_refine_warp(const unsigned long long* __restrict__ list,
-                                                                const unsigned long long* __restrict__ cnt,
-                                                                const uint64_t* __restrict__ pk, idx_t L,
-                                                                idx_t* __restrict__ val, int from,
-                                                                uint8_t* __restrict__ bwt, idx_t* __restrict__ isa,
-                                                                idx_t isa_m, size_t row_base) {
-    constexpr int kChunk = 8;
-    constexpr int N = 32 * E;
+// BWT symbol of the suffix at p: 0 (`$`) at a read start, else the preceding base (1..4)
+__device__ __forceinline__ uint8_t bwt_symbol(const uint64_t* __restrict__ pk, size_t p, const DivL& dl) {
+    if (suffix_bases(p, dl) == int(dl.L)) return 0;
+    const size_t q = p - 1;
+    return uint8_t(((pk[q >> 5] >> (62 - 2 * int(q & 31))) & 3) + 1);
+}
+
+// The warp's 128 slots (slot e * 32 + lane is register set e of that lane) take consecutive listed
+// groups while they fit; one bitonic network on (segment, bases from `from` on, length, slot)
+// sorts every packed group in place.  A group's members arrive in ascending position, so the slot
+// breaks ties exactly as the position does; positions and symbols wait in shared memory and are
+// gathered by slot at the end.  Distances below 32 exchange by shuffle, larger ones swap
+// registers within a lane.
+template <int W>
+__global__ void __launch_bounds__(kRefineThreads, W <= 4 ? 3 : 1)
+k_refine_warp(const unsigned long long* __restrict__ list, const unsigned long long* __restrict__ cnt,
+              const uint64_t* __restrict__ pk, DivL dl, idx_t* __restrict__ val, uint8_t* __restrict__ bwt) {
+    constexpr int kChunk = 8, E = 4, N = 32 * E;
     __shared__ idx_t spos[kRefineThreads / 32][N];
     __shared__ uint8_t ssym[kRefineThreads / 32][N];
     const int lane = threadIdx.x & 31;
@@ -979,14 +1684,16 @@ __global__ void __launch_bounds__(kRefineThreads, E == 1 ? (W <= 3 ? 5 : 1) : (W
             int taken = 0, total = 0;
             uint32_t seg[E];
             size_t at[E];
+            int from[E];
             #pragma unroll
             for (int e = 0; e < E; ++e) {
                 seg[e] = 255;
                 at[e] = 0;
+                from[e] = 0;
             }
             for (int q = next; q < kChunk; ++q) {
                 const unsigned long long x = __shfl_sync(0xffffffffu, mine, q);
-                const int m = int(x & 0xffffff);
+                const int m = group_size(x);
                 if (m == 0 || total + m > N) break;
                 #pragma unroll
                 for (int e = 0; e < E; ++e) {
@@ -994,22 +1701,23 @@ __global__ void __launch_bounds__(kRefineThreads, E == 1 ? (W <= 3 ? 5 : 1) : (W
                     if (slot >= total && slot < total + m) {
                         seg[e] = uint32_t(q - next);
                         at[e] = size_t(x >> 24) + size_t(slot - total);
+                        from[e] = group_from(x);
                     }
                 }
                 total += m;
                 ++taken;
             }
             if (taken == 0) break;
-            RefineItem<W> it[E];
+            SortItem<W, uint32_t> it[E];
             #pragma unroll
             for (int e = 0; e < E; ++e) {
                 if (seg[e] != 255) {
                     const idx_t pos = val[at[e]];
-                    const uint32_t len = uint32_t(L - pos % L);
-                    refine_words<W>(pk, size_t(pos), int(len), from, seg[e], it[e].w);
-                    it[e].tail = (len << 8) | uint32_t(e * 32 + lane);
+                    const int len = suffix_bases(size_t(pos), dl);
+                    sort_words<W, 3>(pk, size_t(pos), len, from[e], seg[e], it[e].w);
+                    it[e].tail = (uint32_t(len) << 8) | uint32_t(e * 32 + lane);
                     mypos[e * 32 + lane] = pos;
-                    if (bwt) mysym[e * 32 + lane] = bwt_symbol(pk, size_t(pos), L);
+                    if (bwt) mysym[e * 32 + lane] = bwt_symbol(pk, size_t(pos), dl);
                 } else {
                     #pragma unroll
                     for (int j = 0; j < W; ++j) it[e].w[j] = ~uint64_t(0);
@@ -1027,7 +1735,7 @@ __global__ void __launch_bounds__(kRefineThreads, E == 1 ? (W <= 3 ? 5 : 1) : (W
                             if (f > e) {
                                 const bool asc = ((e * 32 + lane) & k) == 0;
                                 if (item_less<W>(it[f], it[e]) == asc) {
-                                    const RefineItem<W> t = it[e];
+                                    const SortItem<W, uint32_t> t = it[e];
                                     it[e] = it[f];
                                     it[f] = t;
                                 }
@@ -1036,7 +1744,7 @@ __global__ void __launch_bounds__(kRefineThreads, E == 1 ? (W <= 3 ? 5 : 1) : (W
                     } else {
                         #pragma unroll
                         for (int e = 0; e < E; ++e) {
-                            RefineItem<W> o;
+                            SortItem<W, uint32_t> o;
                             #pragma unroll
                             for (int q = 0; q < W; ++q) o.w[q] = __shfl_xor_sync(0xffffffffu, it[e].w[q], j);
                             o.tail = __shfl_xor_sync(0xffffffffu, it[e].tail, j);
@@ -1050,9 +1758,8 @@ __global__ void __launch_bounds__(kRefineThreads, E == 1 ? (W <= 3 ? 5 : 1) : (W
             #pragma unroll
             for (int e = 0; e < E; ++e) {
                 if (seg[e] != 255) {
-                    const idx_t pos = mypos[it[e].tail & 255u];
-                    val[at[e]] = pos;
-                    row_outputs(bwt, isa, isa_m, row_base + at[e], pos, L, bwt ? mysym[it[e].tail & 255u] : 0);
+                    val[at[e]] = mypos[it[e].tail & 255u];
+                    if (bwt) bwt[at[e]] = mysym[it[e].tail & 255u];
                 }
             }
             __syncwarp();
@@ -1061,7 +1768,18 @@ __global__ void __launch_bounds__(kRefineThreads, E == 1 ? (W <= 3 ? 5 : 1) : (W
     }
 }
 
-// bitonic sort of one group of m suffixes held as columns: words w[j][P2], len[P2], pos[P2]
+// the (words, length, position) order of two suffixes
+template <int W>
+__device__ __forceinline__ bool tuple_less(const uint64_t a[W], uint64_t alen, uint64_t apos, const uint64_t b[W],
+                                           uint64_t blen, uint64_t bpos) {
+    #pragma unroll
+    for (int j = 0; j < W; ++j)
+        if (a[j] != b[j]) return a[j] < b[j];
+    if (alen != blen) return alen < blen;
+    return apos < bpos;
+}
+
+// one CTA's bitonic sort of one group of m suffixes held as columns: words w[j][P2], len[P2], pos[P2]
 template <int W>
 __device__ void cta_bitonic(uint64_t* cols, int P2) {
     uint64_t* lenc = cols + size_t(W) * P2;
@@ -1098,7 +1816,7 @@ __device__ void cta_bitonic(uint64_t* cols, int P2) {
 }
 
 template <int W>
-__device__ void cta_load_group(uint64_t* cols, int P2, size_t start, int m, const uint64_t* __restrict__ pk, idx_t L,
+__device__ void cta_load_group(uint64_t* cols, int P2, size_t start, int m, const uint64_t* __restrict__ pk, const DivL& dl,
                                const idx_t* __restrict__ val, int off) {
     uint64_t* lenc = cols + size_t(W) * P2;
     uint64_t* posc = lenc + P2;
@@ -1107,8 +1825,8 @@ __device__ void cta_load_group(uint64_t* cols, int P2, size_t start, int m, cons
         uint64_t len = ~uint64_t(0), pos = ~uint64_t(0);
         if (i < m) {
             pos = uint64_t(val[start + i]);
-            len = uint64_t(L - idx_t(pos % L));
-            suffix_words<W>(pk, size_t(pos), int(len), off, w);
+            len = uint64_t(suffix_bases(size_t(pos), dl));
+            sort_words<W, 0>(pk, size_t(pos), int(len), off, 0, w);
         } else {
             #pragma unroll
             for (int q = 0; q < W; ++q) w[q] = ~uint64_t(0);
@@ -1123,243 +1841,606 @@ __device__ void cta_load_group(uint64_t* cols, int P2, size_t start, int m, cons
 
 template <int W>
 __global__ void k_refine_cta(const unsigned long long* __restrict__ list, const unsigned long long* __restrict__ cnt,
-                             const uint64_t* __restrict__ pk, idx_t L, idx_t* __restrict__ val, int off,
-                             uint8_t* __restrict__ bwt, idx_t* __restrict__ isa, idx_t isa_m, size_t row_base) {
+                             const uint64_t* __restrict__ pk, DivL dl, idx_t* __restrict__ val, uint8_t* __restrict__ bwt) {
     extern __shared__ uint64_t s_cols[];
     const size_t groups = *cnt;
     for (size_t g = blockIdx.x; g < groups; g += gridDim.x) {
         const unsigned long long e = list[g];
         const size_t start = size_t(e >> 24);
-        const int m = int(e & 0xffffff);
+        const int m = group_size(e);
         int P2 = 32;
         while (P2 < m) P2 <<= 1;
-        cta_load_group<W>(s_cols, P2, start, m, pk, L, val, off);
+        cta_load_group<W>(s_cols, P2, start, m, pk, dl, val, group_from(e));
         cta_bitonic<W>(s_cols, P2);
         const uint64_t* posc = s_cols + size_t(W + 1) * P2;
         for (int i = threadIdx.x; i < m; i += blockDim.x) {
             const idx_t pos = idx_t(posc[i]);
             val[start + i] = pos;
-            row_outputs(bwt, isa, isa_m, row_base + start + i, pos, L, bwt ? bwt_symbol(pk, size_t(pos), L) : 0);
+            if (bwt) bwt[start + i] = bwt_symbol(pk, size_t(pos), dl);
         }
         __syncthreads();
     }
 }
 
-// 64-bit keys of a range of suffixes on their bases [off, off + 29): those bases (padded) and how
-// many of them exist (0..29)
-__global__ void k_range_keys(const uint64_t* __restrict__ pk, const idx_t* __restrict__ val, size_t m, idx_t L,
-                             int off, uint64_t* __restrict__ key, idx_t* __restrict__ out) {
-    const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
-        const idx_t p = val[i];
-        const int rem = int(L - p % L) - off;
-        key[i] = rem > 0 ? make_key<uint64_t>(window(pk, size_t(p) + off), rem) : 0;
-        out[i] = p;
-    }
-}
+// ------------------------------------------------------------------------------ further splits
+//
+// Buckets of more than kLocalLarge suffixes and groups of more than 1024 suffixes equal in all bases
+// of their elements (low-complexity or highly repeated sequence), driven by the host: a range is
+// split by the 10 highest bits in which its elements differ -- text, else length, else, among equal
+// strings, position -- and one whose suffixes all go on past equal heads first gets new elements
+// of its next bases, until every part fits the local kernel.
 
-// the groups of classes 0..2 (c: their counts)
-template <int W>
-static void refine_small_mid(const GroupLists& G, const unsigned long long* c, const uint64_t* pk, idx_t L,
-                             idx_t* val, int off, cudaStream_t st) {
-    if (c[0]) {
-        unsigned g = unsigned(std::min<unsigned long long>((c[0] + 63) / 64, 152ull * 64));
-        { k_refine_warp<W, 1><<<g, kRefineThreads, 0, st>>>(G.list[0], G.counts + 0, pk, L, val, off, G.bwt, G.isa, G.isa_m, G.row_base); note_launch(); }
-    }
-    if (c[1]) {
-        unsigned g = unsigned(std::min<unsigned long long>((c[1] + 15) / 16, 152ull * 64));
-        { k_refine_warp<W, 4><<<g, kRefineThreads, 0, st>>>(G.list[1], G.counts + 1, pk, L, val, off, G.bwt, G.isa, G.isa_m, G.row_base); note_launch(); }
-    }
-    if (c[2]) {
-        const size_t smem = size_t(W + 2) * kGroupCta * sizeof(uint64_t);
-        cudaFuncSetAttribute(k_refine_cta<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        unsigned g = unsigned(std::min<unsigned long long>(c[2], 152ull * 8));
-        { k_refine_cta<W><<<g, 512, smem, st>>>(G.list[2], G.counts + 2, pk, L, val, off, G.bwt, G.isa, G.isa_m, G.row_base); note_launch(); }
-    }
-}
+constexpr int kMoreRanges = 4096;           // ranges described at a time,
+constexpr int kMoreSplits = 64;             // and split at a time
 
-// Groups of up to 1024 suffixes are finished in place by the warp and CTA kernels.  A larger group
-// (low-complexity or highly repeated sequence) gets a device-wide radix sort of its range on the
-// next 29 bases (64-bit keys), and its subgroups are finished the same way, 29 bases further on
-// each time.
-template <int W>
-static int refine_groups_w(const GroupLists& G, const unsigned long long* c0,
-                           const std::vector<unsigned long long>& big, const uint64_t* pk, idx_t L, idx_t* val,
-                           uint64_t* cols, size_t cols_cap, void* rtmp, size_t rtmp_bytes, cudaStream_t st) {
-    refine_small_mid<W>(G, c0, pk, L, val, kHead, st);
-    struct Item {
-        size_t start, m;
-        int off;
-    };
-    std::vector<Item> work;
-    for (size_t i = 0; i + 1 < big.size(); i += 2) work.push_back({size_t(big[i]), size_t(big[i + 1]), kHead});
-    std::vector<unsigned long long> sub;
-    while (!work.empty()) {
-        const Item it = work.back();
-        work.pop_back();
-        const size_t m = it.m;
-        // range scratch in the column area: two key arrays, two value arrays
-        const size_t kw = m, vw = (m * sizeof(idx_t) + 7) / 8;
-        if (2 * kw + 2 * vw + 64 > cols_cap) return -1;
-        uint64_t* ka = cols;
-        uint64_t* kb = cols + kw;
-        idx_t* va = reinterpret_cast<idx_t*>(cols + 2 * kw);
-        idx_t* vb = reinterpret_cast<idx_t*>(cols + 2 * kw + vw);
-        { k_range_keys<<<grid_for(m, 256), 256, 0, st>>>(pk, val + it.start, m, L, it.off, ka, va); note_launch(); }
-        int rc = radix_sort_pairs<uint64_t, idx_t>(&ka, &va, &kb, &vb, m, 0, 64, rtmp, rtmp_bytes, st, true);
-        if (rc) return rc;
-        { k_copy_vals<idx_t><<<grid_for(m, 256), 256, 0, st>>>(va, m, val + it.start); note_launch(); }
-        if (it.off + kWide >= int(L)) continue;          // every suffix is now fully compared
-        cudaMemsetAsync(G.counts, 0, 4 * sizeof(unsigned long long), st);
-        { k_group_lists<uint64_t><<<unsigned(std::min<size_t>((m + kGlTile - 1) / kGlTile, size_t(152) * 64)), 256, 0, st>>>(
-              ka, m, G, it.start); note_launch(); }
-        unsigned long long c[4];
-        cudaMemcpyAsync(c, G.counts, sizeof c, cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) return int(e);
-        for (int z = 0; z < 4; ++z)
-            if (c[z] > G.cap[z]) return -1;
-        refine_small_mid<W>(G, c, pk, L, val, it.off + kWide, st);
-        if (c[3]) {
-            sub.resize(2 * c[3]);
-            cudaMemcpyAsync(sub.data(), G.list[3], sub.size() * 8, cudaMemcpyDeviceToHost, st);
-            e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) return int(e);
-            for (size_t i = 0; i + 1 < sub.size(); i += 2)
-                work.push_back({size_t(sub[i]), size_t(sub[i + 1]), it.off + kWide});
+// new elements for ranges whose suffixes are equal in their first off[range] bases: the next
+// more_bits / 2 of them, left-aligned in the key
+__global__ void __launch_bounds__(kSplitThreads) k_more_rebuild(const uint64_t* __restrict__ pk, MsdPlan a, int more_bits,
+                                                                MsdRanges r, const int* __restrict__ off,
+                                                                uint64_t* __restrict__ buf) {
+    const unsigned tiles = r.tile0[r.count];
+    for (unsigned t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int q = range_of(r, t);
+        const size_t b = r.start[q] + size_t(t - r.tile0[q]) * kSplitTile;
+        const size_t e = zmin(r.end[q], b + kSplitTile);
+        for (size_t i = b + threadIdx.x; i < e; i += kSplitThreads) {
+            const uint64_t low = buf[i] & ((uint64_t(1) << a.len_shift) - 1);
+            const size_t p = size_t(low >> kSymBits);
+            const int rem = suffix_bases(p, a.dl) - off[q];
+            uint64_t key = 0;
+            int w = 0;
+            if (rem > 0) {
+                uint64_t x = window(pk, p + size_t(off[q]));
+                if (rem < 32) x &= ~uint64_t(0) << (64 - 2 * rem);
+                key = (x >> (64 - more_bits)) << (a.kbits - more_bits);
+                w = rem < more_bits / 2 ? rem : more_bits / 2;
+            }
+            buf[i] = (key << a.key_shift) | (uint64_t(w) << a.len_shift) | low;
         }
     }
-    return int(cudaGetLastError());
 }
 
-// lists_mem holds the four group lists: (n/2 + n/33 + n/129 + 2 n/1025 + 5) 64-bit entries,
-// under 0.55 n
-static int refine_groups(const uint32_t* key, idx_t* val, size_t n, idx_t L, const uint64_t* pk, uint64_t* lists_mem,
-                         uint64_t* cols, size_t cols_cap, unsigned long long* counters, void* rtmp, size_t rtmp_bytes,
-                         cudaStream_t st, uint8_t* bwt = nullptr, idx_t* isa = nullptr, idx_t isa_m = 0,
-                         size_t row_base = 0) {
-    // words from base 14 on: 30 bases in the first (beside the segment number), 32 in each other
-    const int W = 1 + int((size_t(L) > size_t(kHead) + 30 ? size_t(L) - kHead - 30 + 31 : 0) / 32);
-    if (W < 1 || W > kRefineMaxWords) return -1;
-    GroupLists G;
-    G.cap[0] = n / 2 + 1;
-    G.cap[1] = n / 33 + 1;
-    G.cap[2] = n / (kGroupWarp4 + 1) + 1;
-    G.cap[3] = n / (kGroupCta + 1) + 1;
-    G.list[0] = reinterpret_cast<unsigned long long*>(lists_mem);
-    G.list[1] = G.list[0] + G.cap[0];
-    G.list[2] = G.list[1] + G.cap[1];
-    G.list[3] = G.list[2] + G.cap[2];
-    G.counts = counters;
-    G.bwt = bwt;
-    G.isa = isa;
-    G.isa_m = isa_m;
-    G.row_base = row_base;
-    cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), st);
-    { k_group_lists<uint32_t><<<unsigned(std::min<size_t>((n + kGlTile - 1) / kGlTile, size_t(152) * 64)), 256, 0, st>>>(
-          key, n, G, 0); note_launch(); }
-    unsigned long long c[4];
-    cudaMemcpyAsync(c, counters, sizeof c, cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return int(e);
-    std::vector<unsigned long long> big(2 * c[3]);
-    if (c[3]) {
-        cudaMemcpyAsync(big.data(), G.list[3], big.size() * 8, cudaMemcpyDeviceToHost, st);
-        e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) return int(e);
+// the bits in which each range's elements differ, and its first element
+__global__ void __launch_bounds__(kSplitThreads) k_more_diff(const uint64_t* __restrict__ buf, MsdRanges r,
+                                                             unsigned long long* __restrict__ diff,
+                                                             unsigned long long* __restrict__ e0) {
+    const unsigned tiles = r.tile0[r.count];
+    for (unsigned t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int q = range_of(r, t);
+        const size_t b = r.start[q] + size_t(t - r.tile0[q]) * kSplitTile;
+        const size_t e = zmin(r.end[q], b + kSplitTile);
+        const uint64_t first = buf[r.start[q]];
+        uint64_t d = 0;
+        for (size_t i = b + threadIdx.x; i < e; i += kSplitThreads) d |= buf[i] ^ first;
+        const unsigned lo = __reduce_or_sync(0xffffffffu, unsigned(d)), hi = __reduce_or_sync(0xffffffffu, unsigned(d >> 32));
+        if ((threadIdx.x & 31) == 0) atomicOr(&diff[q], (unsigned long long)((uint64_t(hi) << 32) | lo));
+        if (threadIdx.x == 0 && b == r.start[q]) e0[q] = first;
     }
-    switch (W) {
-        case 1: return refine_groups_w<1>(G, c, big, pk, L, val, cols, cols_cap, rtmp, rtmp_bytes, st);
-        case 2: return refine_groups_w<2>(G, c, big, pk, L, val, cols, cols_cap, rtmp, rtmp_bytes, st);
-        case 3: return refine_groups_w<3>(G, c, big, pk, L, val, cols, cols_cap, rtmp, rtmp_bytes, st);
-        case 4: return refine_groups_w<4>(G, c, big, pk, L, val, cols, cols_cap, rtmp, rtmp_bytes, st);
-        case 5: return refine_groups_w<5>(G, c, big, pk, L, val, cols, cols_cap, rtmp, rtmp_bytes, st);
-        case 6: return refine_groups_w<6>(G, c, big, pk, L, val, cols, cols_cap, rtmp, rtmp_bytes, st);
-        case 7: return refine_groups_w<7>(G, c, big, pk, L, val, cols, cols_cap, rtmp, rtmp_bytes, st);
-        default: return refine_groups_w<8>(G, c, big, pk, L, val, cols, cols_cap, rtmp, rtmp_bytes, st);
+}
+
+__global__ void __launch_bounds__(kSplitThreads) k_more_copy(const uint64_t* __restrict__ from, MsdRanges r,
+                                                             uint64_t* __restrict__ to) {
+    const unsigned tiles = r.tile0[r.count];
+    for (unsigned t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int q = range_of(r, t);
+        const size_t b = r.start[q] + size_t(t - r.tile0[q]) * kSplitTile;
+        const size_t e = zmin(r.end[q], b + kSplitTile);
+        for (size_t i = b + threadIdx.x; i < e; i += kSplitThreads) to[i] = from[i];
     }
+}
+
+// A k-mer table whose k-mers span buckets is entered by minimum and maximum: prepared so (mode 0;
+// mode 2 only where a k-mer is still absent), then absent ones set as everywhere else (mode 1:
+// kend < kstart)
+__global__ void k_kmer_span(idx_t* __restrict__ kstart, idx_t* __restrict__ kend, size_t c0, size_t c1, int mode) {
+    const size_t stride = size_t(gridDim.x) * blockDim.x;
+    for (size_t i = c0 + size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < c1; i += stride) {
+        if (mode == 0 || (mode == 2 && kend[i] < kstart[i])) {
+            kstart[i] = ~idx_t(0);
+            kend[i] = 0;
+        } else if (mode == 1 && kstart[i] == ~idx_t(0)) {
+            kstart[i] = 1;
+        }
+    }
+}
+
+// rows [r0, r1) all start with k-mer c
+__global__ void k_kmer_rows(idx_t* __restrict__ kstart, idx_t* __restrict__ kend, size_t c, size_t r0, size_t r1) {
+    atomicMin(reinterpret_cast<kmer_int*>(kstart + c), kmer_int(r0));
+    atomicMax(reinterpret_cast<kmer_int*>(kend + c), kmer_int(r1 - 1));
 }
 
 // ------------------------------------------------------------------------------ driver
 
 static size_t al(size_t b) { return (b + 255) & ~size_t(255); }
 
-size_t suffix_sort_tmp_bytes(size_t n) {
-    size_t tiles = (n + HT_TILE - 1) / HT_TILE + 1;
-    return 2 * al(n * sizeof(uint64_t)) + al(n * sizeof(idx_t)) + al(n * sizeof(uint32_t)) +
-           al((n / 32 + 4) * sizeof(uint64_t)) + al(radix_tmp_bytes(n)) + al(3 * tiles * sizeof(unsigned long long)) +
-           al(n) + 1024;
+namespace {
+
+// The working memory of one sort of `m` suffixes at a time out of n.
+struct MsdScratch {
+    uint64_t *a, *b;                                // elements after the first and the second pass
+    unsigned long long *hist, *cnt, *shorts;        // cleared together with the counters
+    MsdCounters* counters;
+    size_t clear_bytes;
+    unsigned long long *start1, *cursor1, *lstart, *cursor, *sfirst;
+    unsigned* tile0;
+    MsdBucket *small, *large, *more;
+    unsigned long long *mid, *big, *huge;
+    size_t cap_list, cap_more, cap_mid, cap_big, cap_huge;
+    uint32_t *sk0, *sk1;                            // short suffixes
+    idx_t *sv0, *sv1;
+    void* rtmp;
+    size_t rtmp_bytes;
+    unsigned long long *r_start, *r_end, *r_diff, *r_e0, *r_cnt, *r_cursor;     // further splits
+    unsigned* r_tile0;
+    int *r_off, *r_shift;
+    uint64_t* pk;
+    uint8_t* bwt;
+    unsigned long long* hist6;
+    size_t bytes;
+};
+
+MsdScratch msd_layout(void* base, const MsdPlan& p, size_t m, size_t nr) {
+    MsdScratch s{};
+    size_t used = 0;
+    auto take = [&](size_t bytes) {
+        char* q = base ? static_cast<char*>(base) + used : nullptr;
+        used += al(bytes);
+        return q;
+    };
+    using U = unsigned long long;
+    const size_t bins1 = size_t(1) << p.d1, buckets = size_t(1) << (p.d1 + p.d2);
+    const bool two = p.d2 > 0;
+    // 64-bit suffix arrays hold the first pass's elements themselves
+    s.a = sizeof(idx_t) == 4 ? reinterpret_cast<uint64_t*>(take(m * 8)) : nullptr;
+    s.b = reinterpret_cast<uint64_t*>(take(m * 8));
+    const size_t z0 = used;
+    s.counters = reinterpret_cast<MsdCounters*>(take(sizeof(MsdCounters)));
+    s.hist = reinterpret_cast<U*>(take(bins1 * 8));
+    s.cnt = reinterpret_cast<U*>(take(two ? buckets * 8 : 0));
+    s.shorts = reinterpret_cast<U*>(take(p.S ? buckets * 8 : 0));
+    s.clear_bytes = used - z0;
+    s.sfirst = reinterpret_cast<U*>(take(p.S ? buckets * 8 : 0));
+    s.start1 = reinterpret_cast<U*>(take(bins1 * 8));
+    s.cursor1 = reinterpret_cast<U*>(take(bins1 * 8));
+    s.tile0 = reinterpret_cast<unsigned*>(take((bins1 + 1) * 4));
+    s.lstart = reinterpret_cast<U*>(take(buckets * 8));
+    s.cursor = reinterpret_cast<U*>(take(buckets * 8));
+    s.cap_list = std::max<size_t>(buckets, kMoreRanges);
+    s.small = reinterpret_cast<MsdBucket*>(take(buckets * sizeof(MsdBucket)));
+    s.large = reinterpret_cast<MsdBucket*>(take(s.cap_list * sizeof(MsdBucket)));
+    s.cap_more = m / (kLocalLarge + 1) + 1;
+    s.cap_mid = m / 33 + 1;
+    s.cap_big = m / 129 + 1;
+    s.cap_huge = m / 1025 + 1;
+    s.more = reinterpret_cast<MsdBucket*>(take(s.cap_more * sizeof(MsdBucket)));
+    s.mid = reinterpret_cast<U*>(take(s.cap_mid * 8));
+    s.big = reinterpret_cast<U*>(take(s.cap_big * 8));
+    s.huge = reinterpret_cast<U*>(take(s.cap_huge * 8));
+    const size_t sh = nr * size_t(p.S);
+    s.sk0 = reinterpret_cast<uint32_t*>(take(sh * 4));
+    s.sk1 = reinterpret_cast<uint32_t*>(take(sh * 4));
+    s.sv0 = reinterpret_cast<idx_t*>(take(sh * sizeof(idx_t)));
+    s.sv1 = reinterpret_cast<idx_t*>(take(sh * sizeof(idx_t)));
+    s.rtmp_bytes = p.S ? radix_tmp_bytes(sh) : 0;
+    s.rtmp = take(s.rtmp_bytes);
+    s.r_start = reinterpret_cast<U*>(take(kMoreRanges * 8));
+    s.r_end = reinterpret_cast<U*>(take(kMoreRanges * 8));
+    s.r_diff = reinterpret_cast<U*>(take(kMoreRanges * 8));
+    s.r_e0 = reinterpret_cast<U*>(take(kMoreRanges * 8));
+    s.r_tile0 = reinterpret_cast<unsigned*>(take((kMoreRanges + 1) * 4));
+    s.r_off = reinterpret_cast<int*>(take(kMoreRanges * 4));
+    s.r_shift = reinterpret_cast<int*>(take(kMoreSplits * 4));
+    s.r_cnt = reinterpret_cast<U*>(take((size_t(kMoreSplits) << kMoreBits) * 8));
+    s.r_cursor = reinterpret_cast<U*>(take((size_t(kMoreSplits) << kMoreBits) * 8));
+    s.pk = reinterpret_cast<uint64_t*>(take((p.n / 32 + 4) * 8));
+    s.bwt = reinterpret_cast<uint8_t*>(take(p.n));
+    s.hist6 = reinterpret_cast<U*>(take(size_t(kBuckets) * 8));
+    s.bytes = used;
+    return s;
 }
 
-int suffix_sort(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa, void* tmp, size_t tmp_bytes,
-                cudaStream_t st, const uint32_t** keys_out, const uint8_t** bwt_out, uint64_t* pk_out,
-                idx_t* isa_out, idx_t isa_m) {
-    if (keys_out) *keys_out = nullptr;
-    if (bwt_out) *bwt_out = nullptr;
-    const size_t n = size_t(num_reads) * size_t(L);
-    if (n == 0) return 0;
-    if (n >= (size_t(1) << 31)) return int(cudaErrorNotSupported);   // 32-bit group ranks
-    if (tmp_bytes < suffix_sort_tmp_bytes(n)) return int(cudaErrorInvalidValue);
+// Working memory of prefix doubling: two 64-bit key arrays, one value array (the other is the
+// suffix array), 32-bit ranks, packed text, per-tile group heads.
+size_t doubling_bytes(size_t n) {
+    const size_t tiles = (n + HT_TILE - 1) / HT_TILE + 1;
+    return 2 * al(n * sizeof(uint64_t)) + al(n * sizeof(idx_t)) + al(n * sizeof(uint32_t)) +
+           al((n / 32 + 4) * sizeof(uint64_t)) + al(radix_tmp_bytes(n)) + al(3 * tiles * sizeof(unsigned long long)) +
+           1024;
+}
+
+// What a sort in chunks of `cap` suffixes may take: 24 bytes and two positions a suffix of a chunk
+// and 3 1/4 bytes a suffix of the index.  One pass over everything is used when it needs no more.
+size_t chunk_budget(size_t n, size_t cap) { return cap * (20 + 2 * sizeof(idx_t)) + 3 * n + n / 4; }
+
+struct SortShape {
+    MsdPlan plan;
+    bool doubling, chunked;
+    size_t m;               // suffixes sorted at a time
+    size_t bytes;
+};
+
+SortShape sort_shape(size_t n, size_t nr, int L, size_t cap) {
+    SortShape s{};
+    s.plan = make_plan(n, nr, idx_t(L), true);
+    s.m = n;
+    if (plan_words(s.plan) > kMaxWords) {
+        s.doubling = true;
+        s.bytes = doubling_bytes(n);
+        return s;
+    }
+    s.bytes = msd_layout(nullptr, s.plan, n, nr).bytes + 1024;
+    if (cap && cap < n && s.bytes > chunk_budget(n, cap)) {
+        s.chunked = true;
+        s.plan = make_plan(n, nr, idx_t(L), false);
+        s.m = cap;
+        s.bytes = msd_layout(nullptr, s.plan, cap, nr).bytes + 1024;
+    }
+    return s;
+}
+
+struct SortRange {
+    unsigned long long start, end;
+    int off;
+    unsigned id;            // off = 0: the bucket it is part of
+    bool rebuild;
+};
+
+template <int W>
+struct MsdKernels {
+    static int local_blocks(bool large, int sms) {
+        static_assert(W >= 1 && W <= kMaxWords, "networks of 1 .. kMaxWords words");
+        int per = 0;
+        const cudaError_t e = large
+            ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_msd_local<W, kLocalLarge, 256>, 256, local_smem<kLocalLarge>())
+            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_msd_local<W, kLocalSmall, 128>, 128, local_smem<kLocalSmall>());
+        if (e != cudaSuccess) cudaGetLastError();
+        return (e == cudaSuccess && per > 0 ? per : 1) * sms;
+    }
+    static void prepare() {
+        cudaFuncSetAttribute(k_msd_local<W, kLocalSmall, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(local_smem<kLocalSmall>()));
+        cudaFuncSetAttribute(k_msd_local<W, kLocalLarge, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(local_smem<kLocalLarge>()));
+        cudaFuncSetAttribute(k_refine_cta<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(size_t(W + 2) * 1024 * sizeof(uint64_t)));
+    }
+    static void local(bool large, MsdLocal a, const MsdScratch& s, size_t most, int sms, cudaStream_t st) {
+        a.list = large ? s.large : s.small;
+        a.count = large ? &s.counters->large : &s.counters->small;
+        a.next = large ? &s.counters->next_large : &s.counters->next_small;
+        const unsigned g = unsigned(std::max<size_t>(1, std::min<size_t>(most, size_t(local_blocks(large, sms)))));
+        if (large) k_msd_local<W, kLocalLarge, 256><<<g, 256, local_smem<kLocalLarge>(), st>>>(a);
+        else k_msd_local<W, kLocalSmall, 128><<<g, 128, local_smem<kLocalSmall>(), st>>>(a);
+        note_launch();
+    }
+    static void groups(const MsdLocal& a, const MsdScratch& s, int sms, cudaStream_t st) {
+        const size_t warps = (s.cap_mid + 7) / 8;
+        const unsigned g = unsigned(std::max<size_t>(1, std::min<size_t>((warps + 7) / 8, size_t(sms) * 4)));
+        k_refine_warp<W><<<g, kRefineThreads, 0, st>>>(s.mid, &s.counters->mid, a.pk, a.plan.dl, a.sa, a.bwt);
+        note_launch();
+        const size_t smem = size_t(W + 2) * 1024 * sizeof(uint64_t);
+        k_refine_cta<W><<<unsigned(std::min<size_t>(s.cap_big, size_t(sms) * 2)), 512, smem, st>>>(
+            s.big, &s.counters->big, a.pk, a.plan.dl, a.sa, a.bwt);
+        note_launch();
+    }
+};
+
+// The further splits (see above) of the listed buckets and groups.
+template <int W>
+int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t* tmp, int sms, cudaStream_t st) {
+    const MsdPlan& P = a.plan;
+    const int k = a.kmer_k, bits = P.d1 + P.d2;
+    const bool own_span = a.kstart && !a.kmer_spans;        // a listed bucket's k-mers span its parts
+    std::vector<unsigned> split_ids;
+    auto h2d = [&](void* d, const void* h, size_t b) { return cudaMemcpyAsync(d, h, b, cudaMemcpyHostToDevice, st); };
+    auto d2h = [&](void* h, const void* d, size_t b) { return cudaMemcpyAsync(h, d, b, cudaMemcpyDeviceToHost, st); };
+    std::vector<SortRange> work;
+    auto take_huge = [&](unsigned long long count) -> int {
+        if (count > s.cap_huge) return int(cudaErrorUnknown);
+        std::vector<unsigned long long> h(count);
+        if (count) d2h(h.data(), s.huge, count * 8);
+        const cudaError_t e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return int(e);
+        for (unsigned long long g : h)
+            work.push_back({g >> 24, (g >> 24) + (g & 0x3fff), int((g >> 14) & 0x3ff), 0, true});
+        return 0;
+    };
+    {
+        if (c0.more > s.cap_more) return int(cudaErrorUnknown);
+        std::vector<MsdBucket> m(c0.more);
+        if (c0.more) d2h(m.data(), s.more, c0.more * sizeof(MsdBucket));
+        const int rc = take_huge(c0.huge);
+        if (rc) return rc;
+        for (const MsdBucket& b : m) {
+            if (b.size == 0xffffffffu) return int(cudaErrorNotSupported);
+            const unsigned id = b.id_off & ((1u << kIdBits) - 1);
+            work.push_back({b.start, b.start + b.size, 0, id, false});
+            if (own_span) {
+                const size_t per = size_t(1) << (2 * k - bits);
+                k_kmer_span<<<grid_for(per, 256), 256, 0, st>>>(a.kstart, a.kend, id * per, (id + 1) * per, 2);
+                note_launch();
+                split_ids.push_back(id);
+            }
+        }
+        if (own_span) a.kmer_spans = 1;
+    }
+    std::vector<SortRange> local;
+    std::vector<unsigned long long> rs, re;
+    std::vector<unsigned> tile0;
+    std::vector<int> ri;
+    // describes ranges v[i0, i1) on the device; false when they are too many tiles for one launch
+    auto describe = [&](const std::vector<SortRange>& v, size_t i0, size_t i1) {
+        rs.clear();
+        re.clear();
+        tile0.assign(1, 0);
+        ri.clear();
+        for (size_t i = i0; i < i1; ++i) {
+            rs.push_back(v[i].start);
+            re.push_back(v[i].end);
+            ri.push_back(v[i].off);
+            tile0.push_back(tile0.back() + unsigned((v[i].end - v[i].start + kSplitTile - 1) / kSplitTile));
+        }
+        h2d(s.r_start, rs.data(), rs.size() * 8);
+        h2d(s.r_end, re.data(), re.size() * 8);
+        h2d(s.r_tile0, tile0.data(), tile0.size() * 4);
+        h2d(s.r_off, ri.data(), ri.size() * 4);
+        MsdRanges r{};
+        r.start = s.r_start;
+        r.end = s.r_end;
+        r.tile0 = s.r_tile0;
+        r.count = int(i1 - i0);
+        return r;
+    };
+    auto grid = [&] { return std::min(tile0.back(), unsigned(sms * 4)); };
+    while (!work.empty() || !local.empty()) {
+        while (!work.empty()) {
+            // new elements where a range's are used up
+            std::vector<SortRange> v;
+            for (SortRange& r : work)
+                if (r.rebuild) v.push_back(r);
+            for (size_t i = 0; i < v.size(); i += kMoreRanges) {
+                const MsdRanges r = describe(v, i, std::min(v.size(), i + kMoreRanges));
+                k_more_rebuild<<<grid(), kSplitThreads, 0, st>>>(a.pk, P, a.more_bits, r, s.r_off, a.buf);
+                note_launch();
+            }
+            v.clear();
+            for (SortRange& r : work) {
+                r.rebuild = false;
+                (r.end - r.start <= size_t(kLocalLarge) ? local : v).push_back(r);
+            }
+            work.clear();
+            // where the others' elements differ
+            std::vector<SortRange> split;
+            std::vector<int> shift;
+            for (size_t i = 0; i < v.size(); i += kMoreRanges) {
+                const size_t i1 = std::min(v.size(), i + kMoreRanges);
+                const MsdRanges r = describe(v, i, i1);
+                cudaMemsetAsync(s.r_diff, 0, r.count * 8, st);
+                k_more_diff<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_diff, s.r_e0);
+                note_launch();
+                std::vector<unsigned long long> d(r.count), e0(r.count);
+                d2h(d.data(), s.r_diff, d.size() * 8);
+                d2h(e0.data(), s.r_e0, e0.size() * 8);
+                const cudaError_t e = cudaStreamSynchronize(st);
+                if (e != cudaSuccess) return int(e);
+                for (int q = 0; q < r.count; ++q) {
+                    SortRange x = v[i + q];
+                    int hb = 63;
+                    while (hb > 0 && !((d[q] >> hb) & 1)) --hb;
+                    const int full = x.off ? a.more_bits / 2 : P.head;
+                    if (hb < P.len_shift && int((e0[q] >> P.len_shift) & 31) == full) {
+                        if (a.kstart && !x.off) {            // one k-mer throughout
+                            const int top = 2 * k - P.d1;
+                            const uint64_t id1 = x.id >> P.d2, key = e0[q] >> P.key_shift;
+                            const uint64_t c = top >= 0 ? (id1 << top) | (key >> (P.kbits - top)) : id1 >> (-top);
+                            k_kmer_rows<<<1, 1, 0, st>>>(a.kstart, a.kend, size_t(c), a.row0 + x.start, a.row0 + x.end);
+                            note_launch();
+                        }
+                        x.off += full;
+                        x.rebuild = true;
+                        work.push_back(x);
+                        continue;
+                    }
+                    int sh = hb - (kMoreBits - 1);
+                    if (hb >= P.key_shift) sh = std::max(sh, P.key_shift);
+                    else if (hb >= P.len_shift) sh = P.len_shift;
+                    split.push_back(x);
+                    shift.push_back(std::max(sh, 0));
+                }
+            }
+            for (size_t i = 0; i < split.size(); i += kMoreSplits) {
+                const size_t i1 = std::min(split.size(), i + kMoreSplits);
+                MsdRanges r = describe(split, i, i1);
+                h2d(s.r_shift, shift.data() + i, (i1 - i) * 4);
+                r.shift = s.r_shift;
+                r.bits = kMoreBits;
+                const size_t nc = (i1 - i) << kMoreBits;
+                cudaMemsetAsync(s.r_cnt, 0, nc * 8, st);
+                k_msd_count<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_cnt);
+                note_launch();
+                std::vector<unsigned long long> cnt(nc), cur(nc);
+                d2h(cnt.data(), s.r_cnt, nc * 8);
+                const cudaError_t e = cudaStreamSynchronize(st);
+                if (e != cudaSuccess) return int(e);
+                for (size_t q = i; q < i1; ++q) {
+                    unsigned long long at = split[q].start;
+                    for (size_t d = 0; d < (size_t(1) << kMoreBits); ++d) {
+                        const size_t c = ((q - i) << kMoreBits) + d;
+                        cur[c] = at;
+                        if (cnt[c])
+                            (cnt[c] <= (unsigned long long)kLocalLarge ? local : work)
+                                .push_back({at, at + cnt[c], split[q].off, split[q].id, false});
+                        at += cnt[c];
+                    }
+                }
+                h2d(s.r_cursor, cur.data(), nc * 8);
+                k_msd_split<<<grid(), kSplitThreads, MsdSmem::bytes(kMoreBits, false), st>>>(a.buf, r, s.r_cursor, tmp);
+                note_launch();
+                k_more_copy<<<grid(), kSplitThreads, 0, st>>>(tmp, r, a.buf);
+                note_launch();
+            }
+        }
+        // every part fits the local kernel; its groups of more than 1024 come back
+        std::vector<SortRange> now;
+        now.swap(local);
+        for (size_t i = 0; i < now.size(); i += s.cap_list) {
+            const size_t i1 = std::min(now.size(), i + s.cap_list);
+            std::vector<MsdBucket> b;
+            for (size_t q = i; q < i1; ++q)
+                b.push_back({now[q].start, unsigned(now[q].end - now[q].start), (unsigned(now[q].off) << kIdBits) | (now[q].off ? 0u : now[q].id)});
+            MsdCounters c{};
+            c.large = b.size();
+            h2d(s.counters, &c, sizeof c);
+            h2d(s.large, b.data(), b.size() * sizeof(MsdBucket));
+            MsdKernels<W>::local(true, a, s, b.size(), sms, st);
+            MsdKernels<W>::groups(a, s, sms, st);
+            d2h(&c, s.counters, sizeof c);
+            const cudaError_t e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess) return int(e);
+            if (c.mid > s.cap_mid || c.big > s.cap_big) return int(cudaErrorUnknown);
+            const int rc = take_huge(c.huge);
+            if (rc) return rc;
+        }
+    }
+    for (unsigned id : split_ids) {
+        const size_t per = size_t(1) << (2 * k - bits);
+        k_kmer_span<<<grid_for(per, 256), 256, 0, st>>>(a.kstart, a.kend, id * per, (id + 1) * per, 1);
+        note_launch();
+    }
+    return int(cudaGetLastError());
+}
+
+struct SortOut {
+    idx_t* sa;
+    uint8_t* bwt;
+    idx_t *kstart, *kend;
+    int kmer_k;
+    bool kmer_spans;        // k-mers shorter than the buckets' prefix (or a chunk boundary's)
+    bool kmer_done;
+};
+
+// One chunk (or everything): the suffixes whose 6-base bucket lies in [c0, c1), m of them from row
+// `row0` on; hist6 (host) holds a chunked sort's 6-base bucket counts.
+template <int W>
+int msd_pass(const MsdPlan& P, size_t nr, const MsdScratch& s, const SortOut& o, size_t row0, size_t m, uint32_t c0, uint32_t c1,
+             const unsigned long long* hist6, size_t cap, bool* listed_more, cudaStream_t st) {
+    const int sms = device_sms();
+    const size_t bins1 = size_t(1) << P.d1;
+    const int bits = P.d1 + P.d2;
+    uint64_t* const ea = sizeof(idx_t) == 8 ? reinterpret_cast<uint64_t*>(o.sa + row0) : s.a;
+    MsdLists G{s.small, s.large, s.more, s.mid, s.big, s.huge, s.cap_more, s.cap_mid, s.cap_big, s.cap_huge, s.counters};
+    const size_t tiles = (P.n + kSplitTile - 1) / kSplitTile;
+    const unsigned wide = unsigned(std::min<size_t>(tiles, size_t(sms) * 2));
+    const size_t smem_text = MsdSmem::bytes(P.d1, true), smem_split = MsdSmem::bytes(std::max(P.d2, kMoreBits), false);
+    cudaFuncSetAttribute(k_msd_text, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_text));
+    cudaFuncSetAttribute(k_msd_split, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_split));
+    MsdKernels<W>::prepare();
+
+    cudaMemsetAsync(s.counters, 0, s.clear_bytes, st);
+    if (hist6) {
+        std::vector<unsigned long long> h(bins1, 0);
+        for (uint32_t c = c0; c < c1; ++c) h[(c >> 3) >> (2 * kBucketBases - P.d1)] += hist6[c];
+        cudaMemcpyAsync(s.hist, h.data(), bins1 * 8, cudaMemcpyHostToDevice, st);
+        const cudaError_t e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return int(e);
+    } else {
+        k_msd_hist<<<unsigned(std::min<size_t>(tiles, size_t(sms) * 4)), kSplitThreads, 0, st>>>(s.pk, P, s.hist);
+        note_launch();
+    }
+    const size_t nshort = nr * size_t(P.S);
+    const unsigned gs = grid_for(nshort, 256);
+    uint32_t *sk0 = s.sk0, *sk1 = s.sk1;
+    idx_t *sv0 = s.sv0, *sv1 = s.sv1;
+    if (P.S) {
+        k_short_keys<<<gs, 256, 0, st>>>(s.pk, nr, P.dl.L, P.S, sk0, sv0);
+        note_launch();
+        const int rc = radix_sort_pairs<uint32_t, idx_t>(&sk0, &sv0, &sk1, &sv1, nshort, 0, P.S <= 3 ? 8 : 16, s.rtmp,
+                                                         s.rtmp_bytes, st, false);
+        if (rc) return rc;
+        cudaMemsetAsync(s.sfirst, 0xff, (size_t(1) << bits) * 8, st);
+        k_short_runs<<<gs, 256, 0, st>>>(s.pk, sk0, sv0, nshort, P.dl, bits, s.shorts, s.sfirst);
+        note_launch();
+    }
+    if (!P.d2) {
+        k_msd_children<<<1, kScanThreads, 0, st>>>(s.hist, P.S ? s.shorts : nullptr, P.d1, 1, nullptr, s.lstart, s.cursor, 1, G);
+        k_msd_text<<<wide, kSplitThreads, smem_text, st>>>(s.pk, P, s.cursor, s.b, c0, c1);
+        note_launch();
+        note_launch();
+    } else {
+        k_msd_children<<<1, kScanThreads, 0, st>>>(s.hist, nullptr, P.d1, 1, nullptr, s.start1, s.cursor1, 0, G);
+        k_msd_text<<<wide, kSplitThreads, smem_text, st>>>(s.pk, P, s.cursor1, ea, c0, c1);
+        k_msd_tiles<<<1, 1024, 0, st>>>(s.start1, s.cursor1, int(bins1), s.tile0);
+        MsdRanges r{};
+        r.start = s.start1;
+        r.end = s.cursor1;
+        r.tile0 = s.tile0;
+        r.ushift = P.key_shift + P.kbits - P.d2;
+        r.count = int(bins1);
+        r.bits = P.d2;
+        k_msd_count<<<unsigned(sms * 4), kSplitThreads, 0, st>>>(ea, r, s.cnt);
+        k_msd_children<<<unsigned(bins1), kScanThreads, 0, st>>>(s.cnt, P.S ? s.shorts : nullptr, P.d2, 0, s.start1, s.lstart,
+                                                                 s.cursor, 1, G);
+        k_msd_split<<<unsigned(sms * 2), kSplitThreads, smem_split, st>>>(ea, r, s.cursor, s.b);
+        for (int i = 0; i < 6; ++i) note_launch();
+    }
+    if (P.S) {
+        k_short_place<<<gs, 256, 0, st>>>(s.pk, sk0, sv0, nshort, P.dl, bits, s.shorts, s.sfirst, s.lstart, o.sa, o.bwt,
+                                          o.kmer_k <= P.S ? o.kstart : nullptr, o.kend, o.kmer_k);
+        note_launch();
+    }
+    MsdLocal a{};
+    a.plan = P;
+    a.pk = s.pk;
+    a.buf = s.b;
+    a.G = G;
+    a.sa = o.sa + row0;
+    a.bwt = o.bwt ? o.bwt + row0 : nullptr;
+    a.kstart = o.kstart;
+    a.kend = o.kend;
+    a.kmer_k = o.kmer_k;
+    a.kmer_spans = o.kmer_spans;
+    a.row0 = row0;
+    a.more_bits = P.kbits & ~1;
+    MsdKernels<W>::local(false, a, s, size_t(1) << bits, sms, st);
+    MsdKernels<W>::local(true, a, s, m / kLocalSmall + 1, sms, st);
+    MsdKernels<W>::groups(a, s, sms, st);
+    MsdCounters c;
+    std::vector<unsigned long long> h(cap ? bins1 : 0);
+    cudaMemcpyAsync(&c, s.counters, sizeof c, cudaMemcpyDeviceToHost, st);
+    if (cap) cudaMemcpyAsync(h.data(), s.hist, bins1 * 8, cudaMemcpyDeviceToHost, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return int(e);
+    if (c.mid > s.cap_mid || c.big > s.cap_big) return int(cudaErrorUnknown);
+    for (unsigned long long x : h)
+        if (x > cap) *listed_more = true;           // (the caller looks at the 6-base buckets)
+    if (c.more || c.huge) {
+        const int rc = more_splits<W>(c, a, s, ea, sms, st);
+        if (rc) return rc;
+    }
+    return int(cudaGetLastError());
+}
+
+}  // namespace
+
+size_t suffix_sort_tmp_bytes(size_t n, size_t num_reads, int L, size_t cap) {
+    return n ? sort_shape(n, num_reads, L, cap).bytes : 0;
+}
+
+// Prefix doubling on 29-base keys (reads longer than the networks' words).
+static int sort_doubling(size_t n, int L, idx_t* sa, const uint64_t* pk, void* tmp, cudaStream_t st) {
     char* p = static_cast<char*>(tmp);
     uint64_t* ka = reinterpret_cast<uint64_t*>(p); p += al(n * sizeof(uint64_t));
     uint64_t* kb = reinterpret_cast<uint64_t*>(p); p += al(n * sizeof(uint64_t));
-    // the values start in the suffix array itself (four radix passes bring them back there)
     idx_t* va = sa;
     idx_t* vb = reinterpret_cast<idx_t*>(p); p += al(n * sizeof(idx_t));
     uint32_t* rank = reinterpret_cast<uint32_t*>(p); p += al(n * sizeof(uint32_t));
-    const size_t nwords = n / 32 + 4;
-    uint64_t* pk = pk_out ? pk_out : reinterpret_cast<uint64_t*>(p);
-    p += al(nwords * sizeof(uint64_t));
+    p += al((n / 32 + 4) * sizeof(uint64_t));           // packed text, when the caller keeps none
     void* rtmp = p; p += al(radix_tmp_bytes(n));
     const size_t tiles = (n + HT_TILE - 1) / HT_TILE;
     unsigned long long* tmax = reinterpret_cast<unsigned long long*>(p);
     unsigned long long* tcnt = tmax + tiles + 1;
     unsigned long long* groups = tcnt + tiles + 1;
-    p += al(3 * (tiles + 1) * sizeof(unsigned long long));
-    // BWT symbols of the refined rows (0xff elsewhere), kept only when asked for
-    uint8_t* bwt = bwt_out ? reinterpret_cast<uint8_t*>(p) : nullptr;
-
-    idx_t* const vb0 = vb;                 // followed by rank in memory
-    auto finish = [&](const uint32_t* keys) {
-        if (va != sa) { k_copy_vals<idx_t><<<grid_for(n, 256), 256, 0, st>>>(va, n, sa); note_launch(); }
-        if (keys_out) *keys_out = keys;
-        return int(cudaGetLastError());
-    };
-    { k_pack_text<<<grid_for(nwords, 256), 256, 0, st>>>(reads, n, idx_t(L), dir, nwords, pk); note_launch(); }
-    // 32-bit head keys in the two 64-bit key buffers
-    uint32_t* ha = reinterpret_cast<uint32_t*>(ka);
-    uint32_t* hb = reinterpret_cast<uint32_t*>(kb);
-    if (reinterpret_cast<uintptr_t>(va) % 16 == 0 && reinterpret_cast<uintptr_t>(ha) % 16 == 0)
-        { k_init_keys4<<<grid_for((n + 3) / 4, 256), 256, 0, st>>>(pk, n, idx_t(L), ha, va); note_launch(); }
-    else    // a caller's suffix array that is not 16-byte aligned
-        { k_init_keys<uint32_t><<<grid_for(n, 256), 256, 0, st>>>(pk, n, idx_t(L), ha, va); note_launch(); }
-    // all four digits vary on any real read set: no histogram pass, no host round trip
-    int rc = radix_sort_pairs<uint32_t, idx_t>(&ha, &va, &hb, &vb, n, 0, 32, rtmp, radix_tmp_bytes(n), st, false);
+    { k_init_keys<<<grid_for(n, 256), 256, 0, st>>>(pk, n, idx_t(L), ka, va); note_launch(); }
+    int rc = radix_sort_pairs<uint64_t, idx_t>(&ka, &va, &kb, &vb, n, 0, 64, rtmp, radix_tmp_bytes(n), st, true);
     if (rc) return rc;
-    if (size_t(L) <= size_t(kHead)) return finish(ha);   // every suffix fits in its key: final order
-    {
-        // finish the groups where they lie; lists go to the free key buffer, big-group scratch to
-        // the free value buffer (and rank behind it when that buffer is the scratch one; when the
-        // values ended in the scratch, the free one is the suffix array, exactly n entries)
-        uint64_t* cols = reinterpret_cast<uint64_t*>(vb);
-        const size_t cols_cap = vb == vb0 ? (al(n * sizeof(idx_t)) + al(n * sizeof(uint32_t))) / sizeof(uint64_t)
-                                          : n * sizeof(idx_t) / sizeof(uint64_t);
-        if (bwt) cudaMemsetAsync(bwt, 0xff, n, st);
-        rc = refine_groups(ha, va, n, idx_t(L), pk, reinterpret_cast<uint64_t*>(hb), cols, cols_cap, tcnt, rtmp,
-                           radix_tmp_bytes(n), st, bwt, isa_out, isa_m);
-        if (rc > 0) return rc;
-        if (rc == 0) {   // the refinement permutes suffixes within groups of equal keys only
-            if (bwt_out) *bwt_out = bwt;
-            return finish(ha);
-        }
-        // a group too large for the scratch (or reads longer than 268 bases): prefix doubling on
-        // 29-base keys
-        ka = reinterpret_cast<uint64_t*>(ha);
-        kb = reinterpret_cast<uint64_t*>(hb);
-        { k_init_keys<uint64_t><<<grid_for(n, 256), 256, 0, st>>>(pk, n, idx_t(L), ka, va); note_launch(); }
-        rc = radix_sort_pairs<uint64_t, idx_t>(&ka, &va, &kb, &vb, n, 0, 64, rtmp, radix_tmp_bytes(n), st, true);
-        if (rc) return rc;
-    }
     for (size_t h = kWide;; h *= 2) {
         { k_head_tiles<<<unsigned(tiles), HT_THREADS, 0, st>>>(ka, n, tmax, tcnt); note_launch(); }
         { k_head_carry<<<1, 1024, 0, st>>>(tmax, tcnt, tiles, groups); note_launch(); }
@@ -1376,378 +2457,128 @@ int suffix_sort(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa
         rc = radix_sort_pairs<uint64_t, idx_t>(&ka, &va, &kb, &vb, n, 0, 32 + bits, rtmp, radix_tmp_bytes(n), st, true);
         if (rc) return rc;
     }
-    return finish(nullptr);
+    if (va != sa) { k_copy_vals<idx_t><<<grid_for(n, 256), 256, 0, st>>>(va, n, sa); note_launch(); }
+    return int(cudaGetLastError());
 }
 
-// ------------------------------------------------------------------------------ chunked sort
-//
-// For indexes too large for one pass (group ranks are 32-bit, and the working memory grows with
-// n): every suffix falls in a bucket by its first 6 bases (padded with A) and min(length, 6),
-// numbered in suffix order, so the suffix array is the concatenation of the buckets' own sorted
-// suffixes.  Consecutive buckets are gathered into chunks of at most `cap` suffixes; each chunk is
-// listed in text order (stable compaction), keyed, radix sorted and refined exactly as a whole
-// sort, and written at its offset.
-
-constexpr int kBucketBases = 6;
-constexpr int kBuckets = (1 << (2 * kBucketBases)) * 8;
-constexpr int kCkTile = 8192;
-
-__device__ __forceinline__ uint32_t bucket_of(const uint64_t* __restrict__ pk, size_t p, const DivL& dl) {
-    const int m = int(dl.L - uint32_t(p - div_l(p, dl) * dl.L));
-    const int w = m < kBucketBases ? m : kBucketBases;
-    const uint32_t pre = uint32_t(window(pk, p) >> (64 - 2 * kBucketBases)) & (~0u << (2 * (kBucketBases - w)));
-    return (pre << 3) | uint32_t(w);
-}
-
-// every position's bucket (kept for the chunk passes, which then read 2 bytes a position) and the
-// bucket histogram, counted in shared memory (kBuckets 32-bit counters, one CTA per SM) and added
-// to the global histogram once per CTA
+// A chunked sort's bucket histogram: 6-base buckets counted in shared memory (kBuckets 32-bit
+// counters, one CTA per SM) and added to the global histogram once per CTA.
 constexpr int kHistThreads = 1024;
 __global__ void __launch_bounds__(kHistThreads) k_bucket_hist(const uint64_t* __restrict__ pk, size_t n, DivL dl,
-                                                              uint16_t* __restrict__ bid,
                                                               unsigned long long* __restrict__ hist) {
     extern __shared__ unsigned s_hist[];
     for (int i = threadIdx.x; i < kBuckets; i += blockDim.x) s_hist[i] = 0;
     __syncthreads();
-    // eight consecutive positions a thread a step: their windows come from the same two words of
-    // the packed text (the first position is a multiple of 8), their read offsets from one
-    // multiply-high, their buckets go out in one 16-byte store
-    const size_t groups = (n + 7) / 8;
-    const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x; g < groups; g += stride) {
-        const size_t p0 = g * 8;
-        const uint64_t a = pk[p0 >> 5], b = pk[(p0 >> 5) + 1];
-        const int s0 = int(p0 & 31);
-        int off = int(uint32_t(p0 - div_l(p0, dl) * dl.L));
-        uint32_t v[8];
-        #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int sh = 2 * (s0 + j);
-            const uint64_t x = sh ? ((a << sh) | (b >> (64 - sh))) : a;
-            const int m = int(dl.L) - off;
-            const int w = m < kBucketBases ? m : kBucketBases;
-            const uint32_t pre = uint32_t(x >> (64 - 2 * kBucketBases)) & (~0u << (2 * (kBucketBases - w)));
-            v[j] = (pre << 3) | uint32_t(w);
-            if (p0 + size_t(j) < n) atomicAdd(&s_hist[v[j]], 1u);
-            off = off + 1 == int(dl.L) ? 0 : off + 1;
-        }
-        if (p0 + 8 <= n) {
-            *reinterpret_cast<uint4*>(bid + p0) =
-                make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
-        } else {
-            for (int j = 0; j < 8; ++j)
-                if (p0 + size_t(j) < n) bid[p0 + j] = uint16_t(v[j]);
-        }
-    }
+    const size_t stride = size_t(gridDim.x) * kHistThreads * 16;
+    for (size_t p0 = (size_t(blockIdx.x) * kHistThreads + threadIdx.x) * 16; p0 < n; p0 += stride)
+        for_positions(pk, p0, n, dl, [&](int, size_t, uint64_t x, int m, int, bool) { atomicAdd(&s_hist[bucket6(x, m)], 1u); });
     __syncthreads();
     for (int i = threadIdx.x; i < kBuckets; i += blockDim.x)
         if (s_hist[i]) atomicAdd(&hist[i], (unsigned long long)s_hist[i]);
 }
 
-// Chunk passes over tiles of kCkTile positions; warp w of a tile takes its positions
-// [w * kCkSpan, (w + 1) * kCkSpan), 32 consecutive ones a step.  A bucket's chunk comes from a
-// kBuckets-byte map (chunk numbers below kNoChunk).
-constexpr int kCkThreads = 256;
-constexpr int kCkWarps = kCkThreads / 32;
-constexpr int kCkSpan = kCkTile / kCkWarps;
-constexpr int kMaxChunks = 255;
-constexpr unsigned kNoChunk = 0xffu;
-
-// per tile and chunk: how many of the tile's positions fall in the chunk, into
-// tcnt[chunk * ntiles + tile]
-__global__ void __launch_bounds__(kCkThreads) k_chunk_tiles(const uint16_t* __restrict__ bid, size_t n,
-                                                            const uint8_t* __restrict__ cmap, int nchunks,
-                                                            size_t ntiles, unsigned long long* __restrict__ tcnt) {
-    __shared__ uint8_t s_map[kBuckets];
-    __shared__ unsigned s_cnt[kMaxChunks];
-    for (int i = threadIdx.x; i < kBuckets; i += blockDim.x) s_map[i] = cmap[i];
-    for (int c = threadIdx.x; c < nchunks; c += blockDim.x) s_cnt[c] = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    for (size_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const size_t t0 = tile * kCkTile;
-        #pragma unroll 4
-        for (int j = threadIdx.x; j < kCkTile; j += kCkThreads) {
-            const size_t p = t0 + size_t(j);
-            const unsigned c = p < n ? unsigned(s_map[bid[p]]) : kNoChunk;
-            const unsigned peers = __match_any_sync(0xffffffffu, c);
-            if (c != kNoChunk && lane == __ffs(peers) - 1) atomicAdd(&s_cnt[c], unsigned(__popc(peers)));
-        }
-        __syncthreads();
-        for (int c = threadIdx.x; c < nchunks; c += blockDim.x) {
-            tcnt[size_t(c) * ntiles + tile] = s_cnt[c];
-            s_cnt[c] = 0;
-        }
-        __syncthreads();
-    }
+static int bucket_hist(const uint64_t* pk, size_t n, const DivL& dl, unsigned long long* dev, std::vector<unsigned long long>& h,
+                       cudaStream_t st) {
+    const size_t hsm = size_t(kBuckets) * sizeof(unsigned);
+    cudaMemsetAsync(dev, 0, size_t(kBuckets) * 8, st);
+    cudaFuncSetAttribute(k_bucket_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, int(hsm));
+    { k_bucket_hist<<<unsigned(device_sms()), kHistThreads, hsm, st>>>(pk, n, dl, dev); note_launch(); }
+    h.resize(kBuckets);
+    cudaMemcpyAsync(h.data(), dev, size_t(kBuckets) * 8, cudaMemcpyDeviceToHost, st);
+    return int(cudaStreamSynchronize(st));
 }
 
-// Every position into its chunk's slice of `out`, in text order within the chunk.  toff is the
-// exclusive scan of tcnt in chunk-major order: the chunk's slice start plus the tile's place in
-// it.  A first walk over the tile counts each warp's positions per chunk, the warps' starts follow
-// from those counts, and a second walk (over the same bytes, from L1) writes, each warp keeping a
-// running offset per chunk.
-template <class V>
-__global__ void __launch_bounds__(kCkThreads) k_chunk_scatter(const uint16_t* __restrict__ bid, size_t n,
-                                                              const uint8_t* __restrict__ cmap, int nchunks,
-                                                              size_t ntiles,
-                                                              const unsigned long long* __restrict__ toff,
-                                                              V* __restrict__ out) {
-    __shared__ uint8_t s_map[kBuckets];
-    __shared__ unsigned s_run[kCkWarps][kMaxChunks];     // per warp and chunk: place within the tile
-    __shared__ unsigned long long s_base[kMaxChunks];    // per chunk: the tile's start in `out`
-    for (int i = threadIdx.x; i < kBuckets; i += blockDim.x) s_map[i] = cmap[i];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned below = (1u << lane) - 1u;
-    for (size_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const size_t w0 = tile * kCkTile + size_t(warp) * kCkSpan;
-        for (int c = lane; c < nchunks; c += 32) s_run[warp][c] = 0;
-        __syncthreads();
-        for (int k = 0; k < kCkSpan; k += 32) {
-            const size_t p = w0 + size_t(k + lane);
-            const unsigned c = p < n ? unsigned(s_map[bid[p]]) : kNoChunk;
-            const unsigned peers = __match_any_sync(0xffffffffu, c);
-            if (c != kNoChunk && lane == __ffs(peers) - 1) s_run[warp][c] += unsigned(__popc(peers));
-            __syncwarp();
-        }
-        __syncthreads();
-        for (int c = threadIdx.x; c < nchunks; c += blockDim.x) {
-            s_base[c] = toff[size_t(c) * ntiles + tile];
-            unsigned run = 0;
-            for (int w = 0; w < kCkWarps; ++w) {
-                const unsigned x = s_run[w][c];
-                s_run[w][c] = run;
-                run += x;
-            }
-        }
-        __syncthreads();
-        for (int k = 0; k < kCkSpan; k += 32) {
-            const size_t p = w0 + size_t(k + lane);
-            const unsigned c = p < n ? unsigned(s_map[bid[p]]) : kNoChunk;
-            const unsigned peers = __match_any_sync(0xffffffffu, c);
-            if (c != kNoChunk) out[s_base[c] + s_run[warp][c] + __popc(peers & below)] = V(p);
-            __syncwarp();
-            if (c != kNoChunk && lane == __ffs(peers) - 1) s_run[warp][c] += unsigned(__popc(peers));
-            __syncwarp();
-        }
-        __syncthreads();
+template <int W>
+static int sort_msd(const SortShape& sh, size_t nr, const MsdScratch& s, SortOut& o, size_t cap, cudaStream_t st) {
+    const MsdPlan& P = sh.plan;
+    const size_t n = P.n;
+    // k-mers entered as the buckets finish: of up to `head` bases; where they span buckets or short
+    // suffixes have them too, by minimum and maximum
+    if (o.kstart && o.kmer_k > P.head) o.kstart = o.kend = nullptr;
+    const bool spans = o.kmer_spans = o.kmer_k <= P.S || 2 * o.kmer_k < std::max(P.d1 + P.d2, sh.chunked ? 2 * kBucketBases : 0);
+    const size_t nk = size_t(1) << (2 * o.kmer_k);
+    if (o.kstart && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kstart, o.kend, 0, nk, 0); note_launch(); }
+    if (o.kstart && !spans) {
+        const cudaError_t e = kmer_table_clear(o.kmer_k, o.kstart, o.kend, st);
+        if (e != cudaSuccess) return int(e);
     }
-}
-
-// The counting pass for at most kFewChunks chunks (every index up to 8 G suffixes at the default
-// capacity), without __match_any_sync: thread tid of a tile takes its 32 consecutive positions
-// [tile * kCkTile + 32 tid, + 32) in four 16-byte loads, and keeps one counter per chunk in its own
-// column of a shared array (no atomics, no bank conflicts): 3.3 times faster than k_chunk_tiles.
-// (Scatters built the same way -- per-thread runs, or per-chunk ballots over 32 consecutive
-// positions -- measured slower than k_chunk_scatter's __match_any_sync groups.)
-constexpr int kFewChunks = 16;
-constexpr int kCkPer = kCkTile / kCkThreads;          // 32 positions a thread
-
-__device__ __forceinline__ void load_bids32(const uint16_t* __restrict__ bid, size_t p0, size_t n, uint32_t (&w)[16]) {
-    if (p0 + kCkPer <= n) {
-        #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 x = *reinterpret_cast<const uint4*>(bid + p0 + 8 * q);
-            w[4 * q] = x.x;
-            w[4 * q + 1] = x.y;
-            w[4 * q + 2] = x.z;
-            w[4 * q + 3] = x.w;
+    bool more = false;
+    std::vector<unsigned long long> h6;
+    if (!sh.chunked) {
+        const int rc = msd_pass<W>(P, nr, s, o, 0, n, 0, uint32_t(kBuckets), nullptr, cap, &more, st);
+        if (rc) return rc;
+        if (more) {       // a first-level bucket above the chunk size: is a 6-base one?
+            const int rh = bucket_hist(s.pk, n, P.dl, s.hist6, h6, st);
+            if (rh) return rh;
+            for (unsigned long long x : h6)
+                if (x > cap) return int(cudaErrorNotSupported);
         }
     } else {
-        #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const uint32_t lo = p0 + 2 * q < n ? bid[p0 + 2 * q] : 0xffffu;
-            const uint32_t hi = p0 + 2 * q + 1 < n ? bid[p0 + 2 * q + 1] : 0xffffu;
-            w[q] = lo | (hi << 16);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kCkThreads) k_chunk_tiles_few(const uint16_t* __restrict__ bid, size_t n,
-                                                                const uint8_t* __restrict__ cmap, int nchunks,
-                                                                size_t ntiles, unsigned long long* __restrict__ tcnt) {
-    __shared__ uint8_t s_map[kBuckets + 1];
-    __shared__ unsigned s_cnt[kFewChunks][kCkThreads];
-    for (int i = threadIdx.x; i < kBuckets; i += blockDim.x) s_map[i] = cmap[i];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (size_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        #pragma unroll
-        for (int c = 0; c < kFewChunks; ++c) s_cnt[c][tid] = 0;
-        __syncthreads();
-        const size_t p0 = tile * kCkTile + size_t(tid) * kCkPer;
-        if (p0 < n) {
-            uint32_t w[16];
-            load_bids32(bid, p0, n, w);
-            #pragma unroll
-            for (int j = 0; j < kCkPer; ++j) {
-                const uint32_t b = (w[j >> 1] >> (16 * (j & 1))) & 0xffffu;
-                if (b != 0xffffu) ++s_cnt[s_map[b]][tid];
-            }
-        }
-        __syncthreads();
-        for (int c = warp; c < nchunks; c += kCkWarps) {
-            unsigned sum = 0;
-            for (int i = lane; i < kCkThreads; i += 32) sum += s_cnt[c][i];
-            #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-            if (lane == 0) tcnt[size_t(c) * ntiles + tile] = sum;
-        }
-        __syncthreads();
-    }
-}
-
-// the chunk's keys, and its positions copied from their slice of the suffix array into the radix
-// sort's value buffer (which starts 16-byte aligned, as the sort's staged tiles want)
-template <class V>
-__global__ void k_init_keys_list(const uint64_t* __restrict__ pk, const V* __restrict__ list, size_t m, DivL dl,
-                                 uint32_t* __restrict__ key, V* __restrict__ val) {
-    const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
-        const V v = list[i];
-        const size_t p = size_t(v);
-        key[i] = make_key<uint32_t>(window(pk, p), int(dl.L - uint32_t(p - div_l(p, dl) * dl.L)));
-        val[i] = v;
-    }
-}
-
-// chunks a greedy packing of buckets into `cap` can make: every chunk but the last is over half
-// full or ends before a bucket of more than half a chunk, so at most 2 n / cap + 2
-static size_t chunk_bound(size_t n, size_t cap) {
-    return std::min<size_t>(size_t(kMaxChunks), 2 * ((n + cap - 1) / cap) + 2);
-}
-
-static size_t chunk_parts(size_t n, size_t cap, size_t (&b)[11]) {
-    const size_t ntiles = (n + kCkTile - 1) / kCkTile;
-    b[0] = cap * sizeof(uint64_t);                    // ka (32-bit head keys; 64-bit for big groups)
-    b[1] = cap * sizeof(uint64_t);                    // kb (also the group lists)
-    b[2] = cap * sizeof(idx_t);                       // va
-    b[3] = cap * sizeof(idx_t);                       // vb (with rank: big-group columns)
-    b[4] = cap * sizeof(uint32_t);                    // rank
-    b[5] = (n / 32 + 4) * sizeof(uint64_t);           // packed text
-    b[6] = radix_tmp_bytes(cap);
-    b[7] = (chunk_bound(n, cap) * ntiles + 1) * sizeof(unsigned long long);   // tile counts / offsets
-    b[8] = (size_t(kBuckets) + 8) * sizeof(unsigned long long) + size_t(kBuckets);   // histogram, counters, map
-    b[9] = n;                                         // BWT symbols of the refined rows
-    b[10] = n * sizeof(uint16_t);                     // every position's 6-base bucket
-    size_t t = 0;
-    for (size_t x : b) t += al(x);
-    return t + 1024;
-}
-
-size_t suffix_sort_chunked_tmp_bytes(size_t n, size_t cap) {
-    size_t b[11];
-    return chunk_parts(n, cap, b);
-}
-
-int suffix_sort_chunked(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa, size_t cap, void* tmp,
-                        size_t tmp_bytes, cudaStream_t st, const uint8_t** bwt_out, uint64_t* pk_out,
-                        idx_t* isa_out, idx_t isa_m, idx_t* kstart, idx_t* kend, int kmer_k) {
-    if (bwt_out) *bwt_out = nullptr;
-    const size_t n = size_t(num_reads) * size_t(L);
-    if (n == 0) return 0;
-    if (cap < 2 || cap >= (size_t(1) << 31)) return int(cudaErrorInvalidValue);
-    size_t b[11];
-    if (tmp_bytes < chunk_parts(n, cap, b)) return int(cudaErrorInvalidValue);
-    char* q = static_cast<char*>(tmp);
-    char* part[11];
-    for (int i = 0; i < 11; ++i) {
-        part[i] = q;
-        q += al(b[i]);
-    }
-    uint64_t* ka0 = reinterpret_cast<uint64_t*>(part[0]);
-    uint64_t* kb0 = reinterpret_cast<uint64_t*>(part[1]);
-    idx_t* va0 = reinterpret_cast<idx_t*>(part[2]);
-    idx_t* vb0 = reinterpret_cast<idx_t*>(part[3]);
-    uint64_t* pk = pk_out ? pk_out : reinterpret_cast<uint64_t*>(part[5]);
-    void* rtmp = part[6];
-    uint8_t* bwt = bwt_out ? reinterpret_cast<uint8_t*>(part[9]) : nullptr;
-    if (bwt) cudaMemsetAsync(bwt, 0xff, n, st);
-    unsigned long long* tcnt = reinterpret_cast<unsigned long long*>(part[7]);
-    unsigned long long* hist = reinterpret_cast<unsigned long long*>(part[8]);
-    unsigned long long* counters = hist + kBuckets;
-    uint16_t* bid = reinterpret_cast<uint16_t*>(part[10]);
-    uint8_t* cmap = reinterpret_cast<uint8_t*>(counters + 8);
-    const DivL dl = make_divl(uint32_t(L));
-    const size_t nwords = n / 32 + 4;
-    const size_t ntiles = (n + kCkTile - 1) / kCkTile;
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    { k_pack_text<<<grid_for(nwords, 256), 256, 0, st>>>(reads, n, idx_t(L), dir, nwords, pk); note_launch(); }
-    cudaMemsetAsync(hist, 0, size_t(kBuckets) * sizeof(unsigned long long), st);
-    const size_t hsm = size_t(kBuckets) * sizeof(unsigned);
-    cudaFuncSetAttribute(k_bucket_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, int(hsm));
-    { k_bucket_hist<<<unsigned(sms), kHistThreads, hsm, st>>>(pk, n, dl, bid, hist); note_launch(); }
-    std::vector<unsigned long long> h(kBuckets);
-    cudaMemcpyAsync(h.data(), hist, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return int(e);
-    // chunks: runs of consecutive buckets that fit the capacity, each a slice of the suffix array
-    std::vector<uint8_t> map(kBuckets, uint8_t(kNoChunk));
-    struct Chunk {
-        size_t offset, m;
-    };
-    std::vector<Chunk> chunks;
-    {
-        size_t offset = 0;
-        uint32_t lo = 0;
-        while (lo < uint32_t(kBuckets)) {
+        const int rh = bucket_hist(s.pk, n, P.dl, s.hist6, h6, st);
+        if (rh) return rh;
+        for (unsigned long long x : h6)
+            if (x > cap) return int(cudaErrorNotSupported);              // one bucket larger than a chunk
+        // chunks: runs of consecutive buckets that fit the capacity, each a slice of the suffix array
+        size_t row = 0;
+        for (uint32_t lo = 0; lo < uint32_t(kBuckets);) {
             uint32_t hi = lo;
             size_t m = 0;
-            while (hi < uint32_t(kBuckets) && m + h[hi] <= cap) m += h[hi++];
-            if (hi == lo) return int(cudaErrorNotSupported);          // one bucket larger than a chunk
+            while (hi < uint32_t(kBuckets) && m + h6[hi] <= cap) m += h6[hi++];
             if (m) {
-                if (chunks.size() >= chunk_bound(n, cap)) return int(cudaErrorNotSupported);
-                for (uint32_t b = lo; b < hi; ++b) map[b] = uint8_t(chunks.size());
-                chunks.push_back({offset, m});
+                const int rc = msd_pass<W>(P, nr, s, o, row, m, lo, hi, h6.data(), 0, &more, st);
+                if (rc) return rc;
             }
-            offset += m;
+            row += m;
             lo = hi;
         }
     }
-    const int nchunks = int(chunks.size());
-    cudaMemcpyAsync(cmap, map.data(), map.size(), cudaMemcpyHostToDevice, st);
-    // every position into its chunk's slice of the suffix array, in text order: tile counts per
-    // chunk, their scan in chunk-major order (the slices' starts included), the scatter
-    const unsigned cgrid = unsigned(std::min<size_t>(ntiles, size_t(sms) * 8));
-    if (nchunks <= kFewChunks) {
-        k_chunk_tiles_few<<<cgrid, kCkThreads, 0, st>>>(bid, n, cmap, nchunks, ntiles, tcnt);
-    } else {
-        k_chunk_tiles<<<cgrid, kCkThreads, 0, st>>>(bid, n, cmap, nchunks, ntiles, tcnt);
-    }
-    note_launch();
-    { k_scan_small<<<1, 1024, 0, st>>>(tcnt, size_t(nchunks) * ntiles); note_launch(); }
-    { k_chunk_scatter<idx_t><<<cgrid, kCkThreads, 0, st>>>(bid, n, cmap, nchunks, ntiles, tcnt, sa); note_launch(); }
-    for (const Chunk& ck : chunks) {
-        const size_t offset = ck.offset, m = ck.m;
-        {
-            uint32_t* ka = reinterpret_cast<uint32_t*>(ka0);
-            uint32_t* kb = reinterpret_cast<uint32_t*>(kb0);
-            { k_init_keys_list<idx_t><<<grid_for(m, 256), 256, 0, st>>>(pk, sa + offset, m, dl, ka, va0); note_launch(); }
-            idx_t* va = va0;
-            idx_t* vb = vb0;
-            int rc = radix_sort_pairs<uint32_t, idx_t>(&ka, &va, &kb, &vb, m, 0, 32, rtmp, radix_tmp_bytes(m), st, false);
-            if (rc) return rc;
-            if (size_t(L) > size_t(kHead)) {
-                // scratch: the free value buffer, and rank behind it when that is the second buffer
-                uint64_t* cols = reinterpret_cast<uint64_t*>(vb);
-                const size_t cols_cap = (vb == vb0 ? al(b[3]) + b[4] : al(b[2])) / sizeof(uint64_t);
-                rc = refine_groups(ka, va, m, idx_t(L), pk, reinterpret_cast<uint64_t*>(kb), cols, cols_cap, counters,
-                                   rtmp, radix_tmp_bytes(m), st, bwt, isa_out, isa_m, offset);
-                if (rc > 0) return rc;
-                if (rc < 0) return int(cudaErrorNotSupported);      // would need prefix doubling
-            }
-            { k_copy_vals<idx_t><<<grid_for(m, 256), 256, 0, st>>>(va, m, sa + offset); note_launch(); }
-            // the chunk's keys are still sorted and aligned with its rows (the refinement only
-            // reorders rows of equal keys): its k-mers' row ranges
-            if (kstart && kmer_k >= 6 && kmer_k <= kSortKeyBases) {
-                const cudaError_t ek = kmer_table_from_keys(ka, m, offset, kmer_k, kstart, kend, st);
-                if (ek != cudaSuccess) return int(ek);
-            }
-        }
-    }
-    if (bwt_out) *bwt_out = bwt;
+    if (o.kstart && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kstart, o.kend, 0, nk, 1); note_launch(); }
+    o.kmer_done = o.kstart != nullptr;
     return int(cudaGetLastError());
+}
+
+int suffix_sort(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa, size_t cap, void* tmp,
+                size_t tmp_bytes, cudaStream_t st, const uint8_t** bwt_out, uint64_t* pk_out, idx_t* kstart, idx_t* kend,
+                int kmer_k, bool* kmer_done) {
+    if (bwt_out) *bwt_out = nullptr;
+    if (kmer_done) *kmer_done = false;
+    const size_t n = size_t(num_reads) * size_t(L);
+    if (n == 0) return 0;
+    if (cap >= n) cap = 0;
+    if (cap == 1) return int(cudaErrorInvalidValue);
+    const SortShape sh = sort_shape(n, num_reads, L, cap);
+    if (tmp_bytes < sh.bytes) return int(cudaErrorInvalidValue);
+    if (cap && L > kChunkMaxLen) return int(cudaErrorNotSupported);
+    if (sh.doubling && n >= (size_t(1) << 31)) return int(cudaErrorNotSupported);      // 32-bit ranks
+    MsdScratch s{};
+    if (!sh.doubling) s = msd_layout(tmp, sh.plan, sh.m, num_reads);
+    uint64_t* pk = pk_out;
+    if (!pk) {
+        if (!sh.doubling) pk = s.pk;
+        else pk = reinterpret_cast<uint64_t*>(static_cast<char*>(tmp) + 2 * al(n * sizeof(uint64_t)) + al(n * sizeof(idx_t)) +
+                                              al(n * sizeof(uint32_t)));
+    }
+    const size_t nwords = n / 32 + 4;
+    { k_pack_text<<<grid_for(nwords, 256), 256, 0, st>>>(reads, n, idx_t(L), dir, nwords, pk); note_launch(); }
+    if (sh.doubling) return sort_doubling(n, L, sa, pk, tmp, st);
+    s.pk = pk;
+    SortOut o{sa, bwt_out ? s.bwt : nullptr, kstart, kend, kmer_k, false, false};
+    int rc = 0;
+    switch (plan_words(sh.plan)) {
+        case 1: rc = sort_msd<1>(sh, num_reads, s, o, cap, st); break;
+        case 2: rc = sort_msd<2>(sh, num_reads, s, o, cap, st); break;
+        case 3: rc = sort_msd<3>(sh, num_reads, s, o, cap, st); break;
+        case 4: rc = sort_msd<4>(sh, num_reads, s, o, cap, st); break;
+        case 5: rc = sort_msd<5>(sh, num_reads, s, o, cap, st); break;
+        case 6: rc = sort_msd<6>(sh, num_reads, s, o, cap, st); break;
+        case 7: rc = sort_msd<7>(sh, num_reads, s, o, cap, st); break;
+        case 8: rc = sort_msd<8>(sh, num_reads, s, o, cap, st); break;
+        default: rc = sort_msd<9>(sh, num_reads, s, o, cap, st); break;
+    }
+    if (rc) return rc;
+    if (bwt_out) *bwt_out = s.bwt;
+    if (kmer_done) *kmer_done = o.kmer_done;
+    return 0;
 }
 
 }  // namespace pq

@@ -1,7 +1,7 @@
 // pq_sort_static.cu — a suffix sort that allocates no device memory.
 //
-// pq_sort() allocates its working memory (keys, values, ranks, packed text, BWT symbols, radix
-// histograms: about 25 bytes per suffix) with cudaMalloc on first use.  Some callers cannot do that: code
+// pq_sort() allocates its working memory (elements of both partition passes, packed text, bucket
+// tables: about 18 bytes per suffix) with cudaMalloc on first use.  Some callers cannot do that: code
 // that runs inside a host application which owns every byte of device memory through its own
 // pool and forbids direct cudaMalloc (an assembler or read-correction tool that embeds this sort
 // for many small per-bucket sorts), and code on latency-critical paths where cudaMalloc's
@@ -30,12 +30,12 @@ namespace {
 constexpr size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kMax = PQ_STATIC_SORT_MAX_SUFFIXES;
 
-// Upper bound of pq::suffix_sort_tmp_bytes(kMax): key double buffer, one value buffer (the other
-// is the caller's suffix array), 32-bit ranks, packed text, radix histograms of up to 608 CTAs
-// plus 8 digit histograms, per-tile head data, one BWT-symbol byte per suffix.
+// Upper bound of pq::suffix_sort_tmp_bytes of up to kMax suffixes: two 64-bit arrays, one idx_t
+// array and one 32-bit array (prefix doubling, the larger layout), packed text, radix histograms of
+// up to 608 CTAs, per-tile head data, one BWT-symbol byte per suffix.
 constexpr size_t kScratchBytes =
     2 * al256(kMax * sizeof(uint64_t)) + al256(kMax * sizeof(idx_t)) + al256(kMax * sizeof(uint32_t)) +
-    al256((kMax / 32 + 4) * sizeof(uint64_t)) + al256((256 * 608 + 8 * 256 + 64) * sizeof(unsigned long long)) +
+    al256((kMax / 32 + 4) * sizeof(uint64_t)) + al256((256 * 608 + 9 * 256 + 64) * sizeof(unsigned long long)) +
     al256(3 * (kMax / 2048 + 2) * sizeof(unsigned long long)) + al256(kMax) + 1024;
 
 __device__ __align__(256) unsigned char g_sort_scratch[kScratchBytes];
@@ -81,7 +81,7 @@ extern "C" int pq_suffix_sort_static(const uint8_t* reads_dev, pq_idx num_reads,
     if (n > kMax) return PQ_ERR_CAPACITY;
     if (n == 0) return PQ_OK;
     if (!reads_dev || !sa_dev) return PQ_ERR_ARG;
-    const size_t need = pq::suffix_sort_tmp_bytes(size_t(n));
+    const size_t need = pq::suffix_sort_tmp_bytes(size_t(n), size_t(num_reads), read_len);
     if (need > kScratchBytes) return PQ_ERR_INTERNAL;
     void* scratch = nullptr;
     int rc = scratch_address(&scratch);
@@ -95,7 +95,7 @@ extern "C" int pq_suffix_sort_static(const uint8_t* reads_dev, pq_idx num_reads,
         cudaStreamSynchronize(st) != cudaSuccess)
         return PQ_ERR_CUDA;
     if (bad) return PQ_ERR_ARG;
-    int e = pq::suffix_sort(reads_dev, idx_t(num_reads), read_len, dir, reinterpret_cast<idx_t*>(sa_dev), scratch,
+    int e = pq::suffix_sort(reads_dev, idx_t(num_reads), read_len, dir, reinterpret_cast<idx_t*>(sa_dev), 0, scratch,
                             kScratchBytes, st);
     if (e != 0) return PQ_ERR_CUDA;
     return cudaStreamSynchronize(st) == cudaSuccess && cudaGetLastError() == cudaSuccess ? PQ_OK : PQ_ERR_CUDA;
