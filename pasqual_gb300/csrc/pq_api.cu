@@ -80,9 +80,10 @@ struct pq_ctx {
     bool have_reads = false;
 
     // per direction
-    DevBuf sa[2], blk[2], sb[2], ri[2], kstart[2], kend[2], pk[2];
+    DevBuf sa[2], blk[2], sb[2], ri[2], kt[2], kx[2], pk[2];
     bool sa_ok[2] = {false, false}, fm_ok[2] = {false, false};
     int fm_k[2] = {0, 0};
+    int kx_bases[2] = {0, 0};  // bases per row kx holds beyond the table's k (0: none)
     DevBuf sort_tmp, counts;
     int kmer_from_sort[2] = {0, 0};                         // k of the k-mer table the last sort entered
     const uint8_t* bwt_hint[2] = {nullptr, nullptr};       // the last sort's BWT symbols, inside sort_tmp
@@ -138,6 +139,12 @@ static inline size_t n_supers(const pq_ctx* c) {
 }
 
 static constexpr int kLxDefaultSteps = 400;
+
+// Rows a k-mer has by chance (n / 4^k) from which on an index build keeps every row's next bases
+// (2 bytes a row): the search then narrows a k-mer's rows in a few sectors of those instead of
+// comparing text (7 rows by chance: 2.1 against 2.9 ms on 1.2 M reads).  With fewer rows the texts
+// saved cost no more than the extra sectors.
+static constexpr size_t kKxRows = 2;
 
 static LearnedView lx_view(const pq_ctx* c, int d) {
     LearnedView v;
@@ -238,8 +245,8 @@ void pq_destroy(pq_ctx* ctx) {
         ctx->blk[d].release();
         ctx->sb[d].release();
         ctx->ri[d].release();
-        ctx->kstart[d].release();
-        ctx->kend[d].release();
+        ctx->kt[d].release();
+        ctx->kx[d].release();
         ctx->pk[d].release();
         ctx->lx_bnd[d].release();
         ctx->lx_base[d].release();
@@ -356,16 +363,18 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
     ctx->bwt_hint[0] = ctx->bwt_hint[1] = nullptr;           // the scratch is about to be reused
     const int kk = ctx->seed_k;
     ctx->kmer_from_sort[dir] = 0;
+    ctx->kx_bases[dir] = 0;
+    const bool want_kx = side_outputs && (n >> (2 * kk)) >= kKxRows;
     if (side_outputs) {
-        const size_t nk = size_t(1) << (2 * kk);
-        CK(ctx->kstart[dir].ensure(nk * sizeof(idx_t)));
-        CK(ctx->kend[dir].ensure(nk * sizeof(idx_t)));
+        CK(ctx->kt[dir].ensure((size_t(2) << (2 * kk)) * sizeof(idx_t)));
+        // the rows' bases past the k-mer where a k-mer has more than a few rows by chance
+        if (want_kx) CK(ctx->kx[dir].ensure(n * sizeof(uint16_t) + 16));
     }
     bool kmer_done = false;
     const int rc = pq::suffix_sort(ctx->reads.as<uint8_t>(), ctx->num_reads, ctx->L, dir, ctx->sa[dir].as<idx_t>(), cap,
                                    ctx->sort_tmp.p, tmp_bytes, ctx->st, side_outputs ? &ctx->bwt_hint[dir] : nullptr,
-                                   ctx->pk[dir].as<uint64_t>(), side_outputs ? ctx->kstart[dir].as<idx_t>() : nullptr,
-                                   side_outputs ? ctx->kend[dir].as<idx_t>() : nullptr, kk, &kmer_done);
+                                   ctx->pk[dir].as<uint64_t>(), side_outputs ? ctx->kt[dir].as<idx_t>() : nullptr, kk, &kmer_done,
+                                   want_kx ? ctx->kx[dir].as<uint16_t>() : nullptr, &ctx->kx_bases[dir]);
     ctx->pk_ok[dir] = rc == 0;
     if (rc == int(cudaErrorNotSupported))
         return fail(ctx, PQ_ERR_CAPACITY, "suffix sort: a 6-base bucket holds more suffixes than a sort chunk");
@@ -495,9 +504,7 @@ int pq_build_fm(pq_ctx* ctx, int dir) {
     CK(ctx->sb[dir].ensure(n_supers(ctx) * 4 * sizeof(idx_t) + 64));
     CK(ctx->ri[dir].ensure(size_t(ctx->num_reads) * sizeof(idx_t) + 64));
     const int k = ctx->seed_k;
-    const size_t nk = size_t(1) << (2 * k);
-    CK(ctx->kstart[dir].ensure(nk * sizeof(idx_t)));
-    CK(ctx->kend[dir].ensure(nk * sizeof(idx_t)));
+    CK(ctx->kt[dir].ensure((size_t(2) << (2 * k)) * sizeof(idx_t)));
     CK(ctx->pk[dir].ensure((n / 32 + 4) * sizeof(uint64_t)));
     CK(cudaEventRecord(ctx->ev0, ctx->st));
     if (!ctx->pk_ok[dir])
@@ -506,10 +513,11 @@ int pq_build_fm(pq_ctx* ctx, int dir) {
     CK(pq::build_occ(ctx->sa[dir].as<idx_t>(), ctx->reads.as<uint8_t>(), ctx->num_reads, idx_t(ctx->L), dir,
                      ctx->blk[dir].as<OccBlock>(), ctx->sb[dir].as<idx_t>(), ctx->ri[dir].as<idx_t>(), ctx->st,
                      ctx->pk[dir].as<uint64_t>(), ctx->bwt_hint[dir]));
-    if (ctx->kmer_from_sort[dir] != k)
-        CK(pq::build_kmer_table(ctx->sa[dir].as<idx_t>(), ctx->num_reads, idx_t(ctx->L), k,
-                                ctx->kstart[dir].as<idx_t>(), ctx->kend[dir].as<idx_t>(), ctx->st,
-                                ctx->pk[dir].as<uint64_t>()));
+    if (ctx->kmer_from_sort[dir] != k) {
+        ctx->kx_bases[dir] = 0;
+        CK(pq::build_kmer_table(ctx->sa[dir].as<idx_t>(), ctx->num_reads, idx_t(ctx->L), k, ctx->kt[dir].as<idx_t>(),
+                                ctx->st, ctx->pk[dir].as<uint64_t>()));
+    }
     ctx->kmer_from_sort[dir] = 0;
     CK(cudaEventRecord(ctx->ev1, ctx->st));
     CK(cudaEventSynchronize(ctx->ev1));
@@ -580,7 +588,7 @@ int pq_get_seeds(pq_ctx* ctx, int dir, pq_idx* start, pq_idx* size, uint16_t* de
     CK(s.ensure(nr * sizeof(idx_t)));
     CK(z.ensure(nr * sizeof(idx_t)));
     CK(pq::read_seeds(ctx->reads.as<uint8_t>(), ctx->num_reads, ctx->L, dir, ctx->fm_k[dir],
-                      ctx->kstart[dir].as<idx_t>(), ctx->kend[dir].as<idx_t>(), s.as<idx_t>(), z.as<idx_t>(), ctx->st));
+                      ctx->kt[dir].as<idx_t>(), s.as<idx_t>(), z.as<idx_t>(), ctx->st));
     if (start) CK(cudaMemcpyAsync(start, s.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
     if (size) CK(cudaMemcpyAsync(size, z.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
@@ -643,11 +651,11 @@ static int search_prepare(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
         f.blk = ctx->blk[d].as<OccBlock>();
         f.sb = ctx->sb[d].as<idx_t>();
         f.reads_index = ctx->ri[d].as<idx_t>();
-        f.kstart = ctx->kstart[d].as<idx_t>();
-        f.kend = ctx->kend[d].as<idx_t>();
+        f.kt = ctx->kt[d].as<idx_t>();
+        f.kx_bases = ctx->kx_bases[d];
+        f.kx = f.kx_bases ? ctx->kx[d].as<uint16_t>() : nullptr;
         f.sa = ctx->sa[d].as<idx_t>();
         f.pk = ctx->pk[d].as<uint64_t>();
-        f.isa = nullptr;          // no inverse suffix array: reads the lean tier hands over walk
         const idx_t* fix = d == 0 ? ctx->sfx : ctx->pfx;
         f.Cf[0] = ctx->C[0];
         for (int c = 1; c <= 4; ++c) f.Cf[c] = ctx->C[c] + fix[c - 1];

@@ -59,12 +59,13 @@ struct FmView {
     const OccBlock* blk;      // n/64 + 1 blocks
     const idx_t* sb;          // 4 per superblock
     const idx_t* reads_index; // read id of the k-th `$` row
-    const idx_t* kstart;      // k-mer seed table: first row of each k-mer (or nullptr)
-    const idx_t* kend;        // last row (kend < kstart when the k-mer is absent)
+    const idx_t* kt;          // k-mer table: (first row, last row) of every k-mer (last < first when
+                              // it is absent), or nullptr
+    const uint16_t* kx;       // per row, the kx_bases <= 7 bases after its first k (2 bits each; of rows
+                              // of at least k bases), or nullptr; whole 16-byte units
+    int kx_bases;
     const idx_t* sa;          // suffix array (for seeds found by binary search), or nullptr
     const uint64_t* pk;       // the text, 32 bases per word, first base in the top bits
-    const idx_t* isa;         // row of the suffix at read offset o (1 <= o <= L - t) of read r at
-                              // isa[r * (L - t) + o - 1], or nullptr
     LearnedView lx;           // learned index of 16-base keys (lx.segs = 0 when absent)
     idx_t Cf[5];              // Cf[0] = C[0]; Cf[c] = C[c] + fix[c]  (LF-mapping base)
 };

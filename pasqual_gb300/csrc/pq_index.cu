@@ -282,7 +282,7 @@ __device__ __forceinline__ uint32_t kmer_at(const idx_t* __restrict__ sa, const 
 }
 
 __global__ void k_kmer_bounds_pk(const idx_t* __restrict__ sa, const uint64_t* __restrict__ pk, size_t n, idx_t L,
-                                 int k, idx_t* __restrict__ kstart, idx_t* __restrict__ kend) {
+                                 int k, idx_t* __restrict__ kt) {
     const int lane = threadIdx.x & 31;
     const size_t warp = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const size_t nwarps = (size_t(gridDim.x) * blockDim.x) >> 5;
@@ -294,15 +294,18 @@ __global__ void k_kmer_bounds_pk(const idx_t* __restrict__ sa, const uint64_t* _
         if (lane == 0) prev = r > 0 && r < n ? kmer_at(sa, pk, r - 1, L, k) : 0xfffffffeu;
         if (lane == 31) next = r + 1 < n ? kmer_at(sa, pk, r + 1, L, k) : 0xfffffffeu;
         if (r < n && c != 0xffffffffu) {
-            if (r == 0 || prev != c) kstart[c] = idx_t(r);
-            if (r + 1 == n || next != c) kend[c] = idx_t(r);
+            if (r == 0 || prev != c) kt[2 * size_t(c)] = idx_t(r);
+            if (r + 1 == n || next != c) kt[2 * size_t(c) + 1] = idx_t(r);
         }
     }
 }
 
-__global__ void k_fill_idx(idx_t* __restrict__ a, size_t m, idx_t v) {
+// every k-mer absent: (1, 0), 16 bytes a store
+__global__ void k_kmer_clear(idx_t* __restrict__ kt, size_t nk) {
+    constexpr int kPer = 16 / (2 * int(sizeof(idx_t)));         // k-mers a store
     const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) a[i] = v;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nk / kPer; i += stride)
+        reinterpret_cast<uint4*>(kt)[i] = kPer == 1 ? make_uint4(1, 0, 0, 0) : make_uint4(1, 0, 1, 0);
 }
 
 // Reference-layout export (src/index.h:26-30): bitmap[c] word b bit j+1 <=> BWT[64b+j] == c for
@@ -338,8 +341,7 @@ __global__ void k_export_ref(const OccBlock* __restrict__ blk, const idx_t* __re
 // Per-read seeds (index_t.interval_start/end/depth, src/index.h:36-41): forward = the read's
 // last k bases, backward = its first k bases reversed; both exact SA intervals from the table.
 __global__ void k_read_seeds(const uint8_t* __restrict__ reads, idx_t nr, int L, int dir, int k,
-                             const idx_t* __restrict__ kstart, const idx_t* __restrict__ kend,
-                             idx_t* __restrict__ start, idx_t* __restrict__ size) {
+                             const idx_t* __restrict__ kt, idx_t* __restrict__ start, idx_t* __restrict__ size) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     for (size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x; r < nr; r += stride) {
         const uint8_t* s = reads + r * size_t(L);
@@ -348,8 +350,8 @@ __global__ void k_read_seeds(const uint8_t* __restrict__ reads, idx_t nr, int L,
             int c = dir == 0 ? s[L - k + j] : s[k - 1 - j];
             code = (code << 2) | uint32_t(c - 1);
         }
-        start[r] = kstart[code];
-        size[r] = kend[code] - kstart[code] + 1;
+        start[r] = kt[2 * size_t(code)];
+        size[r] = kt[2 * size_t(code) + 1] - kt[2 * size_t(code)] + 1;
     }
 }
 
@@ -425,26 +427,25 @@ cudaError_t read_counts(const uint8_t* reads, idx_t num_reads, idx_t L, unsigned
     return cudaGetLastError();
 }
 
-cudaError_t kmer_table_clear(int k, idx_t* kstart, idx_t* kend, cudaStream_t st) {
+cudaError_t kmer_table_clear(int k, idx_t* kt, cudaStream_t st) {
     const size_t nk = size_t(1) << (2 * k);
-    { k_fill_idx<<<grid_for(nk, 256), 256, 0, st>>>(kstart, nk, idx_t(1)); note_launch(); }
-    { k_fill_idx<<<grid_for(nk, 256), 256, 0, st>>>(kend, nk, idx_t(0)); note_launch(); }
+    { k_kmer_clear<<<grid_for(nk / 2, 256), 256, 0, st>>>(kt, nk); note_launch(); }
     return cudaGetLastError();
 }
 
-cudaError_t build_kmer_table(const idx_t* sa, idx_t num_reads, idx_t L, int k, idx_t* kstart, idx_t* kend,
-                             cudaStream_t st, const uint64_t* pk) {
+cudaError_t build_kmer_table(const idx_t* sa, idx_t num_reads, idx_t L, int k, idx_t* kt, cudaStream_t st,
+                             const uint64_t* pk) {
     const size_t n = size_t(num_reads) * L;
-    cudaError_t e = kmer_table_clear(k, kstart, kend, st);
+    cudaError_t e = kmer_table_clear(k, kt, st);
     if (e != cudaSuccess) return e;
-    if (n) { k_kmer_bounds_pk<<<grid_for(n, 256), 256, 0, st>>>(sa, pk, n, L, k, kstart, kend); note_launch(); }
+    if (n) { k_kmer_bounds_pk<<<grid_for(n, 256), 256, 0, st>>>(sa, pk, n, L, k, kt); note_launch(); }
     return cudaGetLastError();
 }
 
-cudaError_t read_seeds(const uint8_t* reads, idx_t num_reads, int L, int dir, int k, const idx_t* kstart,
-                       const idx_t* kend, idx_t* start, idx_t* size, cudaStream_t st) {
+cudaError_t read_seeds(const uint8_t* reads, idx_t num_reads, int L, int dir, int k, const idx_t* kt, idx_t* start,
+                       idx_t* size, cudaStream_t st) {
     if (num_reads)
-        { k_read_seeds<<<grid_for(num_reads, 256), 256, 0, st>>>(reads, num_reads, L, dir, k, kstart, kend, start, size); note_launch(); }
+        { k_read_seeds<<<grid_for(num_reads, 256), 256, 0, st>>>(reads, num_reads, L, dir, k, kt, start, size); note_launch(); }
     return cudaGetLastError();
 }
 

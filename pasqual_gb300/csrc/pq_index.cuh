@@ -17,10 +17,10 @@ cudaError_t kernel_copy(void* dst, const void* src, size_t n, cudaStream_t st);
 cudaError_t read_counts(const uint8_t* reads, idx_t num_reads, idx_t L, unsigned long long* out13,
                         cudaStream_t st);
 // k-mer table of direction dir from the suffix array and the packed text pk (one streaming pass)
-cudaError_t build_kmer_table(const idx_t* sa, idx_t num_reads, idx_t L, int k, idx_t* kstart, idx_t* kend,
-                             cudaStream_t st, const uint64_t* pk);
+cudaError_t build_kmer_table(const idx_t* sa, idx_t num_reads, idx_t L, int k, idx_t* kt, cudaStream_t st,
+                             const uint64_t* pk);
 // the table with every k-mer absent
-cudaError_t kmer_table_clear(int k, idx_t* kstart, idx_t* kend, cudaStream_t st);
+cudaError_t kmer_table_clear(int k, idx_t* kt, cudaStream_t st);
 // The per-read seed intervals the reference's sort records (index_t.interval_start/end/depth,
 // src/sufsort.c:178-209, 322-334) from a finished suffix array and the packed text of its
 // direction (pq_seeds.cu).  seed_init writes the depth-1 seeds build_idx starts from; sort_seeds

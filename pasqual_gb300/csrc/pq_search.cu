@@ -205,6 +205,17 @@ __device__ __forceinline__ int pattern_at(const ReadView& rd, int L, int kind, i
     }
 }
 
+// first and last row of a k-mer (last < first when it is absent)
+__device__ __forceinline__ void kmer_rows(const FmView& f, uint32_t code, idx_t& first, idx_t& last) {
+#ifdef PQ_IDX64
+    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(f.kt) + code);
+#else
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(f.kt) + code);
+#endif
+    first = v.x;
+    last = v.y;
+}
+
 // exact SA interval of pattern pat(hi) pat(hi-1) ... pat(lo) (text order) from the k-mer table
 __device__ __forceinline__ void kmer_seed(const FmView& f, const ReadView& rd, int L, int kind, int first,
                                           int last, int step, idx_t& l, idx_t& u, Tally& probes) {
@@ -213,9 +224,8 @@ __device__ __forceinline__ void kmer_seed(const FmView& f, const ReadView& rd, i
         code = (code << 2) | uint32_t(pattern_at(rd, L, kind, j) - 1);
         if (j == last) break;
     }
-    l = __ldg(f.kstart + code);
-    u = __ldg(f.kend + code);
-    probes.add(1, 2);
+    kmer_rows(f, code, l, u);
+    probes.add(1, 1);
 }
 
 struct ReadResult {
@@ -265,21 +275,16 @@ __device__ __forceinline__ int meta_type(uint32_t m) { return int(m >> 16); }
 // time (the reference's search_2/search_3 loop, src/string_graph.c:226-237), the rows of I_t are
 // read once: one suffix-array entry and one text comparison each, all independent loads.
 //
-// The reference stores, for each depth with candidates, the other index's interval of the
-// reversed pattern restricted to its `$` rows: the rows whose suffix is exactly rev(P_d) followed
-// by end-of-read.  Those are precisely the candidates' suffixes of length d in the other index
-// (text position r' * L + L - d), consecutive and ordered by position, so the interval is
-// [ISA(r'min * L + L - d), + count - 1] with r'min the smallest candidate.
-//
 // Chains are alive at depth d whenever a candidate exists there (a strict kind also holds the
-// read's own suffix, a second row), so the depths reported are the reference's.  I_t itself is
-// found by binary search over the suffix array inside the k-mer table interval of P_t's first k
-// bases, the two chains of a side searched together.  A row compares as its suffix string with
-// end-of-read lowest, the order of the backward search.
+// read's own suffix, a second row), so the depths reported are the reference's.  I_t itself is not
+// needed row for row: any run of rows that holds it serves, since every row is checked against the
+// whole pattern P_d.  That run is the rows of P_t's first k bases (k-mer table) that go on with its
+// next kx_bases bases (FmView::kx); a run of more than kScanDirect rows, or the window of the
+// learned index, is narrowed to I_t by binary search over the suffix array.
 
 constexpr int kScanWords = 2;       // bases of P_t searched by bisection: the first 64 at most
 constexpr int kScanMax = 256;       // larger depth-t intervals walk instead
-constexpr int kScanMaskWords = 4;   // L - t up to 256
+constexpr int kScanDirect = 48;     // rows checked without narrowing them to I_t first
 
 // 64 bases of packed text starting at base p (first base in the top bits)
 __device__ __forceinline__ uint64_t text_window(const uint64_t* __restrict__ pk, size_t p) {
@@ -371,26 +376,53 @@ __device__ __forceinline__ void sa_bounds2(const FmView* f0, const FmView* f1, c
     end[0] = b0[0]; end[1] = b0[1];
 }
 
-// `o` bases of the walked index's text at ra equal those of the pattern source at rs.  The
-// pattern P_d (d = t + o) of a strict kind is the read's own text in the walked index at
-// self * L + L - d; of FF and BB it is the complement of the other index's text there.
-// `sec` counts the sectors loaded from the walked text (the pattern source is the read's own text,
-// counted once by pattern_words).
-__device__ __forceinline__ bool prefix_matches(const uint64_t* __restrict__ pka, size_t ra,
-                                               const uint64_t* __restrict__ pks, size_t rs, int o, bool cmpl,
-                                               uint32_t& sec) {
-    bool ok = true;
-    int c = 0;
-    for (; c < o && ok; c += 32) {
-        const int m = o - c < 32 ? o - c : 32;
-        const uint64_t x = text_window(pka, ra + c);
-        uint64_t y = text_window(pks, rs + c);
-        if (cmpl) y = ~y;
-        ok = ((x ^ y) & top_mask(m)) == 0;
+// 32-byte sectors of packed text that hold the bases [p, p + m), m > 0 (the text starts on a sector)
+__device__ __forceinline__ uint32_t base_sectors(size_t p, int m) { return uint32_t(((p + size_t(m) - 1) >> 7) - (p >> 7)) + 1u; }
+
+// 32 bases from base offset s (0..31) of the words a, b (first base highest) as two 32-bit halves
+__device__ __forceinline__ void shift_bases(uint64_t a, uint64_t b, int s, uint32_t& hi, uint32_t& lo) {
+    const uint32_t r0 = uint32_t(a >> 32), r1 = uint32_t(a), r2 = uint32_t(b >> 32), r3 = uint32_t(b);
+    const bool odd = s >= 16;
+    const uint32_t h0 = odd ? r1 : r0, h1 = odd ? r2 : r1, h2 = odd ? r3 : r2;
+    hi = __funnelshift_l(h1, h0, 2 * s);
+    lo = __funnelshift_l(h2, h1, 2 * s);
+}
+// the bits of half h (0: the higher) of 32 bases that lie within the first `left` of them
+__device__ __forceinline__ uint32_t half_mask(int left, int h) {
+    uint32_t past;
+    asm("shr.u32 %0, %1, %2;" : "=r"(past) : "r"(0xffffffffu), "r"(uint32_t(max(2 * left - 32 * h, 0))));   // 0 from 32 on
+    return ~past;
+}
+
+// The d bases of the walked index's text at ra equal those of the pattern source at rs (their
+// complement for cmpl), 32 at a time.  The pattern P_d of a strict kind is the read's own text in the
+// walked index at self * L + L - d; of FF and BB it is the complement of the other index's text
+// there.  Most rows compared do match, so nothing waits for the first difference: the warp runs to
+// its longest d, each word loaded two steps ahead (no word past the one after the last base's: the
+// text is padded by more).
+__device__ __forceinline__ bool text_matches(const uint64_t* __restrict__ pka, size_t ra,
+                                             const uint64_t* __restrict__ pks, size_t rs, int d, bool cmpl, unsigned lanes) {
+    const uint64_t *wa = pka + (ra >> 5), *wb = pks + (rs >> 5);
+    const int sa = int(ra & 31), sb = int(rs & 31), words = (d + 31) >> 5;
+    const int most = int(__reduce_max_sync(lanes, unsigned(words)));
+    const uint32_t flip = cmpl ? ~0u : 0u;
+    uint64_t a0 = __ldg(wa), b0 = __ldg(wb), a1 = __ldg(wa + 1), b1 = __ldg(wb + 1);
+    uint32_t x = 0;
+    #pragma unroll 1
+    for (int i = 0; i < most; ++i) {
+        const int next = i + 2 < words ? i + 2 : words;
+        const uint64_t a2 = __ldg(wa + next), b2 = __ldg(wb + next);
+        const int left = d - 32 * i;
+        uint32_t ah, al, bh, bl;
+        shift_bases(a0, a1, sa, ah, al);
+        shift_bases(b0, b1, sb, bh, bl);
+        x |= ((ah ^ bh ^ flip) & half_mask(left, 0)) | ((al ^ bl ^ flip) & half_mask(left, 1));
+        a0 = a1;
+        b0 = b1;
+        a1 = a2;
+        b1 = b2;
     }
-    // windows at ra, ra + 32, ..., ra + c - 32: words (ra >> 5) .. ((ra + c - 32) >> 5) + 1
-    if (c > 0) sec += sectors_of(pka + (ra >> 5), 8 * ((((ra + c - 32) >> 5) - (ra >> 5)) + 2));
-    return ok;
+    return !x;
 }
 
 // Slots of the level-0 candidates of the two chains of one side: q * M + i.
@@ -406,11 +438,6 @@ struct SlotsFast {     // fast tier: the warp's global scratch
         uu[p] = b;
         meta[p] = m;
     }
-    __device__ __forceinline__ void get(int q, int i, idx_t& a, idx_t& b) const {
-        const size_t p = base + size_t(q) * M + i;
-        a = ll[p];
-        b = uu[p];
-    }
 };
 struct SlotsStack {    // wide tier: the slot's candidate stack
     Cand* stk;
@@ -422,130 +449,7 @@ struct SlotsStack {    // wide tier: the slot's candidate stack
         c.len = uint16_t(meta_len(m));
         c.type = uint8_t(meta_type(m));
     }
-    __device__ __forceinline__ void get(int q, int i, idx_t& a, idx_t& b) const {
-        a = stk[q * M + i].ll;
-        b = stk[q * M + i].uu;
-    }
 };
-
-// Candidates of both chains by interval scan; false (nothing stored) when a depth-t interval
-// holds more than kScanMax rows, and the caller walks instead.
-template <class Slots>
-__device__ __forceinline__ bool scan_pair(const SearchArgs& A, const FmView* fm, idx_t self, int k0, int k1,
-                                          int (&n)[2], int32_t& olp, Tally& probes, const Slots& slots) {
-    if (!fm[0].isa || !fm[1].isa) return false;      // group intervals need the inverse SA: walk
-    const int L = A.L, t = A.t, k = A.seed_k, M = L - t;
-    const int tb = t < 32 * kScanWords ? t : 32 * kScanWords;    // bases bisected; the rest checked per row
-    uint64_t P0[kScanWords], P1[kScanWords];
-    pattern_words(fm, L, t, k0, self, P0, probes);
-    pattern_words(fm, L, t, k1, self, P1, probes);
-    const FmView* f0 = fm + walked_index(k0);
-    const FmView* f1 = fm + walked_index(k1);
-    idx_t lo[2], hi[2], first[2], end[2];
-    if (A.sa_seed == 2) {
-        // learned window of P_t's first 16 bases: one inference per chain
-        #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const LearnedView& v = (q ? f1 : f0)->lx;
-            const uint32_t K = uint32_t((q ? P1 : P0)[0] >> 32);
-            const int sg = lx_segment(v, K);
-            const long long pr = lx_predict(v, sg, K);
-            const long long b0 = (long long)__ldg(v.base + sg), b1 = (long long)__ldg(v.base + sg + 1);
-            const long long a = pr - (long long)__ldg(v.err + 2 * sg), b = pr + (long long)__ldg(v.err + 2 * sg + 1);
-            lo[q] = idx_t(a > b0 ? a : b0);
-            hi[q] = idx_t(b < b1 ? b : b1);
-            if (hi[q] < lo[q]) hi[q] = lo[q];
-        }
-    } else {
-        const uint32_t c0 = uint32_t(P0[0] >> (64 - 2 * k)), c1 = uint32_t(P1[0] >> (64 - 2 * k));
-        lo[0] = __ldg(f0->kstart + c0);
-        hi[0] = __ldg(f0->kend + c0) + 1;
-        lo[1] = __ldg(f1->kstart + c1);
-        hi[1] = __ldg(f1->kend + c1) + 1;
-        probes.add(2, 4);
-        if (hi[0] < lo[0]) hi[0] = lo[0];
-        if (hi[1] < lo[1]) hi[1] = lo[1];
-    }
-    sa_bounds2(f0, f1, A.dl, P0, P1, tb, lo, hi, first, end, probes);
-    if (A.sa_seed == 2) {
-        // The window holds the answer for every key present in the index; for any other key it
-        // is checked: the rows just outside the window must not start with P_t.
-        const idx_t n_rows = A.num_reads * idx_t(L);
-        bool ok = true;
-        #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const FmView& fa = *(q ? f1 : f0);
-            const uint64_t (&P)[kScanWords] = q ? P1 : P0;
-            if (first[q] == lo[q] && lo[q] > 0) {
-                const idx_t p = __ldg(fa.sa + lo[q] - 1);
-                ok = ok && cmp_row(fa.pk, p, suffix_len(p, A.dl), P, tb) < 0;
-                probes.add(2, 1 + cmp_sectors(fa.pk, p));
-            }
-            if (end[q] == hi[q] && hi[q] < n_rows) {
-                const idx_t p = __ldg(fa.sa + hi[q]);
-                ok = ok && cmp_row(fa.pk, p, suffix_len(p, A.dl), P, tb) > 0;
-                probes.add(2, 1 + cmp_sectors(fa.pk, p));
-            }
-        }
-        if (!ok) {
-            atomicAdd(A.lx_misses, 1ull);
-            return false;           // plain backward search
-        }
-    }
-    if (end[0] - first[0] > idx_t(kScanMax) || end[1] - first[1] > idx_t(kScanMax)) return false;
-    #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int kind = q ? k1 : k0;
-        const FmView& fa = *(q ? f1 : f0);
-        const FmView& fb = fm[1 - walked_index(kind)];
-        const bool cmpl = !(kind == PQ_FB || kind == PQ_BF);
-        const uint64_t* pks = cmpl ? fb.pk : fa.pk;
-        const size_t src = size_t(self) * L + size_t(L - t);     // P_t in the pattern source
-        uint64_t mk0 = 0, mk1 = 0, mk2 = 0, mk3 = 0;              // depths with candidates (o < 256)
-        for (idx_t row = first[q]; row < end[q]; ++row) {
-            const idx_t p = __ldg(fa.sa + row);
-            const idx_t rp = read_of(p, A.dl);
-            const int o = int(p - rp * idx_t(L));
-            probes.add(2, 1);
-            if (o >= M || !prefix_matches(fa.pk, size_t(rp) * L, pks, src - o, o, cmpl, probes.sectors)) continue;
-            if (t > tb && !prefix_matches(fa.pk, size_t(p) + tb, pks, src + tb, t - tb, cmpl, probes.sectors))
-                continue;
-            const uint64_t bit = uint64_t(1) << (o & 63);
-            const int hw = o >> 6;
-            const uint64_t cur = hw == 0 ? mk0 : hw == 1 ? mk1 : hw == 2 ? mk2 : mk3;
-            const bool seen = (cur & bit) != 0;
-            mk0 |= hw == 0 ? bit : 0;
-            mk1 |= hw == 1 ? bit : 0;
-            mk2 |= hw == 2 ? bit : 0;
-            mk3 |= hw == 3 ? bit : 0;
-            if (!seen) {
-                slots.set(q, o, rp, 1, 0);
-            } else {
-                idx_t r0, cnt;
-                slots.get(q, o, r0, cnt);
-                slots.set(q, o, rp < r0 ? rp : r0, cnt + 1, 0);
-            }
-        }
-        int i = 0;
-        #pragma unroll
-        for (int h = 0; h < kScanMaskWords; ++h) {
-            uint64_t m = h == 0 ? mk0 : h == 1 ? mk1 : h == 2 ? mk2 : mk3;
-            while (m) {
-                const int o = 64 * h + __ffsll((long long)m) - 1;
-                m &= m - 1;
-                idx_t r0, cnt;
-                slots.get(q, o, r0, cnt);
-                const int d = t + o;
-                const idx_t l0 = __ldg(fb.isa + (size_t(r0) * M + size_t(L - d - 1)));
-                probes += 1;
-                slots.set(q, i++, l0, l0 + cnt - 1, pack_meta(d, kind));
-                olp = int32_t(uint32_t(olp) + uint32_t(cnt));
-            }
-        }
-        n[q] = i;
-    }
-    return true;
-}
 
 // find_intervals for one side: kinds k0 then k1 (B-F and B-B, or F-B and F-F), searched in
 // lockstep so that each thread keeps two independent chains of loads in flight.
@@ -555,18 +459,13 @@ __device__ __forceinline__ bool scan_pair(const SearchArgs& A, const FmView* fm,
 // only then continues with synchronised search_2 steps.  Here both intervals start from exact
 // k-mer seeds (one per index) and every step is a synchronised step, so the other interval is
 // known at every depth and the rebuild disappears; SA intervals are unique per string, so the
-// intervals at depth t -- and everything after -- are the reference's.  With A.sa_seed the
-// candidates come from the interval scan above instead, unless a depth-t interval is too large.
-// The i-th stored candidate of kind k0 (q = 0) or k1 (q = 1) goes to slot (q, i); n[q] counts them.
-// `need_read()` makes rd valid (the walk reads the read's bases; the scan reads the packed text).
-template <class Slots, class NeedRead>
-__device__ __forceinline__ void chain_pair(const SearchArgs& A, const FmView* fm, const ReadView& rd, idx_t self,
-                                           int k0, int k1, int (&n)[2], int32_t& olp, Tally& probes,
-                                           const Slots& slots, NeedRead need_read) {
+// intervals at depth t -- and everything after -- are the reference's.  The i-th stored candidate
+// of kind k0 (q = 0) or k1 (q = 1) goes to slot (q, i); n[q] counts them.
+template <class Slots>
+__device__ __forceinline__ void chain_pair(const SearchArgs& A, const FmView* fm, const ReadView& rd, int k0, int k1,
+                                           int (&n)[2], int32_t& olp, Tally& probes, const Slots& slots) {
     const int L = A.L, t = A.t, k = A.seed_k;
     n[0] = n[1] = 0;
-    if (A.sa_seed && scan_pair(A, fm, self, k0, k1, n, olp, probes, slots)) return;
-    need_read();
     idx_t l[2], u[2], ll[2], uu[2];
     bool alive[2];
     #pragma unroll
@@ -626,7 +525,7 @@ __device__ __forceinline__ int side_candidates(const SearchArgs& A, const FmView
     const int M = A.L - A.t;
     if (2 * M > cap) return OVF_STACK;
     int n[2];
-    chain_pair(A, fm, rd, self, k0, k1, n, olp, probes, SlotsStack{stk, M}, [] {});
+    chain_pair(A, fm, rd, k0, k1, n, olp, probes, SlotsStack{stk, M});
     for (int i = 0; i < n[1]; ++i) stk[n[0] + i] = stk[M + i];
     n_out = n[0] + n[1];
     return OVF_NONE;
@@ -972,10 +871,21 @@ __device__ __forceinline__ int owner_of(const int* pref, int e) {
 // continuation, then read id: the DFS order.  No FM-index step is taken.
 
 constexpr int kRedMax = 64;          // candidates of one (read, side) reduced this way
+// candidate i of lane l of a warp sits at slot 32 i + l of the warp's arrays, so that the lanes of a
+// warp, each reducing its own read in step with the others, load consecutive words
+constexpr int kRedStride = 32;
 constexpr int kLamWords = 8;         // continuations up to 256 bases (L - t <= 256)
 
 // continuation words the kernels are built for: 2 (L - t <= 64) or kLamWords
 __host__ __device__ constexpr int lam_words(int M) { return M <= 64 ? 2 : kLamWords; }
+
+// word w of the continuation of candidate r' at overlap d (32 w < L - d)
+__device__ __forceinline__ uint64_t continuation_word(const SearchArgs& A, int type, idx_t rp, int d, int w) {
+    const bool fwd = cand_index(type) == 1;
+    const int left = A.L - d - 32 * w;
+    const uint64_t x = text_window(A.fm[fwd ? 0 : 1].pk, size_t(rp) * A.L + size_t(d) + 32 * size_t(w));
+    return (fwd ? x : ~x) & top_mask(left < 32 ? left : 32);
+}
 
 // continuation of candidate r' at overlap d: L - d bases (at most 32 W) in ceil((L - d) / 32)
 // words, first base in the top bits, zero past the end; word w at out[w * plane]
@@ -983,45 +893,35 @@ __host__ __device__ constexpr int lam_words(int M) { return M <= 64 ? 2 : kLamWo
 template <int W>
 __device__ __forceinline__ uint32_t continuation(const SearchArgs& A, int type, idx_t rp, int d, uint64_t* out,
                                                  size_t plane) {
-    const int L = A.L, len = L - d;
-    const bool fwd = cand_index(type) == 1;
-    const uint64_t* pk = A.fm[fwd ? 0 : 1].pk;
-    const size_t pos = size_t(rp) * L + size_t(d);
-    const uint64_t flip = fwd ? 0 : ~uint64_t(0);
-    int nw = 0;
+    const int len = A.L - d;
     #pragma unroll
     for (int w = 0; w < W; ++w) {
-        const int left = len - 32 * w;
-        if (left <= 0) break;
-        out[w * plane] = (text_window(pk, pos + 32 * w) ^ flip) & top_mask(left < 32 ? left : 32);
-        nw = w + 1;
+        if (32 * w >= len) break;
+        out[w * plane] = continuation_word(A, type, rp, d, w);
     }
-    return nw ? sectors_of(pk + (pos >> 5), 8 * ((((pos + 32 * (nw - 1)) >> 5) - (pos >> 5)) + 2)) : 0;
+    return len > 0 ? base_sectors(size_t(rp) * A.L + size_t(d), len) : 0;
 }
 
-// the first n bases (1 <= n <= 32 W) of continuations a and b agree
+// The candidates of one (read, side) as the reduction sees them: read id, (overlap, kind) and
+// continuation words of candidate i, in the warp's global scratch.  (The first 8 or 16 of a read in
+// shared memory instead: 12.0 and 8.9 ms against 7.2 on 5.4 M reads, for want of L1 and of warps.)
+struct Cands {
+    const WarpScratch& S;
+    size_t red;
+    __device__ __forceinline__ size_t at(int i) const { return red + size_t(i) * kRedStride; }
+    __device__ __forceinline__ idx_t id(int i) const { return S.r_id[at(i)]; }
+    __device__ __forceinline__ uint32_t meta(int i) const { return S.r_meta[at(i)]; }
+    __device__ __forceinline__ uint64_t word(int i, int w) const { return S.r_k[w * S.r_plane + at(i)]; }
+};
+// order of candidates i and j, whose continuations (la and lb bases) are equal or not prefixes of
+// one another: their first differing base, else equal
 template <int W>
-__device__ __forceinline__ bool same_prefix(const uint64_t* a, const uint64_t* b, int n, size_t plane) {
-    #pragma unroll
-    for (int w = 0; w < W; ++w) {
-        const int rest = n - 32 * w;
-        if (rest <= 0) return true;
-        const uint64_t x = a[w * plane] ^ b[w * plane];
-        if (rest < 32) return (x & top_mask(rest)) == 0;
-        if (x) return false;
-    }
-    return true;
-}
-
-// order of two continuations of la and lb bases that are equal or not prefixes of one another:
-// their first differing base, else equal
-template <int W>
-__device__ __forceinline__ int cmp_cont(const uint64_t* a, int la, const uint64_t* b, int lb, size_t plane) {
+__device__ __forceinline__ int cmp_cont(const Cands& C, int i, int la, int j, int lb) {
     const int n = la < lb ? la : lb;
     #pragma unroll
     for (int w = 0; w < W; ++w) {
         if (32 * w >= n) break;
-        const uint64_t x = a[w * plane], y = b[w * plane];
+        const uint64_t x = C.word(i, w), y = C.word(j, w);
         if (x != y) return x < y ? -1 : 1;
     }
     return la == lb ? 0 : (la < lb ? -1 : 1);
@@ -1029,7 +929,7 @@ __device__ __forceinline__ int cmp_cont(const uint64_t* a, int la, const uint64_
 
 template <int W>
 __device__ __forceinline__ int reduce_gathered(int L, const WarpScratch& S, idx_t self, int side, size_t red, int m,
-                                               size_t eb, int& ne, int& count);
+                                               size_t eb, int estride, int& ne, int& count);
 
 // Edges of one side of one read from its level-0 candidate groups (na of the first kind, then
 // n0 - na of the second) in the candidate scratch at `cand`; per-lane scratch at `red`.
@@ -1048,69 +948,99 @@ __device__ __forceinline__ int reduce_sorted(const SearchArgs& A, const WarpScra
         for (idx_t row = ll; row <= uu; ++row) {
             const idx_t p = __ldg(fb.sa + row);
             const idx_t rp = read_of(p, A.dl);
-            const uint32_t sec = continuation<W>(A, type, rp, d, S.r_k + red + m, S.r_plane);
-            S.r_id[red + m] = rp;
-            S.r_meta[red + m] = mt;
+            const size_t q = red + size_t(m) * kRedStride;
+            const uint32_t sec = continuation<W>(A, type, rp, d, S.r_k + q, S.r_plane);
+            S.r_id[q] = rp;
+            S.r_meta[q] = mt;
             probes.add(2, 1 + sec);
             ++m;
         }
     }
-    return reduce_gathered<W>(L, S, self, side, red, m, eb, ne, count);
+    return reduce_gathered<W>(L, S, self, side, red, m, eb, 1, ne, count);
 }
 
-// The reduction of reduce_sorted over m gathered candidates: continuations in S.r_k (word w of
-// candidate i at r_k[w * r_plane + red + i]), read ids in S.r_id and (overlap, kind) in S.r_meta,
-// from red on.  Emitted edges go to the edge scratch at eb + ne, in DFS order.
+// The reduction of reduce_sorted over m <= 64 gathered candidates; `red` is the lane's column of the
+// warp's scratch (kRedStride).  Emitted edges go to the edge scratch at eb + estride ne, in DFS order.
+//
+// In rounds: the shortest continuation left, s, has no proper prefix among the others, so its class
+// -- the candidates left whose continuation starts with s -- is emitted where it equals s and covered
+// where it goes on, and trans is the class's size: a candidate of an earlier class starts with a
+// prefix of s only if s itself did.  Most candidates of a read continue one genome locus, so one or
+// two rounds, each a test a candidate, take the place of a test for every pair (the reduction of 5.4
+// M reads at 20x took 3.5 ms by pairs).
 template <int W>
 __device__ __forceinline__ int reduce_gathered(int L, const WarpScratch& S, idx_t self, int side, size_t red, int m,
-                                               size_t eb, int& ne, int& count) {
+                                               size_t eb, int estride, int& ne, int& count) {
+    const Cands C{S, red};
     const int first_kind = side ? PQ_FB : PQ_BF;
+    auto at = [&](int i) { return red + size_t(i) * kRedStride; };
+    auto bit = [](int i) { return 1ull << i; };
     int nemit = 0;
-    for (int c = 0; c < m; ++c) {
-        const uint64_t* kc = S.r_k + red + c;
-        const uint32_t mc = S.r_meta[red + c];
-        const int lc = L - meta_len(mc);
-        bool covered = false, first_same = false;
-        int trans = 0;
-        for (int e = 0; e < m; ++e) {
-            const uint32_t me = S.r_meta[red + e];
-            const int le = L - meta_len(me);
-            if (!same_prefix<W>(kc, S.r_k + red + e, le < lc ? le : lc, S.r_plane)) continue;
-            if (le < lc) {
-                covered = true;
-                break;
+    unsigned long long left = m >= 64 ? ~0ull : bit(m) - 1;
+    while (left) {
+        int ls = 1 << 30, is = 0;
+        for (unsigned long long x = left; x; x &= x - 1) {
+            const int c = __ffsll((long long)x) - 1;
+            const int lc = L - meta_len(C.meta(c));
+            if (lc < ls) {
+                ls = lc;
+                is = c;
             }
-            ++trans;
-            if (le == lc && meta_type(me) == first_kind) first_same = true;
         }
-        if (covered || S.r_id[red + c] == self || (meta_type(mc) != first_kind && first_same)) continue;
-        S.r_emit[red + nemit++] = uint32_t(c) | (uint32_t(trans) << 16);
+        uint64_t ks[W];
+        #pragma unroll
+        for (int w = 0; w < W; ++w) ks[w] = 32 * w < ls ? C.word(is, w) : 0;
+        unsigned long long cls = 0, equal = 0;
+        bool first_same = false;
+        for (unsigned long long x = left; x; x &= x - 1) {
+            const int c = __ffsll((long long)x) - 1;
+            const uint32_t mc = C.meta(c);
+            bool same = true;
+            #pragma unroll
+            for (int w = 0; w < W; ++w) {
+                const int rest = ls - 32 * w;
+                if (rest > 0 && same) same = ((C.word(c, w) ^ ks[w]) & top_mask(rest < 32 ? rest : 32)) == 0;
+            }
+            if (!same) continue;
+            cls |= bit(c);
+            if (L - meta_len(mc) == ls) {
+                equal |= bit(c);
+                first_same = first_same || meta_type(mc) == first_kind;
+            }
+        }
+        left &= ~cls;
+        const uint32_t trans = uint32_t(__popcll(cls));
+        for (; equal; equal &= equal - 1) {
+            const int c = __ffsll((long long)equal) - 1;
+            if (C.id(c) == self || (first_same && meta_type(C.meta(c)) != first_kind)) continue;
+            S.r_emit[at(nemit++)] = uint32_t(c) | (trans << 16);
+        }
     }
     // DFS order: continuation, then read id (insertion sort; a handful of edges)
     for (int i = 1; i < nemit; ++i) {
-        const uint32_t x = S.r_emit[red + i];
+        const uint32_t x = S.r_emit[at(i)];
         const int cx = int(x & 0xffff);
-        const uint64_t* kx = S.r_k + red + cx;
-        const int lx = L - meta_len(S.r_meta[red + cx]);
-        const idx_t xi = S.r_id[red + cx];
+        const int lx = L - meta_len(C.meta(cx));
+        const idx_t xi = C.id(cx);
         int j = i - 1;
         while (j >= 0) {
-            const int cy = int(S.r_emit[red + j] & 0xffff);
-            const int o = cmp_cont<W>(S.r_k + red + cy, L - meta_len(S.r_meta[red + cy]), kx, lx, S.r_plane);
-            const bool greater = o != 0 ? o > 0 : S.r_id[red + cy] > xi;
+            const int cy = int(S.r_emit[at(j)] & 0xffff);
+            const int o = cmp_cont<W>(C, cy, L - meta_len(C.meta(cy)), cx, lx);
+            const bool greater = o != 0 ? o > 0 : C.id(cy) > xi;
             if (!greater) break;
-            S.r_emit[red + j + 1] = S.r_emit[red + j];
+            S.r_emit[at(j + 1)] = S.r_emit[at(j)];
             --j;
         }
-        S.r_emit[red + j + 1] = x;
+        S.r_emit[at(j + 1)] = x;
     }
     for (int i = 0; i < nemit; ++i) {
-        const uint32_t x = S.r_emit[red + i];
+        const uint32_t x = S.r_emit[at(i)];
         const int c = int(x & 0xffff);
         if (ne >= S.ebcap) return OVF_EDGES;
-        S.e_dest[eb + ne] = S.r_id[red + c];
-        S.e_trans[eb + ne] = int32_t(x >> 16);
-        S.e_meta[eb + ne] = S.r_meta[red + c];
+        const size_t q = eb + size_t(ne) * estride;
+        S.e_dest[q] = C.id(c);
+        S.e_trans[q] = int32_t(x >> 16);
+        S.e_meta[q] = C.meta(c);
         ++ne;
     }
     count = nemit;
@@ -1127,108 +1057,109 @@ __device__ __forceinline__ int reduce_gathered(int L, const WarpScratch& S, idx_
 // depth-indexed candidate slots, the inverse-SA load of every candidate depth and the suffix-array
 // reload of every candidate that the group form (scan_pair + reduce_sorted) needs.
 
-// Candidates of both kinds of one side, gathered for reduce_gathered at red + m: false when the
-// scan does not apply to this read (a depth-t interval of more than kScanMax rows, or a learned
-// window that missed) or the side has more than kRedMax candidates -- the fast tier then redoes
-// the read.
-template <int W>
-__device__ __forceinline__ bool scan_planes(const SearchArgs& A, const FmView* fm, idx_t self, int k0, int k1,
-                                            const WarpScratch& S, size_t red, int& m, int32_t& olp, Tally& probes) {
-    const int L = A.L, t = A.t, k = A.seed_k, M = L - t;
-    const int m0 = m;
-    const int tb = t < 32 * kScanWords ? t : 32 * kScanWords;
-    uint64_t P0[kScanWords], P1[kScanWords];
-    pattern_words(fm, L, t, k0, self, P0, probes);
-    pattern_words(fm, L, t, k1, self, P1, probes);
-    const FmView* f0 = fm + walked_index(k0);
-    const FmView* f1 = fm + walked_index(k1);
-    idx_t lo[2], hi[2], first[2], end[2];
-    if (A.sa_seed == 2) {
-        #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const LearnedView& v = (q ? f1 : f0)->lx;
-            const uint32_t K = uint32_t((q ? P1 : P0)[0] >> 32);
-            const int sg = lx_segment(v, K);
-            const long long pr = lx_predict(v, sg, K);
-            const long long b0 = (long long)__ldg(v.base + sg), b1 = (long long)__ldg(v.base + sg + 1);
-            const long long a = pr - (long long)__ldg(v.err + 2 * sg), b = pr + (long long)__ldg(v.err + 2 * sg + 1);
-            lo[q] = idx_t(a > b0 ? a : b0);
-            hi[q] = idx_t(b < b1 ? b : b1);
-            if (hi[q] < lo[q]) hi[q] = lo[q];
-        }
-    } else {
-        const uint32_t c0 = uint32_t(P0[0] >> (64 - 2 * k)), c1 = uint32_t(P1[0] >> (64 - 2 * k));
-        lo[0] = __ldg(f0->kstart + c0);
-        hi[0] = __ldg(f0->kend + c0) + 1;
-        lo[1] = __ldg(f1->kstart + c1);
-        hi[1] = __ldg(f1->kend + c1) + 1;
-        probes.add(2, 4);
-        if (hi[0] < lo[0]) hi[0] = lo[0];
-        if (hi[1] < lo[1]) hi[1] = lo[1];
-    }
-    sa_bounds2(f0, f1, A.dl, P0, P1, tb, lo, hi, first, end, probes);
-    if (A.sa_seed == 2) {
-        const idx_t n_rows = A.num_reads * idx_t(L);
-        bool ok = true;
-        #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const FmView& fa = *(q ? f1 : f0);
-            const uint64_t (&P)[kScanWords] = q ? P1 : P0;
-            if (first[q] == lo[q] && lo[q] > 0) {
-                const idx_t p = __ldg(fa.sa + lo[q] - 1);
-                ok = ok && cmp_row(fa.pk, p, suffix_len(p, A.dl), P, tb) < 0;
-                probes.add(2, 1 + cmp_sectors(fa.pk, p));
-            }
-            if (end[q] == hi[q] && hi[q] < n_rows) {
-                const idx_t p = __ldg(fa.sa + hi[q]);
-                ok = ok && cmp_row(fa.pk, p, suffix_len(p, A.dl), P, tb) > 0;
-                probes.add(2, 1 + cmp_sectors(fa.pk, p));
-            }
-        }
-        if (!ok) {
-            atomicAdd(A.lx_misses, 1ull);
-            return false;
-        }
-    }
-    if (end[0] - first[0] > idx_t(kScanMax) || end[1] - first[1] > idx_t(kScanMax)) return false;
+// Rows [first, end) of each chain's index to check for the patterns P0 and P1 of one side's chains,
+// all rows that start with their first t bases among them; false when the scan does not apply to this
+// read (a depth-t interval of more than kScanMax rows, or a learned window that missed): the fast
+// tier then redoes it.
+
+// The window of the learned index, narrowed to I_t (seed mode 2).
+__device__ __forceinline__ bool learned_rows(const SearchArgs& A, const FmView* f0, const FmView* f1,
+                                             const uint64_t (&P0)[kScanWords], const uint64_t (&P1)[kScanWords],
+                                             idx_t (&first)[2], idx_t (&end)[2], Tally& probes) {
+    const int tb = A.t < 32 * kScanWords ? A.t : 32 * kScanWords;
+    const FmView* fq[2] = {f0, f1};
+    idx_t lo[2], hi[2];
     #pragma unroll
     for (int q = 0; q < 2; ++q) {
-        const int kind = q ? k1 : k0;
-        const FmView& fa = *(q ? f1 : f0);
-        const FmView& fb = fm[1 - walked_index(kind)];
-        const bool cmpl = !(kind == PQ_FB || kind == PQ_BF);
-        const uint64_t* pks = cmpl ? fb.pk : fa.pk;
-        const uint64_t flip = walked_index(kind) ? ~uint64_t(0) : 0;
-        const size_t src = size_t(self) * L + size_t(L - t);
-        for (idx_t row = first[q]; row < end[q]; ++row) {
-            const idx_t p = __ldg(fa.sa + row);
-            const idx_t rp = read_of(p, A.dl);
-            const int o = int(p - rp * idx_t(L));
-            probes.add(2, 1);
-            if (o >= M || !prefix_matches(fa.pk, size_t(rp) * L, pks, src - o, o, cmpl, probes.sectors)) continue;
-            if (t > tb && !prefix_matches(fa.pk, size_t(p) + tb, pks, src + tb, t - tb, cmpl, probes.sectors))
-                continue;
-            if (m - m0 >= kRedMax) return false;
-            // the continuation: M - o bases of the walked text after the pattern
-            const int len = M - o;
-            const size_t pos = size_t(p) + size_t(t);
-            int nw = 0;
-            #pragma unroll
-            for (int w = 0; w < W; ++w) {
-                const int left = len - 32 * w;
-                if (left <= 0) break;
-                S.r_k[w * S.r_plane + red + m] =
-                    (text_window(fa.pk, pos + 32 * w) ^ flip) & top_mask(left < 32 ? left : 32);
-                nw = w + 1;
-            }
-            if (nw) probes.add(0, sectors_of(fa.pk + (pos >> 5), 8 * ((((pos + 32 * (nw - 1)) >> 5) - (pos >> 5)) + 2)));
-            S.r_id[red + m] = rp;
-            S.r_meta[red + m] = pack_meta(t + o, kind);
-            ++m;
-            olp = int32_t(uint32_t(olp) + 1u);
+        const LearnedView& v = fq[q]->lx;
+        const uint32_t K = uint32_t((q ? P1 : P0)[0] >> 32);
+        const int sg = lx_segment(v, K);
+        const long long pr = lx_predict(v, sg, K);
+        const long long b0 = (long long)__ldg(v.base + sg), b1 = (long long)__ldg(v.base + sg + 1);
+        const long long a = pr - (long long)__ldg(v.err + 2 * sg), b = pr + (long long)__ldg(v.err + 2 * sg + 1);
+        lo[q] = idx_t(a > b0 ? a : b0);
+        hi[q] = idx_t(b < b1 ? b : b1);
+        if (hi[q] < lo[q]) hi[q] = lo[q];
+    }
+    sa_bounds2(f0, f1, A.dl, P0, P1, tb, lo, hi, first, end, probes);
+    // The window holds the answer for every key present in the index; for any other key it
+    // is checked: the rows just outside the window must not start with P_t.
+    const idx_t n_rows = A.num_reads * idx_t(A.L);
+    bool ok = true;
+    #pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const FmView& fa = *fq[q];
+        const uint64_t (&P)[kScanWords] = q ? P1 : P0;
+        if (first[q] == lo[q] && lo[q] > 0) {
+            const idx_t p = __ldg(fa.sa + lo[q] - 1);
+            ok = ok && cmp_row(fa.pk, p, suffix_len(p, A.dl), P, tb) < 0;
+            probes.add(2, 1 + cmp_sectors(fa.pk, p));
+        }
+        if (end[q] == hi[q] && hi[q] < n_rows) {
+            const idx_t p = __ldg(fa.sa + hi[q]);
+            ok = ok && cmp_row(fa.pk, p, suffix_len(p, A.dl), P, tb) > 0;
+            probes.add(2, 1 + cmp_sectors(fa.pk, p));
         }
     }
-    return true;
+    if (!ok) atomicAdd(A.lx_misses, 1ull);
+    return ok && end[0] - first[0] <= idx_t(kScanMax) && end[1] - first[1] <= idx_t(kScanMax);
+}
+
+// Of the rows [lo, hi) of a k-mer, those that go on with the next bases of its pattern, whose first
+// 32 bases are `word`.  Up to 64 rows are all read, 8 to a 16-byte load and independent of one
+// another, and compared two to a word (kx values are below 2^15, which leaves each half a guard
+// bit); a binary search would wait for three or four dependent sectors (3.5 ms against 1.2 on 5.4 M
+// reads of 44 rows a k-mer).  More rows are searched.
+__device__ __forceinline__ void narrow_rows(const FmView& f, int k, int t, uint64_t word, idx_t& lo, idx_t& hi, Tally& probes) {
+    const int x = f.kx_bases < t - k ? f.kx_bases : t - k;
+    if (x <= 0 || hi - lo <= 4) return;
+    const int drop = 2 * (f.kx_bases - x);
+    const uint32_t want = uint32_t(word << (2 * k) >> (64 - 2 * x));
+    const uint32_t from = want << drop, past = (want + 1) << drop;          // the values of the rows wanted
+    if (hi - lo <= 64) {
+        const idx_t base = lo & ~idx_t(7);
+        const int chunks = int(hi - base + 7) >> 3, skip = int(lo - base), held = int(hi - base) - 8 * (chunks - 1);
+        const uint4* v = reinterpret_cast<const uint4*>(f.kx + base);
+        // a chunk's rows 0, 2, 4, 6 in bits 0..3 and 1, 3, 5, 7 in bits 16..19: those from `skip` on
+        // in the first, the first `held` in the last
+        const uint32_t head = ((0xfu << ((skip + 1) >> 1)) & 0xfu) | (((0xfu << (skip >> 1)) & 0xfu) << 16);
+        const uint32_t tail = ((1u << ((held + 1) >> 1)) - 1u) | (((1u << (held >> 1)) - 1u) << 16);
+        const uint32_t from2 = from * 0x10001u, past2 = past * 0x10001u;
+        constexpr uint32_t H = 0x80008000u;
+        int below = 0, upto = 0;
+        #pragma unroll 3
+        for (int c = 0; c < chunks; ++c) {
+            const uint4 q = __ldg(v + c);
+            const uint32_t in = (c ? 0xf000fu : head) & (c + 1 < chunks ? 0xf000fu : tail);
+            auto less = [&](uint32_t w, uint32_t than) { return ~((w | H) - than) & H; };
+            auto rows = [&](uint32_t than) {
+                return (less(q.x, than) >> 15) | (less(q.y, than) >> 14) | (less(q.z, than) >> 13) | (less(q.w, than) >> 12);
+            };
+            below += __popc(rows(from2) & in);
+            upto += __popc(rows(past2) & in);
+        }
+        probes.add(0, uint32_t(chunks + 1) / 2);
+        hi = lo + idx_t(upto);
+        lo += idx_t(below);
+        return;
+    }
+    idx_t first = lo, b = hi;
+    while (first < b) {
+        const idx_t m = first + (b - first) / 2;
+        if (__ldg(f.kx + m) < from) first = m + 1;
+        else b = m;
+        probes.add(0, 1);
+    }
+    idx_t end = first;
+    b = hi;
+    while (end < b) {
+        const idx_t m = end + (b - end) / 2;
+        if (__ldg(f.kx + m) < past) end = m + 1;
+        else b = m;
+        probes.add(0, 1);
+    }
+    lo = first;
+    hi = end;
 }
 
 // warp-cooperative copy of one batch description into shared memory
@@ -1314,10 +1245,9 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
             const size_t cb = cbase_w + size_t(lane) * 4 * size_t(S.mstride);
             int nb[2], nf[2];
             int32_t ob = 0, of = 0;
-            chain_pair(A, A.fm, rd, self, PQ_BF, PQ_BB, nb, ob, probes, SlotsFast{S.c_ll, S.c_uu, S.c_meta, cb, M},
-                       [] {});
-            chain_pair(A, A.fm, rd, self, PQ_FB, PQ_FF, nf, of, probes,
-                       SlotsFast{S.c_ll, S.c_uu, S.c_meta, cb + 2 * size_t(M), M}, [] {});
+            chain_pair(A, A.fm, rd, PQ_BF, PQ_BB, nb, ob, probes, SlotsFast{S.c_ll, S.c_uu, S.c_meta, cb, M});
+            chain_pair(A, A.fm, rd, PQ_FB, PQ_FF, nf, of, probes,
+                       SlotsFast{S.c_ll, S.c_uu, S.c_meta, cb + 2 * size_t(M), M});
             s_n[wid][lane][0] = nb[0];
             s_n[wid][lane][1] = nb[1];
             s_n[wid][lane][2] = nf[0];
@@ -1340,7 +1270,7 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
             int sc_sorted = -1;
             if (active && A.sorted_reduce && s_olp[wid][lane][side] <= kRedMax) {
                 const int st = reduce_sorted<W>(A, S, self, side, cbase_w + size_t(lane) * 4 * size_t(S.mstride), na,
-                                             n0, rbase_w + size_t(lane) * kRedMax, eb, ne, sc_sorted, probes);
+                                             n0, rbase_w + lane, eb, ne, sc_sorted, probes);
                 if (st != OVF_NONE) status = st;
                 active = false;
             }
@@ -1609,25 +1539,37 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
 
 // ------------------------------------------------------------------------------ lean tier
 //
-// One thread per read, no warp-level phases: each side's candidates by the interval scan as a list
-// of records, and its edges by sorted continuations.  A read the scan does not serve (a depth-t
-// interval beyond kScanMax rows, a learned window that missed) or with more than kRedMax
-// candidates on a side is listed in `defer` for the fast tier (which walks and runs the DFS there).
-// With no shared-memory DFS state and fewer registers, more warps stay resident to hide the latency
-// of the independent suffix-array and text loads.
+// A warp takes 32 reads.  The rows to check of each read's two chains of a side are found lane by
+// lane (k-mer table, narrow_rows); then the rows of all 32 reads are taken one a lane, so that 32 suffix-array entries are in flight at once whatever the reads' own numbers
+// of rows.  Rows at an offset that can be a candidate wait in a queue until a warp's worth is there
+// to compare its texts, and a row that is a candidate takes the next slot of its read.  Each lane
+// then reduces its read by sorted continuations.  A read the scan does not serve or with more than
+// kRedMax candidates on a side is listed in `defer` for the fast tier, which walks and runs the DFS.
+//
+// Bound by DRAM at random sectors (4.1 TB/s, of which every second sector of a 64-byte fetch goes
+// unused): k-mer table, kx, suffix array, text.  5.4 M reads of 100 bases, 566 M suffixes, 64-bit
+// index: 7.3 ms, against 13.5 with one thread per read throughout (10 of 32 lanes active) and I_t
+// found by bisection; 1.2 M reads, 123 M suffixes: 1.5 against 2.4.  Eight CTAs of 64 registers per
+// SM; six or ten were 3 to 10 % slower.
 constexpr int kLeanThreads = 128;
 
 template <int W>
 __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, SearchOut O0, WarpScratch S,
                                                                 SearchQueue Q) {
-    extern __shared__ uint32_t s_reads[];
     __shared__ SearchBatch s_b[kLeanThreads / 32];
+    __shared__ int s_pref[kLeanThreads / 32][33], s_m[kLeanThreads / 32][32];
+    __shared__ idx_t s_qid[kLeanThreads / 32][64];              // rows waiting for their text to be checked:
+    __shared__ uint32_t s_qo[kLeanThreads / 32][64];            // read, and offset | lane << 16 | chain << 21
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const size_t gw = size_t(blockIdx.x) * (kLeanThreads / 32) + wid;
     const size_t nw = size_t(gridDim.x) * (kLeanThreads / 32);
     SearchBatch& B = s_b[wid];
     const SearchArgs& A = B.a;
     const SearchOut& O = B.o;
+    int* const pref = s_pref[wid];
+    int* const slots = s_m[wid];
+    idx_t* const qid = s_qid[wid];
+    uint32_t* const qo = s_qo[wid];
     if (Q.count == 0) {
         if (lane == 0) {
             B.a = A0;
@@ -1635,9 +1577,8 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
         }
         __syncwarp();
     }
-    const size_t tid = gw * 32 + lane;
-    const size_t eb = tid * size_t(S.ebcap);
-    const size_t red = tid * size_t(kRedMax);
+    const size_t ebase = gw * 32 * size_t(S.ebcap) + lane;      // edge i of a lane at ebase + 32 i
+    const size_t rbase = gw * 32 * size_t(kRedMax);
     Tally probes;
     int cur = -1;
     for (size_t iter = 0;; ++iter) {
@@ -1663,53 +1604,171 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
             if (group * 32 >= size_t(A.num_reads)) break;
         }
         for (; group < gend && group * 32 < size_t(A.num_reads); ++group) {
+            const int L = A.L, t = A.t, M = L - t;
             const size_t r = group * 32 + lane;
-            if (r >= size_t(A.num_reads)) continue;
             const idx_t self = idx_t(r);
+            const bool have = r < size_t(A.num_reads);
+            bool ok = have;
+            int ne = 0, status = OVF_NONE;
+            int count_b = 0, count_f = 0;
+            int32_t olp_b = 0, olp_f = 0;
             // B side: B-F then B-B candidates, then extract_bw_edges (src/string_graph.c:824-825);
-            // then the F side: F-B, F-F, extract_fw_edges (:828-829)
-            int32_t ob = 0, of = 0;
-            int m = 0, ne = 0, count_b = 0, count_f = 0;
-            int status = OVF_NONE;
-            bool ok = scan_planes<W>(A, A.fm, self, PQ_BF, PQ_BB, S, red, m, ob, probes);
-            if (ok && ob != 0) status = reduce_gathered<W>(A.L, S, self, 0, red, m, eb, ne, count_b);
-            m = 0;
-            if (ok) ok = scan_planes<W>(A, A.fm, self, PQ_FB, PQ_FF, S, red, m, of, probes);
-            if (ok && of != 0 && status == OVF_NONE)
-                status = reduce_gathered<W>(A.L, S, self, 1, red, m, eb, ne, count_f);
-            if (!ok) {              // the fast tier redoes this read (walk, or more candidates)
+            // then the F side: F-B, F-F, extract_fw_edges (:828-829).  Both kinds of a side take
+            // their pattern from the same text: the first as it is, the second its complement.
+            #pragma unroll 1
+            for (int side = 0; side < 2; ++side) {
+                const int k0 = side ? PQ_FB : PQ_BF, k1 = side ? PQ_FF : PQ_BB;
+                const FmView* f0 = A.fm + walked_index(k0);
+                const FmView* f1 = A.fm + walked_index(k1);
+                idx_t first[2] = {0, 0}, end[2] = {0, 0};
+                uint64_t P0[kScanWords] = {}, P1[kScanWords] = {};
+                if (ok) {
+                    pattern_words(A.fm, L, t, k0, self, P0, probes);
+                    #pragma unroll
+                    for (int w = 0; w < kScanWords; ++w) P1[w] = ~P0[w];
+                }
+                if (A.sa_seed == 2) {
+                    if (ok) ok = learned_rows(A, f0, f1, P0, P1, first, end, probes);
+                    __syncwarp();
+                } else {
+                    const int k = A.seed_k;
+                    if (ok) {
+                        kmer_rows(*f0, uint32_t(P0[0] >> (64 - 2 * k)), first[0], end[0]);
+                        kmer_rows(*f1, uint32_t(P1[0] >> (64 - 2 * k)), first[1], end[1]);
+                        probes.add(2, 2);
+                        #pragma unroll
+                        for (int q = 0; q < 2; ++q) end[q] = end[q] < first[q] ? first[q] : end[q] + 1;
+                    }
+                    narrow_rows(*f0, k, t, P0[0], first[0], end[0], probes);
+                    narrow_rows(*f1, k, t, P1[0], first[1], end[1], probes);
+                    if (ok && (end[0] - first[0] > idx_t(kScanDirect) || end[1] - first[1] > idx_t(kScanDirect))) {
+                        const idx_t lo[2] = {first[0], first[1]}, hi[2] = {end[0], end[1]};
+                        sa_bounds2(f0, f1, A.dl, P0, P1, t < 32 * kScanWords ? t : 32 * kScanWords, lo, hi, first, end, probes);
+                        ok = end[0] - first[0] <= idx_t(kScanMax) && end[1] - first[1] <= idx_t(kScanMax);
+                    }
+                }
+                slots[lane] = 0;
+                __syncwarp();
+                // a row that passed the offset test: its read against the whole pattern, and its
+                // continuation (M - o bases of the walked text after the pattern) if it matches
+                const uint64_t* const pks = f0->pk;             // both patterns' source
+                auto check = [&](int i, unsigned lanes) {
+                    const idx_t rp = qid[i];
+                    const uint32_t v = qo[i];
+                    const int o = int(v & 0xffffu), j = int((v >> 16) & 31u), d = t + o, len = M - o;
+                    const bool cmpl = (v >> 21) != 0;
+                    const FmView& fa = cmpl ? *f1 : *f0;
+                    const size_t text = size_t(rp) * size_t(L);
+                    const size_t src = (group * 32 + size_t(j)) * size_t(L) + size_t(len);
+                    probes.add(0, base_sectors(text, d));
+                    if (!text_matches(fa.pk, text, pks, src, d, cmpl, lanes)) return;
+                    const int slot = atomicAdd(&slots[j], 1);
+                    if (slot >= kRedMax) return;
+                    const size_t pos = text + size_t(d), at = rbase + size_t(slot) * kRedStride + size_t(j);
+                    const uint32_t flip = walked_index(cmpl ? k1 : k0) ? ~0u : 0u;
+                    const uint64_t* w = fa.pk + (pos >> 5);
+                    const int s = int(pos & 31);
+                    uint64_t a0 = __ldg(w);
+                    #pragma unroll
+                    for (int q = 0; q < W; ++q) {
+                        const int left = len - 32 * q;
+                        if (left <= 0) break;
+                        const uint64_t a1 = __ldg(w + q + 1);
+                        uint32_t h, l;
+                        shift_bases(a0, a1, s, h, l);
+                        S.r_k[q * S.r_plane + at] = (uint64_t((h ^ flip) & half_mask(left, 0)) << 32) |
+                                                    ((l ^ flip) & half_mask(left, 1));
+                        a0 = a1;
+                    }
+                    probes.add(0, base_sectors(pos, len));
+                    S.r_id[at] = rp;
+                    S.r_meta[at] = pack_meta(d, cmpl ? k1 : k0);
+                };
+                int waiting = 0;
+                #pragma unroll 1
+                for (int q = 0; q < 2; ++q) {
+                    const idx_t* const sa = q ? f1->sa : f0->sa;
+                    const idx_t mine = q ? first[1] : first[0];
+                    const int total = warp_prefix(ok ? int((q ? end[1] : end[0]) - mine) : 0, pref);
+                    for (int e0 = 0; e0 < total; e0 += 32) {
+                        const int e = e0 + lane;
+                        const int j = owner_of(pref, e < total ? e : total - 1);
+                        const idx_t row = __shfl_sync(0xffffffffu, mine, j) + idx_t(e - pref[j]);
+                        int o = M;
+                        idx_t rp = 0;
+                        if (e < total) {
+                            const idx_t p = __ldg(sa + row);
+                            rp = read_of(p, A.dl);
+                            o = int(p - rp * idx_t(L));
+                            probes.add(2, 1);
+                        }
+                        const unsigned pass = __ballot_sync(0xffffffffu, o < M);
+                        if (o < M) {
+                            const int i = waiting + __popc(pass & ((1u << lane) - 1u));
+                            qid[i] = rp;
+                            qo[i] = uint32_t(o) | (uint32_t(j) << 16) | (uint32_t(q) << 21);
+                        }
+                        __syncwarp();
+                        waiting += __popc(pass);
+                        if (waiting >= 32) {                    // a full warp's worth
+                            waiting -= 32;
+                            check(waiting + lane, 0xffffffffu);
+                            __syncwarp();
+                        }
+                    }
+                    __syncwarp();
+                }
+                if (lane < waiting) check(lane, (1u << waiting) - 1u);
+                __syncwarp();
+                const int m = slots[lane];
+                if (m > kRedMax) ok = false;
+                int count = 0;
+                if (ok && m && status == OVF_NONE)
+                    status = reduce_gathered<W>(L, S, self, side, rbase + lane, m, ebase, 32, ne, count);
+                if (side == 0) {
+                    olp_b = m;
+                    count_b = count;
+                } else {
+                    olp_f = m;
+                    count_f = count;
+                }
+                __syncwarp();
+            }
+            if (have && !ok) {          // the fast tier redoes this read (walk, or more candidates)
                 const unsigned k = atomicAdd(A.defer_count, 1u);
                 A.defer[k] = self;
-                continue;
-            }
-            if (status != OVF_NONE) {
+            } else if (have && status != OVF_NONE) {
                 O.status[r] = uint8_t(status);
+                const unsigned k = atomicAdd(O.ovf_count, 1u);
+                O.ovf_list[k] = self;
+            }
+            // one reservation of edge slots for the warp's reads
+            const int mine = have && ok && status == OVF_NONE ? ne : 0;
+            const int edges = warp_prefix(mine, pref);
+            unsigned long long base = 0;
+            if (lane == 0 && edges) base = atomicAdd(O.e_count, (unsigned long long)edges);
+            base = __shfl_sync(0xffffffffu, base, 0) + (unsigned long long)pref[lane];
+            __syncwarp();
+            if (!have || !ok || status != OVF_NONE) continue;
+            if (ne && base + ne > O.e_cap) {
+                O.status[r] = OVF_POOL;
                 const unsigned k = atomicAdd(O.ovf_count, 1u);
                 O.ovf_list[k] = self;
                 continue;
             }
-            unsigned long long base = 0;
-            if (ne) {
-                base = atomicAdd(O.e_count, (unsigned long long)ne);
-                if (base + ne > O.e_cap) {
-                    O.status[r] = OVF_POOL;
-                    const unsigned k = atomicAdd(O.ovf_count, 1u);
-                    O.ovf_list[k] = self;
-                    continue;
-                }
-                for (int e = 0; e < ne; ++e) {
-                    const uint32_t mt = S.e_meta[eb + e];
-                    O.e_dest[base + e] = S.e_dest[eb + e];
-                    O.e_trans[base + e] = S.e_trans[eb + e];
-                    O.e_len[base + e] = uint16_t(meta_len(mt));
-                    O.e_type[base + e] = uint8_t(meta_type(mt));
-                }
+            for (int e = 0; e < ne; ++e) {
+                const size_t q = ebase + size_t(e) * 32;
+                const uint32_t mt = S.e_meta[q];
+                O.e_dest[base + e] = S.e_dest[q];
+                O.e_trans[base + e] = S.e_trans[q];
+                O.e_len[base + e] = uint16_t(meta_len(mt));
+                O.e_type[base + e] = uint8_t(meta_type(mt));
             }
             O.status[r] = OVF_NONE;
             O.num_B[r] = uint16_t(count_b);
             O.num_F[r] = uint16_t(count_f);
-            O.olp_B[r] = ob;
-            O.olp_F[r] = of;
+            O.olp_B[r] = olp_b;
+            O.olp_F[r] = olp_f;
             O.edge_src[r] = base;
         }
         __syncwarp();
@@ -1718,12 +1777,11 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
 }
 
 int search_lean_blocks(int L, int M, int num_sms) {
-    const int words = (L + 15) / 16;
-    const size_t smem = size_t(words) * kLeanThreads * sizeof(uint32_t);
+    (void)L;
     int per_sm = 0;
     const cudaError_t e = lam_words(M) == 2
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search_lean<2>, kLeanThreads, smem)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search_lean<kLamWords>, kLeanThreads, smem);
+        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search_lean<2>, kLeanThreads, 0)
+        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search_lean<kLamWords>, kLeanThreads, 0);
     if (e != cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
@@ -1809,10 +1867,10 @@ cudaError_t search_lean(const SearchArgs& a, const SearchOut& o, int lean_blocks
     const int words = (a.L + 15) / 16;
     cudaError_t e = cudaMemsetAsync(a.defer_count, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
-    const size_t lsm = size_t(words) * kLeanThreads * 4, fsm = size_t(words) * 32 * kWarpsPerCta * 4;
+    const size_t fsm = size_t(words) * 32 * kWarpsPerCta * 4;
     SearchQueue none{};
-    if (lam_words(a.L - a.t) == 2) k_search_lean<2><<<lean_blocks, kLeanThreads, lsm, st>>>(a, o, S, none);
-    else k_search_lean<kLamWords><<<lean_blocks, kLeanThreads, lsm, st>>>(a, o, S, none);
+    if (lam_words(a.L - a.t) == 2) k_search_lean<2><<<lean_blocks, kLeanThreads, 0, st>>>(a, o, S, none);
+    else k_search_lean<kLamWords><<<lean_blocks, kLeanThreads, 0, st>>>(a, o, S, none);
     note_launch();
     // the handed-over reads, whatever their number (read on the device): the fast tier's DFS
     SearchQueue Q{};
@@ -1834,12 +1892,12 @@ cudaError_t search_lean_queue(const SearchQueue& q, const SearchBatch* host_batc
     WarpScratch S;
     if (scratch_bytes < scratch_layout(M_max, nwarps, ebcap, scratch, &S)) return cudaErrorInvalidValue;
     const int words = (L_max + 15) / 16;
-    const size_t lsm = size_t(words) * kLeanThreads * 4, fsm = size_t(words) * 32 * kWarpsPerCta * 4;
+    const size_t fsm = size_t(words) * 32 * kWarpsPerCta * 4;
     const bool two = lam_words(M_max) == 2;
     SearchArgs a0{};
     SearchOut o0{};
-    if (two) k_search_lean<2><<<lean_blocks, kLeanThreads, lsm, st>>>(a0, o0, S, q);
-    else k_search_lean<kLamWords><<<lean_blocks, kLeanThreads, lsm, st>>>(a0, o0, S, q);
+    if (two) k_search_lean<2><<<lean_blocks, kLeanThreads, 0, st>>>(a0, o0, S, q);
+    else k_search_lean<kLamWords><<<lean_blocks, kLeanThreads, 0, st>>>(a0, o0, S, q);
     note_launch();
     for (int i = 0; i < nbatch; ++i) {
         const SearchBatch& hbt = host_batches[batches[i]];
@@ -2176,8 +2234,8 @@ __global__ void __launch_bounds__(kBlockThreads) k_search_block(SearchArgs A, Se
             ReadView rd{rdw, 1};
             int n[2];
             int32_t olp = 0;
-            chain_pair(A, A.fm, rd, self, side ? PQ_FB : PQ_BF, side ? PQ_FF : PQ_BB, n, olp, probes,
-                       SlotsStack{grp + size_t(side) * 2 * M, M}, [] {});
+            chain_pair(A, A.fm, rd, side ? PQ_FB : PQ_BF, side ? PQ_FF : PQ_BB, n, olp, probes,
+                       SlotsStack{grp + size_t(side) * 2 * M, M});
             s_n[side][0] = n[0];
             s_n[side][1] = n[1];
             s_olp[side] = olp;

@@ -1063,12 +1063,12 @@ __global__ void k_short_runs(const uint64_t* __restrict__ pk, const uint32_t* __
 }
 
 // the rows of the short suffixes: before their bucket's long ones; those of at least k bases also
-// belong to a k-mer (k <= S only: kstart null otherwise)
+// belong to a k-mer (k <= S only: kt null otherwise)
 __global__ void k_short_place(const uint64_t* __restrict__ pk, const uint32_t* __restrict__ key,
                               const idx_t* __restrict__ val, size_t m, DivL dl, int bits,
                               const unsigned long long* __restrict__ count, const unsigned long long* __restrict__ first,
                               const unsigned long long* __restrict__ lstart, idx_t* __restrict__ sa,
-                              uint8_t* __restrict__ bwt, idx_t* __restrict__ kstart, idx_t* __restrict__ kend, int k) {
+                              uint8_t* __restrict__ bwt, idx_t* __restrict__ kt, int k) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
         const idx_t p = val[i];
@@ -1076,10 +1076,10 @@ __global__ void k_short_place(const uint64_t* __restrict__ pk, const uint32_t* _
         const size_t row = size_t(lstart[b] - count[b] + (i - first[b]));
         sa[row] = p;
         if (bwt) bwt[row] = uint8_t(key[i] >> kShortSym);
-        if (kstart && suffix_bases(size_t(p), dl) >= k) {
+        if (kt && suffix_bases(size_t(p), dl) >= k) {
             const size_t c = size_t(window(pk, size_t(p)) >> (64 - 2 * k));
-            atomicMin(reinterpret_cast<kmer_int*>(kstart + c), kmer_int(row));
-            atomicMax(reinterpret_cast<kmer_int*>(kend + c), kmer_int(row));
+            atomicMin(reinterpret_cast<kmer_int*>(kt + 2 * c), kmer_int(row));
+            atomicMax(reinterpret_cast<kmer_int*>(kt + 2 * c + 1), kmer_int(row));
         }
     }
 }
@@ -1261,7 +1261,9 @@ struct MsdLocal {
     MsdLists G;
     idx_t* sa;                          // rows of element 0 on
     uint8_t* bwt;                       // or null
-    idx_t *kstart, *kend;               // k-mer table, or null
+    idx_t* kt;                          // k-mer table, or null
+    uint16_t* kx;                       // every row's next bases, or null: kx_bits bits of an element
+    int kx_bits, kx_shift;              // from bit kx_shift on
     int kmer_k;
     int kmer_spans;                     // a k-mer's rows may lie in several buckets
     size_t row0;                        // suffix-array row of element 0
@@ -1596,8 +1598,9 @@ __global__ void __launch_bounds__(T, T == 128 ? (W <= 4 ? 8 : 6) : 3) k_msd_loca
             const uint64_t e = se[j];
             a.sa[bk.start + j] = idx_t((e >> kSymBits) & pos_mask);
             if (a.bwt) a.bwt[bk.start + j] = uint8_t(e & 7u);
+            if (a.kx && !off) a.kx[bk.start + j] = uint16_t((e >> a.kx_shift) & ((1u << a.kx_bits) - 1u));
         }
-        if (a.kstart && !off) {
+        if (a.kt && !off) {
             // k-mer of a row (k <= head): the bucket's first d1 bits and the key; absent in a
             // suffix of fewer bases.  Buckets of whole k-mers write each one's two rows; when a
             // k-mer spans buckets its rows are agreed on by minimum and maximum.
@@ -1620,15 +1623,15 @@ __global__ void __launch_bounds__(T, T == 128 ? (W <= 4 ? 8 : 6) : 3) k_msd_loca
                 }
                 if (!begins && !ends) continue;
                 const uint64_t key = e >> P.key_shift;
-                const unsigned c = unsigned(top >= 0 ? (id1 << top) | (key >> (P.kbits - top)) : id1 >> (-top));
+                const size_t c = size_t(top >= 0 ? (id1 << top) | (key >> (P.kbits - top)) : id1 >> (-top));
                 const idx_t row = idx_t(a.row0 + bk.start + j);
                 if (begins) {
-                    if (spans) atomicMin(reinterpret_cast<kmer_int*>(a.kstart + c), kmer_int(row));
-                    else a.kstart[c] = row;
+                    if (spans) atomicMin(reinterpret_cast<kmer_int*>(a.kt + 2 * c), kmer_int(row));
+                    else a.kt[2 * c] = row;
                 }
                 if (ends) {
-                    if (spans) atomicMax(reinterpret_cast<kmer_int*>(a.kend + c), kmer_int(row));
-                    else a.kend[c] = row;
+                    if (spans) atomicMax(reinterpret_cast<kmer_int*>(a.kt + 2 * c + 1), kmer_int(row));
+                    else a.kt[2 * c + 1] = row;
                 }
             }
         }
@@ -1931,23 +1934,29 @@ __global__ void __launch_bounds__(kSplitThreads) k_more_copy(const uint64_t* __r
 
 // A k-mer table whose k-mers span buckets is entered by minimum and maximum: prepared so (mode 0;
 // mode 2 only where a k-mer is still absent), then absent ones set as everywhere else (mode 1:
-// kend < kstart)
-__global__ void k_kmer_span(idx_t* __restrict__ kstart, idx_t* __restrict__ kend, size_t c0, size_t c1, int mode) {
+// last < first)
+__global__ void k_kmer_span(idx_t* __restrict__ kt, size_t c0, size_t c1, int mode) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     for (size_t i = c0 + size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < c1; i += stride) {
-        if (mode == 0 || (mode == 2 && kend[i] < kstart[i])) {
-            kstart[i] = ~idx_t(0);
-            kend[i] = 0;
-        } else if (mode == 1 && kstart[i] == ~idx_t(0)) {
-            kstart[i] = 1;
+        idx_t* const k = kt + 2 * i;
+        if (mode == 0 || (mode == 2 && k[1] < k[0])) {
+            k[0] = ~idx_t(0);
+            k[1] = 0;
+        } else if (mode == 1 && k[0] == ~idx_t(0)) {
+            k[0] = 1;
         }
     }
 }
 
 // rows [r0, r1) all start with k-mer c
-__global__ void k_kmer_rows(idx_t* __restrict__ kstart, idx_t* __restrict__ kend, size_t c, size_t r0, size_t r1) {
-    atomicMin(reinterpret_cast<kmer_int*>(kstart + c), kmer_int(r0));
-    atomicMax(reinterpret_cast<kmer_int*>(kend + c), kmer_int(r1 - 1));
+__global__ void k_kmer_rows(idx_t* __restrict__ kt, size_t c, size_t r0, size_t r1) {
+    atomicMin(reinterpret_cast<kmer_int*>(kt + 2 * c), kmer_int(r0));
+    atomicMax(reinterpret_cast<kmer_int*>(kt + 2 * c + 1), kmer_int(r1 - 1));
+}
+// and go on with the same bases
+__global__ void k_kx_rows(uint16_t* __restrict__ kx, size_t m, uint16_t v) {
+    const size_t stride = size_t(gridDim.x) * blockDim.x;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) kx[i] = v;
 }
 
 // ------------------------------------------------------------------------------ driver
@@ -2128,7 +2137,7 @@ template <int W>
 int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t* tmp, int sms, cudaStream_t st) {
     const MsdPlan& P = a.plan;
     const int k = a.kmer_k, bits = P.d1 + P.d2;
-    const bool own_span = a.kstart && !a.kmer_spans;        // a listed bucket's k-mers span its parts
+    const bool own_span = a.kt && !a.kmer_spans;        // a listed bucket's k-mers span its parts
     std::vector<unsigned> split_ids;
     auto h2d = [&](void* d, const void* h, size_t b) { return cudaMemcpyAsync(d, h, b, cudaMemcpyHostToDevice, st); };
     auto d2h = [&](void* h, const void* d, size_t b) { return cudaMemcpyAsync(h, d, b, cudaMemcpyDeviceToHost, st); };
@@ -2155,7 +2164,7 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
             work.push_back({b.start, b.start + b.size, 0, id, false});
             if (own_span) {
                 const size_t per = size_t(1) << (2 * k - bits);
-                k_kmer_span<<<grid_for(per, 256), 256, 0, st>>>(a.kstart, a.kend, id * per, (id + 1) * per, 2);
+                k_kmer_span<<<grid_for(per, 256), 256, 0, st>>>(a.kt, id * per, (id + 1) * per, 2);
                 note_launch();
                 split_ids.push_back(id);
             }
@@ -2227,12 +2236,18 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
                     while (hb > 0 && !((d[q] >> hb) & 1)) --hb;
                     const int full = x.off ? a.more_bits / 2 : P.head;
                     if (hb < P.len_shift && int((e0[q] >> P.len_shift) & 31) == full) {
-                        if (a.kstart && !x.off) {            // one k-mer throughout
+                        if (a.kt && !x.off) {                // one k-mer throughout
                             const int top = 2 * k - P.d1;
                             const uint64_t id1 = x.id >> P.d2, key = e0[q] >> P.key_shift;
                             const uint64_t c = top >= 0 ? (id1 << top) | (key >> (P.kbits - top)) : id1 >> (-top);
-                            k_kmer_rows<<<1, 1, 0, st>>>(a.kstart, a.kend, size_t(c), a.row0 + x.start, a.row0 + x.end);
+                            k_kmer_rows<<<1, 1, 0, st>>>(a.kt, size_t(c), a.row0 + x.start, a.row0 + x.end);
                             note_launch();
+                            if (a.kx) {
+                                const size_t m = size_t(x.end - x.start);
+                                k_kx_rows<<<grid_for(m, 256), 256, 0, st>>>(
+                                    a.kx + x.start, m, uint16_t((e0[q] >> a.kx_shift) & ((1u << a.kx_bits) - 1u)));
+                                note_launch();
+                            }
                         }
                         x.off += full;
                         x.rebuild = true;
@@ -2302,7 +2317,7 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
     }
     for (unsigned id : split_ids) {
         const size_t per = size_t(1) << (2 * k - bits);
-        k_kmer_span<<<grid_for(per, 256), 256, 0, st>>>(a.kstart, a.kend, id * per, (id + 1) * per, 1);
+        k_kmer_span<<<grid_for(per, 256), 256, 0, st>>>(a.kt, id * per, (id + 1) * per, 1);
         note_launch();
     }
     return int(cudaGetLastError());
@@ -2311,7 +2326,9 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
 struct SortOut {
     idx_t* sa;
     uint8_t* bwt;
-    idx_t *kstart, *kend;
+    idx_t* kt;
+    uint16_t* kx;
+    int kx_bases;
     int kmer_k;
     bool kmer_spans;        // k-mers shorter than the buckets' prefix (or a chunk boundary's)
     bool kmer_done;
@@ -2383,7 +2400,7 @@ int msd_pass(const MsdPlan& P, size_t nr, const MsdScratch& s, const SortOut& o,
     }
     if (P.S) {
         k_short_place<<<gs, 256, 0, st>>>(s.pk, sk0, sv0, nshort, P.dl, bits, s.shorts, s.sfirst, s.lstart, o.sa, o.bwt,
-                                          o.kmer_k <= P.S ? o.kstart : nullptr, o.kend, o.kmer_k);
+                                          o.kmer_k <= P.S ? o.kt : nullptr, o.kmer_k);
         note_launch();
     }
     MsdLocal a{};
@@ -2393,8 +2410,10 @@ int msd_pass(const MsdPlan& P, size_t nr, const MsdScratch& s, const SortOut& o,
     a.G = G;
     a.sa = o.sa + row0;
     a.bwt = o.bwt ? o.bwt + row0 : nullptr;
-    a.kstart = o.kstart;
-    a.kend = o.kend;
+    a.kt = o.kt;
+    a.kx = o.kx ? o.kx + row0 : nullptr;
+    a.kx_bits = 2 * o.kx_bases;
+    a.kx_shift = P.key_shift + P.kbits - (2 * o.kmer_k - P.d1) - 2 * o.kx_bases;
     a.kmer_k = o.kmer_k;
     a.kmer_spans = o.kmer_spans;
     a.row0 = row0;
@@ -2494,12 +2513,14 @@ static int sort_msd(const SortShape& sh, size_t nr, const MsdScratch& s, SortOut
     const size_t n = P.n;
     // k-mers entered as the buckets finish: of up to `head` bases; where they span buckets or short
     // suffixes have them too, by minimum and maximum
-    if (o.kstart && o.kmer_k > P.head) o.kstart = o.kend = nullptr;
+    if (o.kt && o.kmer_k > P.head) o.kt = nullptr;
+    o.kx_bases = o.kt && o.kx && 2 * o.kmer_k >= P.d1 ? std::min(7, P.head - o.kmer_k) : 0;
+    if (!o.kx_bases) o.kx = nullptr;
     const bool spans = o.kmer_spans = o.kmer_k <= P.S || 2 * o.kmer_k < std::max(P.d1 + P.d2, sh.chunked ? 2 * kBucketBases : 0);
     const size_t nk = size_t(1) << (2 * o.kmer_k);
-    if (o.kstart && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kstart, o.kend, 0, nk, 0); note_launch(); }
-    if (o.kstart && !spans) {
-        const cudaError_t e = kmer_table_clear(o.kmer_k, o.kstart, o.kend, st);
+    if (o.kt && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kt, 0, nk, 0); note_launch(); }
+    if (o.kt && !spans) {
+        const cudaError_t e = kmer_table_clear(o.kmer_k, o.kt, st);
         if (e != cudaSuccess) return int(e);
     }
     bool more = false;
@@ -2532,16 +2553,17 @@ static int sort_msd(const SortShape& sh, size_t nr, const MsdScratch& s, SortOut
             lo = hi;
         }
     }
-    if (o.kstart && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kstart, o.kend, 0, nk, 1); note_launch(); }
-    o.kmer_done = o.kstart != nullptr;
+    if (o.kt && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kt, 0, nk, 1); note_launch(); }
+    o.kmer_done = o.kt != nullptr;
     return int(cudaGetLastError());
 }
 
 int suffix_sort(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa, size_t cap, void* tmp,
-                size_t tmp_bytes, cudaStream_t st, const uint8_t** bwt_out, uint64_t* pk_out, idx_t* kstart, idx_t* kend,
-                int kmer_k, bool* kmer_done) {
+                size_t tmp_bytes, cudaStream_t st, const uint8_t** bwt_out, uint64_t* pk_out, idx_t* kt, int kmer_k, bool* kmer_done,
+                uint16_t* kx, int* kx_bases) {
     if (bwt_out) *bwt_out = nullptr;
     if (kmer_done) *kmer_done = false;
+    if (kx_bases) *kx_bases = 0;
     const size_t n = size_t(num_reads) * size_t(L);
     if (n == 0) return 0;
     if (cap >= n) cap = 0;
@@ -2562,7 +2584,7 @@ int suffix_sort(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa
     { k_pack_text<<<grid_for(nwords, 256), 256, 0, st>>>(reads, n, idx_t(L), dir, nwords, pk); note_launch(); }
     if (sh.doubling) return sort_doubling(n, L, sa, pk, tmp, st);
     s.pk = pk;
-    SortOut o{sa, bwt_out ? s.bwt : nullptr, kstart, kend, kmer_k, false, false};
+    SortOut o{sa, bwt_out ? s.bwt : nullptr, kt, kx, 0, kmer_k, false, false};
     int rc = 0;
     switch (plan_words(sh.plan)) {
         case 1: rc = sort_msd<1>(sh, num_reads, s, o, cap, st); break;
@@ -2578,6 +2600,7 @@ int suffix_sort(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa
     if (rc) return rc;
     if (bwt_out) *bwt_out = s.bwt;
     if (kmer_done) *kmer_done = o.kmer_done;
+    if (kx_bases) *kx_bases = o.kx_bases;
     return 0;
 }
 

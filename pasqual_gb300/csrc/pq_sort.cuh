@@ -11,17 +11,18 @@ namespace pq {
 // 6-base bucket exceeds it.  When bwt_out is given it receives the BWT symbol (0 = `$`, 1..4) of
 // every row, inside tmp (valid until tmp is reused), or nullptr when the sort went by prefix
 // doubling.  pk_out (n/32 + 4 words), when given, receives the packed text of the direction (see
-// pack_text) instead of tmp.  kstart/kend, when given, receive the table of kmer_k-mers;
-// *kmer_done tells whether they are complete (else the caller builds the table).
+// pack_text) instead of tmp.  kt, when given, receives the table of kmer_k-mers (FmView::kt) and kx
+// (n entries), when given beside it, every row's next bases (FmView::kx); *kmer_done tells whether
+// the table is complete (else the caller builds it) and *kx_bases how many bases kx holds (0: none).
 constexpr int kSortKeyBases = 14;           // longest k-mers of the table
 size_t suffix_sort_tmp_bytes(size_t n, size_t num_reads, int L, size_t cap = 0);
 int suffix_sort(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa, size_t cap, void* tmp,
                 size_t tmp_bytes, cudaStream_t st, const uint8_t** bwt_out = nullptr, uint64_t* pk_out = nullptr,
-                idx_t* kstart = nullptr, idx_t* kend = nullptr, int kmer_k = 0, bool* kmer_done = nullptr);
+                idx_t* kt = nullptr, int kmer_k = 0, bool* kmer_done = nullptr, uint16_t* kx = nullptr, int* kx_bases = nullptr);
 
 // Per-read seeds from a k-mer table (pq_index.cu).
-cudaError_t read_seeds(const uint8_t* reads, idx_t num_reads, int L, int dir, int k, const idx_t* kstart,
-                       const idx_t* kend, idx_t* start, idx_t* size, cudaStream_t st);
+cudaError_t read_seeds(const uint8_t* reads, idx_t num_reads, int L, int dir, int k, const idx_t* kt,
+                       idx_t* start, idx_t* size, cudaStream_t st);
 
 // Stable LSD radix sort of (key, value) pairs on the bits [lo_bit, hi_bit) of the key (K is
 // uint32_t or uint64_t).  Buffers are ping-ponged; the sorted result ends in (*k0, *v0) (pointers
