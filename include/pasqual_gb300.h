@@ -295,7 +295,7 @@ PQ_API int pq_autotune_batched (pq_ctx ** ctxs, int count, int flags, float *bes
 
 /* How the last pq_overlaps divided its reads among its tiers: reads[0] = reads the lean tier (one
  * thread a read, interval scan) handed to the fast tier (warp-level walk and DFS), reads[1] = reads
- * the block tier (one CTA a read, all-pairs reduction in shared memory) finished of those the fast
+ * the block tier (one CTA a read, candidates sorted in shared memory) finished of those the fast
  * tier handed over, reads[2] = reads the heavy tier (the fast tier's DFS with larger capacities)
  * took, reads[3] = reads the wide tier (the reference's own bounds) took; ms[0] = the lean and
  * fast kernels (CUDA events), ms[1..3] = the block, heavy and wide tiers (host time, their

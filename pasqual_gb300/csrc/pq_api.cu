@@ -738,74 +738,74 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
     ctx->block_reads = 0;
     ctx->ms_block = 0;
     if (ovf && A.sorted_reduce) {
-        // block tier (one CTA a read, all-pairs reduction in shared memory) over the reads the fast
+        // block tier (one CTA a read, candidates sorted in shared memory) over the reads the fast
         // tier could not hold; the ones it cannot hold either go on to the heavy tier.  Seed mode 0
         // keeps the reference's DFS for every read and skips it.
         const float tb0 = wall_ms();
         CK(ctx->ovf3.ensure(nrp * sizeof(idx_t)));
         CK(cudaMemsetAsync(ctr + 7, 0, sizeof(unsigned long long), ctx->st));
-        CK(pq::search_block(A, O, ctx->ovf_list.as<idx_t>(), reinterpret_cast<const unsigned*>(ctr + 2), ovf,
-                            ctx->ovf3.as<idx_t>(), reinterpret_cast<unsigned*>(ctr + 7), ctx->st));
+        const size_t bbytes = pq::block_scratch_bytes(ctx->L, ctx->t, ovf);
+        CK(ctx->block_scratch.ensure(bbytes));
+        CK(pq::search_block(A, O, ctx->ovf_list.as<idx_t>(), ovf, ctx->block_scratch.p, bbytes, ctx->ovf3.as<idx_t>(),
+                            reinterpret_cast<unsigned*>(ctr + 7), ctx->st));
         unsigned long long h7 = 0;
         CK(cudaMemcpyAsync(&h7, ctr + 7, sizeof h7, cudaMemcpyDeviceToHost, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
         const unsigned left = unsigned(h7 & 0xffffffffu);
-        if (pq::block_tier_holds(ctx->L, ctx->t)) {
-            ctx->block_reads = ovf - left;
-            ovf = left;
-            ovf_src = ctx->ovf3.as<idx_t>();
-            ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 7);
+        ctx->block_reads = ovf - left;
+        ovf = left;
+        ovf_src = ctx->ovf3.as<idx_t>();
+        ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 7);
+        if (ovf) {
+            // the same tier with its candidate arrays in global memory, for sides of up to
+            // 32768 candidates
+            const int gb = pq::block_global_blocks(ovf);
+            const size_t gbytes = pq::block_global_bytes(ctx->L, ctx->t, gb);
+            CK(ctx->block_scratch.ensure(gbytes));
+            CK(ctx->ovf4.ensure(nrp * sizeof(idx_t)));
+            CK(cudaMemsetAsync(ctr + 8, 0, sizeof(unsigned long long), ctx->st));
+            CK(pq::search_block_global(A, O, ovf_src, ovf_cnt, ovf, gb, ctx->block_scratch.p, gbytes,
+                                       ctx->ovf4.as<idx_t>(), reinterpret_cast<unsigned*>(ctr + 8), ctx->st));
+            unsigned long long h8 = 0;
+            CK(cudaMemcpyAsync(&h8, ctr + 8, sizeof h8, cudaMemcpyDeviceToHost, ctx->st));
+            CK(cudaStreamSynchronize(ctx->st));
+            const unsigned left2 = unsigned(h8 & 0xffffffffu);
+            ctx->block_reads += ovf - left2;
+            ovf = left2;
+            ovf_src = ctx->ovf4.as<idx_t>();
+            ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 8);
+            // reads that found the edge pool full: grow it past everything reserved so far
+            // (twice that covers every failed reservation made again) and run them once more
+            unsigned long long reserved = 0;
             if (ovf) {
-                // the same tier with its candidate arrays in global memory, for sides of up to
-                // 32768 candidates
-                const int gb = pq::block_global_blocks(ovf);
-                const size_t gbytes = pq::block_global_bytes(ctx->L, ctx->t, gb);
-                CK(ctx->block_scratch.ensure(gbytes));
-                CK(ctx->ovf4.ensure(nrp * sizeof(idx_t)));
-                CK(cudaMemsetAsync(ctr + 8, 0, sizeof(unsigned long long), ctx->st));
-                CK(pq::search_block_global(A, O, ovf_src, ovf_cnt, ovf, gb, ctx->block_scratch.p, gbytes,
-                                           ctx->ovf4.as<idx_t>(), reinterpret_cast<unsigned*>(ctr + 8), ctx->st));
-                unsigned long long h8 = 0;
-                CK(cudaMemcpyAsync(&h8, ctr + 8, sizeof h8, cudaMemcpyDeviceToHost, ctx->st));
+                CK(cudaMemcpyAsync(&reserved, ctr + 0, sizeof reserved, cudaMemcpyDeviceToHost, ctx->st));
                 CK(cudaStreamSynchronize(ctx->st));
-                const unsigned left2 = unsigned(h8 & 0xffffffffu);
-                ctx->block_reads += ovf - left2;
-                ovf = left2;
-                ovf_src = ctx->ovf4.as<idx_t>();
-                ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 8);
-                // reads that found the edge pool full: grow it past everything reserved so far
-                // (twice that covers every failed reservation made again) and run them once more
-                unsigned long long reserved = 0;
-                if (ovf) {
-                    CK(cudaMemcpyAsync(&reserved, ctr + 0, sizeof reserved, cudaMemcpyDeviceToHost, ctx->st));
-                    CK(cudaStreamSynchronize(ctx->st));
-                }
-                if (ovf && reserved > O.e_cap) {
-                    const size_t need = size_t(2 * reserved + 4096), keep = O.e_cap;
-                    CK(ctx->e_dest.grow(need * sizeof(idx_t), keep * sizeof(idx_t), ctx->st));
-                    CK(ctx->e_trans.grow(need * 4, keep * 4, ctx->st));
-                    CK(ctx->e_len.grow(need * 2, keep * 2, ctx->st));
-                    CK(ctx->e_type.grow(need, keep, ctx->st));
-                    O.e_dest = ctx->e_dest.as<idx_t>();
-                    O.e_trans = ctx->e_trans.as<int32_t>();
-                    O.e_len = ctx->e_len.as<uint16_t>();
-                    O.e_type = ctx->e_type.as<uint8_t>();
-                    O.e_cap = need;
-                    const int gb2 = pq::block_global_blocks(ovf);
-                    const size_t gbytes2 = pq::block_global_bytes(ctx->L, ctx->t, gb2);
-                    CK(ctx->block_scratch.ensure(gbytes2));
-                    CK(cudaMemsetAsync(ctr + 7, 0, sizeof(unsigned long long), ctx->st));
-                    CK(pq::search_block_global(A, O, ovf_src, ovf_cnt, ovf, gb2, ctx->block_scratch.p, gbytes2,
-                                               ctx->ovf3.as<idx_t>(), reinterpret_cast<unsigned*>(ctr + 7), ctx->st));
-                    unsigned long long h7b = 0;
-                    CK(cudaMemcpyAsync(&h7b, ctr + 7, sizeof h7b, cudaMemcpyDeviceToHost, ctx->st));
-                    CK(cudaStreamSynchronize(ctx->st));
-                    const unsigned left3 = unsigned(h7b & 0xffffffffu);
-                    ctx->block_reads += ovf - left3;
-                    ovf = left3;
-                    ovf_src = ctx->ovf3.as<idx_t>();
-                    ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 7);
-                }
+            }
+            if (ovf && reserved > O.e_cap) {
+                const size_t need = size_t(2 * reserved + 4096), keep = O.e_cap;
+                CK(ctx->e_dest.grow(need * sizeof(idx_t), keep * sizeof(idx_t), ctx->st));
+                CK(ctx->e_trans.grow(need * 4, keep * 4, ctx->st));
+                CK(ctx->e_len.grow(need * 2, keep * 2, ctx->st));
+                CK(ctx->e_type.grow(need, keep, ctx->st));
+                O.e_dest = ctx->e_dest.as<idx_t>();
+                O.e_trans = ctx->e_trans.as<int32_t>();
+                O.e_len = ctx->e_len.as<uint16_t>();
+                O.e_type = ctx->e_type.as<uint8_t>();
+                O.e_cap = need;
+                const int gb2 = pq::block_global_blocks(ovf);
+                const size_t gbytes2 = pq::block_global_bytes(ctx->L, ctx->t, gb2);
+                CK(ctx->block_scratch.ensure(gbytes2));
+                CK(cudaMemsetAsync(ctr + 7, 0, sizeof(unsigned long long), ctx->st));
+                CK(pq::search_block_global(A, O, ovf_src, ovf_cnt, ovf, gb2, ctx->block_scratch.p, gbytes2,
+                                           ctx->ovf3.as<idx_t>(), reinterpret_cast<unsigned*>(ctr + 7), ctx->st));
+                unsigned long long h7b = 0;
+                CK(cudaMemcpyAsync(&h7b, ctr + 7, sizeof h7b, cudaMemcpyDeviceToHost, ctx->st));
+                CK(cudaStreamSynchronize(ctx->st));
+                const unsigned left3 = unsigned(h7b & 0xffffffffu);
+                ctx->block_reads += ovf - left3;
+                ovf = left3;
+                ovf_src = ctx->ovf3.as<idx_t>();
+                ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 7);
             }
         }
         ctx->ms_block = wall_ms() - tb0;

@@ -1919,34 +1919,415 @@ size_t lean_scratch_bytes(int L, int t, int lean_blocks, int fast_blocks, int eb
 // ------------------------------------------------------------------------------ block tier
 //
 // Reads the fast tier hands over are the ones with many candidates -- low-complexity sequence,
-// where a read's side can have thousands.  The block tier gives each such read one CTA: two
-// threads walk the two sides (chain_pair, from exact k-mer seeds, with the reference's depths),
-// the CTA expands every candidate group into its candidates (read id from the suffix array,
-// continuation from the packed text), and reduces each side as reduce_gathered does, with the
-// m x m ordered pairs of candidates spread over the CTA's threads: candidate c is covered when
-// another candidate's continuation is a proper prefix of its own, trans(c) counts the
-// continuations that start with c's, first_same(c) tells whether a candidate of the side's first
-// kind has exactly c's continuation.  The emitted candidates are then ranked in DFS order
-// (continuation, read id) by counting, again over pairs.  In this variant everything lives in
-// shared memory; a side with more candidates than fit goes to the variant with its arrays in
-// global memory, which reduces by sorting (block_sorted_side), and only a side beyond that one's
-// capacity goes on to the heavy and wide tiers.
+// where a read's side can have thousands.  One thread per (read, side) walks the chains of all of
+// them first (k_block_walk: chain_pair, from exact k-mer seeds, with the reference's depths), so
+// that the dependent steps of thousands of walks overlap.  Then one CTA takes each read: every
+// candidate group is expanded into its candidates (read id from the suffix array, continuation from
+// the packed text) and each side is reduced in shared memory by sorting (k_search_block).  A side
+// with more candidates than the larger of its two sizes goes to the variant with everything in
+// global memory (k_search_block_global), and only one beyond that variant's capacity to the heavy
+// and wide tiers.
+
+// The candidate groups of one (read, side): n[q] of kind q at grp[q * M ..], their candidates' number
+// (0xffffffff: more than any block kernel holds) and the overlaps counted.
+struct BlockSide {
+    int n[2];
+    int32_t olp;
+    unsigned m;
+};
+constexpr int kWalkThreads = 64;
+
+__global__ void __launch_bounds__(kWalkThreads) k_block_walk(SearchArgs A, SearchOut O, const idx_t* list, unsigned count,
+                                                             Cand* groups, BlockSide* sides) {
+    extern __shared__ uint32_t s_reads[];
+    const unsigned i = (blockIdx.x * kWalkThreads + threadIdx.x);
+    Tally probes;
+    if (i < 2 * count) {
+        const int side = int(i & 1u), M = A.L - A.t;
+        load_read(A, list[i >> 1], s_reads + threadIdx.x, kWalkThreads, probes);
+        const ReadView rd{s_reads + threadIdx.x, kWalkThreads};
+        Cand* g = groups + size_t(i) * size_t(2 * M);
+        BlockSide b{};
+        chain_pair(A, A.fm, rd, side ? PQ_FB : PQ_BF, side ? PQ_FF : PQ_BB, b.n, b.olp, probes, SlotsStack{g, M});
+        unsigned long long m = 0;               // group sizes are index-wide: summed in 64 bits, stopped past 2^31
+        for (int q = 0; q < 2; ++q)
+            for (int j = 0; j < b.n[q] && m < (1ull << 31); ++j) {
+                const Cand& c = g[q * M + j];
+                m += (unsigned long long)(c.uu - c.ll) + 1ull;
+            }
+        b.m = m < (1ull << 31) ? unsigned(m) : 0xffffffffu;
+        sides[i] = b;
+    }
+    add_probes(O, probes);
+}
+
+// What k_search_block keeps per candidate in its CTA's region of global memory (L2-resident), each
+// an array of CAP: continuation words, read id, (overlap, kind) and, of either side, the emitted
+// edges.
+__host__ __device__ constexpr size_t block_region_bytes(int cap, int nw) {
+    return size_t(cap) * (size_t(nw) * 8 + sizeof(idx_t) + 4 + 2 * (sizeof(idx_t) + 4 + 4));
+}
+// and in shared memory: the sort key (the walk's record after the sort), the order, and the group
+// prefix sums
+constexpr size_t block_smem_bytes(int cap) { return size_t(cap) * 10 + (2 * 256 + 1 + 31) * 4; }
+constexpr int kBlockSmall = 4096, kBlockMid = 8192, kBlockLarge = 16384;    // candidates a side, by 256, 512 and 512 threads
+
+// One read a CTA.  Each side's candidates are ordered by (continuation words, zero past the end;
+// length; read id) with a bitonic sort in shared memory.  In low-complexity sequence most
+// continuations start with the same long run, so a key of their first words would seldom tell them
+// apart: the key is relative to one of them, the pivot p.  With l the common prefix of a continuation
+// and p, its highest 10 bits are l where the continuation ends there or is smaller than p, 1023 - l
+// where it is larger, and the next 53 the 26 1/2 bases from l on: continuations of one side and one l
+// share their first l bases, and of two that leave p at different places the one that leaves it later
+// is nearer to p.  (One that ends at l is a prefix of every other that shares more than l bases with p
+// and sorts before it: its padding is the smallest base.)  The lowest bit is clear in a prefix of
+// p, which sorts before what goes on with the smallest base; equal keys without it are equal strings,
+// other equal keys are compared by all words.
+//
+// In that order a continuation is followed by its extensions: its class, found for all places at once
+// by a prefix scan (below).  The candidates equal to their class's shortest are emitted, in DFS order.
+//
+// Bound by the sort's instructions and its barriers.  The 3,645 run reads of the 200 Mbp workload at
+// 1/100 genome (150 bases, up to 6.7 thousand candidates of a kind) took 58 ms by pair tests in shared
+// memory and radix passes in global memory; 19 with the first words as keys; 16 with keys relative to
+// a pivot and one warp walking from class to class; 6 with the classes found by the scan.
+template <int CAP, int T>
+__global__ void __launch_bounds__(T) k_search_block(SearchArgs A, SearchOut O, const idx_t* list, unsigned count, const Cand* groups,
+                                                    const BlockSide* sides, unsigned* next, unsigned char* region,
+                                                    unsigned lowest, unsigned highest, idx_t* next_list, unsigned* next_count) {
+    extern __shared__ __align__(16) unsigned char smem_dyn[];
+    uint64_t* const key = reinterpret_cast<uint64_t*>(smem_dyn);
+    uint16_t* const ord = reinterpret_cast<uint16_t*>(key + CAP);
+    unsigned* const pref = reinterpret_cast<unsigned*>(ord + CAP);
+    __shared__ unsigned s_item, s_sum[T / 32];
+    __shared__ int s_ne[2], s_pivot;
+    __shared__ unsigned long long s_base;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    constexpr int NW = T / 32;
+    const int L = A.L, M = L - A.t, nw = (M + 31) / 32;
+    unsigned char* at = region + size_t(blockIdx.x) * block_region_bytes(CAP, nw);
+    uint64_t* const cw = reinterpret_cast<uint64_t*>(at); at += size_t(CAP) * nw * 8;
+    idx_t* const cid = reinterpret_cast<idx_t*>(at); at += size_t(CAP) * sizeof(idx_t);
+    idx_t* const e_id = reinterpret_cast<idx_t*>(at); at += size_t(2 * CAP) * sizeof(idx_t);
+    uint32_t* const cmeta = reinterpret_cast<uint32_t*>(at); at += size_t(CAP) * 4;
+    uint32_t* const e_meta = reinterpret_cast<uint32_t*>(at); at += size_t(2 * CAP) * 4;
+    int32_t* const e_trans = reinterpret_cast<int32_t*>(at);
+    Tally probes;
+    while (true) {
+        if (tid == 0) s_item = atomicAdd(next, 1u);
+        __syncthreads();
+        const unsigned item = s_item;
+        if (item >= count) break;
+        const BlockSide sb[2] = {sides[2 * item], sides[2 * item + 1]};
+        const unsigned most = max(sb[0].olp ? sb[0].m : 0u, sb[1].olp ? sb[1].m : 0u);
+        __syncthreads();
+        if (most < lowest || most > highest) continue;          // the other size's, or the next tier's
+        const idx_t self = list[item];
+        if (tid < 2) s_ne[tid] = 0;
+        for (int side = 0; side < 2; ++side) {
+            if (sb[side].olp == 0) continue;                    // src/string_graph.c:824, 828
+            const int n0 = sb[side].n[0], ng = n0 + sb[side].n[1], m = int(sb[side].m);
+            const Cand* g = groups + (size_t(2 * item) + side) * size_t(2 * M);
+            // exclusive prefix of the group sizes, two groups a thread (ng <= 2 M <= 512)
+            {
+                unsigned v[2] = {0, 0};
+                #pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int i = 2 * tid + q;
+                    if (i < ng) {
+                        const Cand& c = g[i < n0 ? i : M + (i - n0)];
+                        v[q] = unsigned(c.uu - c.ll) + 1u;
+                    }
+                }
+                unsigned x = v[0] + v[1];
+                #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (lane == 31) s_sum[wid] = x;
+                __syncthreads();
+                unsigned run = x - v[0] - v[1];
+                for (int w = 0; w < wid; ++w) run += s_sum[w];
+                if (2 * tid <= ng) pref[2 * tid] = run;
+                if (2 * tid + 1 <= ng) pref[2 * tid + 1] = run + v[0];
+                __syncthreads();
+            }
+            // every candidate's read id and continuation
+            for (int i = tid; i < m; i += T) {
+                int lo = 0, hi = ng - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (pref[mid] <= unsigned(i)) lo = mid;
+                    else hi = mid - 1;
+                }
+                const Cand& c = g[lo < n0 ? lo : M + (lo - n0)];
+                const idx_t row = c.ll + idx_t(unsigned(i) - pref[lo]);
+                const int type = int(c.type), d = int(c.len);
+                const idx_t rp = read_of(__ldg(A.fm[cand_index(type)].sa + row), A.dl);
+                for (int w = 0; w < nw; ++w) {
+                    const uint64_t x = 32 * w < L - d ? continuation_word(A, type, rp, d, w) : 0;
+                    cw[size_t(w) * CAP + i] = x;
+                }
+                probes.add(2, 1 + base_sectors(size_t(rp) * L + size_t(d), L - d));
+                cid[i] = rp;
+                cmeta[i] = pack_meta(d, type);
+                ord[i] = uint16_t(i);
+            }
+            __syncthreads();
+            auto length = [&](int i) { return L - meta_len(cmeta[i]); };
+            // common prefix of candidates i and j
+            auto shared_prefix = [&](int i, int j) {
+                const int n = min(length(i), length(j));
+                for (int w = 0; 32 * w < n; ++w) {
+                    const uint64_t z = cw[size_t(w) * CAP + i] ^ cw[size_t(w) * CAP + j];
+                    if (z) return min(n, 32 * w + (__clzll((long long)z) >> 1));
+                }
+                return n;
+            };
+            // the pivot: of 32 candidates, the one that shares most with 8 of them
+            if (wid == 0) {
+                const int mine = int((unsigned long long)lane * unsigned(m) >> 5);
+                unsigned sum = 0;
+                for (int j = 2; j < 32; j += 4) sum += unsigned(shared_prefix(mine, int((unsigned long long)j * unsigned(m) >> 5)));
+                const unsigned best = __reduce_max_sync(0xffffffffu, (sum << 5) | unsigned(lane));
+                if (lane == 0) s_pivot = int((unsigned long long)(best & 31u) * unsigned(m) >> 5);
+            }
+            __syncthreads();
+            const int pivot = s_pivot, lp = length(pivot);
+            for (int i = tid; i < m; i += T) {
+                const int n = length(i), l = shared_prefix(i, pivot);
+                const int w = l >> 5, sh = 2 * (l & 31);
+                const uint64_t x0 = w < nw ? cw[size_t(w) * CAP + i] : 0;
+                const uint64_t x1 = w + 1 < nw ? cw[size_t(w + 1) * CAP + i] : 0;
+                const uint64_t rest = sh ? (x0 << sh) | (x1 >> (64 - sh)) : x0;     // zero past the end
+                bool larger = false;
+                if (l < n) larger = l == lp || rest >> 62 > ((cw[size_t(w) * CAP + pivot] << sh) >> 62);
+                key[i] = (uint64_t(unsigned(larger ? 1023 - l : l)) << 54) | ((rest >> 11) << 1) | uint64_t(l != n);
+            }
+            __syncthreads();
+            // a before b, whose keys are equal
+            auto before = [&](int a, int b, uint64_t k) {
+                if (k & 1) {
+                    for (int w = 0; w < nw; ++w) {
+                        const uint64_t x = cw[size_t(w) * CAP + a], y = cw[size_t(w) * CAP + b];
+                        if (x != y) return x < y;
+                    }
+                    const int la = length(a), lb = length(b);
+                    if (la != lb) return la < lb;
+                }
+                return cid[a] < cid[b];
+            };
+            auto exchange = [&](int a, int b) {
+                if (b >= m) return;
+                const uint64_t x = key[a], y = key[b];
+                if (x < y) return;
+                const int p = ord[a], q = ord[b];
+                if (x == y && before(p, q, x)) return;
+                key[a] = y;
+                key[b] = x;
+                ord[a] = uint16_t(q);
+                ord[b] = uint16_t(p);
+            };
+            for (int k = 2; k < 2 * m; k <<= 1) {
+                const int half = k >> 1, pairs = (m + k - 1) / k * half;
+                for (int i = tid; i < pairs; i += T) {          // the mirrored step: every comparator points up
+                    const int q = i / half, o = i - q * half;
+                    exchange(q * k + o, q * k + k - 1 - o);
+                }
+                __syncthreads();
+                for (int j = half >> 1; j > 0; j >>= 1) {
+                    for (int i = tid; i < pairs; i += T) {
+                        const int a = ((i & ~(j - 1)) << 1) | (i & (j - 1));
+                        exchange(a, a + j);
+                    }
+                    __syncthreads();
+                }
+            }
+            // per place of the order, in the key's four 16-bit fields: common prefix with the place
+            // before (later the class), length, flags, and (by class) the class's first place
+            const int first_kind = side ? PQ_FB : PQ_BF;
+            constexpr unsigned kSelf = 1, kFirst = 2, kEqual = 4, kFirstSame = 8;
+            ushort4* const at4 = reinterpret_cast<ushort4*>(key);
+            for (int k = tid; k < m; k += T) {
+                const int c = ord[k];
+                const int lcp = k > 0 ? shared_prefix(int(ord[k - 1]), c) : 0;
+                at4[k] = make_ushort4(uint16_t(lcp), uint16_t(length(c)),
+                                      uint16_t((cid[c] == self ? kSelf : 0u) | (meta_type(cmeta[c]) == first_kind ? kFirst : 0u)), 0);
+            }
+            // The shortest candidate that is a prefix of place k's, H(k) its length, starts k's class:
+            // H(k) = H(k - 1) where that is at most k's common prefix with k - 1, else k's own length
+            // (a longer prefix of k - 1 than H(k - 1) cannot reach k either).  Such steps compose,
+            // (a1, b1) then (a2, b2) to (min(a1, a2), b1 <= a2 ? b1 : b2), so H is a prefix scan.
+            const int rows = (m + 32 * NW - 1) / (32 * NW), k0 = wid * rows * 32;
+            auto then = [](unsigned f, unsigned g) {            // a << 16 | b
+                const unsigned a1 = f >> 16, b1 = f & 0xffffu, a2 = g >> 16, b2 = g & 0xffffu;
+                return (min(a1, a2) << 16) | (b1 <= a2 ? b1 : b2);
+            };
+            auto step = [&](int k) {
+                if (k >= m) return 0xffffffffu;                 // nothing
+                const ushort4 v = at4[k];
+                return (unsigned(v.x) << 16) | v.y;
+            };
+            __syncthreads();
+            {
+                unsigned f = 0xffffffffu;
+                for (int q = 0; q < rows; ++q) {
+                    unsigned x = step(k0 + 32 * q + lane);
+                    #pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const unsigned y = __shfl_down_sync(0xffffffffu, x, o);
+                        if (lane + o < 32) x = then(x, y);      // lane 0: the row's steps in order
+                    }
+                    f = then(f, __shfl_sync(0xffffffffu, x, 0));
+                }
+                if (lane == 0) s_sum[wid] = f;
+            }
+            __syncthreads();
+            {
+                unsigned f = 0xffffffffu;
+                for (int w = 0; w < wid; ++w) f = then(f, s_sum[w]);
+                int heads = 0;
+                for (int q = 0; q < rows; ++q) {
+                    const int k = k0 + 32 * q + lane;
+                    unsigned x = step(k);
+                    const unsigned lcp = x >> 16, len = x & 0xffffu;
+                    #pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+                        if (lane >= o) x = then(y, x);
+                    }
+                    x = then(f, x);
+                    const unsigned up = __shfl_up_sync(0xffffffffu, x, 1);
+                    const bool head = k < m && ((lane ? up : f) & 0xffffu) > lcp;
+                    const bool equal = k < m && len == (x & 0xffffu);
+                    const unsigned hb = __ballot_sync(0xffffffffu, head);
+                    if (k < m) {                                // class within the warp's places, for now
+                        ushort4 v = at4[k];
+                        v.x = uint16_t(heads + __popc(hb & (0xffffffffu >> (31 - lane))));
+                        v.z = uint16_t(v.z | (equal ? kEqual : 0u) | (head ? 0x8000u : 0u));
+                        at4[k] = v;
+                    }
+                    heads += __popc(hb);
+                    f = __shfl_sync(0xffffffffu, x, 31);
+                }
+                __syncthreads();
+                if (lane == 0) s_sum[wid] = unsigned(heads);
+            }
+            __syncthreads();
+            int classes = 0;
+            {
+                int before_me = 0;
+                for (int w = 0; w < NW; ++w) {
+                    before_me += w < wid ? int(s_sum[w]) : 0;
+                    classes += int(s_sum[w]);
+                }
+                for (int q = 0; q < rows; ++q) {
+                    const int k = k0 + 32 * q + lane;
+                    if (k >= m) break;
+                    const int c = before_me + int(at4[k].x) - 1;
+                    at4[k].x = uint16_t(c);
+                    if (at4[k].z & 0x8000u) at4[c].w = uint16_t(k);
+                }
+            }
+            __syncthreads();
+            // a class with a first-kind candidate of exactly its continuation
+            for (int k = tid; k < m; k += T) {
+                const ushort4 v = at4[k];
+                if ((v.z & (kEqual | kFirst)) == (kEqual | kFirst))
+                    atomicOr(reinterpret_cast<unsigned*>(key + v.x) + 1, kFirstSame);
+            }
+            __syncthreads();
+            auto emitted = [&](int k) {
+                if (k >= m) return false;
+                const ushort4 v = at4[k];
+                return (v.z & kEqual) && !(v.z & kSelf) && ((v.z & kFirst) || !(at4[v.x].z & kFirstSame));
+            };
+            {
+                int n = 0;
+                for (int q = 0; q < rows; ++q) n += __popc(__ballot_sync(0xffffffffu, emitted(k0 + 32 * q + lane)));
+                if (lane == 0) s_sum[wid] = unsigned(n);
+            }
+            __syncthreads();
+            {
+                const int ne0 = side ? s_ne[0] : 0;             // the F side's edges follow the B side's
+                int ne = ne0, all = 0;
+                for (int w = 0; w < NW; ++w) {
+                    ne += w < wid ? int(s_sum[w]) : 0;
+                    all += int(s_sum[w]);
+                }
+                for (int q = 0; q < rows; ++q) {
+                    const int k = k0 + 32 * q + lane;
+                    const bool em = emitted(k);
+                    const unsigned e = __ballot_sync(0xffffffffu, em);
+                    if (em) {
+                        const int z = ne + __popc(e & ((1u << lane) - 1u)), c = ord[k], cls = at4[k].x;
+                        e_id[z] = cid[c];
+                        e_meta[z] = cmeta[c];
+                        e_trans[z] = (cls + 1 < classes ? int(at4[cls + 1].w) : m) - int(at4[cls].w);
+                    }
+                    ne += __popc(e);
+                }
+                if (tid == 0) s_ne[side] = all;
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+        const int nb = s_ne[0], nf = s_ne[1], ne = nb + nf;
+        if (tid == 0) {
+            s_base = ne ? atomicAdd(O.e_count, (unsigned long long)ne) : 0ull;
+            if (s_base + ne > O.e_cap) {         // edge pool full: the host grows it, runs the read again
+                O.status[self] = OVF_POOL;
+                const unsigned k = atomicAdd(next_count, 1u);
+                next_list[k] = self;
+            } else {
+                O.status[self] = OVF_NONE;
+                O.num_B[self] = uint16_t(nb);
+                O.num_F[self] = uint16_t(nf);
+                O.olp_B[self] = sb[0].olp;
+                O.olp_F[self] = sb[1].olp;
+                O.edge_src[self] = s_base;
+            }
+        }
+        __syncthreads();
+        const unsigned long long base = s_base;
+        if (base + ne <= O.e_cap) {
+            for (int e = tid; e < ne; e += T) {
+                const uint32_t mt = e_meta[e];
+                O.e_dest[base + e] = e_id[e];
+                O.e_trans[base + e] = e_trans[e];
+                O.e_len[base + e] = uint16_t(meta_len(mt));
+                O.e_type[base + e] = uint8_t(meta_type(mt));
+            }
+        }
+        __syncthreads();
+    }
+    add_probes(O, probes);
+}
+
+// reads with a side beyond `highest` candidates: to the next list
+__global__ void k_block_beyond(const idx_t* list, unsigned count, const BlockSide* sides, unsigned highest, idx_t* next_list,
+                               unsigned* next_count) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const BlockSide a = sides[2 * i], b = sides[2 * i + 1];
+    if (max(a.olp ? a.m : 0u, b.olp ? b.m : 0u) > highest) next_list[atomicAdd(next_count, 1u)] = list[i];
+}
 
 constexpr int kBlockThreads = 256;
-constexpr size_t kBlockSmemBudget = 200 * 1024;     // dynamic shared memory of one block-tier CTA
 
-struct BlockSmem {      // the block tier's dynamic shared memory (offsets in bytes)
+struct BlockSmem {      // a CTA's region of the global variant (offsets in bytes)
     size_t words, ids, metas, cnts, elist, e_ids, e_metas, e_trans, groups, prefs, read, bytes;
-    size_t perm0, perm1, info;      // the sorted reduction's order and walk arrays (global variant)
+    size_t perm0, perm1, info;      // the sorted reduction's order and walk arrays
     int cap;            // candidates a side (and B-side edges kept while the F side is reduced)
     int nw;             // continuation words per candidate
 };
 
-// bytes a candidate takes (continuation words, read id, meta, counter, emitted list, B-side edge;
-// with `sorted`, two order arrays and the walk's array) and the fixed part (both sides' candidate
+// bytes a candidate takes (continuation words, read id, meta, counter, emitted list, B-side edge, two
+// order arrays and the walk's array) and the fixed part (both sides' candidate
 // groups, their prefix sums, the read)
-size_t block_per_cand(int L, int t, bool sorted = false) {
-    return size_t((L - t + 31) / 32) * 8 + sizeof(idx_t) + 4 + 4 + 4 + sizeof(idx_t) + 4 + 4 + (sorted ? 12 : 0);
+size_t block_per_cand(int L, int t) {
+    return size_t((L - t + 31) / 32) * 8 + sizeof(idx_t) + 4 + 4 + 4 + sizeof(idx_t) + 4 + 4 + 12;
 }
 size_t block_fixed(int L, int t) {
     const int M = L - t;
@@ -1954,14 +2335,14 @@ size_t block_fixed(int L, int t) {
            size_t((L + 15) / 16) * sizeof(uint32_t) + 16 * 16;
 }
 
-BlockSmem block_smem_layout(int L, int t, size_t budget, bool sorted = false) {
+BlockSmem block_smem_layout(int L, int t, size_t budget) {
     BlockSmem b{};
     const int M = L - t;
     b.nw = (M + 31) / 32;
     const size_t groups = size_t(2) * size_t(2 * M) * sizeof(Cand);
     const size_t prefs = size_t(2 * M + 1) * sizeof(unsigned);
     const size_t read = size_t((L + 15) / 16) * sizeof(uint32_t);
-    const size_t per = block_per_cand(L, t, sorted);
+    const size_t per = block_per_cand(L, t);
     const size_t fixed = block_fixed(L, t);
     int cap = budget > fixed ? int(std::min<size_t>((budget - fixed) / per, 65535)) : 0;
     cap &= ~31;
@@ -1983,33 +2364,11 @@ BlockSmem block_smem_layout(int L, int t, size_t budget, bool sorted = false) {
     b.groups = take(groups);
     b.prefs = take(prefs);
     b.read = take(read);
-    b.perm0 = b.perm1 = b.info = 0;
-    if (sorted) {
-        b.perm0 = take(size_t(cap) * 4);
-        b.perm1 = take(size_t(cap) * 4);
-        b.info = take(size_t(cap) * 4);
-    }
+    b.perm0 = take(size_t(cap) * 4);
+    b.perm1 = take(size_t(cap) * 4);
+    b.info = take(size_t(cap) * 4);
     b.bytes = o;
     return b;
-}
-
-// the first n bases of continuations a and b (word k of candidate i at w[k * cap + i]) agree
-__device__ __forceinline__ bool block_same_prefix(const uint64_t* w, int cap, int a, int b, int n) {
-    for (int k = 0; n > 0; ++k, n -= 32) {
-        const uint64_t x = w[size_t(k) * cap + a] ^ w[size_t(k) * cap + b];
-        if (n < 32) return (x & top_mask(n)) == 0;
-        if (x) return false;
-    }
-    return true;
-}
-// order of two continuations that are equal or not prefixes of one another
-__device__ __forceinline__ int block_cmp(const uint64_t* w, int cap, int nw, int a, int la, int b, int lb) {
-    const int n = la < lb ? la : lb;
-    for (int k = 0; k < nw && 32 * k < n; ++k) {
-        const uint64_t x = w[size_t(k) * cap + a], y = w[size_t(k) * cap + b];
-        if (x != y) return x < y ? -1 : 1;
-    }
-    return la == lb ? 0 : (la < lb ? -1 : 1);
 }
 
 constexpr int kBlockMaxWords = 8;       // continuation words a candidate (L - t <= 256)
@@ -2186,21 +2545,19 @@ __device__ int block_sorted_side(int m, int L, int nw, int cap, const uint64_t* 
     return ne;
 }
 
-// kGlobal: the candidate arrays live in a per-CTA region of `scratch` (global memory, cached in
-// L1/L2) instead of shared memory, for sides with more candidates than shared memory holds; each
-// side is then reduced by sorting (block_sorted_side) instead of by pair tests.
-template <bool kGlobal>
-__global__ void __launch_bounds__(kBlockThreads) k_search_block(SearchArgs A, SearchOut O, const idx_t* list,
-                                                                const unsigned* list_count, BlockSmem lay,
-                                                                idx_t* next_list, unsigned* next_count,
-                                                                unsigned char* scratch) {
+// The block tier with its candidate arrays in a per-CTA region of `scratch` (global memory, cached in
+// L1/L2), for sides of up to kBlockGlobalCap candidates; each side is reduced by block_sorted_side.
+__global__ void __launch_bounds__(kBlockThreads) k_search_block_global(SearchArgs A, SearchOut O, const idx_t* list,
+                                                                       const unsigned* list_count, BlockSmem lay,
+                                                                       idx_t* next_list, unsigned* next_count,
+                                                                       unsigned char* scratch) {
     extern __shared__ __align__(16) unsigned char smem_dyn[];
-    unsigned char* smem = kGlobal ? scratch + size_t(blockIdx.x) * lay.bytes : smem_dyn;
+    unsigned char* smem = scratch + size_t(blockIdx.x) * lay.bytes;
     uint64_t* cw = reinterpret_cast<uint64_t*>(smem + lay.words);
     uint32_t* perm0 = reinterpret_cast<uint32_t*>(smem + lay.perm0);
     uint32_t* perm1 = reinterpret_cast<uint32_t*>(smem + lay.perm1);
     uint32_t* sinfo = reinterpret_cast<uint32_t*>(smem + lay.info);
-    unsigned* scnt = reinterpret_cast<unsigned*>(smem_dyn);              // global variant: 16 x 256 counts, padded
+    unsigned* scnt = reinterpret_cast<unsigned*>(smem_dyn);              // 16 x 256 counts, padded
     unsigned* smisc = scnt + 16 * kBlockThreads + 16 * kBlockThreads / 16;
     idx_t* cid = reinterpret_cast<idx_t*>(smem + lay.ids);
     uint32_t* cmeta = reinterpret_cast<uint32_t*>(smem + lay.metas);
@@ -2214,10 +2571,9 @@ __global__ void __launch_bounds__(kBlockThreads) k_search_block(SearchArgs A, Se
     uint32_t* rdw = reinterpret_cast<uint32_t*>(smem + lay.read);
     __shared__ int s_n[2][2];
     __shared__ int32_t s_olp[2];
-    __shared__ int s_ok, s_ne, s_cnt[2];
-    __shared__ unsigned s_wsum[kBlockThreads / 32];
+    __shared__ int s_ok, s_cnt[2];
     __shared__ unsigned long long s_base;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int tid = threadIdx.x;
     const int L = A.L, M = L - A.t, cap = lay.cap, nw = lay.nw;
     const unsigned count = *list_count;
     Tally probes;
@@ -2297,74 +2653,9 @@ __global__ void __launch_bounds__(kBlockThreads) k_search_block(SearchArgs A, Se
             }
             __syncthreads();
             const int first_kind = side ? PQ_FB : PQ_BF;
-            if constexpr (kGlobal) {
-                const int nsorted = block_sorted_side(m, L, nw, cap, cw, cid, cmeta, perm0, perm1, sinfo, scnt, smisc,
-                                                      first_kind, self, side, e_id, e_meta, e_trans, elist, ccnt);
-                if (tid == 0) s_cnt[side] = nsorted;
-                __syncthreads();
-                continue;
-            }
-            // all pairs: covered (bit 0), first_same (bit 1), trans (bits 2..)
-            for (int c = tid; c < m; c += kBlockThreads) {
-                const int lc = L - meta_len(cmeta[c]);
-                uint32_t v = 0;
-                for (int x = 0; x < m; ++x) {
-                    const uint32_t mx = cmeta[x];
-                    const int lx = L - meta_len(mx);
-                    if (!block_same_prefix(cw, cap, c, x, lx < lc ? lx : lc)) continue;
-                    if (lx < lc) {
-                        v |= 1u;
-                        break;
-                    }
-                    v += 4u;
-                    if (lx == lc && meta_type(mx) == first_kind) v |= 2u;
-                }
-                ccnt[c] = v;
-            }
-            if (tid == 0) s_ne = 0;
-            __syncthreads();
-            // the emitted candidates, listed (index | trans << 16) in candidate order
-            for (int c0 = 0; c0 < m; c0 += kBlockThreads) {
-                const int c = c0 + tid;
-                bool em = false;
-                if (c < m) {
-                    const uint32_t v = ccnt[c];
-                    em = !(v & 1u) && cid[c] != self && (meta_type(cmeta[c]) == first_kind || !(v & 2u));
-                }
-                const unsigned bal = __ballot_sync(0xffffffffu, em);
-                if (lane == 0) s_wsum[wid] = __popc(bal);
-                __syncthreads();
-                unsigned before = 0, all = 0;
-                for (int w = 0; w < kBlockThreads / 32; ++w) {
-                    before += w < wid ? s_wsum[w] : 0u;
-                    all += s_wsum[w];
-                }
-                if (em) elist[s_ne + int(before) + __popc(bal & ((1u << lane) - 1))] = uint32_t(c) | ((ccnt[c] >> 2) << 16);
-                __syncthreads();
-                if (tid == 0) s_ne += int(all);
-                __syncthreads();
-            }
-            const int ne = s_ne;
-            // DFS order: each emitted candidate's rank among the emitted ones; B-side edges are
-            // kept in place, F-side ranks wait in ccnt for the pool reservation
-            for (int i = tid; i < ne; i += kBlockThreads) {
-                const uint32_t v = elist[i];
-                const int c = int(v & 0xffff), lc = L - meta_len(cmeta[c]);
-                int rank = 0;
-                for (int j = 0; j < ne; ++j) {
-                    const int x = int(elist[j] & 0xffff);
-                    const int o = block_cmp(cw, cap, nw, x, L - meta_len(cmeta[x]), c, lc);
-                    rank += (o != 0 ? o < 0 : cid[x] < cid[c]) ? 1 : 0;
-                }
-                if (side == 0) {
-                    e_id[rank] = cid[c];
-                    e_meta[rank] = cmeta[c];
-                    e_trans[rank] = int32_t(v >> 16);
-                } else {
-                    ccnt[c] = uint32_t(rank);
-                }
-            }
-            if (tid == 0) s_cnt[side] = ne;
+            const int nsorted = block_sorted_side(m, L, nw, cap, cw, cid, cmeta, perm0, perm1, sinfo, scnt, smisc, first_kind,
+                                                  self, side, e_id, e_meta, e_trans, elist, ccnt);
+            if (tid == 0) s_cnt[side] = nsorted;
             __syncthreads();
         }
         if (!s_ok) {             // more candidates than fit: the next tier
@@ -2415,22 +2706,70 @@ __global__ void __launch_bounds__(kBlockThreads) k_search_block(SearchArgs A, Se
     add_probes(O, probes);
 }
 
-bool block_tier_holds(int L, int t) { return block_smem_layout(L, t, kBlockSmemBudget).cap >= 128; }
+constexpr unsigned kWalkBatch = 8192;       // reads walked (and then reduced) at a time
 
-cudaError_t search_block(const SearchArgs& a, const SearchOut& o, const idx_t* list, const unsigned* count,
-                         unsigned count_host, idx_t* next_list, unsigned* next_count, cudaStream_t st) {
-    const BlockSmem lay = block_smem_layout(a.L, a.t, kBlockSmemBudget);
-    if (lay.cap < 128 || !count_host) return cudaSuccess;     // nothing this tier can hold
-    cudaError_t e = cudaFuncSetAttribute(k_search_block<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(lay.bytes));
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 152;
+template <int CAP, int T>
+static int block_ctas(unsigned count) {
+    int dev = 0, sms = 152, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned blocks = count_host < unsigned(sms) ? count_host : unsigned(sms);
-    k_search_block<false><<<blocks, kBlockThreads, lay.bytes, st>>>(a, o, list, count, lay, next_list, next_count,
-                                                                    nullptr);
-    note_launch();
+    cudaFuncSetAttribute(k_search_block<CAP, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(block_smem_bytes(CAP)));
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_search_block<CAP, T>, T, block_smem_bytes(CAP));
+    if (e != cudaSuccess) cudaGetLastError();
+    return int(std::min<unsigned>(count, unsigned(sms * (e == cudaSuccess && per > 0 ? per : 1))));
+}
+
+// queue counters, walked sides, their groups, and the CTAs' regions: one area, since the three sizes
+// run one after the other
+static size_t block_layout(int L, int t, unsigned count, size_t (&o)[4]) {
+    const unsigned nb = std::min(count, kWalkBatch);
+    const int M = L - t, nw = (M + 31) / 32;
+    const size_t region = std::max({size_t(block_ctas<kBlockSmall, 256>(nb)) * block_region_bytes(kBlockSmall, nw),
+                                    size_t(block_ctas<kBlockMid, 512>(nb)) * block_region_bytes(kBlockMid, nw),
+                                    size_t(block_ctas<kBlockLarge, 512>(nb)) * block_region_bytes(kBlockLarge, nw)});
+    const size_t part[4] = {256, size_t(2 * nb) * sizeof(BlockSide), size_t(2 * nb) * size_t(2 * M) * sizeof(Cand), region};
+    size_t used = 0;
+    for (int i = 0; i < 4; ++i) {
+        o[i] = used;
+        used += (part[i] + 255) & ~size_t(255);
+    }
+    return used;
+}
+
+size_t block_scratch_bytes(int L, int t, unsigned count) {
+    size_t o[4];
+    return block_layout(L, t, count, o);
+}
+
+cudaError_t search_block(const SearchArgs& a, const SearchOut& o, const idx_t* list, unsigned count, void* scratch,
+                         size_t scratch_bytes, idx_t* next_list, unsigned* next_count, cudaStream_t st) {
+    size_t at[4];
+    if (!count) return cudaSuccess;
+    if (scratch_bytes < block_layout(a.L, a.t, count, at)) return cudaErrorInvalidValue;
+    char* p = static_cast<char*>(scratch);
+    unsigned* next = reinterpret_cast<unsigned*>(p + at[0]);
+    BlockSide* sides = reinterpret_cast<BlockSide*>(p + at[1]);
+    Cand* groups = reinterpret_cast<Cand*>(p + at[2]);
+    const size_t rd = size_t((a.L + 15) / 16) * kWalkThreads * 4;
+    cudaError_t e = cudaFuncSetAttribute(k_block_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rd));
+    if (e != cudaSuccess) return e;
+    for (unsigned b = 0; b < count; b += kWalkBatch) {
+        const unsigned nb = std::min(count - b, kWalkBatch);
+        e = cudaMemsetAsync(next, 0, 256, st);
+        if (e != cudaSuccess) return e;
+        k_block_walk<<<(2 * nb + kWalkThreads - 1) / kWalkThreads, kWalkThreads, rd, st>>>(a, o, list + b, nb, groups, sides);
+        note_launch();
+        unsigned char* region = reinterpret_cast<unsigned char*>(p + at[3]);
+        k_search_block<kBlockSmall, 256><<<block_ctas<kBlockSmall, 256>(nb), 256, block_smem_bytes(kBlockSmall), st>>>(
+            a, o, list + b, nb, groups, sides, next, region, 0, kBlockSmall, next_list, next_count);
+        k_search_block<kBlockMid, 512><<<block_ctas<kBlockMid, 512>(nb), 512, block_smem_bytes(kBlockMid), st>>>(
+            a, o, list + b, nb, groups, sides, next + 1, region, kBlockSmall + 1, kBlockMid, next_list, next_count);
+        k_search_block<kBlockLarge, 512><<<block_ctas<kBlockLarge, 512>(nb), 512, block_smem_bytes(kBlockLarge), st>>>(
+            a, o, list + b, nb, groups, sides, next + 2, region, kBlockMid + 1, kBlockLarge, next_list, next_count);
+        for (int i = 0; i < 3; ++i) note_launch();
+        k_block_beyond<<<(nb + 255) / 256, 256, 0, st>>>(list + b, nb, sides, kBlockLarge, next_list, next_count);
+        note_launch();
+    }
     return cudaGetLastError();
 }
 
@@ -2447,7 +2786,7 @@ int block_global_blocks(unsigned count) {
 }
 
 BlockSmem block_global_layout(int L, int t) {
-    return block_smem_layout(L, t, block_per_cand(L, t, true) * kBlockGlobalCap + block_fixed(L, t), true);
+    return block_smem_layout(L, t, block_per_cand(L, t) * kBlockGlobalCap + block_fixed(L, t));
 }
 // the global variant's dynamic shared memory: the sort's 16 x kBlockThreads digit counts and a
 // few words of scan state
@@ -2461,7 +2800,7 @@ cudaError_t search_block_global(const SearchArgs& a, const SearchOut& o, const i
     if (!count_host || blocks <= 0) return cudaSuccess;
     const BlockSmem lay = block_global_layout(a.L, a.t);
     if (scratch_bytes < size_t(blocks) * lay.bytes) return cudaErrorInvalidValue;
-    k_search_block<true><<<blocks, kBlockThreads, kBlockSortSmem, st>>>(a, o, list, count, lay, next_list, next_count,
+    k_search_block_global<<<blocks, kBlockThreads, kBlockSortSmem, st>>>(a, o, list, count, lay, next_list, next_count,
                                                                         static_cast<unsigned char*>(scratch));
     note_launch();
     return cudaGetLastError();
