@@ -110,7 +110,7 @@ struct pq_ctx {
 
     // overlap-search output
     DevBuf nB, nF, oB, oF, status, esrc, e_dest, e_trans, e_len, e_type, ctrs, ovf_list;
-    DevBuf off, g_dest, g_len, g_type, g_trans, asm_tmp, wide, warp_scratch, defer, heavy_scratch, ovf2, ovf3, ovf4, block_scratch;
+    DevBuf off, g_dest, g_len, g_type, g_trans, asm_tmp, wide, warp_scratch, heavy_scratch, ovf2, ovf3, ovf4, block_scratch;
     uint64_t block_reads = 0;               // reads the block tier finished
     float ms_block = 0;
     uint64_t heavy_reads = 0, deferred_reads = 0;
@@ -237,7 +237,7 @@ void pq_destroy(pq_ctx* ctx) {
     DevBuf* bufs[] = {&ctx->reads, &ctx->sort_tmp, &ctx->counts, &ctx->nB, &ctx->nF, &ctx->oB,
                       &ctx->oF, &ctx->status, &ctx->esrc, &ctx->e_dest, &ctx->e_trans, &ctx->e_len,
                       &ctx->e_type, &ctx->ctrs, &ctx->ovf_list, &ctx->off, &ctx->g_dest, &ctx->g_len,
-                      &ctx->g_type, &ctx->g_trans, &ctx->asm_tmp, &ctx->wide, &ctx->warp_scratch, &ctx->defer,
+                      &ctx->g_type, &ctx->g_trans, &ctx->asm_tmp, &ctx->wide, &ctx->warp_scratch,
                       &ctx->heavy_scratch, &ctx->ovf2, &ctx->ovf3, &ctx->ovf4, &ctx->block_scratch};
     for (DevBuf* b : bufs) b->release();
     for (int d = 0; d < 2; ++d) {
@@ -690,7 +690,7 @@ static int search_prepare(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
     // sorted continuations wherever those fit in 256 bases
     A.sorted_reduce = (ctx->seed_mode != 0 && ctx->L - ctx->t <= 256) ? 1 : 0;
 
-    // [0] e_count [1] probes [2] ovf (u32) [3] learned misses [4] defer (u32) [5] heavy ovf [6] sectors
+    // [0] e_count [1] probes [2] ovf (u32) [3] learned misses [5] heavy ovf [6] sectors
     unsigned long long* ctr = ctx->ctrs.as<unsigned long long>();
     O.num_B = ctx->nB.as<uint16_t>();
     O.num_F = ctx->nF.as<uint16_t>();
@@ -709,16 +709,29 @@ static int search_prepare(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
     O.probes = ctr + 1;
     O.sectors = ctr + 6;
     A.lx_misses = ctr + 3;
-    CK(ctx->defer.ensure((nr + 1) * sizeof(idx_t)));
-    A.defer = ctx->defer.as<idx_t>();
-    A.defer_count = reinterpret_cast<unsigned*>(ctr + 4);
 
     CK(cudaMemsetAsync(ctr, 0, 64, ctx->st));
     return PQ_OK;
 }
 
-// After the fast kernel: the wide tier for the reads it handed over, then the CSR in read order.
-static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
+// The edge pool with room for `need` edges, its first `keep` kept.
+static cudaError_t grow_pool(pq_ctx* ctx, pq::SearchOut& O, size_t need, size_t keep) {
+    cudaError_t e = ctx->e_dest.grow(need * sizeof(idx_t), keep * sizeof(idx_t), ctx->st);
+    if (e == cudaSuccess) e = ctx->e_trans.grow(need * 4, keep * 4, ctx->st);
+    if (e == cudaSuccess) e = ctx->e_len.grow(need * 2, keep * 2, ctx->st);
+    if (e == cudaSuccess) e = ctx->e_type.grow(need, keep, ctx->st);
+    if (e != cudaSuccess) return e;
+    O.e_dest = ctx->e_dest.as<idx_t>();
+    O.e_trans = ctx->e_trans.as<int32_t>();
+    O.e_len = ctx->e_len.as<uint16_t>();
+    O.e_type = ctx->e_type.as<uint8_t>();
+    O.e_cap = need;
+    return cudaSuccess;
+}
+
+// After the first kernel (lean or fast): the other tiers for the reads it handed over, then the CSR
+// in read order.
+static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool lean) {
     const size_t nr = ctx->num_reads;
     const size_t nrp = nr + 1;
     unsigned long long* ctr = ctx->ctrs.as<unsigned long long>();
@@ -726,8 +739,8 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
     CK(cudaMemcpyAsync(hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     ctx->lx_misses = hc[3];
-    ctx->deferred_reads = A.sorted_reduce ? (hc[4] & 0xffffffffu) : 0;
     unsigned ovf = unsigned(hc[2] & 0xffffffffu);
+    ctx->deferred_reads = lean ? ovf : 0;
     const idx_t* ovf_src = ctx->ovf_list.as<idx_t>();
     const unsigned* ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 2);     // device count of ovf_src
     ctx->heavy_reads = 0;
@@ -738,41 +751,53 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
     ctx->block_reads = 0;
     ctx->ms_block = 0;
     if (ovf && A.sorted_reduce) {
-        // block tier (one CTA a read, candidates sorted in shared memory) over the reads the fast
-        // tier could not hold; the ones it cannot hold either go on to the heavy tier.  Seed mode 0
+        // block tier (one CTA a read, candidates sorted in shared memory) over the reads the lean
+        // tier handed over; the ones it cannot hold either go on to the heavy tier.  Seed mode 0
         // keeps the reference's DFS for every read and skips it.
         const float tb0 = wall_ms();
         CK(ctx->ovf3.ensure(nrp * sizeof(idx_t)));
-        CK(cudaMemsetAsync(ctr + 7, 0, sizeof(unsigned long long), ctx->st));
-        const size_t bbytes = pq::block_scratch_bytes(ctx->L, ctx->t, ovf);
-        CK(ctx->block_scratch.ensure(bbytes));
-        CK(pq::search_block(A, O, ctx->ovf_list.as<idx_t>(), ovf, ctx->block_scratch.p, bbytes, ctx->ovf3.as<idx_t>(),
-                            reinterpret_cast<unsigned*>(ctr + 7), ctx->st));
-        unsigned long long h7 = 0;
-        CK(cudaMemcpyAsync(&h7, ctr + 7, sizeof h7, cudaMemcpyDeviceToHost, ctx->st));
-        CK(cudaStreamSynchronize(ctx->st));
-        const unsigned left = unsigned(h7 & 0xffffffffu);
-        ctx->block_reads = ovf - left;
-        ovf = left;
-        ovf_src = ctx->ovf3.as<idx_t>();
-        ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 7);
+        CK(ctx->ovf4.ensure(nrp * sizeof(idx_t)));
+        // A pass's leftovers go to the other list.  Reads that found the edge pool full: it grows past
+        // everything reserved so far (twice that covers every failed reservation made again), and they
+        // run once more.
+        for (int pass = 0; pass < 2; ++pass) {
+            const size_t bbytes = pq::block_scratch_bytes(ctx->L, ctx->t, ovf);
+            CK(ctx->block_scratch.ensure(bbytes));
+            CK(cudaMemsetAsync(ctr + 7, 0, sizeof(unsigned long long), ctx->st));
+            idx_t* next = pass ? ctx->ovf4.as<idx_t>() : ctx->ovf3.as<idx_t>();
+            CK(pq::search_block(A, O, ovf_src, ovf, ctx->block_scratch.p, bbytes, next,
+                                reinterpret_cast<unsigned*>(ctr + 7), ctx->st));
+            unsigned long long h7 = 0, reserved = 0;
+            CK(cudaMemcpyAsync(&h7, ctr + 7, sizeof h7, cudaMemcpyDeviceToHost, ctx->st));
+            CK(cudaMemcpyAsync(&reserved, ctr + 0, sizeof reserved, cudaMemcpyDeviceToHost, ctx->st));
+            CK(cudaStreamSynchronize(ctx->st));
+            const unsigned left = unsigned(h7 & 0xffffffffu);
+            ctx->block_reads += ovf - left;
+            ovf = left;
+            ovf_src = next;
+            ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 7);
+            if (!ovf || reserved <= O.e_cap) break;
+            CK(grow_pool(ctx, O, size_t(2 * reserved + 4096), O.e_cap));
+        }
         if (ovf) {
             // the same tier with its candidate arrays in global memory, for sides of up to
             // 32768 candidates
             const int gb = pq::block_global_blocks(ovf);
             const size_t gbytes = pq::block_global_bytes(ctx->L, ctx->t, gb);
             CK(ctx->block_scratch.ensure(gbytes));
-            CK(ctx->ovf4.ensure(nrp * sizeof(idx_t)));
+            idx_t* const last = ctx->ovf3.as<idx_t>();
+            idx_t* const gnext = ovf_src == last ? ctx->ovf4.as<idx_t>() : last;
+            idx_t* const gagain = ovf_src == last ? last : ctx->ovf4.as<idx_t>();
             CK(cudaMemsetAsync(ctr + 8, 0, sizeof(unsigned long long), ctx->st));
             CK(pq::search_block_global(A, O, ovf_src, ovf_cnt, ovf, gb, ctx->block_scratch.p, gbytes,
-                                       ctx->ovf4.as<idx_t>(), reinterpret_cast<unsigned*>(ctr + 8), ctx->st));
+                                       gnext, reinterpret_cast<unsigned*>(ctr + 8), ctx->st));
             unsigned long long h8 = 0;
             CK(cudaMemcpyAsync(&h8, ctr + 8, sizeof h8, cudaMemcpyDeviceToHost, ctx->st));
             CK(cudaStreamSynchronize(ctx->st));
             const unsigned left2 = unsigned(h8 & 0xffffffffu);
             ctx->block_reads += ovf - left2;
             ovf = left2;
-            ovf_src = ctx->ovf4.as<idx_t>();
+            ovf_src = gnext;
             ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 8);
             // reads that found the edge pool full: grow it past everything reserved so far
             // (twice that covers every failed reservation made again) and run them once more
@@ -782,29 +807,20 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
                 CK(cudaStreamSynchronize(ctx->st));
             }
             if (ovf && reserved > O.e_cap) {
-                const size_t need = size_t(2 * reserved + 4096), keep = O.e_cap;
-                CK(ctx->e_dest.grow(need * sizeof(idx_t), keep * sizeof(idx_t), ctx->st));
-                CK(ctx->e_trans.grow(need * 4, keep * 4, ctx->st));
-                CK(ctx->e_len.grow(need * 2, keep * 2, ctx->st));
-                CK(ctx->e_type.grow(need, keep, ctx->st));
-                O.e_dest = ctx->e_dest.as<idx_t>();
-                O.e_trans = ctx->e_trans.as<int32_t>();
-                O.e_len = ctx->e_len.as<uint16_t>();
-                O.e_type = ctx->e_type.as<uint8_t>();
-                O.e_cap = need;
+                CK(grow_pool(ctx, O, size_t(2 * reserved + 4096), O.e_cap));
                 const int gb2 = pq::block_global_blocks(ovf);
                 const size_t gbytes2 = pq::block_global_bytes(ctx->L, ctx->t, gb2);
                 CK(ctx->block_scratch.ensure(gbytes2));
                 CK(cudaMemsetAsync(ctr + 7, 0, sizeof(unsigned long long), ctx->st));
                 CK(pq::search_block_global(A, O, ovf_src, ovf_cnt, ovf, gb2, ctx->block_scratch.p, gbytes2,
-                                           ctx->ovf3.as<idx_t>(), reinterpret_cast<unsigned*>(ctr + 7), ctx->st));
+                                           gagain, reinterpret_cast<unsigned*>(ctr + 7), ctx->st));
                 unsigned long long h7b = 0;
                 CK(cudaMemcpyAsync(&h7b, ctr + 7, sizeof h7b, cudaMemcpyDeviceToHost, ctx->st));
                 CK(cudaStreamSynchronize(ctx->st));
                 const unsigned left3 = unsigned(h7b & 0xffffffffu);
                 ctx->block_reads += ovf - left3;
                 ovf = left3;
-                ovf_src = ctx->ovf3.as<idx_t>();
+                ovf_src = gagain;
                 ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 7);
             }
         }
@@ -888,15 +904,7 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
             // grow the pool past everything reserved so far plus a full worst case per retried read
             size_t need = size_t(hc[0]) + again.size() * size_t(2 * 65535 + 2);
             size_t keep = std::min<size_t>(size_t(hc[0]), O.e_cap);
-            CK(ctx->e_dest.grow(need * sizeof(idx_t), keep * sizeof(idx_t), ctx->st));
-            CK(ctx->e_trans.grow(need * 4, keep * 4, ctx->st));
-            CK(ctx->e_len.grow(need * 2, keep * 2, ctx->st));
-            CK(ctx->e_type.grow(need, keep, ctx->st));
-            O.e_dest = ctx->e_dest.as<idx_t>();
-            O.e_trans = ctx->e_trans.as<int32_t>();
-            O.e_len = ctx->e_len.as<uint16_t>();
-            O.e_type = ctx->e_type.as<uint8_t>();
-            O.e_cap = need;
+            CK(grow_pool(ctx, O, need, keep));
             list.swap(again);
         }
         dlist.release();
@@ -948,13 +956,12 @@ int pq_overlaps(pq_ctx* ctx) {
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device);
     CK(cudaEventRecord(ctx->evk0, ctx->st));
     if (nr && A.sorted_reduce) {
-        // lean tier over every read (thread per read), then the fast tier over what it hands over
+        // lean tier over every read; what it hands over is taken in search_finish
         const int ebcap = 64;
         const int lean = int(std::min<size_t>((nr + 127) / 128, size_t(pq::search_lean_blocks(ctx->L, ctx->L - ctx->t, dev_sms))));
-        const int fast = pq::search_fast_blocks(ctx->L, ctx->L - ctx->t, dev_sms);
-        const size_t wsb = pq::lean_scratch_bytes(ctx->L, ctx->t, lean, fast, ebcap);
+        const size_t wsb = pq::lean_scratch_bytes(ctx->L, ctx->t, lean, ebcap);
         CK(ctx->warp_scratch.ensure(wsb));
-        CK(pq::search_lean(A, O, lean, fast, ctx->warp_scratch.p, wsb, ebcap, ctx->st));
+        CK(pq::search_lean(A, O, lean, ctx->warp_scratch.p, wsb, ebcap, ctx->st));
     } else if (nr) {
         // 4 warps per block, each warp 32 reads per batch; enough blocks to fill every SM
         const int ebcap = 64;
@@ -964,7 +971,7 @@ int pq_overlaps(pq_ctx* ctx) {
         CK(pq::search_fast(A, O, blocks, ctx->warp_scratch.p, wsb, ebcap, ctx->st));
     }
     CK(cudaEventRecord(ctx->evk1, ctx->st));
-    return search_finish(ctx, A, O);
+    return search_finish(ctx, A, O, A.sorted_reduce != 0);
 }
 
 int pq_get_graph_sizes(pq_ctx* ctx, uint64_t* num_edges, uint64_t* probes, uint64_t* wide_reads) {
@@ -1254,15 +1261,18 @@ static uint64_t fnv1a(const void* p, size_t n) {
 // One queued search over the batch descriptions already on the device (lead->q_batches, copies
 // of hb).  Lean path (every batch reduces by sorted continuations): the batches are split by the
 // continuation words their kernels are built for (L - t <= 64 or not); each class is one
-// persistent lean launch over its own queue, followed by the fast tier over its batches'
-// handed-over reads.  Otherwise one fast-kernel launch over the whole queue.
+// persistent lean launch over its own queue.  Otherwise one fast-kernel launch over the whole queue.
+// The reads they hand over are taken batch by batch afterwards (search_finish).
+static bool all_lean(const std::vector<pq::SearchBatch>& hb) {
+    return std::all_of(hb.begin(), hb.end(), [](const pq::SearchBatch& b) { return b.a.sorted_reduce != 0; });
+}
+
 static int queue_launch(pq_ctx* lead, const std::vector<pq::SearchBatch>& hb, const std::vector<int>& order,
                         int use_graph) {
     pq_ctx* ctx = lead;
     int dev_sms = 152;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, lead->device);
-    bool lean = true;
-    for (const auto& b : hb) lean = lean && b.a.sorted_reduce;
+    const bool lean = all_lean(hb);
     const unsigned gpi = unsigned(std::max(1, lead->q_groups_per_item));
     // classes of batches, each with its items (batch, first group), longest reads first
     struct Class {
@@ -1285,7 +1295,7 @@ static int queue_launch(pq_ctx* lead, const std::vector<pq::SearchBatch>& hb, co
     }
     size_t nitems = 0, scratch = 0;
     struct Plan {
-        int blocks, fast_blocks;
+        int blocks;
         size_t wsb, first;
     };
     std::vector<Plan> plan(cls.size());
@@ -1297,9 +1307,7 @@ static int queue_launch(pq_ctx* lead, const std::vector<pq::SearchBatch>& hb, co
         if (lead->q_ctas_per_sm > 0) per_sm = std::min(lead->q_ctas_per_sm, per_sm);
         Plan& p = plan[k];
         p.blocks = int(std::max<size_t>(1, std::min<size_t>(size_t(per_sm) * dev_sms, (c.ib.size() + 3) / 4)));
-        p.fast_blocks = fast_max * dev_sms;
-        const size_t nwarps = size_t(lean ? std::max(p.blocks, p.fast_blocks) : p.blocks) * 4;
-        p.wsb = pq::queue_scratch_bytes(c.L_max, c.M_max, nwarps, lead->q_ebcap);
+        p.wsb = pq::queue_scratch_bytes(c.L_max, c.M_max, size_t(p.blocks) * 4, lead->q_ebcap);
         p.first = nitems;
         nitems += c.ib.size();
         scratch = std::max(scratch, p.wsb);
@@ -1328,9 +1336,7 @@ static int queue_launch(pq_ctx* lead, const std::vector<pq::SearchBatch>& hb, co
             Q.groups_per_item = gpi;
             Q.next = lead->q_next.as<unsigned>() + k;
             if (lean)
-                e = pq::search_lean_queue(Q, hb.data(), c.batches.data(), int(c.batches.size()), c.L_max, c.M_max,
-                                          plan[k].blocks, plan[k].fast_blocks, lead->warp_scratch.p, plan[k].wsb,
-                                          lead->q_ebcap, lead->st);
+                e = pq::search_lean_queue(Q, c.M_max, plan[k].blocks, lead->warp_scratch.p, plan[k].wsb, lead->q_ebcap, lead->st);
             else
                 e = pq::search_fast_queue(Q, c.L_max, c.M_max, plan[k].blocks, lead->warp_scratch.p, plan[k].wsb,
                                           lead->q_ebcap, lead->st);
@@ -1421,7 +1427,7 @@ int pq_overlaps_batched(pq_ctx** ctxs, int count, int flags) {
     }
     CK(cudaStreamSynchronize(lead->st));
     for (int b = 0; b < count; ++b) {
-        const int rc = search_finish(ctxs[b], hb[b].a, hb[b].o);
+        const int rc = search_finish(ctxs[b], hb[b].a, hb[b].o, all_lean(hb));
         if (rc != PQ_OK) {
             if (b) fail(lead, rc, std::string("batch ") + std::to_string(b) + ": " + ctxs[b]->err);
             return rc;

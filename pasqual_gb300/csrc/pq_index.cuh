@@ -66,8 +66,6 @@ struct SearchArgs {
                                 // 2: the same with learned windows (needs fm[].lx)
     unsigned long long* lx_misses;  // learned windows that missed (those chains walk)
     int sorted_reduce;          // 1: edges from sorted continuations (L - t <= 256)
-    idx_t* defer;               // lean tier: reads handed to the fast tier ...
-    unsigned* defer_count;      //   ... and their number (zero before the search)
 };
 
 // Global scratch of the fast kernel, per warp of 32 reads: level-0 candidates (4 kinds x (L - t)
@@ -119,12 +117,12 @@ int search_fast_blocks(int L, int M, int num_sms);   // resident blocks of the f
 // the frame count are listed for the wide kernel.
 cudaError_t search_fast(const SearchArgs& a, const SearchOut& o, int blocks, void* scratch, size_t scratch_bytes,
                         int ebcap, cudaStream_t st);
-// Lean tier (thread per read, sorted reduction) over every read, then the fast tier over the reads
-// it hands over (more than 64 candidates on a side); needs a.sorted_reduce.
+// Lean tier (sorted reduction) over every read; the ones it does not serve (more than 64 candidates
+// on a side, a missed window, a full edge pool) are listed in o.ovf_list; needs a.sorted_reduce.
 int search_lean_blocks(int L, int M, int num_sms);
-size_t lean_scratch_bytes(int L, int t, int lean_blocks, int fast_blocks, int ebcap);
-cudaError_t search_lean(const SearchArgs& a, const SearchOut& o, int lean_blocks, int fast_blocks, void* scratch,
-                        size_t scratch_bytes, int ebcap, cudaStream_t st);
+size_t lean_scratch_bytes(int L, int t, int blocks, int ebcap);
+cudaError_t search_lean(const SearchArgs& a, const SearchOut& o, int blocks, void* scratch, size_t scratch_bytes, int ebcap,
+                        cudaStream_t st);
 // Block tier over list[0, count): one CTA a read, each side's candidates sorted in shared memory;
 // reads it cannot hold (or whose edges overflow the pool) are appended to next_list.
 size_t block_scratch_bytes(int L, int t, unsigned count);
@@ -137,15 +135,13 @@ size_t block_global_bytes(int L, int t, int blocks);
 cudaError_t search_block_global(const SearchArgs& a, const SearchOut& o, const idx_t* list, const unsigned* count,
                                 unsigned count_host, int blocks, void* scratch, size_t scratch_bytes,
                                 idx_t* next_list, unsigned* next_count, cudaStream_t st);
-// Heavy tier over reads[0, *count) with a wider DFS (reads the fast tier could not hold).
+// Heavy tier over reads[0, *count) with a wider DFS (reads the fast or block tiers could not hold).
 size_t heavy_scratch_bytes(int L, int t, int blocks, int ebcap);
 cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* list, const unsigned* count, int blocks,
                          void* scratch, size_t scratch_bytes, int ebcap, cudaStream_t st);
-// One persistent lean launch over a queue of batches, then the fast tier over the handed-over
-// reads of the batches listed in `batches` (host_batches: the descriptions the queue holds).
-cudaError_t search_lean_queue(const SearchQueue& q, const SearchBatch* host_batches, const int* batches, int nbatch,
-                              int L_max, int M_max, int lean_blocks, int fast_blocks, void* scratch,
-                              size_t scratch_bytes, int ebcap, cudaStream_t st);
+// One persistent lean launch over a queue of batches (M_max: the largest L - t).
+cudaError_t search_lean_queue(const SearchQueue& q, int M_max, int blocks, void* scratch, size_t scratch_bytes, int ebcap,
+                              cudaStream_t st);
 constexpr int lam_words_host(int M) { return M <= 64 ? 2 : 8; }
 // One persistent launch over a queue of batches (L_max, M_max: the largest L and L - t).
 size_t queue_scratch_bytes(int L_max, int M_max, size_t nwarps, int ebcap);

@@ -1540,11 +1540,15 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
 // ------------------------------------------------------------------------------ lean tier
 //
 // A warp takes 32 reads.  The rows to check of each read's two chains of a side are found lane by
-// lane (k-mer table, narrow_rows); then the rows of all 32 reads are taken one a lane, so that 32 suffix-array entries are in flight at once whatever the reads' own numbers
-// of rows.  Rows at an offset that can be a candidate wait in a queue until a warp's worth is there
+// lane (k-mer table, narrow_rows); then the rows of all 32 reads are taken one a lane, so that 32
+// suffix-array entries are in flight at once whatever the reads' own numbers of rows.  Rows at an offset that can be a candidate wait in a queue until a warp's worth is there
 // to compare its texts, and a row that is a candidate takes the next slot of its read.  Each lane
 // then reduces its read by sorted continuations.  A read the scan does not serve or with more than
-// kRedMax candidates on a side is listed in `defer` for the fast tier, which walks and runs the DFS.
+// kRedMax candidates on a side is listed for the block tier: the fast tier's walk and DFS in between
+// was slower for every kind of such reads, whether it could hold them or not (1.5 M bases of 100-base
+// reads with 2 % dinucleotide runs, 2,165 such reads, 431 of which it could: 36 ms with it, 1.6
+// without; with half the genome in repeats, 565 and 555: 3.4 and 1.9; 400x coverage, 38 thousand and
+// 6 thousand: 8.6 and 5.3).
 //
 // Bound by DRAM at random sectors (4.1 TB/s, of which every second sector of a 64-byte fetch goes
 // unused): k-mer table, kx, suffix array, text.  5.4 M reads of 100 bases, 566 M suffixes, 64-bit
@@ -1734,11 +1738,8 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                 }
                 __syncwarp();
             }
-            if (have && !ok) {          // the fast tier redoes this read (walk, or more candidates)
-                const unsigned k = atomicAdd(A.defer_count, 1u);
-                A.defer[k] = self;
-            } else if (have && status != OVF_NONE) {
-                O.status[r] = uint8_t(status);
+            if (have && (!ok || status != OVF_NONE)) {   // the block tier redoes this read
+                if (ok) O.status[r] = uint8_t(status);
                 const unsigned k = atomicAdd(O.ovf_count, 1u);
                 O.ovf_list[k] = self;
             }
@@ -1859,66 +1860,39 @@ cudaError_t search_fast(const SearchArgs& a, const SearchOut& o, int blocks, voi
     return cudaGetLastError();
 }
 
-cudaError_t search_lean(const SearchArgs& a, const SearchOut& o, int lean_blocks, int fast_blocks, void* scratch,
-                        size_t scratch_bytes, int ebcap, cudaStream_t st) {
-    const size_t nwarps = size_t(std::max(lean_blocks * (kLeanThreads / 32), fast_blocks * kWarpsPerCta));
+cudaError_t search_lean(const SearchArgs& a, const SearchOut& o, int blocks, void* scratch, size_t scratch_bytes, int ebcap,
+                        cudaStream_t st) {
     WarpScratch S;
-    if (scratch_bytes < scratch_layout(a.L - a.t, nwarps, ebcap, scratch, &S)) return cudaErrorInvalidValue;
-    const int words = (a.L + 15) / 16;
-    cudaError_t e = cudaMemsetAsync(a.defer_count, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
-    const size_t fsm = size_t(words) * 32 * kWarpsPerCta * 4;
+    if (scratch_bytes < scratch_layout(a.L - a.t, size_t(blocks) * (kLeanThreads / 32), ebcap, scratch, &S))
+        return cudaErrorInvalidValue;
     SearchQueue none{};
-    if (lam_words(a.L - a.t) == 2) k_search_lean<2><<<lean_blocks, kLeanThreads, 0, st>>>(a, o, S, none);
-    else k_search_lean<kLamWords><<<lean_blocks, kLeanThreads, 0, st>>>(a, o, S, none);
-    note_launch();
-    // the handed-over reads, whatever their number (read on the device): the fast tier's DFS
-    SearchQueue Q{};
-    Q.read_list = a.defer;
-    Q.list_count = a.defer_count;
-    if (lam_words(a.L - a.t) == 2) k_search_fast<2, kTaskCap, kTaskFrames, kPMax><<<fast_blocks, 32 * kWarpsPerCta, fsm, st>>>(a, o, S, Q);
-    else k_search_fast<kLamWords, kTaskCap, kTaskFrames, kPMax><<<fast_blocks, 32 * kWarpsPerCta, fsm, st>>>(a, o, S, Q);
+    if (lam_words(a.L - a.t) == 2) k_search_lean<2><<<blocks, kLeanThreads, 0, st>>>(a, o, S, none);
+    else k_search_lean<kLamWords><<<blocks, kLeanThreads, 0, st>>>(a, o, S, none);
     note_launch();
     return cudaGetLastError();
 }
 
 // Queued lean search: one persistent lean launch over the queue (kernel built for the words of
-// M_max), then the fast tier over the handed-over reads of each batch in `batches` (one launch per
-// batch, counts read on the device; no host sync).
-cudaError_t search_lean_queue(const SearchQueue& q, const SearchBatch* host_batches, const int* batches, int nbatch,
-                              int L_max, int M_max, int lean_blocks, int fast_blocks, void* scratch,
-                              size_t scratch_bytes, int ebcap, cudaStream_t st) {
-    const size_t nwarps = size_t(std::max(lean_blocks * (kLeanThreads / 32), fast_blocks * kWarpsPerCta));
+// M_max; no host sync).
+cudaError_t search_lean_queue(const SearchQueue& q, int M_max, int blocks, void* scratch, size_t scratch_bytes, int ebcap,
+                              cudaStream_t st) {
     WarpScratch S;
-    if (scratch_bytes < scratch_layout(M_max, nwarps, ebcap, scratch, &S)) return cudaErrorInvalidValue;
-    const int words = (L_max + 15) / 16;
-    const size_t fsm = size_t(words) * 32 * kWarpsPerCta * 4;
-    const bool two = lam_words(M_max) == 2;
+    if (scratch_bytes < scratch_layout(M_max, size_t(blocks) * (kLeanThreads / 32), ebcap, scratch, &S)) return cudaErrorInvalidValue;
     SearchArgs a0{};
     SearchOut o0{};
-    if (two) k_search_lean<2><<<lean_blocks, kLeanThreads, 0, st>>>(a0, o0, S, q);
-    else k_search_lean<kLamWords><<<lean_blocks, kLeanThreads, 0, st>>>(a0, o0, S, q);
+    if (lam_words(M_max) == 2) k_search_lean<2><<<blocks, kLeanThreads, 0, st>>>(a0, o0, S, q);
+    else k_search_lean<kLamWords><<<blocks, kLeanThreads, 0, st>>>(a0, o0, S, q);
     note_launch();
-    for (int i = 0; i < nbatch; ++i) {
-        const SearchBatch& hbt = host_batches[batches[i]];
-        SearchQueue Q{};
-        Q.read_list = hbt.a.defer;
-        Q.list_count = hbt.a.defer_count;
-        if (two) k_search_fast<2, kTaskCap, kTaskFrames, kPMax><<<fast_blocks, 32 * kWarpsPerCta, fsm, st>>>(hbt.a, hbt.o, S, Q);
-        else k_search_fast<kLamWords, kTaskCap, kTaskFrames, kPMax><<<fast_blocks, 32 * kWarpsPerCta, fsm, st>>>(hbt.a, hbt.o, S, Q);
-        note_launch();
-    }
     return cudaGetLastError();
 }
 
-size_t lean_scratch_bytes(int L, int t, int lean_blocks, int fast_blocks, int ebcap) {
-    const size_t nwarps = size_t(std::max(lean_blocks * (kLeanThreads / 32), fast_blocks * kWarpsPerCta));
-    return scratch_layout(L - t, nwarps, ebcap, nullptr, nullptr);
+size_t lean_scratch_bytes(int L, int t, int blocks, int ebcap) {
+    return scratch_layout(L - t, size_t(blocks) * (kLeanThreads / 32), ebcap, nullptr, nullptr);
 }
 
 // ------------------------------------------------------------------------------ block tier
 //
-// Reads the fast tier hands over are the ones with many candidates -- low-complexity sequence,
+// Reads the lean tier hands over are mostly the ones with many candidates -- low-complexity sequence,
 // where a read's side can have thousands.  One thread per (read, side) walks the chains of all of
 // them first (k_block_walk: chain_pair, from exact k-mer seeds, with the reference's depths), so
 // that the dependent steps of thousands of walks overlap.  Then one CTA takes each read: every
@@ -2991,16 +2965,30 @@ size_t assemble_tmp_bytes(idx_t num_reads) {
     return (total + 64) * sizeof(unsigned long long);
 }
 
+// A warp copies the edges of 32 reads, an edge a lane whatever read it belongs to: a read of a thousand
+// edges does not hold one thread, and the CSR arrays are written in whole sectors.  Bound by memory;
+// with a thread a read, the 3,645 run reads of the 200 Mbp workload at 1/100 genome took 0.95 ms, now 0.37.
 __global__ void k_gather_edges(const SearchOut O, idx_t n, const unsigned long long* off, idx_t* dest,
                                uint16_t* len, uint8_t* type, int32_t* trans) {
-    const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += stride) {
-        unsigned long long o = off[r], m = off[r + 1] - o, s = O.edge_src[r];
-        for (unsigned long long j = 0; j < m; ++j) {
-            dest[o + j] = O.e_dest[s + j];
-            len[o + j] = O.e_len[s + j];
-            type[o + j] = O.e_type[s + j];
-            trans[o + j] = O.e_trans[s + j];
+    const int lane = int(threadIdx.x & 31u);
+    const size_t warps = size_t(gridDim.x) * blockDim.x / 32, nn = size_t(n);
+    for (size_t r0 = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; r0 < nn; r0 += warps * 32) {
+        const size_t r = r0 + size_t(lane);
+        const unsigned long long lo = off[r < nn ? r : nn], src = r < nn ? O.edge_src[r] : 0;
+        const unsigned long long first = __shfl_sync(0xffffffffu, lo, 0), last = off[r0 + 32 < nn ? r0 + 32 : nn];
+        for (unsigned long long e0 = first; e0 < last; e0 += 32) {
+            const unsigned long long e = e0 + unsigned(lane);
+            int q = 0;                                          // the last of the 32 reads to start at or before e
+            #pragma unroll
+            for (int w = 16; w; w >>= 1)
+                if (__shfl_sync(0xffffffffu, lo, q + w) <= e) q += w;
+            const unsigned long long s = __shfl_sync(0xffffffffu, src, q) + (e - __shfl_sync(0xffffffffu, lo, q));
+            if (e < last) {
+                dest[e] = O.e_dest[s];
+                len[e] = O.e_len[s];
+                type[e] = O.e_type[s];
+                trans[e] = O.e_trans[s];
+            }
         }
     }
 }
