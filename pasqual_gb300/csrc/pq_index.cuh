@@ -72,9 +72,14 @@ struct SearchArgs {
 // slots per read), ebcap edge slots per read, and per (read, side) task a DFS stack, sparse
 // extension slots, emission bounds and DFS frames.
 struct TFrame;
+struct FastTask;
 struct WarpScratch {
     idx_t *c_ll, *c_uu;
     uint32_t* c_meta;
+    idx_t *p_ll, *p_uu;         // candidates of the queued reads, `pool` of them
+    uint32_t* p_meta;
+    FastTask* queue;
+    int pool;
     idx_t* e_dest;
     int32_t* e_trans;
     uint32_t* e_meta;

@@ -426,14 +426,14 @@ __device__ __forceinline__ bool text_matches(const uint64_t* __restrict__ pka, s
 }
 
 // Slots of the level-0 candidates of the two chains of one side: q * M + i.
-struct SlotsFast {     // fast tier: the warp's global scratch
+struct SlotsFast {     // fast tier: the warp's global scratch, the lanes' slots interleaved
     idx_t* ll;
     idx_t* uu;
     uint32_t* meta;
     size_t base;
     int M;
     __device__ __forceinline__ void set(int q, int i, idx_t a, idx_t b, uint32_t m) const {
-        const size_t p = base + size_t(q) * M + i;
+        const size_t p = base + (size_t(q) * M + i) * 32;
         ll[p] = a;
         uu[p] = b;
         meta[p] = m;
@@ -748,22 +748,39 @@ __device__ __forceinline__ void add_probes(const SearchOut& O, const Tally& t) {
 
 // ------------------------------------------------------------------------------ fast tier
 //
-// A warp takes 32 reads.  Phase A: each lane runs the candidate searches of its read (two chains
-// at a time, B side then F side) and stores the level-0 candidates in the warp's scratch.
-// Phase B: the whole warp reduces one (read, side) at a time -- the extract_*_edges DFS with the
-// intervals of a level spread over the lanes: every lane loads the blocks of its interval, the
-// four extension sets are packed with ballots, the emission check finds the first completing
-// interval with a ballot, and the edge reads are fetched by all lanes at once.  Control flow of
-// phase B is uniform across the warp (all decisions come from ballots, shuffles and the frames
-// in shared memory), and the stack lives in global memory as three coalesced arrays.
-// Phase C: each lane publishes its read (edge-pool reservation, copy, per-read counts).
+// Phase A: each lane runs the candidate searches of a read (two chains at a time, B side then F
+// side); the level-0 candidates of up to kFastQueue reads are packed into the warp's pool.
+// Phase B: the (read, side) DFS of extract_*_edges, one a lane, advance together, one level per step;
+// a lane whose read is done publishes it (edge-pool reservation, copy, per-read counts) and takes
+// the next of the queue.  Each lane owns the control of its read's DFS (frames, emission,
+// backtracking); the intervals of all tasks expanding in a step are spread over the lanes, so the
+// block loads of up to 32 intervals are in flight together.  The order of the extension sets, the
+// first emitting interval and the DFS order of the edges are fixed by entry index (ballots, bit masks
+// with population counts, an atomic minimum), never by the order in which lanes happen to run, so
+// every edge list is the reference's.
+//
+// Bound by the latency of the walks' and intervals' blocks (two random sectors each) and by the
+// instructions of a step.  1.23 M reads of 100 bases at 30x, 302 M chain steps and 86 M intervals:
+// 11.2 ms, 7 of them the chains.  Was 21.2: extensions went through sparse slots and a second pass
+// over all four sets of every interval, and a frame was kept at every level (both now only where
+// needed: 12.9), with 32 reads at a time in step (15.8 with a queue of 32, 12.5 with 256); five CTAs
+// of 96 registers, where six of 80 spill, gave the rest, seven took 16.0, four 12.0.
 
 constexpr int kWarpsPerCta = 4;
 constexpr int kTaskCap = 512;       // stack intervals per (read, side) task
-constexpr int kTaskFrames = 48;     // DFS levels per task (deeper reads go to the wide kernel)
+constexpr int kTaskFrames = 48;     // DFS frames kept per task (reads with more go to the wide kernel)
 constexpr int kPMax = 128;          // intervals of one level of one task
 
 __device__ __forceinline__ int csz_at(uint64_t c4, int i) { return int((c4 >> (16 * i)) & 0xffff); }
+
+// A read of the warp's queue: its level-0 candidates are at `at` in the warp's pool, n[side] of them.
+struct FastTask {
+    idx_t read;
+    uint32_t at;
+    int n[2];
+};
+constexpr int kFastQueue = 128;     // reads a warp walks before it reduces them
+constexpr int kFastPool = 4096;     // candidates kept for them (at least one read's most)
 
 // One DFS level of one task (the reference's recursion frame of extract_*_edges).
 struct TFrame {
@@ -772,14 +789,14 @@ struct TFrame {
     uint32_t cbase;     // first slot of the four extension sets (back to back, A..T)
     int32_t trans;      // sum of this level's interval sizes (path_t.trans of its edges)
     uint16_t size, maxlen;
-    uint32_t next_a;
+    uint16_t next_a, level;
     uint64_t csz4;      // sizes of the four sets, 16 bits each (A lowest)
     uint64_t cml4;      // largest overlap length in each set, 16 bits each
     int32_t ctr[4];     // interval-size sum of each set
 };
 
 // Shared memory of one warp for the level-synchronous DFS of its 32 tasks (MW 64-bit mask words
-// per task and base: one bit per interval of a level, up to 64 MW intervals).
+// per larger task and base: one bit per interval of a level, up to 64 MW intervals).
 template <int MW>
 struct MultiSmem {
     unsigned long long mask[32][4][MW];  // extension present, by entry index
@@ -789,7 +806,10 @@ struct MultiSmem {
     int setoff[32][4];
     int pref[33];
     uint32_t pos[32], cbase[32];
-    int lvl[32], chk[32], size[32], na[32];
+    int lvl[32], chk[32], size[32];
+    uint32_t src[32];                    // pool position of a task's level 0
+    int list[32];                        // the tasks of up to 32 intervals, in lane order
+    uint32_t cnt[32];                    // their four sets' sizes, 8 bits each
 };
 
 template <int MW>
@@ -837,19 +857,6 @@ __device__ __forceinline__ int owner_of(const int* pref, int e) {
     }
     return lo;
 }
-
-// ------------------------------------------------------------------------------ fast tier
-//
-// A warp takes 32 reads.  Phase A: each lane runs the candidate searches of its read (two chains
-// at a time, B side then F side) and stores the level-0 candidates in the warp's scratch.
-// Phase B, once for the B side and once for the F side: the 32 (read, side) DFS of
-// extract_*_edges advance together, one level per step.  Each lane owns the control of its
-// read's DFS (frames, emission, backtracking); the intervals of all tasks expanding in a step
-// are spread over the lanes, so the block loads of up to 32 tasks are in flight together.  The
-// order of the extension sets, the first emitting interval and the DFS order of the edges are
-// fixed by entry index (bit masks with population counts, an atomic minimum), never by the order
-// in which lanes happen to run, so every edge list is the reference's.
-// Phase C: each lane publishes its read (edge-pool reservation, copy, per-read counts).
 
 // ------------------------------------------------------------------------------ sorted reduction
 //
@@ -935,14 +942,13 @@ __device__ __forceinline__ int reduce_gathered(int L, const WarpScratch& S, idx_
 // n0 - na of the second) in the candidate scratch at `cand`; per-lane scratch at `red`.
 template <int W>
 __device__ __forceinline__ int reduce_sorted(const SearchArgs& A, const WarpScratch& S, idx_t self, int side,
-                                             size_t cand, int na, int n0, size_t red, size_t eb, int& ne,
+                                             size_t cand, int n0, size_t red, size_t eb, int& ne,
                                              int& count, Tally& probes) {
-    const int L = A.L, M = L - A.t;
+    const int L = A.L;
     int m = 0;
     for (int g = 0; g < n0; ++g) {
-        const size_t src = cand + (g < na ? size_t(2 * side) * M + g : size_t(2 * side + 1) * M + (g - na));
-        const idx_t ll = S.c_ll[src], uu = S.c_uu[src];
-        const uint32_t mt = S.c_meta[src];
+        const idx_t ll = S.p_ll[cand + g], uu = S.p_uu[cand + g];
+        const uint32_t mt = S.p_meta[cand + g];
         const int d = meta_len(mt), type = meta_type(mt);
         const FmView& fb = A.fm[cand_index(type)];
         for (idx_t row = ll; row <= uu; ++row) {
@@ -1171,18 +1177,45 @@ __device__ __forceinline__ void load_batch(SearchBatch& dst, const SearchBatch* 
     __syncwarp();
 }
 
+// A lane's read is done: its edges (eb .. eb + ne: B side, then F side) to the pool and its counts, or
+// the next tier's list.
+__device__ __forceinline__ void publish_lane(const SearchOut& O, const WarpScratch& S, idx_t r, int status, size_t eb, int ne,
+                                             int count_b, int count_f) {
+    unsigned long long base = 0;
+    if (status == OVF_NONE && ne) {
+        base = atomicAdd(O.e_count, (unsigned long long)ne);
+        if (base + ne > O.e_cap) status = OVF_POOL;
+    }
+    O.status[r] = uint8_t(status);
+    if (status != OVF_NONE) {
+        if (status != ERR_TOO_MANY) {
+            const unsigned k = atomicAdd(O.ovf_count, 1u);
+            O.ovf_list[k] = r;
+        }
+        return;
+    }
+    for (int e = 0; e < ne; ++e) {
+        const uint32_t mt = S.e_meta[eb + e];
+        O.e_dest[base + e] = S.e_dest[eb + e];
+        O.e_trans[base + e] = S.e_trans[eb + e];
+        O.e_len[base + e] = uint16_t(meta_len(mt));
+        O.e_type[base + e] = uint8_t(meta_type(mt));
+    }
+    O.num_B[r] = uint16_t(count_b);
+    O.num_F[r] = uint16_t(count_f);
+    O.edge_src[r] = base;
+}
+
 // Without a queue (Q.count == 0) the kernel searches the one read set of (A0, O0), warp w taking
 // groups of 32 reads w, w + #warps, ...  With a queue, each warp takes the next item (a batch and
 // a group of its reads) from a shared counter until the queue is empty; the batch's description
 // (index pair, L, t, outputs) is loaded into the warp's shared memory when it changes.
 template <int W, int CAP, int FRAMES, int PMAX>
-__global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut O0, WarpScratch S, SearchQueue Q) {
+__global__ void __launch_bounds__(128, 5) k_search_fast(SearchArgs A0, SearchOut O0, WarpScratch S, SearchQueue Q) {
     constexpr int MW = PMAX / 64;
     extern __shared__ uint32_t s_reads[];
     __shared__ SearchBatch s_b[kWarpsPerCta];
     __shared__ MultiSmem<MW> s_ms[kWarpsPerCta];
-    __shared__ int s_n[kWarpsPerCta][32][4];
-    __shared__ int32_t s_olp[kWarpsPerCta][32][2];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const size_t gw = size_t(blockIdx.x) * kWarpsPerCta + wid;
     const size_t nw = size_t(gridDim.x) * kWarpsPerCta;
@@ -1197,7 +1230,9 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
         __syncwarp();
     }
     MultiSmem<MW>& sm = s_ms[wid];
-    const size_t cbase_w = gw * 32 * 4 * size_t(S.mstride);    // level-0 candidates of this warp
+    const size_t cbase_w = gw * 32 * 4 * size_t(S.mstride);    // level-0 candidates of 32 reads
+    const size_t pbase_w = gw * size_t(S.pool);                // and of the queued reads, packed
+    FastTask* const queue = S.queue + gw * kFastQueue;
     const size_t ebase_w = gw * 32 * size_t(S.ebcap);          // edge slots of this warp
     const size_t tbase_w = gw * 32 * size_t(CAP);         // task stacks
     const size_t xbase_w = gw * 32 * 4 * size_t(PMAX);        // sparse extension slots
@@ -1208,8 +1243,8 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
     int cur = -1;
     // reads of the current batch (or of the list of reads handed over by the lean tier)
     const size_t list_n = Q.read_list ? size_t(*Q.list_count) : 0;
-    for (size_t iter = 0;; ++iter) {
-        size_t group, gend;
+    while (true) {
+        size_t group = gw, gend = 0, step = nw;
         if (Q.count) {
             unsigned it = 0;
             if (lane == 0) it = atomicAdd(Q.next, 1u);
@@ -1218,6 +1253,7 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
             const int b = int(Q.item_batch[it]);
             group = Q.item_group[it];
             gend = group + Q.groups_per_item;
+            step = 1;
             if (b != cur) {
                 if (cur >= 0) add_probes(O, probes);
                 probes = Tally{};
@@ -1225,117 +1261,181 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
                 load_batch(B, Q.batches + b, lane);
                 cur = b;
             }
-        } else {
-            group = gw + iter * nw;
-            gend = group + 1;
-            if (group * 32 >= (Q.read_list ? list_n : size_t(A.num_reads))) break;
         }
         const size_t n_items = Q.read_list ? list_n : size_t(A.num_reads);
-        for (; group < gend && group * 32 < n_items; ++group) {
+        const size_t groups = (n_items + 31) / 32;
+        if (!Q.count || gend > groups) gend = groups;
         const int M = A.L - A.t;
         const int L = A.L;
-        const size_t item = group * 32 + lane;
-        const bool have = item < n_items;
-        const size_t r = Q.read_list ? (have ? size_t(Q.read_list[item]) : 0) : item;
-        const idx_t self = idx_t(r);
+        bool pend = false;          // this lane's read of the last group walked waits for room in the queue
+        idx_t pr = 0;
+        int pn[4] = {0, 0, 0, 0};
+        while (true) {
         // ---- phase A
-        if (have) {
-            load_read(A, idx_t(r), s_reads + threadIdx.x, blockDim.x, probes);
-            ReadView rd{s_reads + threadIdx.x, int(blockDim.x)};
-            const size_t cb = cbase_w + size_t(lane) * 4 * size_t(S.mstride);
-            int nb[2], nf[2];
-            int32_t ob = 0, of = 0;
-            chain_pair(A, A.fm, rd, PQ_BF, PQ_BB, nb, ob, probes, SlotsFast{S.c_ll, S.c_uu, S.c_meta, cb, M});
-            chain_pair(A, A.fm, rd, PQ_FB, PQ_FF, nf, of, probes,
-                       SlotsFast{S.c_ll, S.c_uu, S.c_meta, cb + 2 * size_t(M), M});
-            s_n[wid][lane][0] = nb[0];
-            s_n[wid][lane][1] = nb[1];
-            s_n[wid][lane][2] = nf[0];
-            s_n[wid][lane][3] = nf[1];
-            s_olp[wid][lane][0] = ob;
-            s_olp[wid][lane][1] = of;
+        int nq = 0, used = 0;
+        while (true) {
+            if (!__any_sync(0xffffffffu, pend)) {
+                if (group >= gend || nq + 32 > kFastQueue) break;
+                const size_t item = group * 32 + lane;
+                pend = item < n_items;
+                group += step;
+                if (pend) {
+                    pr = Q.read_list ? Q.read_list[item] : idx_t(item);
+                    load_read(A, pr, s_reads + threadIdx.x, blockDim.x, probes);
+                    const ReadView rd{s_reads + threadIdx.x, int(blockDim.x)};
+                    const size_t cb = cbase_w + size_t(lane);
+                    int n[2];
+                    int32_t olp = 0;
+                    chain_pair(A, A.fm, rd, PQ_BF, PQ_BB, n, olp, probes, SlotsFast{S.c_ll, S.c_uu, S.c_meta, cb, M});
+                    O.olp_B[pr] = olp;
+                    pn[0] = n[0];
+                    pn[1] = n[1];
+                    olp = 0;
+                    chain_pair(A, A.fm, rd, PQ_FB, PQ_FF, n, olp, probes,
+                               SlotsFast{S.c_ll, S.c_uu, S.c_meta, cb + size_t(2 * M) * 32, M});
+                    O.olp_F[pr] = olp;
+                    pn[2] = n[0];
+                    pn[3] = n[1];
+                }
+                __syncwarp();
+            }
+            const int mine = pend ? pn[0] + pn[1] + pn[2] + pn[3] : 0;
+            int incl = mine;
+            #pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const bool fits = pend && used + incl <= S.pool;
+            const unsigned take = __ballot_sync(0xffffffffu, fits);
+            if (!take) break;
+            if (fits) {
+                uint32_t to = uint32_t(used + incl - mine);
+                queue[nq + __popc(take & ((1u << lane) - 1u))] = FastTask{pr, to, {pn[0] + pn[1], pn[2] + pn[3]}};
+                #pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    for (int i = 0; i < pn[q]; ++i, ++to) {
+                        const size_t src = cbase_w + (size_t(q) * M + i) * 32 + size_t(lane);
+                        S.p_ll[pbase_w + to] = S.c_ll[src];
+                        S.p_uu[pbase_w + to] = S.c_uu[src];
+                        S.p_meta[pbase_w + to] = S.c_meta[src];
+                    }
+                pend = false;
+            }
+            nq += __popc(take);
+            used += __shfl_sync(0xffffffffu, incl, 31 - __clz(int(take)));
+            __syncwarp();
+            if (__any_sync(0xffffffffu, pend)) break;
         }
-        __syncwarp();
+        if (!nq) break;
         // ---- phase B
-        int status = have ? OVF_NONE : -1;
-        int ne = 0, count_b = 0, count_f = 0;
+        int next_q = 0, qi = 0, side = 0;
+        bool busy = false, active = false, entering = false;
+        idx_t self = 0;
+        int status = OVF_NONE, ne = 0, count_b = 0, level = 0, sp = 0, sc = 0;
         const size_t tb = tbase_w + size_t(lane) * CAP;    // this lane's task stack
         TFrame* const fr = frw + lane * FRAMES;
         const size_t eb = ebase_w + size_t(lane) * S.ebcap;
-        #pragma unroll 1
-        for (int side = 0; side < 2; ++side) {
-            bool active = have && status == OVF_NONE && s_olp[wid][lane][side] != 0;   // src/string_graph.c:824, 828
-            const int na = active ? s_n[wid][lane][2 * side] : 0;
-            const int n0 = active ? na + s_n[wid][lane][2 * side + 1] : 0;
-            int sc_sorted = -1;
-            if (active && A.sorted_reduce && s_olp[wid][lane][side] <= kRedMax) {
-                const int st = reduce_sorted<W>(A, S, self, side, cbase_w + size_t(lane) * 4 * size_t(S.mstride), na,
-                                             n0, rbase_w + lane, eb, ne, sc_sorted, probes);
-                if (st != OVF_NONE) status = st;
-                active = false;
+        TFrame F{};
+        while (true) {
+            // (0) lanes without a task take the next: the read's other side, or the next read's first
+            bool fresh = false;
+            uint32_t src = 0;
+            while (__any_sync(0xffffffffu, (busy && !active) || (!busy && next_q < nq))) {
+                bool setup = false;
+                if (busy && !active) {
+                    if (side == 0 && status == OVF_NONE) {
+                        count_b = sc;
+                        side = 1;
+                        setup = true;
+                    } else {
+                        publish_lane(O, S, self, status, eb, ne, side ? count_b : sc, side ? sc : 0);
+                        busy = false;
+                    }
+                }
+                const unsigned idle = __ballot_sync(0xffffffffu, !busy);
+                if (!busy) {
+                    qi = next_q + __popc(idle & ((1u << lane) - 1u));
+                    if (qi < nq) {
+                        self = queue[qi].read;
+                        busy = setup = true;
+                        side = 0;
+                        status = OVF_NONE;
+                        ne = 0;
+                    }
+                }
+                next_q = min(nq, next_q + __popc(idle));
+                if (setup) {
+                    const FastTask task = queue[qi];
+                    const int n0 = side ? task.n[1] : task.n[0];
+                    const int32_t olp = side ? O.olp_F[self] : O.olp_B[self];
+                    src = task.at + uint32_t(side ? task.n[0] : 0);
+                    sc = 0;
+                    active = olp != 0;                                  // src/string_graph.c:824, 828
+                    if (active && A.sorted_reduce && olp <= kRedMax) {
+                        const int st = reduce_sorted<W>(A, S, self, side, pbase_w + src, n0, rbase_w + lane, eb, ne, sc, probes);
+                        if (st != OVF_NONE) status = st;
+                        active = false;
+                    } else if (active && n0 > CAP) {
+                        status = OVF_STACK;
+                        active = false;
+                    }
+                    fresh = active;
+                    F = TFrame{};
+                    F.free = uint32_t(n0);
+                    F.size = uint16_t(n0);
+                    F.next_a = 1;
+                    entering = true;
+                    level = sp = 0;
+                }
             }
-            if (active && n0 > CAP) { status = OVF_STACK; active = false; }
-            // level 0 = kind-0 candidates then kind-1 candidates, copied into the task stacks
-            sm.na[lane] = na;
-            const int tot0 = warp_prefix(active ? n0 : 0, sm.pref);
-            for (int e = lane; e < tot0; e += 32) {
-                const int j = owner_of(sm.pref, e);
-                const int i = e - sm.pref[j];
-                const int nj = sm.na[j];
-                const size_t src = cbase_w + size_t(j) * 4 * size_t(S.mstride) +
-                                   (i < nj ? size_t(2 * side) * M + i : size_t(2 * side + 1) * M + (i - nj));
-                const size_t dst = tbase_w + size_t(j) * CAP + i;
-                S.t_ll[dst] = S.c_ll[src];
-                S.t_uu[dst] = S.c_uu[src];
-                S.t_meta[dst] = S.c_meta[src];
+            if (!__any_sync(0xffffffffu, busy)) break;
+            // level 0: kind-0 candidates then kind-1 candidates
+            if (__any_sync(0xffffffffu, fresh)) {
+                sm.src[lane] = src;
+                const int tot0 = warp_prefix(fresh ? int(F.size) : 0, sm.pref);
+                for (int e = lane; e < tot0; e += 32) {
+                    const int j = owner_of(sm.pref, e);
+                    const int i = e - sm.pref[j];
+                    const size_t from = pbase_w + sm.src[j] + i, dst = tbase_w + size_t(j) * CAP + i;
+                    S.t_ll[dst] = S.p_ll[from];
+                    S.t_uu[dst] = S.p_uu[from];
+                    S.t_meta[dst] = S.p_meta[from];
+                }
+                __syncwarp();
             }
-            __syncwarp();
-            TFrame F;
-            F.pos = 0;
-            F.free = uint32_t(n0);
-            F.cbase = 0;
-            F.trans = 0;
-            F.size = uint16_t(n0);
-            F.maxlen = 0;
-            F.next_a = 1;
-            F.csz4 = 0;
-            F.cml4 = 0;
-            F.ctr[0] = F.ctr[1] = F.ctr[2] = F.ctr[3] = 0;
-            bool entering = true;
-            int level = 0, sc = 0;
-            while (__any_sync(0xffffffffu, active)) {
-                // (1) own control: backtrack / descend until this task needs an expansion
+            {
+                // (1) own control: backtrack / descend until this task needs an expansion.  A frame
+                // is kept only while sets of it remain: the last one is entered in its place.
                 if (active && !entering) {
                     while (true) {
                         int a = int(F.next_a);
                         while (a <= 4 && csz_at(F.csz4, a - 1) == 0) ++a;
                         if (a > 4) {
-                            if (level == 0) { active = false; break; }
-                            --level;
-                            F = fr[level];
+                            if (sp == 0) { active = false; break; }
+                            F = fr[--sp];
+                            level = F.level;
                             continue;
                         }
-                        if (level + 1 >= FRAMES) { status = OVF_LEVELS; active = false; break; }
-                        F.next_a = uint32_t(a + 1);
-                        fr[level] = F;
                         uint32_t before = 0, all = 0;
                         #pragma unroll
                         for (int b = 0; b < 4; ++b) {
                             before += (b < a - 1) ? csz_at(F.csz4, b) : 0;
                             all += csz_at(F.csz4, b);
                         }
-                        TFrame G;
-                        G.pos = F.cbase + before;
-                        G.free = F.cbase + all;      // below it: the parent's four sets, still pending
-                        G.cbase = 0;
-                        G.size = uint16_t(csz_at(F.csz4, a - 1));
-                        G.maxlen = uint16_t(csz_at(F.cml4, a - 1));
-                        G.trans = a == 1 ? F.ctr[0] : (a == 2 ? F.ctr[1] : (a == 3 ? F.ctr[2] : F.ctr[3]));
-                        G.next_a = 1;
-                        G.csz4 = 0;
-                        G.cml4 = 0;
-                        G.ctr[0] = G.ctr[1] = G.ctr[2] = G.ctr[3] = 0;
-                        F = G;
+                        if (all > before + csz_at(F.csz4, a - 1)) {
+                            if (sp >= FRAMES) { status = OVF_LEVELS; active = false; break; }
+                            F.next_a = uint16_t(a + 1);
+                            F.level = uint16_t(level);
+                            fr[sp++] = F;
+                        }
+                        F.size = uint16_t(csz_at(F.csz4, a - 1));
+                        F.maxlen = uint16_t(csz_at(F.cml4, a - 1));
+                        F.trans = a == 1 ? F.ctr[0] : (a == 2 ? F.ctr[1] : (a == 3 ? F.ctr[2] : F.ctr[3]));
+                        F.pos = F.cbase + before;
+                        F.free = F.cbase + all;      // below it: the parent's four sets, still pending
+                        F.next_a = 1;
+                        F.csz4 = 0;
                         ++level;
                         entering = true;
                         break;
@@ -1344,21 +1444,124 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
                 const bool expand = active && entering;
                 if (expand && F.size > PMAX) { status = OVF_STACK; active = false; }
                 const bool go = active && entering;
-                sm.size[lane] = go ? int(F.size) : 0;
-                sm.pos[lane] = F.pos;
-                sm.lvl[lane] = level;
-                sm.chk[lane] = int(F.maxlen) + level == L;
+                const bool narrow = go && F.size > 0 && F.size <= 32;
+                const bool chk = int(F.maxlen) + level == L;
                 sm.hit[lane] = 0x7fffffff;
+                sm.cnt[lane] = 0;
                 #pragma unroll
                 for (int a = 0; a < 4; ++a) {
-                    #pragma unroll
-                    for (int w = 0; w < MW; ++w) sm.mask[lane][a][w] = 0;
                     sm.cml[lane][a] = 0;
                     sm.ctr[lane][a] = 0;
                 }
                 // (2) every interval of every expanding task: one pair of block loads serves the
-                // emission check and the four extensions
-                const int tot = warp_prefix(go ? int(F.size) : 0, sm.pref);
+                // emission check and the four extensions.  Tasks of up to 32 intervals, as many
+                // whole ones as fit the lanes at a time: their sets are counted by ballots and
+                // written where they belong.
+                {
+                    const int size = narrow ? int(F.size) : 0;
+                    int end = size;
+                    #pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(0xffffffffu, end, o);
+                        if (lane >= o) end += y;
+                    }
+                    const int total = __shfl_sync(0xffffffffu, end, 31), mine = end - size;
+                    const unsigned all = __ballot_sync(0xffffffffu, narrow);
+                    if (narrow) sm.list[__popc(all & ((1u << lane) - 1u))] = lane;
+                    __syncwarp();
+                    for (int base = 0, first = 0; base < total;) {
+                        const bool in = narrow && mine >= base && end <= base + 32;
+                        const unsigned starts = __reduce_or_sync(0xffffffffu, in ? 1u << (mine - base) : 0u);
+                        const unsigned tasks = __ballot_sync(0xffffffffu, in);
+                        const int n = __shfl_sync(0xffffffffu, end, 31 - __clz(int(tasks))) - base;
+                        const unsigned at = starts & (0xffffffffu >> (31 - lane));
+                        const int s = 31 - __clz(int(at)), j = sm.list[first + __popc(at) - 1];
+                        const unsigned over = starts & (0xfffffffeu << lane);
+                        const int e = over ? __ffs(int(over)) - 1 : n;
+                        const unsigned seg = (e < 32 ? (1u << e) - 1u : 0xffffffffu) & (0xffffffffu << s);
+                        const uint32_t pos = __shfl_sync(0xffffffffu, F.pos, j), free = __shfl_sync(0xffffffffu, F.free, j);
+                        const int lc = __shfl_sync(0xffffffffu, chk ? level : -1, j);
+                        const size_t tj = tbase_w + size_t(j) * CAP;
+                        bool emits = false;
+                        idx_t lo[4], hi[4], ea = 0, eb2 = 0;
+                        unsigned has = 0;
+                        uint32_t m = 0;
+                        if (lane < n) {
+                            const size_t from = tj + pos + (lane - s);
+                            const idx_t cl = S.t_ll[from], cu = S.t_uu[from];
+                            m = S.t_meta[from];
+                            const bool ext = idx_t(cu - cl + 1) != 0;   // wrapped [0, all-ones]: kept, never extended
+                            const bool ends = lc >= 0 && meta_len(m) + lc == L;
+                            const int o = cand_index(meta_type(m));
+                            const FmView& f = A.fm[o];
+                            idx_t rl[4] = {0, 0, 0, 0}, ru[4] = {0, 0, 0, 0};
+                            if (ext || ends) {
+                                rank_all(f, cl, rl);
+                                rank_all(f, cu + 1, ru);
+                                probes += 2;
+                            }
+                            if (ends) {
+                                ea = f.Cf[0] + (cl - (rl[0] + rl[1] + rl[2] + rl[3]));
+                                eb2 = f.Cf[0] + ((cu + 1) - (ru[0] + ru[1] + ru[2] + ru[3])) - 1;
+                                emits = ea <= eb2;
+                            }
+                            if (ext) {
+                                #pragma unroll
+                                for (int a = 1; a <= 4; ++a) {
+                                    const int ch = o == 0 ? complement(a) : a;
+                                    lo[a - 1] = f.Cf[ch] + pick4(rl, ch);
+                                    hi[a - 1] = f.Cf[ch] + pick4(ru, ch) - 1;
+                                    has |= lo[a - 1] <= hi[a - 1] ? 1u << (a - 1) : 0u;
+                                }
+                            }
+                        }
+                        const unsigned em = __ballot_sync(0xffffffffu, emits) & seg;
+                        if (emits && !(em & ((1u << lane) - 1u))) {
+                            const size_t me = mbase_w + size_t(j) * PMAX + (lane - s);
+                            S.em_l[me] = ea;
+                            S.em_u[me] = eb2;
+                            sm.hit[j] = lane - s;
+                        }
+                        unsigned to = free, cnt = 0, b[4];
+                        #pragma unroll
+                        for (int a = 0; a < 4; ++a) {
+                            b[a] = __ballot_sync(0xffffffffu, (has >> a) & 1u) & seg;
+                            cnt |= unsigned(__popc(b[a])) << (8 * a);
+                        }
+                        if (lane < n) {
+                            if (lane == s) sm.cnt[j] = cnt;
+                            const bool room = free + __popc(b[0]) + __popc(b[1]) + __popc(b[2]) + __popc(b[3]) <= unsigned(CAP);
+                            #pragma unroll
+                            for (int a = 0; a < 4; ++a) {
+                                if (((has >> a) & 1u) && room) {
+                                    const size_t x = tj + to + __popc(b[a] & ((1u << lane) - 1u));
+                                    S.t_ll[x] = lo[a];
+                                    S.t_uu[x] = hi[a];
+                                    S.t_meta[x] = m;
+                                    atomicMax(&sm.cml[j][a], meta_len(m));
+                                    atomicAdd(&sm.ctr[j][a], unsigned(hi[a] - lo[a] + 1));
+                                }
+                                to += __popc(b[a]);
+                            }
+                        }
+                        first += __popc(tasks);
+                        base += n;
+                    }
+                }
+                // larger tasks: the intervals of all of them one after the other, extensions by
+                // entry first, packed below
+                const bool broad = go && F.size > 32, any_broad = __any_sync(0xffffffffu, broad);
+                if (any_broad) {
+                    sm.size[lane] = broad ? int(F.size) : 0;
+                    sm.pos[lane] = F.pos;
+                    sm.lvl[lane] = level;
+                    sm.chk[lane] = chk;
+                    #pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        #pragma unroll
+                        for (int w = 0; w < MW; ++w) sm.mask[lane][a][w] = 0;
+                    }
+                const int tot = warp_prefix(broad ? int(F.size) : 0, sm.pref);
                 for (int e = lane; e < tot; e += 32) {
                     const int j = owner_of(sm.pref, e);
                     const int i = e - sm.pref[j];
@@ -1403,6 +1606,7 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
                         }
                     }
                 }
+                }
                 __syncwarp();
                 // (3) own control: emit, or record the four sets
                 bool place = false;
@@ -1433,10 +1637,10 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
                         } else if (cnt > 0) {           // flag: this branch is finished
                             popped = true;
                             entering = false;
-                            if (level == 0) active = false;
+                            if (sp == 0) active = false;
                             else {
-                                --level;
-                                F = fr[level];
+                                F = fr[--sp];
+                                level = F.level;
                             }
                         }
                     }
@@ -1445,7 +1649,7 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
                         int run = 0;
                         #pragma unroll
                         for (int a = 0; a < 4; ++a) {
-                            c[a] = popc_words<MW>(sm.mask[lane][a]);
+                            c[a] = broad ? popc_words<MW>(sm.mask[lane][a]) : int((sm.cnt[lane] >> (8 * a)) & 0xffu);
                             sm.setoff[lane][a] = run;
                             run += c[a];
                         }
@@ -1464,11 +1668,12 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
                             F.ctr[3] = int32_t(sm.ctr[lane][3]);
                             F.next_a = 1;
                             entering = false;
-                            place = true;
+                            place = broad;
                         }
                     }
                 }
-                // (4) pack the sets of every expanded task into its stack, in entry order
+                if (any_broad) {
+                // (4) pack the sets of every larger task into its stack, in entry order
                 sm.cbase[lane] = F.cbase;
                 const int totx = warp_prefix(place ? 4 * int(F.size) : 0, sm.pref);
                 __syncwarp();
@@ -1487,52 +1692,12 @@ __global__ void __launch_bounds__(128, 6) k_search_fast(SearchArgs A0, SearchOut
                         S.t_meta[t] = S.x_meta[x];
                     }
                 }
+                }
                 __syncwarp();
             }
-            if (sc_sorted >= 0) sc = sc_sorted;
-            if (side == 0) count_b = sc;
-            else count_f = sc;
         }
-        // ---- phase C: publish
-        if (have) {
-            if (status != OVF_NONE) {
-                O.status[r] = uint8_t(status);
-                if (status != ERR_TOO_MANY) {
-                    unsigned k = atomicAdd(O.ovf_count, 1u);
-                    O.ovf_list[k] = idx_t(r);
-                }
-            } else {
-                unsigned long long base = 0;
-                bool ok = true;
-                if (ne) {
-                    base = atomicAdd(O.e_count, (unsigned long long)ne);
-                    if (base + ne > O.e_cap) {
-                        ok = false;
-                        O.status[r] = OVF_POOL;
-                        unsigned k = atomicAdd(O.ovf_count, 1u);
-                        O.ovf_list[k] = idx_t(r);
-                    } else {
-                        for (int e = 0; e < ne; ++e) {
-                            const uint32_t mt = S.e_meta[eb + e];
-                            O.e_dest[base + e] = S.e_dest[eb + e];
-                            O.e_trans[base + e] = S.e_trans[eb + e];
-                            O.e_len[base + e] = uint16_t(meta_len(mt));
-                            O.e_type[base + e] = uint8_t(meta_type(mt));
-                        }
-                    }
-                }
-                if (ok) {
-                    O.status[r] = OVF_NONE;
-                    O.num_B[r] = uint16_t(count_b);
-                    O.num_F[r] = uint16_t(count_f);
-                    O.olp_B[r] = s_olp[wid][lane][0];
-                    O.olp_F[r] = s_olp[wid][lane][1];
-                    O.edge_src[r] = base;
-                }
-            }
         }
-        __syncwarp();
-        }
+        if (!Q.count) break;
     }
     if (Q.count == 0 || cur >= 0) add_probes(O, probes);
 }
@@ -1803,7 +1968,7 @@ int search_fast_blocks(int L, int M, int num_sms) {
 
 static size_t scratch_layout(int M_max, size_t nwarps, int ebcap, void* base, WarpScratch* S, int cap = kTaskCap,
                              int frames = kTaskFrames, int pmax = kPMax) {
-    const size_t M = size_t(M_max);
+    const size_t M = size_t(M_max), pool = std::max(size_t(kFastPool), 4 * M);
     const size_t cand = nwarps * 32 * 4 * M, edg = nwarps * 32 * size_t(ebcap);
     const size_t tsk = nwarps * 32 * size_t(cap), spr = nwarps * 32 * 4 * size_t(pmax);
     const size_t emb = nwarps * 32 * size_t(pmax), frm = nwarps * 32 * size_t(frames);
@@ -1818,6 +1983,11 @@ static size_t scratch_layout(int M_max, size_t nwarps, int ebcap, void* base, Wa
     T.c_ll = reinterpret_cast<idx_t*>(take(cand * sizeof(idx_t)));
     T.c_uu = reinterpret_cast<idx_t*>(take(cand * sizeof(idx_t)));
     T.c_meta = reinterpret_cast<uint32_t*>(take(cand * 4));
+    T.p_ll = reinterpret_cast<idx_t*>(take(nwarps * pool * sizeof(idx_t)));
+    T.p_uu = reinterpret_cast<idx_t*>(take(nwarps * pool * sizeof(idx_t)));
+    T.p_meta = reinterpret_cast<uint32_t*>(take(nwarps * pool * 4));
+    T.queue = reinterpret_cast<FastTask*>(take(nwarps * kFastQueue * sizeof(FastTask)));
+    T.pool = int(pool);
     T.e_dest = reinterpret_cast<idx_t*>(take(edg * sizeof(idx_t)));
     T.e_trans = reinterpret_cast<int32_t*>(take(edg * 4));
     T.e_meta = reinterpret_cast<uint32_t*>(take(edg * 4));
