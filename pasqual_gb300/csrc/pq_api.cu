@@ -455,12 +455,12 @@ int pq_apply_sort_seeds(pq_ctx* ctx, int dir, uint64_t r0, uint64_t r1, pq_idx* 
     CK(s.ensure(nr * sizeof(idx_t)));
     CK(z.ensure(nr * sizeof(idx_t)));
     CK(d.ensure(nr * sizeof(uint16_t)));
-    const size_t tb = pq::sort_seeds_tmp_bytes(size_t(r1 - r0));
+    const size_t tb = pq::sort_seeds_tmp_bytes(size_t(r1 - r0), nr);
     CK(tmp.ensure(tb));
     CK(cudaMemcpyAsync(s.p, start, nr * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(z.p, size, nr * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(d.p, depth, nr * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->st));
-    CK(pq::sort_seeds(ctx->sa[dir].as<idx_t>(), ctx->pk[dir].as<uint64_t>(), idx_t(ctx->L), ctx->t, size_t(r0),
+    CK(pq::sort_seeds(ctx->sa[dir].as<idx_t>(), ctx->pk[dir].as<uint64_t>(), ctx->num_reads, idx_t(ctx->L), ctx->t, size_t(r0),
                       size_t(r1), d.as<uint16_t>(), s.as<idx_t>(), z.as<idx_t>(), tmp.p, tb, ctx->st));
     CK(cudaMemcpyAsync(start, s.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(size, z.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
@@ -612,11 +612,11 @@ int pq_get_sort_seeds(pq_ctx* ctx, int dir, pq_idx* start, pq_idx* size, uint16_
     CK(s.ensure(nr * sizeof(idx_t)));
     CK(z.ensure(nr * sizeof(idx_t)));
     CK(d.ensure(nr * sizeof(uint16_t)));
-    const size_t tb = pq::sort_seeds_tmp_bytes(n);
+    const size_t tb = pq::sort_seeds_tmp_bytes(n, nr);
     CK(tmp.ensure(tb));
     CK(pq::seed_init(ctx->reads.as<uint8_t>(), ctx->num_reads, idx_t(ctx->L), dir, ctx->C, d.as<uint16_t>(),
                      s.as<idx_t>(), z.as<idx_t>(), ctx->st));
-    CK(pq::sort_seeds(ctx->sa[dir].as<idx_t>(), ctx->pk[dir].as<uint64_t>(), idx_t(ctx->L), ctx->t, 0, n,
+    CK(pq::sort_seeds(ctx->sa[dir].as<idx_t>(), ctx->pk[dir].as<uint64_t>(), ctx->num_reads, idx_t(ctx->L), ctx->t, 0, n,
                       d.as<uint16_t>(), s.as<idx_t>(), z.as<idx_t>(), tmp.p, tb, ctx->st));
     if (start) CK(cudaMemcpyAsync(start, s.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
     if (size) CK(cudaMemcpyAsync(size, z.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));

@@ -27,8 +27,8 @@ cudaError_t kmer_table_clear(int k, idx_t* kt, cudaStream_t st);
 // then deepens them with the records of the buckets in rows [r0, r1).
 cudaError_t seed_init(const uint8_t* reads, idx_t num_reads, idx_t L, int dir, const idx_t C[6], uint16_t* depth,
                       idx_t* start, idx_t* size, cudaStream_t st);
-size_t sort_seeds_tmp_bytes(size_t rows);
-cudaError_t sort_seeds(const idx_t* sa, const uint64_t* pk, idx_t L, int t, size_t r0, size_t r1, uint16_t* depth,
+size_t sort_seeds_tmp_bytes(size_t rows, size_t num_reads);
+cudaError_t sort_seeds(const idx_t* sa, const uint64_t* pk, idx_t num_reads, idx_t L, int t, size_t r0, size_t r1, uint16_t* depth,
                        idx_t* start, idx_t* size, void* tmp, size_t tmp_bytes, cudaStream_t st);
 cudaError_t export_ref_layout(const OccBlock* blk, const idx_t* sb, idx_t num_reads, idx_t L,
                               const idx_t fix[4], uint64_t* bitmap, idx_t* sample, cudaStream_t st);
