@@ -710,7 +710,9 @@ __device__ __forceinline__ unsigned bins_exclusive(const unsigned* cnt, unsigned
 
 // ------------------------------------------------------------------------------ partition passes
 
-// how many suffixes start with each d1-bit prefix (padded with A)
+// how many suffixes start with each d1-bit prefix (padded with A).  Bound by integer instructions: 16
+// positions a thread from two 32-bit halves of the packed text; with 64-bit windows 113 M positions
+// took 0.15 ms, now 0.08.
 __global__ void __launch_bounds__(kSplitThreads) k_msd_hist(const uint64_t* __restrict__ pk, MsdPlan a,
                                                             unsigned long long* __restrict__ cnt) {
     __shared__ unsigned h[1 << kMaxDigit];
@@ -718,11 +720,20 @@ __global__ void __launch_bounds__(kSplitThreads) k_msd_hist(const uint64_t* __re
     for (int i = threadIdx.x; i < bins; i += kSplitThreads) h[i] = 0;
     __syncthreads();
     const size_t stride = size_t(gridDim.x) * kSplitThreads * 16;
-    for (size_t p0 = (size_t(blockIdx.x) * kSplitThreads + threadIdx.x) * 16; p0 < a.n; p0 += stride)
-        for_positions(pk, p0, a.n, a.dl, [&](int, size_t, uint64_t x, int m, int, bool) {
-            const uint64_t xm = m < 32 ? x & (~uint64_t(0) << (64 - 2 * m)) : x;
-            atomicAdd(&h[xm >> (64 - a.d1)], 1u);
-        });
+    const uint32_t* const half = reinterpret_cast<const uint32_t*>(pk);     // the words' halves, lower first
+    for (size_t p0 = (size_t(blockIdx.x) * kSplitThreads + threadIdx.x) * 16; p0 < a.n; p0 += stride) {
+        const uint32_t w0 = half[(p0 >> 4) ^ 1], w1 = half[((p0 >> 4) + 1) ^ 1];
+        const int left = int(a.n - p0 < 16 ? a.n - p0 : 16);
+        int m = suffix_bases(p0, a.dl);
+        #pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            uint32_t past;
+            asm("shr.u32 %0, %1, %2;" : "=r"(past) : "r"(0xffffffffu), "r"(2u * unsigned(m)));      // 0 from 32 on
+            const uint32_t x = __funnelshift_l(w1, w0, 2 * j) & ~past;
+            if (j < left) atomicAdd(&h[x >> (32 - a.d1)], 1u);
+            m = m == 1 ? int(a.dl.L) : m - 1;
+        }
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < bins; i += kSplitThreads)
         if (h[i]) atomicAdd(&cnt[i], (unsigned long long)h[i]);
@@ -741,12 +752,14 @@ __device__ __forceinline__ uint32_t bucket6(uint64_t x, int m) {
 // [c0, c1)) as an element into its d1-bit bucket.  Bound by the 8 bytes written per suffix (the
 // text is a quarter byte): a tile of 8192 positions is ranked with one shared-memory atomic a
 // suffix, takes its place in every bucket with one global atomic a bucket, and leaves through
-// shared memory in runs.
+// shared memory in runs.  That, not the 8 bytes, takes the time: the ranking, the way through shared
+// memory and their barriers; 113 M suffixes take 0.58 ms (0.65 with 64-bit windows), 0.16 at the rate of
+// a copy.
 struct MsdSmem {            // dynamic shared memory of the partition passes
     static constexpr size_t bins = size_t(1) << kMaxDigit;
     static constexpr size_t elems = size_t(kSplitTile) * 8;
     static constexpr size_t bytes(int bits, bool digits) {
-        return elems + (size_t(1) << bits) * (8 + 4 + 4) + (digits ? size_t(kSplitTile) * 2 : 0);
+        return elems + (size_t(1) << bits) * (sizeof(idx_t) + 4 + 4) + (digits ? size_t(kSplitTile) * 2 : 0);
     }
 };
 
@@ -757,10 +770,11 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_msd_text(const uint64_t* _
     __shared__ unsigned wsum[kSplitThreads / 32];
     const int bins = 1 << a.d1, tid = threadIdx.x;
     uint64_t* se = reinterpret_cast<uint64_t*>(msd_smem);
-    unsigned long long* gb = reinterpret_cast<unsigned long long*>(se + kSplitTile);
+    idx_t* gb = reinterpret_cast<idx_t*>(se + kSplitTile);          // element j of bucket d to out[gb[d] + j]
     unsigned* cnt = reinterpret_cast<unsigned*>(gb + bins);
     unsigned* start = cnt + bins;
     uint16_t* sd = reinterpret_cast<uint16_t*>(start + bins);
+    const uint32_t* const half = reinterpret_cast<const uint32_t*>(pk);     // the words' halves, lower first
     const bool chunk = c1 < uint32_t(kBuckets) || c0 > 0;
     const size_t tiles = (a.n + kSplitTile - 1) / kSplitTile;
     for (size_t t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -770,23 +784,45 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_msd_text(const uint64_t* _
         unsigned dr[16];                        // digit << 16 | rank within the tile's bucket
         #pragma unroll
         for (int j = 0; j < 16; ++j) dr[j] = ~0u;
-        for_positions(pk, t * kSplitTile + size_t(tid) * 16, a.n, a.dl,
-                      [&](int j, size_t p, uint64_t x, int m, int prev, bool dollar) {
-            if (m <= a.S) return;
-            if (chunk) {
-                const uint32_t c = bucket6(x, m);
-                if (c < c0 || c >= c1) return;
+        const size_t p0 = t * kSplitTile + size_t(tid) * 16;
+        if (p0 < a.n) {
+            // three halves of the packed text hold the windows of the 16 positions
+            const size_t w = p0 >> 4;
+            const uint32_t w0 = half[w ^ 1], w1 = half[(w + 1) ^ 1], w2 = half[(w + 2) ^ 1];
+            uint32_t prev = w ? half[(w - 1) ^ 1] & 3u : 0u;
+            const int left = int(a.n - p0 < 16 ? a.n - p0 : 16);
+            int m = suffix_bases(p0, a.dl);
+            #pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                uint32_t past0, past1;          // bits past the suffix's end
+                asm("shr.u32 %0, %1, %2;" : "=r"(past0) : "r"(0xffffffffu), "r"(2u * unsigned(m)));        // 0 from 32 on
+                asm("shr.u32 %0, %1, %2;" : "=r"(past1) : "r"(0xffffffffu), "r"(unsigned(max(2 * m - 32, 0))));
+                const uint32_t x0 = __funnelshift_l(w1, w0, 2 * j), x1 = __funnelshift_l(w2, w1, 2 * j);
+                const uint32_t y0 = x0 & ~past0, y1 = x1 & ~past1;
+                bool in = j < left && m > a.S;
+                if (chunk) {
+                    const uint32_t c = bucket6(uint64_t(y0) << 32, m);
+                    in = in && c >= c0 && c < c1;
+                }
+                if (in) {
+                    const unsigned d = y0 >> (32 - a.d1);
+                    const uint32_t k0 = __funnelshift_l(y1, y0, a.d1), k1 = y1 << a.d1;
+                    const uint64_t key = (((uint64_t(k0) << 32) | k1) >> (64 - a.kbits)) << a.key_shift;
+                    const uint32_t sym = m == int(a.dl.L) ? 0u : prev + 1u;
+                    v[j] = key | (uint64_t(unsigned(min(m, a.head))) << a.len_shift) | (uint64_t(p0) << kSymBits) |
+                           uint64_t((unsigned(j) << kSymBits) | sym);
+                    dr[j] = (d << 16) | atomicAdd(&cnt[d], 1u);
+                }
+                prev = x0 >> 30;
+                m = m == 1 ? int(a.dl.L) : m - 1;
             }
-            unsigned d;
-            v[j] = make_element(a, p, m, x, prev, dollar, d);
-            dr[j] = (d << 16) | atomicAdd(&cnt[d], 1u);
-        });
+        }
         __syncthreads();
         const unsigned total = bins_exclusive<kSplitThreads>(cnt, start, bins, wsum);
         __syncthreads();
         for (int d = tid; d < bins; d += kSplitThreads) {
             const unsigned c = cnt[d];
-            if (c) gb[d] = atomicAdd(&cursor[d], (unsigned long long)c) - start[d];
+            if (c) gb[d] = idx_t(atomicAdd(&cursor[d], (unsigned long long)c) - start[d]);
         }
         #pragma unroll
         for (int j = 0; j < 16; ++j)
@@ -796,7 +832,8 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_msd_text(const uint64_t* _
                 sd[q] = uint16_t(dr[j] >> 16);
             }
         __syncthreads();
-        for (unsigned j = tid; j < total; j += kSplitThreads) out[gb[sd[j]] + j] = se[j];
+        #pragma unroll 4
+        for (unsigned j = tid; j < total; j += kSplitThreads) out[idx_t(gb[sd[j]] + j)] = se[j];
         __syncthreads();
     }
 }
@@ -879,7 +916,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_msd_split(const uint64_t* 
     __shared__ unsigned wsum[kSplitThreads / 32];
     const int bins = 1 << r.bits, tid = threadIdx.x;
     uint64_t* se = reinterpret_cast<uint64_t*>(msd_smem);
-    unsigned long long* gb = reinterpret_cast<unsigned long long*>(se + kSplitTile);
+    idx_t* gb = reinterpret_cast<idx_t*>(se + kSplitTile);          // element j of bucket d to out[gb[d] + j]
     unsigned* cnt = reinterpret_cast<unsigned*>(gb + bins);
     unsigned* start = cnt + bins;
     const unsigned tiles = r.tile0[r.count];
@@ -906,15 +943,16 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_msd_split(const uint64_t* 
         __syncthreads();
         for (int d = tid; d < bins; d += kSplitThreads) {
             const unsigned c = cnt[d];
-            if (c) gb[d] = atomicAdd(&cursor[(size_t(q) << r.bits) + d], (unsigned long long)c) - start[d];
+            if (c) gb[d] = idx_t(atomicAdd(&cursor[(size_t(q) << r.bits) + d], (unsigned long long)c) - start[d]);
         }
         #pragma unroll
         for (int j = 0; j < kPer; ++j)
             if (tid + j * kSplitThreads < m) se[start[unsigned(v[j] >> shift) & (bins - 1)] + rk[j]] = v[j];
         __syncthreads();
+        #pragma unroll 4
         for (int j = tid; j < m; j += kSplitThreads) {
             const uint64_t e = se[j];
-            out[gb[unsigned(e >> shift) & (bins - 1)] + j] = e;
+            out[idx_t(gb[unsigned(e >> shift) & (bins - 1)] + idx_t(j))] = e;
         }
         __syncthreads();
     }
