@@ -117,7 +117,9 @@ struct pq_ctx {
     float ms_heavy = 0, ms_wide = 0;        // host time of the heavy and wide tiers
     bool graph_ok = false;
     uint64_t num_edges = 0, probes = 0, sectors = 0, wide_reads = 0;
+    unsigned long long* h_ctr = nullptr;    // the search's counters (ctrs), page-locked
 };
+constexpr size_t kCtrBytes = 64;
 
 static int fail(pq_ctx* c, int code, const std::string& msg) {
     if (c) c->err = msg;
@@ -222,6 +224,12 @@ int pq_create(pq_ctx** out, int device, void* cuda_stream) {
         }
         ctx->own_stream = true;
     }
+    if (cudaMallocHost(reinterpret_cast<void**>(&ctx->h_ctr), kCtrBytes) != cudaSuccess) {
+        cudaGetLastError();
+        if (ctx->own_stream) cudaStreamDestroy(ctx->st);
+        delete ctx;
+        return PQ_ERR_NOMEM;
+    }
     cudaEventCreate(&ctx->ev0);
     cudaEventCreate(&ctx->ev1);
     cudaEventCreate(&ctx->evk0);
@@ -255,6 +263,7 @@ void pq_destroy(pq_ctx* ctx) {
         ctx->lx_err_root[d].release();
         ctx->lx_segof[d].release();
     }
+    if (ctx->h_ctr) cudaFreeHost(ctx->h_ctr);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->evk0) cudaEventDestroy(ctx->evk0);
@@ -729,17 +738,21 @@ static cudaError_t grow_pool(pq_ctx* ctx, pq::SearchOut& O, size_t need, size_t 
     return cudaSuccess;
 }
 
-// After the first kernel (lean or fast): the other tiers for the reads it handed over, then the CSR
-// in read order.
+static cudaError_t read_counters(pq_ctx* ctx, cudaStream_t st) {
+    return cudaMemcpyAsync(ctx->h_ctr, ctx->ctrs.p, kCtrBytes, cudaMemcpyDeviceToHost, st);
+}
+
+// After the first kernel (lean or fast), its counters read: the other tiers for the reads it handed
+// over, then the CSR in read order, enqueued.  search_end waits for it.
 static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool lean) {
     const size_t nr = ctx->num_reads;
     const size_t nrp = nr + 1;
     unsigned long long* ctr = ctx->ctrs.as<unsigned long long>();
     unsigned long long hc[5];
-    CK(cudaMemcpyAsync(hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
+    std::memcpy(hc, ctx->h_ctr, sizeof hc);
     ctx->lx_misses = hc[3];
     unsigned ovf = unsigned(hc[2] & 0xffffffffu);
+    const bool more = ovf != 0;
     ctx->deferred_reads = lean ? ovf : 0;
     const idx_t* ovf_src = ctx->ovf_list.as<idx_t>();
     const unsigned* ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 2);     // device count of ovf_src
@@ -911,16 +924,16 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool 
         if (!list.empty()) return fail(ctx, PQ_ERR_INTERNAL, "edge pool retries exhausted");
     }
     if (ctx->wide_reads) ctx->ms_wide = wall_ms() - tw0;
-    // CSR in read order
+    // CSR in read order.  Its size is the edges reserved when one kernel took every read, else it is
+    // read back after the scan of the counts.
     CK(ctx->off.ensure(nrp * 8));
-    unsigned long long total = 0;
+    unsigned long long total = hc[0];
     size_t atb = pq::assemble_tmp_bytes(ctx->num_reads);
     CK(ctx->asm_tmp.ensure(atb));
-    // size the CSR from the per-read counts
-    {
-        CK(pq::assemble_counts_total(O, ctx->num_reads, ctx->off.as<unsigned long long>(), ctx->asm_tmp.p, atb,
-                                     ctx->st));
+    CK(pq::assemble_counts_total(O, ctx->num_reads, ctx->off.as<unsigned long long>(), ctx->asm_tmp.p, atb, ctx->st));
+    if (more) {
         CK(cudaMemcpyAsync(&total, ctx->off.as<unsigned long long>() + nr, 8, cudaMemcpyDeviceToHost, ctx->st));
+        CK(read_counters(ctx, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
     }
     CK(ctx->g_dest.ensure((total + 1) * sizeof(idx_t)));
@@ -930,16 +943,15 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool 
     CK(pq::assemble_gather(O, ctx->num_reads, ctx->off.as<unsigned long long>(), ctx->g_dest.as<idx_t>(),
                            ctx->g_len.as<uint16_t>(), ctx->g_type.as<uint8_t>(), ctx->g_trans.as<int32_t>(), ctx->st));
     CK(cudaEventRecord(ctx->ev1, ctx->st));
-    CK(cudaMemcpyAsync(hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, ctx->st));
-    unsigned long long sec = 0;
-    CK(cudaMemcpyAsync(&sec, ctr + 6, sizeof sec, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaEventSynchronize(ctx->ev1));
+    ctx->num_edges = total;
+    ctx->probes = ctx->h_ctr[1];
+    ctx->sectors = ctx->h_ctr[6];
+    return PQ_OK;
+}
+
+static int search_end(pq_ctx* ctx) {
     CK(cudaStreamSynchronize(ctx->st));
     cudaEventElapsedTime(&ctx->ms_search, ctx->ev0, ctx->ev1);
-    cudaEventElapsedTime(&ctx->ms_fast, ctx->evk0, ctx->evk1);
-    ctx->num_edges = total;
-    ctx->probes = hc[1];
-    ctx->sectors = sec;
     ctx->graph_ok = true;
     return PQ_OK;
 }
@@ -971,7 +983,12 @@ int pq_overlaps(pq_ctx* ctx) {
         CK(pq::search_fast(A, O, blocks, ctx->warp_scratch.p, wsb, ebcap, ctx->st));
     }
     CK(cudaEventRecord(ctx->evk1, ctx->st));
-    return search_finish(ctx, A, O, A.sorted_reduce != 0);
+    CK(read_counters(ctx, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
+    rc = search_finish(ctx, A, O, A.sorted_reduce != 0);
+    if (rc == PQ_OK) rc = search_end(ctx);
+    if (rc == PQ_OK) cudaEventElapsedTime(&ctx->ms_fast, ctx->evk0, ctx->evk1);
+    return rc;
 }
 
 int pq_get_graph_sizes(pq_ctx* ctx, uint64_t* num_edges, uint64_t* probes, uint64_t* wide_reads) {
@@ -999,10 +1016,15 @@ int pq_get_graph(pq_ctx* ctx, uint16_t* num_B, uint16_t* num_F, int32_t* olp_B, 
     if (!ctx->graph_ok) return fail(ctx, PQ_ERR_STATE, "pq_overlaps first");
     const size_t nr = ctx->num_reads, ne = ctx->num_edges;
     cudaStream_t s = ctx->st;
-    // page-locked destinations are written by the copy kernel, pageable ones by cudaMemcpy
+    // page-locked destinations are written by the copy kernel, all in one launch; pageable ones by
+    // cudaMemcpy
+    pq::CopyList locked{};
     auto d2h = [&](void* h, const DevBuf& b, size_t bytes) -> cudaError_t {
         if (!h || !bytes) return cudaSuccess;
-        if (void* locked = locked_device_ptr(h)) return pq::kernel_copy(locked, b.p, bytes, s);
+        if (void* p = locked_device_ptr(h)) {
+            locked.add(p, b.p, bytes);
+            return cudaSuccess;
+        }
         return cudaMemcpyAsync(h, b.p, bytes, cudaMemcpyDeviceToHost, s);
     };
     CK(d2h(num_B, ctx->nB, nr * 2));
@@ -1014,6 +1036,7 @@ int pq_get_graph(pq_ctx* ctx, uint16_t* num_B, uint16_t* num_F, int32_t* olp_B, 
     CK(d2h(len, ctx->g_len, ne * 2));
     CK(d2h(type, ctx->g_type, ne));
     CK(d2h(trans, ctx->g_trans, ne * 4));
+    CK(pq::kernel_copy(locked, s));
     CK(cudaStreamSynchronize(s));
     return PQ_OK;
 }
@@ -1425,16 +1448,26 @@ int pq_overlaps_batched(pq_ctx** ctxs, int count, int flags) {
     } else {
         lead->q_kernel_ms = 0;
     }
+    // every set's counters in one wait; then the sets' other tiers and CSRs, each on its own stream
+    for (int b = 0; b < count; ++b) CK(read_counters(ctxs[b], lead->st));
     CK(cudaStreamSynchronize(lead->st));
-    for (int b = 0; b < count; ++b) {
-        const int rc = search_finish(ctxs[b], hb[b].a, hb[b].o, all_lean(hb));
+    int rc = PQ_OK, done = 0;
+    for (; done < count; ++done) {
+        rc = search_finish(ctxs[done], hb[done].a, hb[done].o, all_lean(hb));
         if (rc != PQ_OK) {
+            if (done) fail(lead, rc, std::string("batch ") + std::to_string(done) + ": " + ctxs[done]->err);
+            break;
+        }
+    }
+    for (int b = 0; b < done; ++b) {
+        const int re = search_end(ctxs[b]);
+        if (re != PQ_OK && rc == PQ_OK) {
+            rc = re;
             if (b) fail(lead, rc, std::string("batch ") + std::to_string(b) + ": " + ctxs[b]->err);
-            return rc;
         }
         ctxs[b]->ms_fast = lead->q_kernel_ms;
     }
-    return PQ_OK;
+    return rc;
 }
 
 int pq_set_batch_plan(pq_ctx* lead, int ctas_per_sm, int groups_per_item, int edge_slots) {

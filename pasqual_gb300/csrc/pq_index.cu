@@ -428,9 +428,8 @@ cudaError_t build_occ(const idx_t* sa, const uint8_t* reads, idx_t num_reads, id
 // (cudaHostAlloc'd) buffer was measured at ~10 GB/s.  Bytes before the first 16-byte boundary
 // and after the last go one by one; when the two sides are not equally aligned the whole copy
 // goes byte by byte.
-__global__ void __launch_bounds__(256) k_copy_bytes(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src,
-                                                    size_t n) {
-    const size_t tid = size_t(blockIdx.x) * blockDim.x + threadIdx.x, stride = size_t(gridDim.x) * blockDim.x;
+__device__ __forceinline__ void copy_bytes(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, size_t n, size_t tid,
+                                           size_t stride) {
     const size_t mis = reinterpret_cast<uintptr_t>(src) & 15;
     if (mis != (reinterpret_cast<uintptr_t>(dst) & 15)) {
         for (size_t i = tid; i < n; i += stride) dst[i] = src[i];
@@ -453,16 +452,31 @@ __global__ void __launch_bounds__(256) k_copy_bytes(uint8_t* __restrict__ dst, c
     for (; i < n16; i += stride) d[i] = s[i];
 }
 
-cudaError_t kernel_copy(void* dst, const void* src, size_t n, cudaStream_t st) {
-    if (!n) return cudaSuccess;
+// several copies, one after the other (arrays of a few kilobytes to gigabytes: one launch for all)
+__global__ void __launch_bounds__(256) k_copy_bytes(CopyList c) {
+    const size_t tid = size_t(blockIdx.x) * blockDim.x + threadIdx.x, stride = size_t(gridDim.x) * blockDim.x;
+    for (int i = 0; i < c.count; ++i)
+        copy_bytes(static_cast<uint8_t*>(c.dst[i]), static_cast<const uint8_t*>(c.src[i]), c.bytes[i], tid, stride);
+}
+
+cudaError_t kernel_copy(const CopyList& c, cudaStream_t st) {
+    size_t most = 0;
+    for (int i = 0; i < c.count; ++i) most = std::max(most, c.bytes[i]);
+    if (!most) return cudaSuccess;
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const size_t want = (n / 16 + 255) / 256;
+    const size_t want = (most / 16 + 255) / 256;
     const unsigned blocks = unsigned(std::max<size_t>(1, std::min<size_t>(want, size_t(sms) * 32)));
-    k_copy_bytes<<<blocks, 256, 0, st>>>(static_cast<uint8_t*>(dst), static_cast<const uint8_t*>(src), n);
+    k_copy_bytes<<<blocks, 256, 0, st>>>(c);
     note_launch();
     return cudaGetLastError();
+}
+
+cudaError_t kernel_copy(void* dst, const void* src, size_t n, cudaStream_t st) {
+    CopyList c{};
+    c.add(dst, src, n);
+    return kernel_copy(c, st);
 }
 
 cudaError_t read_counts(const uint8_t* reads, idx_t num_reads, idx_t L, unsigned long long* out13,

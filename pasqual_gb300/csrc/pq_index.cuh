@@ -10,10 +10,22 @@ namespace pq {
 cudaError_t build_occ(const idx_t* sa, const uint8_t* reads, idx_t num_reads, idx_t L, int dir,
                       OccBlock* blk, idx_t* sb, idx_t* reads_index, cudaStream_t st, const uint64_t* pk = nullptr,
                       const uint8_t* hint = nullptr);
-// out13: base counts [4], last-base counts [4], first-base counts [4], bytes outside 1..4
 // n bytes between device memory and page-locked host memory (at its device-accessible address),
 // copied by a kernel
+struct CopyList {               // of kernel_copy: up to 9 copies in one launch
+    void* dst[9];
+    const void* src[9];
+    size_t bytes[9];
+    int count;
+    void add(void* d, const void* s, size_t n) {
+        dst[count] = d;
+        src[count] = s;
+        bytes[count++] = n;
+    }
+};
+cudaError_t kernel_copy(const CopyList& copies, cudaStream_t st);
 cudaError_t kernel_copy(void* dst, const void* src, size_t n, cudaStream_t st);
+// out13: base counts [4], last-base counts [4], first-base counts [4], bytes outside 1..4
 cudaError_t read_counts(const uint8_t* reads, idx_t num_reads, idx_t L, unsigned long long* out13,
                         cudaStream_t st);
 // k-mer table of direction dir from the suffix array and the packed text pk (one streaming pass)

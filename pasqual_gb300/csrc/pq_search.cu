@@ -3073,15 +3073,15 @@ cudaError_t search_wide(const SearchArgs& a, const SearchOut& o, const idx_t* li
 
 // ------------------------------------------------------------------------------ CSR assembly
 
-__global__ void k_edge_counts(const uint16_t* nB, const uint16_t* nF, idx_t n, unsigned long long* cnt) {
-    const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += stride)
-        cnt[r] = (unsigned long long)nB[r] + nF[r];
-}
-
 // exclusive scan of 64-bit counts: tiles of 1024 per CTA (3 passes)
-__global__ void k_scan_tiles(const unsigned long long* in, size_t n, unsigned long long* out,
-                             unsigned long long* tile_sums) {
+// of `in`, or of the reads' edge counts (the last entry is none)
+struct EdgeCounts {
+    const uint16_t *nB, *nF;
+    size_t reads;
+    __device__ unsigned long long operator[](size_t i) const { return i < reads ? (unsigned long long)nB[i] + nF[i] : 0ull; }
+};
+template <class In>
+__global__ void k_scan_tiles(In in, size_t n, unsigned long long* out, unsigned long long* tile_sums) {
     __shared__ unsigned long long warp_sum[32];
     const size_t tile = blockIdx.x;
     const size_t i = tile * 1024 + threadIdx.x;
@@ -3113,7 +3113,8 @@ __global__ void k_scan_add(unsigned long long* out, size_t n, const unsigned lon
     if (i < n) out[i] += tile_off[blockIdx.x];
 }
 
-static void scan_u64(const unsigned long long* in, size_t n, unsigned long long* out, unsigned long long* tmp,
+template <class In>
+static void scan_u64(In in, size_t n, unsigned long long* out, unsigned long long* tmp,
                      cudaStream_t st) {
     if (n == 0) return;
     size_t tiles = (n + 1023) / 1024;
@@ -3124,12 +3125,12 @@ static void scan_u64(const unsigned long long* in, size_t n, unsigned long long*
     unsigned long long* sums = tmp;
     unsigned long long* sums_scan = tmp + tiles;
     { k_scan_tiles<<<unsigned(tiles), 1024, 0, st>>>(in, n, out, sums); note_launch(); }
-    scan_u64(sums, tiles, sums_scan, tmp + 2 * tiles, st);
+    scan_u64<const unsigned long long*>(sums, tiles, sums_scan, tmp + 2 * tiles, st);
     { k_scan_add<<<unsigned(tiles), 1024, 0, st>>>(out, n, sums_scan); note_launch(); }
 }
 
 size_t assemble_tmp_bytes(idx_t num_reads) {
-    size_t n = size_t(num_reads) + 1, total = n;   // counts
+    size_t n = size_t(num_reads) + 1, total = 0;
     size_t t = (n + 1023) / 1024;
     while (t > 1) { total += 2 * t; t = (t + 1023) / 1024; }
     return (total + 64) * sizeof(unsigned long long);
@@ -3167,12 +3168,7 @@ cudaError_t assemble_counts_total(const SearchOut& o, idx_t num_reads, unsigned 
                                   size_t scan_tmp_bytes, cudaStream_t st) {
     const size_t n = size_t(num_reads);
     if (scan_tmp_bytes < assemble_tmp_bytes(num_reads)) return cudaErrorInvalidValue;
-    unsigned long long* cnt = reinterpret_cast<unsigned long long*>(scan_tmp);
-    unsigned long long* tmp = cnt + n + 1;
-    cudaMemsetAsync(cnt, 0, (n + 1) * sizeof(unsigned long long), st);
-    unsigned g = unsigned(std::min<size_t>((n + 255) / 256 + 1, 152 * 32));
-    if (n) { k_edge_counts<<<g, 256, 0, st>>>(o.num_B, o.num_F, idx_t(n), cnt); note_launch(); }
-    scan_u64(cnt, n + 1, out_off, tmp, st);
+    scan_u64(EdgeCounts{o.num_B, o.num_F, n}, n + 1, out_off, reinterpret_cast<unsigned long long*>(scan_tmp), st);
     return cudaGetLastError();
 }
 
