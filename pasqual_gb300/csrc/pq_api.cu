@@ -970,7 +970,7 @@ int pq_overlaps(pq_ctx* ctx) {
     if (nr && A.sorted_reduce) {
         // lean tier over every read; what it hands over is taken in search_finish
         const int ebcap = 64;
-        const int lean = int(std::min<size_t>((nr + 127) / 128, size_t(pq::search_lean_blocks(ctx->L, ctx->L - ctx->t, dev_sms))));
+        const int lean = int(std::min<size_t>((nr + 15) / 16, size_t(pq::search_lean_blocks(ctx->L, ctx->L - ctx->t, dev_sms))));
         const size_t wsb = pq::lean_scratch_bytes(ctx->L, ctx->t, lean, ebcap);
         CK(ctx->warp_scratch.ensure(wsb));
         CK(pq::search_lean(A, O, lean, ctx->warp_scratch.p, wsb, ebcap, ctx->st));

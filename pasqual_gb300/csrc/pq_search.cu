@@ -1724,7 +1724,7 @@ constexpr int kLeanThreads = 128;
 
 template <int W>
 __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, SearchOut O0, WarpScratch S,
-                                                                SearchQueue Q) {
+                                                                SearchQueue Q, int per) {
     __shared__ SearchBatch s_b[kLeanThreads / 32];
     __shared__ int s_pref[kLeanThreads / 32][33], s_m[kLeanThreads / 32][32];
     __shared__ idx_t s_qid[kLeanThreads / 32][64];              // rows waiting for their text to be checked:
@@ -1770,13 +1770,13 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
         } else {
             group = gw + iter * nw;
             gend = group + 1;
-            if (group * 32 >= size_t(A.num_reads)) break;
+            if (group * per >= size_t(A.num_reads)) break;
         }
-        for (; group < gend && group * 32 < size_t(A.num_reads); ++group) {
+        for (; group < gend && group * per < size_t(A.num_reads); ++group) {
             const int L = A.L, t = A.t, M = L - t;
-            const size_t r = group * 32 + lane;
+            const size_t r = group * per + lane;
             const idx_t self = idx_t(r);
-            const bool have = r < size_t(A.num_reads);
+            const bool have = lane < per && r < size_t(A.num_reads);
             bool ok = have;
             int ne = 0, status = OVF_NONE;
             int count_b = 0, count_f = 0;
@@ -1828,7 +1828,7 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                     const bool cmpl = (v >> 21) != 0;
                     const FmView& fa = cmpl ? *f1 : *f0;
                     const size_t text = size_t(rp) * size_t(L);
-                    const size_t src = (group * 32 + size_t(j)) * size_t(L) + size_t(len);
+                    const size_t src = (group * per + size_t(j)) * size_t(L) + size_t(len);
                     probes.add(0, base_sectors(text, d));
                     if (!text_matches(fa.pk, text, pks, src, d, cmpl, lanes)) return;
                     const int slot = atomicAdd(&slots[j], 1);
@@ -2030,14 +2030,24 @@ cudaError_t search_fast(const SearchArgs& a, const SearchOut& o, int blocks, voi
     return cudaGetLastError();
 }
 
+// Reads a warp takes: 32, or 16, 8 or 4 where there are not 32 for every warp resident.  A warp takes the
+// rows of its reads 32 at a time, so a quarter of the reads is nearly a quarter of its time (4.9
+// thousand reads of 100 bases: 87 us with 32 a warp, 31 with 4).
+static int lean_reads(size_t num_reads, int blocks) {
+    int per = 32;
+    while (per > 4 && num_reads <= size_t(blocks) * (kLeanThreads / 32) * size_t(per / 2)) per /= 2;
+    return per;
+}
+
 cudaError_t search_lean(const SearchArgs& a, const SearchOut& o, int blocks, void* scratch, size_t scratch_bytes, int ebcap,
                         cudaStream_t st) {
     WarpScratch S;
     if (scratch_bytes < scratch_layout(a.L - a.t, size_t(blocks) * (kLeanThreads / 32), ebcap, scratch, &S))
         return cudaErrorInvalidValue;
     SearchQueue none{};
-    if (lam_words(a.L - a.t) == 2) k_search_lean<2><<<blocks, kLeanThreads, 0, st>>>(a, o, S, none);
-    else k_search_lean<kLamWords><<<blocks, kLeanThreads, 0, st>>>(a, o, S, none);
+    const int per = lean_reads(size_t(a.num_reads), blocks);
+    if (lam_words(a.L - a.t) == 2) k_search_lean<2><<<blocks, kLeanThreads, 0, st>>>(a, o, S, none, per);
+    else k_search_lean<kLamWords><<<blocks, kLeanThreads, 0, st>>>(a, o, S, none, per);
     note_launch();
     return cudaGetLastError();
 }
@@ -2050,8 +2060,8 @@ cudaError_t search_lean_queue(const SearchQueue& q, int M_max, int blocks, void*
     if (scratch_bytes < scratch_layout(M_max, size_t(blocks) * (kLeanThreads / 32), ebcap, scratch, &S)) return cudaErrorInvalidValue;
     SearchArgs a0{};
     SearchOut o0{};
-    if (lam_words(M_max) == 2) k_search_lean<2><<<blocks, kLeanThreads, 0, st>>>(a0, o0, S, q);
-    else k_search_lean<kLamWords><<<blocks, kLeanThreads, 0, st>>>(a0, o0, S, q);
+    if (lam_words(M_max) == 2) k_search_lean<2><<<blocks, kLeanThreads, 0, st>>>(a0, o0, S, q, 32);
+    else k_search_lean<kLamWords><<<blocks, kLeanThreads, 0, st>>>(a0, o0, S, q, 32);
     note_launch();
     return cudaGetLastError();
 }

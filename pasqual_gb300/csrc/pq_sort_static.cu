@@ -15,7 +15,7 @@
 // scratch it reads back, and clears the histogram it accumulates, before use.
 //
 // Each call first counts the read bytes outside the base codes 1..4 (a count kept in a second
-// fixed device variable, cleared by the call) and refuses such input with PQ_ERR_ARG: the sort
+// fixed device variable, zero between calls: a call that counts any clears it) and refuses such input with PQ_ERR_ARG: the sort
 // packs 2 bits a base, so another byte would corrupt its neighbours' bits and give a wrong order.
 // The call synchronises its stream before it returns, so the suffix array is complete and any
 // kernel error is reported as PQ_ERR_CUDA.
@@ -88,13 +88,17 @@ extern "C" int pq_suffix_sort_static(const uint8_t* reads_dev, pq_idx num_reads,
     if (rc != PQ_OK) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
     const size_t nn = size_t(n);
-    k_clear_bad_codes<<<1, 1, 0, st>>>();
     k_count_bad_codes<<<unsigned((nn + 255) / 256 < 1024 ? (nn + 255) / 256 : 1024), 256, 0, st>>>(reads_dev, nn);
     unsigned long long bad = 0;
     if (cudaMemcpyFromSymbolAsync(&bad, g_bad_codes, sizeof bad, 0, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
+        cudaStreamSynchronize(st) != cudaSuccess) {
+        k_clear_bad_codes<<<1, 1, 0, st>>>();
         return PQ_ERR_CUDA;
-    if (bad) return PQ_ERR_ARG;
+    }
+    if (bad) {
+        k_clear_bad_codes<<<1, 1, 0, st>>>();
+        return cudaStreamSynchronize(st) == cudaSuccess ? PQ_ERR_ARG : PQ_ERR_CUDA;
+    }
     int e = pq::suffix_sort(reads_dev, idx_t(num_reads), read_len, dir, reinterpret_cast<idx_t*>(sa_dev), 0, scratch,
                             kScratchBytes, st);
     if (e != 0) return PQ_ERR_CUDA;

@@ -38,3 +38,19 @@ def test_rows_selected_give_the_oracles_graph(name, k, width):
         out = P.construct_string_graph()
     for f in ("num_B", "num_F", "olp_B", "olp_F", "edge_off", "dest", "length", "etype", "trans"):
         assert np.array_equal(getattr(out, f), getattr(ref, f)), f
+
+
+@pytest.mark.parametrize("count", [3, 33, 4_000, 30_000, 60_000, 120_000, 200_000])
+def test_reads_a_warp_by_their_number(count):
+    """A warp takes 4 to 32 reads by the number of reads: the graph is the walk's (seed mode 0)."""
+    gen = synth.genome(length=400 + count * 3, gc=0.45, repeat_frac=0.1, divergence=(0.0, 0.02), seed=71)
+    rd = synth.dedup(synth.reads_for_coverage(gen, 60, 22, 0.003, seed=72))[:count]
+    out = {}
+    for mode in (0, 1):
+        with pq.Pasqual(32) as P:
+            P.set_reads(rd, 30)
+            P.set_seed_mode(mode)
+            P.build_index()
+            out[mode] = P.construct_string_graph()
+    for f in ("num_B", "num_F", "olp_B", "olp_F", "edge_off", "dest", "length", "etype", "trans"):
+        assert np.array_equal(getattr(out[0], f), getattr(out[1], f)), f
