@@ -635,7 +635,7 @@ static int plan_words(const MsdPlan& p) {
 // multiply-high by floor(2^32 / L): the quotient is short by at most one below 2^32
 __device__ __forceinline__ int suffix_bases(size_t p, const DivL& dl) {
 #ifdef PQ_IDX64
-    return int(dl.L - uint32_t(p - div_l(p, dl) * dl.L));
+    return dl.L == 1 ? 1 : int(dl.L - uint32_t(p - div_l(p, dl) * dl.L));      // div_l: L of 2 and more
 #else
     const uint32_t x = uint32_t(p), q = __umulhi(x, dl.m32), r = x - q * dl.L;
     return int((r >= dl.L ? 2 * dl.L : dl.L) - r);
