@@ -2144,7 +2144,8 @@ constexpr int kBlockSmall = 4096, kBlockMid = 8192, kBlockLarge = 16384;    // c
 // Bound by the sort's instructions and its barriers.  The 3,645 run reads of the 200 Mbp workload at
 // 1/100 genome (150 bases, up to 6.7 thousand candidates of a kind) took 58 ms by pair tests in shared
 // memory and radix passes in global memory; 19 with the first words as keys; 16 with keys relative to
-// a pivot and one warp walking from class to class; 6 with the classes found by the scan.
+// a pivot and one warp walking from class to class; 6 with the classes found by the scan, 5.2 with
+// equal keys compared only from where they may differ.  (Two steps of the network at a time gave 5.0.)
 template <int CAP, int T>
 __global__ void __launch_bounds__(T) k_search_block(SearchArgs A, SearchOut O, const idx_t* list, unsigned count, const Cand* groups,
                                                     const BlockSide* sides, unsigned* next, unsigned char* region,
@@ -2260,17 +2261,19 @@ __global__ void __launch_bounds__(T) k_search_block(SearchArgs A, SearchOut O, c
                 key[i] = (uint64_t(unsigned(larger ? 1023 - l : l)) << 54) | ((rest >> 11) << 1) | uint64_t(l != n);
             }
             __syncthreads();
-            // a before b, whose keys are equal
+            // a before b, whose keys are equal.  Equal continuations of one kind stay as they were expanded,
+            // in row order, which is ascending read id; of two kinds only one is emitted.
             auto before = [&](int a, int b, uint64_t k) {
-                if (k & 1) {
-                    for (int w = 0; w < nw; ++w) {
+                if (k & 1) {                // equal up to 26 bases past where both leave the pivot
+                    const int l = int(k >> 54);
+                    for (int w = ((l < 512 ? l : 1023 - l) + 26) >> 5; w < nw; ++w) {
                         const uint64_t x = cw[size_t(w) * CAP + a], y = cw[size_t(w) * CAP + b];
                         if (x != y) return x < y;
                     }
                     const int la = length(a), lb = length(b);
                     if (la != lb) return la < lb;
                 }
-                return cid[a] < cid[b];
+                return a < b;
             };
             auto exchange = [&](int a, int b) {
                 if (b >= m) return;
