@@ -5,7 +5,7 @@ index with the batched (queued, graph-replayed) search against the plain GPU bac
 Workload (default): 250 Mbp synthetic genome, GC 42 %, 15 % repeat copies of 1-5 kbp segments at
 0.5-2 % divergence; 100 bp reads at 20x from both strands (50 M reads) with 0.5 % substitution
 errors; t = 55; 64-bit index, 4.8 G suffixes per index after de-duplication (equal or
-reverse-complement reads dropped), sorted in chunks.  Data is seeded synthetic.
+reverse-complement reads dropped).  Data is seeded synthetic.
 
 A step is one overlap search (find_intervals + transitive reduction + edge CSR) over every read,
 with both indexes resident in HBM, in the library's default seed mode (1: depth-t interval scan

@@ -144,11 +144,10 @@ PQ_API int pq_set_seed_k (pq_ctx * ctx, int k);
 
 /* How the candidates of each read are found.  0 walks from the depth-k seed to depth L with one
  * synchronised backward-search step per base, as the reference does from its sort-recorded seed
- * (src/string_graph.c:207-237).  1 (default) finds the depth-t interval of the walked index by
- * binary search over its suffix array inside the k-mer table interval of the pattern's first k
- * bases, reads that interval's rows once (a read r' whose suffix at offset o matches, and whose
- * first o bases continue the pattern, is a candidate at depth t + o) and takes the other index's
- * interval from the inverse suffix array.  2 is mode 1 with the learned index's window in place
+ * (src/string_graph.c:207-237).  1 (default) takes the rows of the walked index that start with the
+ * pattern's first k bases, narrowed by the bases kept beside them, and checks each against the
+ * pattern (a read r' whose suffix at offset o matches the first t bases, and whose first o bases
+ * continue the pattern, is a candidate at depth t + o).  2 is mode 1 with the learned index's window in place
  * of the k-mer table's (t >= 16).  Modes 1 and 2 apply when L - t <= 256 and
  * 4^min(t, 64) > 64 * num_reads * read_len (depth-t intervals are small; beyond 64 bases the
  * pattern is checked row by row); a read whose depth-t interval exceeds 256 rows walks.  All

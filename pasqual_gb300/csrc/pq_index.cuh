@@ -74,7 +74,7 @@ struct SearchArgs {
     int t;
     DivL dl;                    // division by L
     int seed_k;                 // k-mer seed depth (0 = start at depth 1 from C[])
-    int sa_seed;                // 1: candidates by depth-t interval scan (needs fm[].sa/pk/isa),
+    int sa_seed;                // 1: candidates by depth-t interval scan (needs fm[].sa/pk),
                                 // 2: the same with learned windows (needs fm[].lx)
     unsigned long long* lx_misses;  // learned windows that missed (those chains walk)
     int sorted_reduce;          // 1: edges from sorted continuations (L - t <= 256)

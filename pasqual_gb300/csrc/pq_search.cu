@@ -1059,13 +1059,11 @@ __device__ __forceinline__ int reduce_gathered(int L, const WarpScratch& S, idx_
 // (r', o) of I_t is a candidate at depth t + o -- and its continuation is the rest of r' after the
 // overlap: the walked index's text right after the matched pattern, at the row's text position
 // plus t (complemented for the kinds walked on the backward index, B-F and F-F).  So the lean tier
-// gathers each side's candidates for reduce_gathered straight from the scan, without the
-// depth-indexed candidate slots, the inverse-SA load of every candidate depth and the suffix-array
-// reload of every candidate that the group form (scan_pair + reduce_sorted) needs.
+// gathers each side's candidates for reduce_gathered straight from the scan.
 
 // Rows [first, end) of each chain's index to check for the patterns P0 and P1 of one side's chains,
 // all rows that start with their first t bases among them; false when the scan does not apply to this
-// read (a depth-t interval of more than kScanMax rows, or a learned window that missed): the fast
+// read (a depth-t interval of more than kScanMax rows, or a learned window that missed): the block
 // tier then redoes it.
 
 // The window of the learned index, narrowed to I_t (seed mode 2).
