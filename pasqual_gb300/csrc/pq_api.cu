@@ -1330,7 +1330,7 @@ static int queue_launch(pq_ctx* lead, const std::vector<pq::SearchBatch>& hb, co
         if (lead->q_ctas_per_sm > 0) per_sm = std::min(lead->q_ctas_per_sm, per_sm);
         Plan& p = plan[k];
         p.blocks = int(std::max<size_t>(1, std::min<size_t>(size_t(per_sm) * dev_sms, (c.ib.size() + 3) / 4)));
-        p.wsb = pq::queue_scratch_bytes(c.L_max, c.M_max, size_t(p.blocks) * 4, lead->q_ebcap);
+        p.wsb = pq::queue_scratch_bytes(c.M_max, size_t(p.blocks) * 4, lead->q_ebcap, lean);
         p.first = nitems;
         nitems += c.ib.size();
         scratch = std::max(scratch, p.wsb);

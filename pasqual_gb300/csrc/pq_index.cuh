@@ -161,7 +161,7 @@ cudaError_t search_lean_queue(const SearchQueue& q, int M_max, int blocks, void*
                               cudaStream_t st);
 constexpr int lam_words_host(int M) { return M <= 64 ? 2 : 8; }
 // One persistent launch over a queue of batches (L_max, M_max: the largest L and L - t).
-size_t queue_scratch_bytes(int L_max, int M_max, size_t nwarps, int ebcap);
+size_t queue_scratch_bytes(int M_max, size_t nwarps, int ebcap, bool lean);
 cudaError_t search_fast_queue(const SearchQueue& q, int L_max, int M_max, int blocks, void* scratch,
                               size_t scratch_bytes, int ebcap, cudaStream_t st);
 

@@ -1965,11 +1965,11 @@ int search_fast_blocks(int L, int M, int num_sms) {
 }
 
 static size_t scratch_layout(int M_max, size_t nwarps, int ebcap, void* base, WarpScratch* S, int cap = kTaskCap,
-                             int frames = kTaskFrames, int pmax = kPMax) {
-    const size_t M = size_t(M_max), pool = std::max(size_t(kFastPool), 4 * M);
-    const size_t cand = nwarps * 32 * 4 * M, edg = nwarps * 32 * size_t(ebcap);
-    const size_t tsk = nwarps * 32 * size_t(cap), spr = nwarps * 32 * 4 * size_t(pmax);
-    const size_t emb = nwarps * 32 * size_t(pmax), frm = nwarps * 32 * size_t(frames);
+                             int frames = kTaskFrames, int pmax = kPMax, bool lean = false) {
+    const size_t M = size_t(M_max), pool = std::max(size_t(kFastPool), 4 * M), edg = nwarps * 32 * size_t(ebcap);
+    const size_t dfs = lean ? 0 : nwarps;                   // warps that walk and run the DFS
+    const size_t cand = dfs * 32 * 4 * M, tsk = dfs * 32 * size_t(cap), spr = dfs * 32 * 4 * size_t(pmax);
+    const size_t emb = dfs * 32 * size_t(pmax), frm = dfs * 32 * size_t(frames);
     char* p = static_cast<char*>(base);
     size_t used = 0;
     auto take = [&](size_t bytes) {
@@ -1981,10 +1981,10 @@ static size_t scratch_layout(int M_max, size_t nwarps, int ebcap, void* base, Wa
     T.c_ll = reinterpret_cast<idx_t*>(take(cand * sizeof(idx_t)));
     T.c_uu = reinterpret_cast<idx_t*>(take(cand * sizeof(idx_t)));
     T.c_meta = reinterpret_cast<uint32_t*>(take(cand * 4));
-    T.p_ll = reinterpret_cast<idx_t*>(take(nwarps * pool * sizeof(idx_t)));
-    T.p_uu = reinterpret_cast<idx_t*>(take(nwarps * pool * sizeof(idx_t)));
-    T.p_meta = reinterpret_cast<uint32_t*>(take(nwarps * pool * 4));
-    T.queue = reinterpret_cast<FastTask*>(take(nwarps * kFastQueue * sizeof(FastTask)));
+    T.p_ll = reinterpret_cast<idx_t*>(take(dfs * pool * sizeof(idx_t)));
+    T.p_uu = reinterpret_cast<idx_t*>(take(dfs * pool * sizeof(idx_t)));
+    T.p_meta = reinterpret_cast<uint32_t*>(take(dfs * pool * 4));
+    T.queue = reinterpret_cast<FastTask*>(take(dfs * kFastQueue * sizeof(FastTask)));
     T.pool = int(pool);
     T.e_dest = reinterpret_cast<idx_t*>(take(edg * sizeof(idx_t)));
     T.e_trans = reinterpret_cast<int32_t*>(take(edg * 4));
@@ -2008,6 +2008,10 @@ static size_t scratch_layout(int M_max, size_t nwarps, int ebcap, void* base, Wa
     T.mstride = int(M);
     if (S) *S = T;
     return used;
+}
+
+static size_t lean_layout(int M_max, size_t nwarps, int ebcap, void* base, WarpScratch* S) {
+    return scratch_layout(M_max, nwarps, ebcap, base, S, kTaskCap, kTaskFrames, kPMax, true);
 }
 
 size_t warp_scratch_bytes(int L, int t, size_t nwarps, int ebcap) {
@@ -2040,7 +2044,7 @@ static int lean_reads(size_t num_reads, int blocks) {
 cudaError_t search_lean(const SearchArgs& a, const SearchOut& o, int blocks, void* scratch, size_t scratch_bytes, int ebcap,
                         cudaStream_t st) {
     WarpScratch S;
-    if (scratch_bytes < scratch_layout(a.L - a.t, size_t(blocks) * (kLeanThreads / 32), ebcap, scratch, &S))
+    if (scratch_bytes < lean_layout(a.L - a.t, size_t(blocks) * (kLeanThreads / 32), ebcap, scratch, &S))
         return cudaErrorInvalidValue;
     SearchQueue none{};
     const int per = lean_reads(size_t(a.num_reads), blocks);
@@ -2055,7 +2059,7 @@ cudaError_t search_lean(const SearchArgs& a, const SearchOut& o, int blocks, voi
 cudaError_t search_lean_queue(const SearchQueue& q, int M_max, int blocks, void* scratch, size_t scratch_bytes, int ebcap,
                               cudaStream_t st) {
     WarpScratch S;
-    if (scratch_bytes < scratch_layout(M_max, size_t(blocks) * (kLeanThreads / 32), ebcap, scratch, &S)) return cudaErrorInvalidValue;
+    if (scratch_bytes < lean_layout(M_max, size_t(blocks) * (kLeanThreads / 32), ebcap, scratch, &S)) return cudaErrorInvalidValue;
     SearchArgs a0{};
     SearchOut o0{};
     if (lam_words(M_max) == 2) k_search_lean<2><<<blocks, kLeanThreads, 0, st>>>(a0, o0, S, q, 32);
@@ -2065,7 +2069,7 @@ cudaError_t search_lean_queue(const SearchQueue& q, int M_max, int blocks, void*
 }
 
 size_t lean_scratch_bytes(int L, int t, int blocks, int ebcap) {
-    return scratch_layout(L - t, size_t(blocks) * (kLeanThreads / 32), ebcap, nullptr, nullptr);
+    return lean_layout(L - t, size_t(blocks) * (kLeanThreads / 32), ebcap, nullptr, nullptr);
 }
 
 // ------------------------------------------------------------------------------ block tier
@@ -2998,9 +3002,8 @@ cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* l
     return cudaGetLastError();
 }
 
-size_t queue_scratch_bytes(int L_max, int M_max, size_t nwarps, int ebcap) {
-    (void)L_max;
-    return scratch_layout(M_max, nwarps, ebcap, nullptr, nullptr);
+size_t queue_scratch_bytes(int M_max, size_t nwarps, int ebcap, bool lean) {
+    return lean ? lean_layout(M_max, nwarps, ebcap, nullptr, nullptr) : scratch_layout(M_max, nwarps, ebcap, nullptr, nullptr);
 }
 
 cudaError_t search_fast_queue(const SearchQueue& q, int L_max, int M_max, int blocks, void* scratch,
