@@ -1132,12 +1132,13 @@ __global__ void k_short_runs(const uint64_t* __restrict__ pk, const uint32_t* __
 }
 
 // the rows of the short suffixes: before their bucket's long ones; those of at least k bases also
-// belong to a k-mer (k <= S only: kt null otherwise)
+// belong to a k-mer (k <= S only: kt null otherwise), and where it has them (kx_bits) its rows' next
+// bases, padded with A as in an element
 __global__ void k_short_place(const uint64_t* __restrict__ pk, const uint32_t* __restrict__ key,
                               const idx_t* __restrict__ val, size_t m, DivL dl, int bits,
                               const unsigned long long* __restrict__ count, const unsigned long long* __restrict__ first,
                               const unsigned long long* __restrict__ lstart, idx_t* __restrict__ sa,
-                              uint8_t* __restrict__ bwt, idx_t* __restrict__ kt, int k) {
+                              uint8_t* __restrict__ bwt, idx_t* __restrict__ kt, int k, uint16_t* __restrict__ kx, int kx_bits) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
         const idx_t p = val[i];
@@ -1145,8 +1146,11 @@ __global__ void k_short_place(const uint64_t* __restrict__ pk, const uint32_t* _
         const size_t row = size_t(lstart[b] - count[b] + (i - first[b]));
         sa[row] = p;
         if (bwt) bwt[row] = uint8_t(key[i] >> kShortSym);
-        if (kt && suffix_bases(size_t(p), dl) >= k) {
-            const size_t c = size_t(window(pk, size_t(p)) >> (64 - 2 * k));
+        const int left = suffix_bases(size_t(p), dl);
+        if (kt && left >= k) {
+            const uint64_t x = window(pk, size_t(p)) & (~uint64_t(0) << (64 - 2 * left));
+            const size_t c = size_t(x >> (64 - 2 * k));
+            if (kx_bits) kx[row] = uint16_t((x << (2 * k)) >> (64 - kx_bits));
             atomicMin(reinterpret_cast<kmer_int*>(kt + 2 * c), kmer_int(row));
             atomicMax(reinterpret_cast<kmer_int*>(kt + 2 * c + 1), kmer_int(row));
         }
@@ -2469,7 +2473,7 @@ int msd_pass(const MsdPlan& P, size_t nr, const MsdScratch& s, const SortOut& o,
     }
     if (P.S) {
         k_short_place<<<gs, 256, 0, st>>>(s.pk, sk0, sv0, nshort, P.dl, bits, s.shorts, s.sfirst, s.lstart, o.sa, o.bwt,
-                                          o.kmer_k <= P.S ? o.kt : nullptr, o.kmer_k);
+                                          o.kmer_k <= P.S ? o.kt : nullptr, o.kmer_k, o.kx, 2 * o.kx_bases);
         note_launch();
     }
     MsdLocal a{};
