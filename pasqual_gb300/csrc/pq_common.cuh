@@ -83,6 +83,16 @@ inline DivL make_divl(uint32_t L) { return DivL{~uint64_t(0) / L + 1, L, ~uint32
 __device__ __forceinline__ uint64_t div_l(uint64_t p, const DivL& d) { return __umul64hi(p, d.m); }
 
 namespace pq {
+// Lets `kernel` be launched with up to Bytes of dynamic shared memory.  The limit belongs to the
+// function on the device, so to every thread and context of the process: Bytes is the kernel's own
+// largest, known at compile time, and never the size of one call, which another thread's smaller one
+// could take back between this and the launch.
+template <size_t Bytes, class... Args>
+inline cudaError_t allow_smem(void (*kernel)(Args...)) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Bytes));
+}
+constexpr size_t kMaxSmem = 227 * 1024;     // of a block, static and dynamic
+
 // Count of kernels this library has launched (reported through pq_get_kernel_stats).
 void note_launch();
 unsigned long long launch_count();

@@ -2872,7 +2872,8 @@ static int block_ctas(unsigned count) {
     int dev = 0, sms = 152, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(k_search_block<CAP, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(block_smem_bytes(CAP)));
+    const cudaError_t allowed = allow_smem<block_smem_bytes(CAP)>(k_search_block<CAP, T>);
+    if (allowed != cudaSuccess) cudaGetLastError();         // the launch reports it
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_search_block<CAP, T>, T, block_smem_bytes(CAP));
     if (e != cudaSuccess) cudaGetLastError();
     return int(std::min<unsigned>(count, unsigned(sms * (e == cudaSuccess && per > 0 ? per : 1))));
@@ -2910,13 +2911,16 @@ cudaError_t search_block(const SearchArgs& a, const SearchOut& o, const idx_t* l
     BlockSide* sides = reinterpret_cast<BlockSide*>(p + at[1]);
     Cand* groups = reinterpret_cast<Cand*>(p + at[2]);
     const size_t rd = size_t((a.L + 15) / 16) * kWalkThreads * 4;
-    cudaError_t e = cudaFuncSetAttribute(k_block_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rd));
+    if (rd > kMaxSmem) return cudaErrorInvalidValue;
+    cudaError_t e = allow_smem<kMaxSmem>(k_block_walk);
     if (e != cudaSuccess) return e;
     for (unsigned b = 0; b < count; b += kWalkBatch) {
         const unsigned nb = std::min(count - b, kWalkBatch);
         e = cudaMemsetAsync(next, 0, 256, st);
         if (e != cudaSuccess) return e;
         k_block_walk<<<(2 * nb + kWalkThreads - 1) / kWalkThreads, kWalkThreads, rd, st>>>(a, o, list + b, nb, groups, sides);
+        e = cudaGetLastError();                             // the next kernels index by what this leaves
+        if (e != cudaSuccess) return e;
         note_launch();
         unsigned char* region = reinterpret_cast<unsigned char*>(p + at[3]);
         k_search_block<kBlockSmall, 256><<<block_ctas<kBlockSmall, 256>(nb), 256, block_smem_bytes(kBlockSmall), st>>>(
@@ -2986,12 +2990,12 @@ cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* l
     SearchQueue Q{};
     Q.read_list = list;
     Q.list_count = count;
-    // static shared memory (~47 KB) plus the reads: past the 48 KB a launch may take unasked
+    // static shared memory (~46 KB) plus the reads: past the 48 KB a launch may take unasked
+    constexpr size_t kReadSmem = 180 * 1024;            // reads of up to 5760 bases
+    if (smem > kReadSmem) return cudaErrorInvalidValue;
     cudaError_t e = lam_words(a.L - a.t) == 2
-        ? cudaFuncSetAttribute(k_search_fast<2, kHeavyCap, kHeavyFrames, kHeavyPMax>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))
-        : cudaFuncSetAttribute(k_search_fast<kLamWords, kHeavyCap, kHeavyFrames, kHeavyPMax>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        ? allow_smem<kReadSmem>(k_search_fast<2, kHeavyCap, kHeavyFrames, kHeavyPMax>)
+        : allow_smem<kReadSmem>(k_search_fast<kLamWords, kHeavyCap, kHeavyFrames, kHeavyPMax>);
     if (e != cudaSuccess) return e;
     if (lam_words(a.L - a.t) == 2)
         k_search_fast<2, kHeavyCap, kHeavyFrames, kHeavyPMax><<<blocks, 32 * kWarpsPerCta, smem, st>>>(a, o, S, Q);

@@ -395,7 +395,7 @@ k_rs_downsweep(const K* __restrict__ kin, const V* __restrict__ vin, K* __restri
 }
 
 template <class K, class V>
-static size_t rs_down_smem() {
+static constexpr size_t rs_down_smem() {
     constexpr int T = RsCfg<K, V>::threads, TILE = RsCfg<K, V>::tile;
     return 2 * size_t(TILE) * (sizeof(K) + sizeof(V)) + size_t(T / 32 + 2) * 256 * 4 + 32 * 4 + 256 * 8;
 }
@@ -431,8 +431,9 @@ int radix_sort_pairs(K** k0, V** v0, K** k1, V** v1, size_t n, int lo_bit, int h
     size_t tiles = (n + RS_TILE_MAX - 1) / RS_TILE_MAX;
     // one wave of resident CTAs: as many per SM as the downsweep's shared memory and registers
     // allow (a grid sized for more ran a second, partial wave on a fraction of the SMs)
-    const size_t smem = rs_down_smem<K, V>();
-    cudaFuncSetAttribute(k_rs_downsweep<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    constexpr size_t smem = rs_down_smem<K, V>();
+    const cudaError_t allowed = allow_smem<smem>(k_rs_downsweep<K, V>);
+    if (allowed != cudaSuccess) return int(allowed);
     int dev = 0, sms = 152, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2179,10 +2180,14 @@ struct MsdKernels {
         if (e != cudaSuccess) cudaGetLastError();
         return (e == cudaSuccess && per > 0 ? per : 1) * sms;
     }
-    static void prepare() {
-        cudaFuncSetAttribute(k_msd_local<W, kLocalSmall, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(local_smem<kLocalSmall>()));
-        cudaFuncSetAttribute(k_msd_local<W, kLocalLarge, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(local_smem<kLocalLarge>()));
-        cudaFuncSetAttribute(k_refine_cta<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(size_t(W + 2) * 1024 * sizeof(uint64_t)));
+    static constexpr size_t kCtaSmem = size_t(W + 2) * 1024 * sizeof(uint64_t);
+    static cudaError_t prepare() {
+        cudaError_t e = allow_smem<local_smem<kLocalSmall>()>(k_msd_local<W, kLocalSmall, 128>);
+        if (e == cudaSuccess) e = allow_smem<local_smem<kLocalLarge>()>(k_msd_local<W, kLocalLarge, 256>);
+        if (e == cudaSuccess) e = allow_smem<kCtaSmem>(k_refine_cta<W>);
+        if (e == cudaSuccess) e = allow_smem<MsdSmem::bytes(kMaxDigit, true)>(k_msd_text);
+        if (e == cudaSuccess) e = allow_smem<MsdSmem::bytes(kMaxDigit, false)>(k_msd_split);
+        return e;
     }
     static void local(bool large, MsdLocal a, const MsdScratch& s, size_t most, int sms, cudaStream_t st) {
         a.list = large ? s.large : s.small;
@@ -2198,8 +2203,7 @@ struct MsdKernels {
         const unsigned g = unsigned(std::max<size_t>(1, std::min<size_t>((warps + 7) / 8, size_t(sms) * 4)));
         k_refine_warp<W><<<g, kRefineThreads, 0, st>>>(s.mid, &s.counters->mid, a.pk, a.plan.dl, a.sa, a.bwt);
         note_launch();
-        const size_t smem = size_t(W + 2) * 1024 * sizeof(uint64_t);
-        k_refine_cta<W><<<unsigned(std::min<size_t>(s.cap_big, size_t(sms) * 2)), 512, smem, st>>>(
+        k_refine_cta<W><<<unsigned(std::min<size_t>(s.cap_big, size_t(sms) * 2)), 512, kCtaSmem, st>>>(
             s.big, &s.counters->big, a.pk, a.plan.dl, a.sa, a.bwt);
         note_launch();
     }
@@ -2361,6 +2365,8 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
                 }
                 h2d(s.r_cursor, cur.data(), nc * 8);
                 k_msd_split<<<grid(), kSplitThreads, MsdSmem::bytes(kMoreBits, false), st>>>(a.buf, r, s.r_cursor, tmp);
+                const cudaError_t es = cudaGetLastError();
+                if (es != cudaSuccess) return int(es);
                 note_launch();
                 k_more_copy<<<grid(), kSplitThreads, 0, st>>>(tmp, r, a.buf);
                 note_launch();
@@ -2420,9 +2426,8 @@ int msd_pass(const MsdPlan& P, size_t nr, const MsdScratch& s, const SortOut& o,
     const size_t tiles = (P.n + kSplitTile - 1) / kSplitTile;
     const unsigned wide = unsigned(std::min<size_t>(tiles, size_t(sms) * 2));
     const size_t smem_text = MsdSmem::bytes(P.d1, true), smem_split = MsdSmem::bytes(std::max(P.d2, kMoreBits), false);
-    cudaFuncSetAttribute(k_msd_text, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_text));
-    cudaFuncSetAttribute(k_msd_split, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_split));
-    MsdKernels<W>::prepare();
+    const cudaError_t allowed = MsdKernels<W>::prepare();
+    if (allowed != cudaSuccess) return int(allowed);
 
     cudaMemsetAsync(s.counters, 0, s.clear_bytes, st);
     if (hist6) {
@@ -2452,11 +2457,15 @@ int msd_pass(const MsdPlan& P, size_t nr, const MsdScratch& s, const SortOut& o,
     if (!P.d2) {
         k_msd_children<<<1, kScanThreads, 0, st>>>(s.hist, P.S ? s.shorts : nullptr, P.d1, 1, nullptr, s.lstart, s.cursor, 1, G);
         k_msd_text<<<wide, kSplitThreads, smem_text, st>>>(s.pk, P, s.cursor, s.b, c0, c1);
+        const cudaError_t e = cudaGetLastError();           // the next kernels index by what these leave
+        if (e != cudaSuccess) return int(e);
         note_launch();
         note_launch();
     } else {
         k_msd_children<<<1, kScanThreads, 0, st>>>(s.hist, nullptr, P.d1, 1, nullptr, s.start1, s.cursor1, 0, G);
         k_msd_text<<<wide, kSplitThreads, smem_text, st>>>(s.pk, P, s.cursor1, ea, c0, c1);
+        const cudaError_t et = cudaGetLastError();          // the next kernels index by what these leave
+        if (et != cudaSuccess) return int(et);
         k_msd_tiles<<<1, 1024, 0, st>>>(s.start1, s.cursor1, int(bins1), s.tile0);
         MsdRanges r{};
         r.start = s.start1;
@@ -2469,6 +2478,8 @@ int msd_pass(const MsdPlan& P, size_t nr, const MsdScratch& s, const SortOut& o,
         k_msd_children<<<unsigned(bins1), kScanThreads, 0, st>>>(s.cnt, P.S ? s.shorts : nullptr, P.d2, 0, s.start1, s.lstart,
                                                                  s.cursor, 1, G);
         k_msd_split<<<unsigned(sms * 2), kSplitThreads, smem_split, st>>>(ea, r, s.cursor, s.b);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return int(e);
         for (int i = 0; i < 6; ++i) note_launch();
     }
     if (P.S) {
@@ -2571,9 +2582,10 @@ __global__ void __launch_bounds__(kHistThreads) k_bucket_hist(const uint64_t* __
 
 static int bucket_hist(const uint64_t* pk, size_t n, const DivL& dl, unsigned long long* dev, std::vector<unsigned long long>& h,
                        cudaStream_t st) {
-    const size_t hsm = size_t(kBuckets) * sizeof(unsigned);
+    constexpr size_t hsm = size_t(kBuckets) * sizeof(unsigned);
+    const cudaError_t allowed = allow_smem<hsm>(k_bucket_hist);
+    if (allowed != cudaSuccess) return int(allowed);
     cudaMemsetAsync(dev, 0, size_t(kBuckets) * 8, st);
-    cudaFuncSetAttribute(k_bucket_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, int(hsm));
     { k_bucket_hist<<<unsigned(device_sms()), kHistThreads, hsm, st>>>(pk, n, dl, dev); note_launch(); }
     h.resize(kBuckets);
     cudaMemcpyAsync(h.data(), dev, size_t(kBuckets) * 8, cudaMemcpyDeviceToHost, st);
