@@ -22,6 +22,7 @@
 // 64-bit keys: ranks by (rank(p), rank(p+h) or "empty" past the read end) for h = 29, 58, 116, ...
 #include "pq_sort.cuh"
 #include "pq_index.cuh"
+#include "pq_ranges.h"
 
 #include <algorithm>
 #include <vector>
@@ -2054,9 +2055,8 @@ struct MsdScratch {
     idx_t *sv0, *sv1;
     void* rtmp;
     size_t rtmp_bytes;
-    unsigned long long *r_start, *r_end, *r_diff, *r_e0, *r_cnt, *r_cursor;     // further splits
-    unsigned* r_tile0;
-    int *r_off, *r_shift;
+    unsigned char* r_desc;                          // further splits: a RangeBlock,
+    unsigned long long *r_diff, *r_e0, *r_cnt, *r_cursor;
     uint64_t* pk;
     uint8_t* bwt;
     unsigned long long* hist6;
@@ -2107,13 +2107,9 @@ MsdScratch msd_layout(void* base, const MsdPlan& p, size_t m, size_t nr) {
     s.sv1 = reinterpret_cast<idx_t*>(take(sh * sizeof(idx_t)));
     s.rtmp_bytes = p.S ? radix_tmp_bytes(sh) : 0;
     s.rtmp = take(s.rtmp_bytes);
-    s.r_start = reinterpret_cast<U*>(take(kMoreRanges * 8));
-    s.r_end = reinterpret_cast<U*>(take(kMoreRanges * 8));
+    s.r_desc = reinterpret_cast<unsigned char*>(take(RangeBlock{size_t(kMoreRanges)}.bytes()));
     s.r_diff = reinterpret_cast<U*>(take(kMoreRanges * 8));
     s.r_e0 = reinterpret_cast<U*>(take(kMoreRanges * 8));
-    s.r_tile0 = reinterpret_cast<unsigned*>(take((kMoreRanges + 1) * 4));
-    s.r_off = reinterpret_cast<int*>(take(kMoreRanges * 4));
-    s.r_shift = reinterpret_cast<int*>(take(kMoreSplits * 4));
     s.r_cnt = reinterpret_cast<U*>(take((size_t(kMoreSplits) << kMoreBits) * 8));
     s.r_cursor = reinterpret_cast<U*>(take((size_t(kMoreSplits) << kMoreBits) * 8));
     s.pk = reinterpret_cast<uint64_t*>(take((p.n / 32 + 4) * 8));
@@ -2216,14 +2212,18 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
     const int k = a.kmer_k, bits = P.d1 + P.d2;
     const bool own_span = a.kt && !a.kmer_spans;        // a listed bucket's k-mers span its parts
     std::vector<unsigned> split_ids;
-    auto h2d = [&](void* d, const void* h, size_t b) { return cudaMemcpyAsync(d, h, b, cudaMemcpyHostToDevice, st); };
+    auto wait_stream = [st] { return cudaStreamSynchronize(st); };
+    HeldBlocks<decltype(wait_stream)> held(wait_stream);        // the sources of copies to the device
+    auto h2d = [&](void* d, const void* h, size_t b) {
+        return cudaMemcpyAsync(d, std::memcpy(held.take(b), h, b), b, cudaMemcpyHostToDevice, st);
+    };
     auto d2h = [&](void* h, const void* d, size_t b) { return cudaMemcpyAsync(h, d, b, cudaMemcpyDeviceToHost, st); };
     std::vector<SortRange> work;
     auto take_huge = [&](unsigned long long count) -> int {
         if (count > s.cap_huge) return int(cudaErrorUnknown);
         std::vector<unsigned long long> h(count);
         if (count) d2h(h.data(), s.huge, count * 8);
-        const cudaError_t e = cudaStreamSynchronize(st);
+        const cudaError_t e = held.wait();
         if (e != cudaSuccess) return int(e);
         for (unsigned long long g : h)
             work.push_back({g >> 24, (g >> 24) + (g & 0x3fff), int((g >> 14) & 0x3ff), 0, true});
@@ -2249,33 +2249,24 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
         if (own_span) a.kmer_spans = 1;
     }
     std::vector<SortRange> local;
-    std::vector<unsigned long long> rs, re;
-    std::vector<unsigned> tile0;
-    std::vector<int> ri;
-    // describes ranges v[i0, i1) on the device; false when they are too many tiles for one launch
-    auto describe = [&](const std::vector<SortRange>& v, size_t i0, size_t i1) {
-        rs.clear();
-        re.clear();
-        tile0.assign(1, 0);
-        ri.clear();
-        for (size_t i = i0; i < i1; ++i) {
-            rs.push_back(v[i].start);
-            re.push_back(v[i].end);
-            ri.push_back(v[i].off);
-            tile0.push_back(tile0.back() + unsigned((v[i].end - v[i].start + kSplitTile - 1) / kSplitTile));
-        }
-        h2d(s.r_start, rs.data(), rs.size() * 8);
-        h2d(s.r_end, re.data(), re.size() * 8);
-        h2d(s.r_tile0, tile0.data(), tile0.size() * 4);
-        h2d(s.r_off, ri.data(), ri.size() * 4);
+    // describes ranges v[i0, i1) (at most kMoreRanges) and their shifts on the device, one copy for all
+    unsigned tiles = 0;
+    const int* r_off = nullptr;
+    auto describe = [&](const std::vector<SortRange>& v, size_t i0, size_t i1, const int* shift) {
+        const RangeBlock b{i1 - i0};
+        unsigned char* const h = held.take(b.bytes());
+        tiles = fill_ranges(h, v.data() + i0, i1 - i0, shift, size_t(kSplitTile));
+        cudaMemcpyAsync(s.r_desc, h, b.bytes(), cudaMemcpyHostToDevice, st);
+        r_off = reinterpret_cast<const int*>(s.r_desc + b.offs());
         MsdRanges r{};
-        r.start = s.r_start;
-        r.end = s.r_end;
-        r.tile0 = s.r_tile0;
+        r.start = reinterpret_cast<const unsigned long long*>(s.r_desc);
+        r.end = reinterpret_cast<const unsigned long long*>(s.r_desc + b.ends());
+        r.tile0 = reinterpret_cast<const unsigned*>(s.r_desc + b.tiles());
+        r.shift = shift ? reinterpret_cast<const int*>(s.r_desc + b.shifts()) : nullptr;
         r.count = int(i1 - i0);
         return r;
     };
-    auto grid = [&] { return std::min(tile0.back(), unsigned(sms * 4)); };
+    auto grid = [&] { return std::min(tiles, unsigned(sms * 4)); };
     while (!work.empty() || !local.empty()) {
         while (!work.empty()) {
             // new elements where a range's are used up
@@ -2283,8 +2274,8 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
             for (SortRange& r : work)
                 if (r.rebuild) v.push_back(r);
             for (size_t i = 0; i < v.size(); i += kMoreRanges) {
-                const MsdRanges r = describe(v, i, std::min(v.size(), i + kMoreRanges));
-                k_more_rebuild<<<grid(), kSplitThreads, 0, st>>>(a.pk, P, a.more_bits, r, s.r_off, a.buf);
+                const MsdRanges r = describe(v, i, std::min(v.size(), i + kMoreRanges), nullptr);
+                k_more_rebuild<<<grid(), kSplitThreads, 0, st>>>(a.pk, P, a.more_bits, r, r_off, a.buf);
                 note_launch();
             }
             v.clear();
@@ -2298,14 +2289,14 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
             std::vector<int> shift;
             for (size_t i = 0; i < v.size(); i += kMoreRanges) {
                 const size_t i1 = std::min(v.size(), i + kMoreRanges);
-                const MsdRanges r = describe(v, i, i1);
+                const MsdRanges r = describe(v, i, i1, nullptr);
                 cudaMemsetAsync(s.r_diff, 0, r.count * 8, st);
                 k_more_diff<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_diff, s.r_e0);
                 note_launch();
                 std::vector<unsigned long long> d(r.count), e0(r.count);
                 d2h(d.data(), s.r_diff, d.size() * 8);
                 d2h(e0.data(), s.r_e0, e0.size() * 8);
-                const cudaError_t e = cudaStreamSynchronize(st);
+                const cudaError_t e = held.wait();
                 if (e != cudaSuccess) return int(e);
                 for (int q = 0; q < r.count; ++q) {
                     SortRange x = v[i + q];
@@ -2338,38 +2329,42 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
                     shift.push_back(std::max(sh, 0));
                 }
             }
-            for (size_t i = 0; i < split.size(); i += kMoreSplits) {
-                const size_t i1 = std::min(split.size(), i + kMoreSplits);
-                MsdRanges r = describe(split, i, i1);
-                h2d(s.r_shift, shift.data() + i, (i1 - i) * 4);
-                r.shift = s.r_shift;
-                r.bits = kMoreBits;
-                const size_t nc = (i1 - i) << kMoreBits;
-                cudaMemsetAsync(s.r_cnt, 0, nc * 8, st);
-                k_msd_count<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_cnt);
-                note_launch();
-                std::vector<unsigned long long> cnt(nc), cur(nc);
-                d2h(cnt.data(), s.r_cnt, nc * 8);
-                const cudaError_t e = cudaStreamSynchronize(st);
+            // split, the children's places from the counts on the device; the host learns the counts of
+            // kSplitBatch ranges (8 KB each) at a time
+            constexpr size_t kSplitBatch = 16 * kMoreSplits;
+            for (size_t z = 0; z < split.size(); z += kSplitBatch) {
+                const size_t z1 = std::min(split.size(), z + kSplitBatch);
+                std::vector<unsigned long long> cnt((z1 - z) << kMoreBits);
+                for (size_t i = z; i < z1; i += kMoreSplits) {
+                    const size_t i1 = std::min(z1, i + kMoreSplits);
+                    MsdRanges r = describe(split, i, i1, shift.data() + i);
+                    r.bits = kMoreBits;
+                    const size_t nc = (i1 - i) << kMoreBits;
+                    cudaMemsetAsync(s.r_cnt, 0, nc * 8, st);
+                    k_msd_count<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_cnt);
+                    k_msd_children<<<unsigned(i1 - i), kScanThreads, 0, st>>>(s.r_cnt, nullptr, kMoreBits, 0, r.start,
+                                                                             s.r_cursor, s.r_cursor, 0, a.G);
+                    k_msd_split<<<grid(), kSplitThreads, MsdSmem::bytes(kMoreBits, false), st>>>(a.buf, r, s.r_cursor, tmp);
+                    const cudaError_t e = cudaGetLastError();
+                    if (e != cudaSuccess) {
+                        held.wait();
+                        return int(e);
+                    }
+                    k_more_copy<<<grid(), kSplitThreads, 0, st>>>(tmp, r, a.buf);
+                    for (int q = 0; q < 4; ++q) note_launch();
+                    d2h(cnt.data() + ((i - z) << kMoreBits), s.r_cnt, nc * 8);
+                }
+                const cudaError_t e = held.wait();
                 if (e != cudaSuccess) return int(e);
-                for (size_t q = i; q < i1; ++q) {
+                for (size_t q = z; q < z1; ++q) {
                     unsigned long long at = split[q].start;
-                    for (size_t d = 0; d < (size_t(1) << kMoreBits); ++d) {
-                        const size_t c = ((q - i) << kMoreBits) + d;
-                        cur[c] = at;
+                    for (size_t c = (q - z) << kMoreBits; c < (q - z + 1) << kMoreBits; ++c) {
                         if (cnt[c])
                             (cnt[c] <= (unsigned long long)kLocalLarge ? local : work)
                                 .push_back({at, at + cnt[c], split[q].off, split[q].id, false});
                         at += cnt[c];
                     }
                 }
-                h2d(s.r_cursor, cur.data(), nc * 8);
-                k_msd_split<<<grid(), kSplitThreads, MsdSmem::bytes(kMoreBits, false), st>>>(a.buf, r, s.r_cursor, tmp);
-                const cudaError_t es = cudaGetLastError();
-                if (es != cudaSuccess) return int(es);
-                note_launch();
-                k_more_copy<<<grid(), kSplitThreads, 0, st>>>(tmp, r, a.buf);
-                note_launch();
             }
         }
         // every part fits the local kernel; its groups of more than 1024 come back
@@ -2387,7 +2382,7 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
             MsdKernels<W>::local(true, a, s, b.size(), sms, st);
             MsdKernels<W>::groups(a, s, sms, st);
             d2h(&c, s.counters, sizeof c);
-            const cudaError_t e = cudaStreamSynchronize(st);
+            const cudaError_t e = held.wait();
             if (e != cudaSuccess) return int(e);
             if (c.mid > s.cap_mid || c.big > s.cap_big) return int(cudaErrorUnknown);
             const int rc = take_huge(c.huge);
