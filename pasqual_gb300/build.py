@@ -19,7 +19,7 @@ SOURCES = ["pq_index.cu", "pq_search.cu", "pq_sort.cu", "pq_api.cu", "pq_dropin.
            "pq_sort_static.cu", "pq_learned.cu", "pq_seeds.cu",
            "pq_sufsort.cu"]
 HEADERS = ["pq_common.cuh", "pq_index.cuh", "pq_sort.cuh", "pq_learned.cuh", "pq_learned_build.cuh", "pq_slots.h",
-           "pq_ranges.h"]
+           "pq_ranges.h", "pq_pack.h"]
 PUBLIC = ["pasqual_gb300.h", "pasqual_gb300_dropin.h"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

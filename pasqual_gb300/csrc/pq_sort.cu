@@ -22,6 +22,7 @@
 // 64-bit keys: ranks by (rank(p), rank(p+h) or "empty" past the read end) for h = 29, 58, 116, ...
 #include "pq_sort.cuh"
 #include "pq_index.cuh"
+#include "pq_pack.h"
 #include "pq_ranges.h"
 
 #include <algorithm>
@@ -51,27 +52,11 @@ static int device_sms() {
 // 32 bases per word, first base in the top two bits (A=0 .. T=3).  The forward text of a whole
 // word comes in two 16-byte loads; the backward text in steps of eight bases with one division for
 // the first (the read offset then steps and wraps).
-// eight bytes of codes 1..4, the first base highest, as 16 bits
-__device__ __forceinline__ uint32_t pack8(uint64_t x) {
-    x -= 0x0101010101010101ull;
-    x = (x | (x >> 6)) & 0x000f000f000f000full;
-    x = (x | (x >> 12)) & 0x000000ff000000ffull;
-    return uint32_t((x | (x >> 24)) & 0xffffu);
-}
 __device__ __forceinline__ uint64_t swap8(uint32_t lo, uint32_t hi) {
     return (uint64_t(__byte_perm(lo, 0, 0x0123)) << 32) | __byte_perm(hi, 0, 0x0123);
 }
-// the eight bytes at p, from the aligned words that hold them
-__device__ __forceinline__ uint64_t load8(const uint8_t* __restrict__ p) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const uint64_t* w = reinterpret_cast<const uint64_t*>(a & ~uintptr_t(7));
-    const int s = 8 * int(a & 7);
-    const uint64_t lo = w[0];
-    return s ? (lo >> s) | (w[1] << (64 - s)) : lo;
-}
-
-// Bound by the bytes read: backward, the eight bases of a step lie in one read, last first, or in the
-// start of one and the end of the next (1.13 G bases, both directions: 0.70 ms, 1.43 a base at a time).
+// Bound by the bytes read (1.13 G bases, both directions: 0.70 ms, 1.43 a base at a time).  No byte outside
+// the reads is read: at their ends, where the words of eight would hold others, a base at a time.
 __global__ void k_pack_text(const uint8_t* __restrict__ reads, size_t n, DivL dl, int dir, size_t nwords,
                             uint64_t* __restrict__ pk) {
     const size_t stride = size_t(gridDim.x) * blockDim.x, L = dl.L;
@@ -86,19 +71,9 @@ __global__ void k_pack_text(const uint8_t* __restrict__ reads, size_t n, DivL dl
                 (uint64_t(pack8(swap8(b.x, b.y))) << 16) | pack8(swap8(b.z, b.w));
         } else if (p0 < n) {
             size_t r = L == 1 ? p0 : size_t(div_l(p0, dl)), off = p0 - r * L;
-            if (dir == 1 && L >= 8 && p0 + 32 <= n) {
-                #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const size_t k = L - off;                   // bases left in read r
-                    uint64_t x = load8(reads + r * L + (k < 8 ? 0 : k - 8));
-                    if (k < 8) x = (x << (64 - 8 * k)) | (load8(reads + (r + 2) * L - 8) >> (8 * k));
-                    v = (v << 16) | pack8(x);
-                    off += 8;
-                    if (off >= L) {
-                        off -= L;
-                        ++r;
-                    }
-                }
+            if (dir == 1 && L >= 8 && pack_inside(reinterpret_cast<uintptr_t>(reads), n, p0, L)) {
+                v = pack_backward(reinterpret_cast<uintptr_t>(reads), r, off, L,
+                                  [](uintptr_t a) { return *reinterpret_cast<const uint64_t*>(a); });
             } else {
                 for (int j = 0; j < 32; ++j) {
                     const size_t p = p0 + size_t(j);
