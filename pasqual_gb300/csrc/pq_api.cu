@@ -374,7 +374,10 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
     ctx->kmer_from_sort[dir] = 0;
     ctx->kx_bases[dir] = 0;
     const bool want_kx = side_outputs && (n >> (2 * kk)) >= kKxRows;
+    const bool had_sa = ctx->sa_ok[dir];
+    ctx->sa_ok[dir] = false;            // until the sort is done: what fails on the way leaves neither this
     if (side_outputs) {
+        ctx->fm_ok[dir] = false;        // nor, its k-mer table rewritten, the FM-index
         CK(ctx->kt[dir].ensure((size_t(2) << (2 * kk)) * sizeof(idx_t)));
         // the rows' bases past the k-mer where a k-mer has more than a few rows by chance
         if (want_kx) CK(ctx->kx[dir].ensure(n * sizeof(uint16_t) + 16));
@@ -385,9 +388,14 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
                                    ctx->pk[dir].as<uint64_t>(), side_outputs ? ctx->kt[dir].as<idx_t>() : nullptr, kk, &kmer_done,
                                    want_kx ? ctx->kx[dir].as<uint16_t>() : nullptr, &ctx->kx_bases[dir]);
     ctx->pk_ok[dir] = rc == 0;
-    if (rc == int(cudaErrorNotSupported))
+    if (rc == int(cudaErrorNotSupported)) {
+        ctx->sa_ok[dir] = had_sa;       // a refusal leaves the rows as they were
         return fail(ctx, PQ_ERR_CAPACITY, "suffix sort: a 6-base bucket holds more suffixes than a sort chunk");
-    if (rc != 0) return fail(ctx, PQ_ERR_CUDA, std::string("suffix sort failed: ") + cudaGetErrorString(cudaGetLastError()));
+    }
+    if (rc != 0) {
+        ctx->fm_ok[dir] = false;
+        return fail(ctx, PQ_ERR_CUDA, std::string("suffix sort failed: ") + cudaGetErrorString(cudaGetLastError()));
+    }
     CK(cudaEventRecord(ctx->ev1, ctx->st));
     CK(cudaEventSynchronize(ctx->ev1));
     cudaEventElapsedTime(&ctx->ms_sort, ctx->ev0, ctx->ev1);

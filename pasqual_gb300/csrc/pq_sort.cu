@@ -2237,7 +2237,7 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
         const int rc = take_huge(c0.huge);
         if (rc) return rc;
         for (const MsdBucket& b : m) {
-            if (b.size == 0xffffffffu) return int(cudaErrorNotSupported);
+            if (b.size == 0xffffffffu) return int(cudaErrorInvalidValue);       // 2^32 and more in one bucket
             const unsigned id = b.id_off & ((1u << kIdBits) - 1);
             work.push_back({b.start, b.start + b.size, 0, id, false});
             if (own_span) {
