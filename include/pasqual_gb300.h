@@ -95,14 +95,15 @@ PQ_API int pq_get_counts (pq_ctx * ctx, pq_idx C[6], pq_idx suffix_count[4], pq_
  * by text position.  Replaces transform_to_triplet[_reverse] + initial_sort + suf_sort over the
  * five slots (src/sufsort.h:29-46, driven by src/index.c:558-585). */
 PQ_API int pq_sort (pq_ctx * ctx, int dir);
-/* Largest number of suffixes pq_sort is to sort at a time (0, the default: no limit).  Every suffix
+/* Largest number of suffixes pq_sort is to sort at a time (0, the default: as the memory allows).  Every suffix
  * falls in a bucket by its first 6 bases and min(length, 6), numbered in suffix order; runs of
  * consecutive buckets of at most this many suffixes are chunks -- the sort the reference does over
  * its 5 first-character slots (src/index.c:558-585), at a finer grain.  The limit bounds the sort's
  * working memory: one pass over everything is taken while it needs no more than chunks of this size
  * may (20 bytes and two positions a suffix of a chunk, 3 1/4 bytes a suffix of the index), else the
  * chunks are sorted one after the other into their place.  A bucket larger than a chunk makes
- * pq_sort return PQ_ERR_CAPACITY.  Same suffix array either way. */
+ * pq_sort return PQ_ERR_CAPACITY.  Without a limit, chunks are taken where the working memory of one
+ * pass does not fit the device.  Same suffix array either way. */
 PQ_API int pq_set_sort_chunk (pq_ctx * ctx, uint64_t max_suffixes);
 
 /* Use a given suffix array instead of sorting (testing and external sorters). */

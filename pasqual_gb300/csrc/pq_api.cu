@@ -37,6 +37,7 @@ struct DevBuf {
         bytes = 0;
         cudaError_t e = cudaMalloc(&p, want ? want : 16);
         if (e == cudaSuccess) bytes = want;
+        else cudaGetLastError();            // the caller may go on with less
         return e;
     }
     // grow keeping the first `keep` bytes
@@ -44,7 +45,10 @@ struct DevBuf {
         if (want <= bytes && p) return cudaSuccess;
         void* q = nullptr;
         cudaError_t e = cudaMalloc(&q, want);
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return e;
+        }
         if (p && keep) cudaMemcpyAsync(q, p, std::min(keep, bytes), cudaMemcpyDeviceToDevice, st);
         cudaStreamSynchronize(st);
         if (p) cudaFree(p);
@@ -133,6 +137,26 @@ static int fail(pq_ctx* c, int code, const std::string& msg) {
             return fail(ctx, e_ == cudaErrorMemoryAllocation ? PQ_ERR_NOMEM : PQ_ERR_CUDA,        \
                         std::string(#call) + ": " + cudaGetErrorString(e_));                      \
     } while (0)
+
+// Gives back the device memory that the context holds but can do without: the last sort's working
+// memory, and the rows' next bases (the search then compares texts).  Not while a kernel that uses either
+// is about to be launched.  False where there was none.
+static bool give_back(pq_ctx* c) {
+    bool any = c->sort_tmp.p != nullptr;
+    c->sort_tmp.release();
+    c->bwt_hint[0] = c->bwt_hint[1] = nullptr;
+    for (int d = 0; d < 2; ++d) {
+        any = any || c->kx[d].p;
+        c->kx[d].release();
+        c->kx_bases[d] = 0;
+    }
+    return any;
+}
+// b (neither of those two) with `bytes` bytes, if need be after giving them back
+static cudaError_t need(pq_ctx* c, DevBuf& b, size_t bytes) {
+    const cudaError_t e = b.ensure(bytes);
+    return e == cudaErrorMemoryAllocation && give_back(c) ? b.ensure(bytes) : e;
+}
 
 static inline size_t n_rows(const pq_ctx* c) { return size_t(c->num_reads) * size_t(c->L); }
 static inline size_t n_blocks(const pq_ctx* c) { return n_rows(c) / 64 + 1; }
@@ -303,7 +327,7 @@ int pq_set_reads(pq_ctx* ctx, const uint8_t* reads, pq_idx num_reads, int read_l
     }
     ctx->seed_k = std::min(ctx->seed_k, min_overlap);
     size_t bytes = size_t(num_reads) * read_len;
-    CK(ctx->reads.ensure(bytes + 64));
+    CK(need(ctx, ctx->reads, bytes + 64));
     if (bytes) {
         // page-locked host memory (cudaHostAlloc'd or registered) is read by the copy kernel;
         // pageable memory goes through cudaMemcpy
@@ -314,7 +338,7 @@ int pq_set_reads(pq_ctx* ctx, const uint8_t* reads, pq_idx num_reads, int read_l
             CK(cudaMemcpyAsync(ctx->reads.p, reads, bytes,
                                from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->st));
     }
-    CK(ctx->counts.ensure(13 * sizeof(unsigned long long)));
+    CK(need(ctx, ctx->counts, 13 * sizeof(unsigned long long)));
     CK(pq::read_counts(ctx->reads.as<uint8_t>(), num_reads, idx_t(read_len),
                        ctx->counts.as<unsigned long long>(), ctx->st));
     unsigned long long h[13];
@@ -363,25 +387,40 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
     if (!ctx->have_reads) return fail(ctx, PQ_ERR_STATE, "pq_set_reads first");
     cudaSetDevice(ctx->device);
     const size_t n = n_rows(ctx);
-    CK(ctx->sa[dir].ensure(n * sizeof(idx_t) + 64));
-    CK(ctx->pk[dir].ensure((n / 32 + 4) * sizeof(uint64_t)));
-    const size_t cap = size_t(ctx->sort_chunk);
-    const size_t tmp_bytes = pq::suffix_sort_tmp_bytes(n, ctx->num_reads, ctx->L, cap);
-    CK(ctx->sort_tmp.ensure(tmp_bytes));
-    CK(cudaEventRecord(ctx->ev0, ctx->st));
-    ctx->bwt_hint[0] = ctx->bwt_hint[1] = nullptr;           // the scratch is about to be reused
     const int kk = ctx->seed_k;
-    ctx->kmer_from_sort[dir] = 0;
-    ctx->kx_bases[dir] = 0;
-    const bool want_kx = side_outputs && (n >> (2 * kk)) >= kKxRows;
-    const bool had_sa = ctx->sa_ok[dir];
-    ctx->sa_ok[dir] = false;            // until the sort is done: what fails on the way leaves neither this
+    CK(need(ctx, ctx->sa[dir], n * sizeof(idx_t) + 64));
+    CK(need(ctx, ctx->pk[dir], (n / 32 + 4) * sizeof(uint64_t)));
     if (side_outputs) {
-        ctx->fm_ok[dir] = false;        // nor, its k-mer table rewritten, the FM-index
-        CK(ctx->kt[dir].ensure((size_t(2) << (2 * kk)) * sizeof(idx_t)));
-        // the rows' bases past the k-mer where a k-mer has more than a few rows by chance
-        if (want_kx) CK(ctx->kx[dir].ensure(n * sizeof(uint16_t) + 16));
+        ctx->fm_ok[dir] = false;        // the k-mer table is rewritten
+        CK(need(ctx, ctx->kt[dir], (size_t(2) << (2 * kk)) * sizeof(idx_t)));
     }
+    // the rows' bases past the k-mer where a k-mer has more than a few rows by chance, if they fit
+    bool want_kx = side_outputs && (n >> (2 * kk)) >= kKxRows;
+    ctx->kx_bases[dir] = 0;
+    if (want_kx) want_kx = ctx->kx[dir].ensure(n * sizeof(uint16_t) + 16) == cudaSuccess;
+    // One pass, or as many suffixes at a time as the caller allows.  Where the working memory does not fit,
+    // without the next bases of either direction, and then in chunks small enough.
+    size_t cap = size_t(ctx->sort_chunk), tmp_bytes = pq::suffix_sort_tmp_bytes(n, ctx->num_reads, ctx->L, cap);
+    ctx->bwt_hint[0] = ctx->bwt_hint[1] = nullptr;           // the scratch is about to be reused
+    cudaError_t room = ctx->sort_tmp.ensure(tmp_bytes);
+    if (room == cudaErrorMemoryAllocation && give_back(ctx)) {
+        want_kx = false;
+        room = ctx->sort_tmp.ensure(tmp_bytes);
+    }
+    bool too_small = false;             // chunks by the memory, not by the caller
+    for (size_t c = std::min(n / 2, size_t(1) << 30); room == cudaErrorMemoryAllocation && !ctx->sort_chunk && c > n / 512; c /= 2) {
+        const size_t b = pq::suffix_sort_tmp_bytes(n, ctx->num_reads, ctx->L, c);
+        if (b >= tmp_bytes) continue;
+        too_small = true;
+        cap = c;
+        tmp_bytes = b;
+        room = ctx->sort_tmp.ensure(b);
+    }
+    CK(room);
+    CK(cudaEventRecord(ctx->ev0, ctx->st));
+    ctx->kmer_from_sort[dir] = 0;
+    const bool had_sa = ctx->sa_ok[dir];
+    ctx->sa_ok[dir] = false;            // until the sort is done: what fails on the way leaves none
     bool kmer_done = false;
     const int rc = pq::suffix_sort(ctx->reads.as<uint8_t>(), ctx->num_reads, ctx->L, dir, ctx->sa[dir].as<idx_t>(), cap,
                                    ctx->sort_tmp.p, tmp_bytes, ctx->st, side_outputs ? &ctx->bwt_hint[dir] : nullptr,
@@ -390,6 +429,7 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
     ctx->pk_ok[dir] = rc == 0;
     if (rc == int(cudaErrorNotSupported)) {
         ctx->sa_ok[dir] = had_sa;       // a refusal leaves the rows as they were
+        if (too_small) return fail(ctx, PQ_ERR_NOMEM, "suffix sort: no room for its working memory");
         return fail(ctx, PQ_ERR_CAPACITY, "suffix sort: a 6-base bucket holds more suffixes than a sort chunk");
     }
     if (rc != 0) {
@@ -417,7 +457,7 @@ int pq_set_sa(pq_ctx* ctx, int dir, const pq_idx* sa, int from_device) {
     if (!ctx->have_reads) return fail(ctx, PQ_ERR_STATE, "pq_set_reads first");
     cudaSetDevice(ctx->device);
     const size_t n = n_rows(ctx);
-    CK(ctx->sa[dir].ensure(n * sizeof(idx_t) + 64));
+    CK(need(ctx, ctx->sa[dir], n * sizeof(idx_t) + 64));
     if (n)
         CK(cudaMemcpyAsync(ctx->sa[dir].p, sa, n * sizeof(idx_t),
                            from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->st));
@@ -464,16 +504,16 @@ int pq_apply_sort_seeds(pq_ctx* ctx, int dir, uint64_t r0, uint64_t r1, pq_idx* 
     if (!nr || r0 == r1) return PQ_OK;
     cudaSetDevice(ctx->device);
     if (!ctx->pk_ok[dir]) {
-        CK(ctx->pk[dir].ensure((n / 32 + 4) * sizeof(uint64_t)));
+        CK(need(ctx, ctx->pk[dir], (n / 32 + 4) * sizeof(uint64_t)));
         CK(pq::pack_text(ctx->reads.as<uint8_t>(), n, idx_t(ctx->L), dir, ctx->pk[dir].as<uint64_t>(), ctx->st));
         ctx->pk_ok[dir] = true;
     }
     DevBuf s, z, d, tmp;
-    CK(s.ensure(nr * sizeof(idx_t)));
-    CK(z.ensure(nr * sizeof(idx_t)));
-    CK(d.ensure(nr * sizeof(uint16_t)));
+    CK(need(ctx, s, nr * sizeof(idx_t)));
+    CK(need(ctx, z, nr * sizeof(idx_t)));
+    CK(need(ctx, d, nr * sizeof(uint16_t)));
     const size_t tb = pq::sort_seeds_tmp_bytes(size_t(r1 - r0), nr);
-    CK(tmp.ensure(tb));
+    CK(need(ctx, tmp, tb));
     CK(cudaMemcpyAsync(s.p, start, nr * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(z.p, size, nr * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(d.p, depth, nr * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->st));
@@ -517,12 +557,12 @@ int pq_build_fm(pq_ctx* ctx, int dir) {
     if (!ctx->sa_ok[dir]) return fail(ctx, PQ_ERR_STATE, "no suffix array for this direction");
     cudaSetDevice(ctx->device);
     const size_t n = n_rows(ctx);
-    CK(ctx->blk[dir].ensure(n_blocks(ctx) * sizeof(OccBlock)));
-    CK(ctx->sb[dir].ensure(n_supers(ctx) * 4 * sizeof(idx_t) + 64));
-    CK(ctx->ri[dir].ensure(size_t(ctx->num_reads) * sizeof(idx_t) + 64));
+    CK(need(ctx, ctx->blk[dir], n_blocks(ctx) * sizeof(OccBlock)));
+    CK(need(ctx, ctx->sb[dir], n_supers(ctx) * 4 * sizeof(idx_t) + 64));
+    CK(need(ctx, ctx->ri[dir], size_t(ctx->num_reads) * sizeof(idx_t) + 64));
     const int k = ctx->seed_k;
-    CK(ctx->kt[dir].ensure((size_t(2) << (2 * k)) * sizeof(idx_t)));
-    CK(ctx->pk[dir].ensure((n / 32 + 4) * sizeof(uint64_t)));
+    CK(need(ctx, ctx->kt[dir], (size_t(2) << (2 * k)) * sizeof(idx_t)));
+    CK(need(ctx, ctx->pk[dir], (n / 32 + 4) * sizeof(uint64_t)));
     CK(cudaEventRecord(ctx->ev0, ctx->st));
     if (!ctx->pk_ok[dir])
         CK(pq::pack_text(ctx->reads.as<uint8_t>(), n, idx_t(ctx->L), dir, ctx->pk[dir].as<uint64_t>(), ctx->st));
@@ -577,8 +617,8 @@ int pq_get_index_ref(pq_ctx* ctx, int dir, uint64_t* bitmap, pq_idx* sample, pq_
     const size_t nblk = n_blocks(ctx);
     if (bitmap || sample) {
         DevBuf bm, smp;
-        CK(bm.ensure(nblk * 5 * sizeof(uint64_t)));
-        CK(smp.ensure(nblk * 5 * sizeof(idx_t)));
+        CK(need(ctx, bm, nblk * 5 * sizeof(uint64_t)));
+        CK(need(ctx, smp, nblk * 5 * sizeof(idx_t)));
         const idx_t* fix = dir == 0 ? ctx->sfx : ctx->pfx;
         CK(pq::export_ref_layout(ctx->blk[dir].as<OccBlock>(), ctx->sb[dir].as<idx_t>(), ctx->num_reads,
                                  idx_t(ctx->L), fix, bm.as<uint64_t>(), smp.as<idx_t>(), ctx->st));
@@ -602,8 +642,8 @@ int pq_get_seeds(pq_ctx* ctx, int dir, pq_idx* start, pq_idx* size, uint16_t* de
     const size_t nr = ctx->num_reads;
     if (!nr) return PQ_OK;
     DevBuf s, z;
-    CK(s.ensure(nr * sizeof(idx_t)));
-    CK(z.ensure(nr * sizeof(idx_t)));
+    CK(need(ctx, s, nr * sizeof(idx_t)));
+    CK(need(ctx, z, nr * sizeof(idx_t)));
     CK(pq::read_seeds(ctx->reads.as<uint8_t>(), ctx->num_reads, ctx->L, dir, ctx->fm_k[dir],
                       ctx->kt[dir].as<idx_t>(), s.as<idx_t>(), z.as<idx_t>(), ctx->st));
     if (start) CK(cudaMemcpyAsync(start, s.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
@@ -621,16 +661,16 @@ int pq_get_sort_seeds(pq_ctx* ctx, int dir, pq_idx* start, pq_idx* size, uint16_
     const size_t nr = ctx->num_reads, n = n_rows(ctx);
     if (!nr) return PQ_OK;
     if (!ctx->pk_ok[dir]) {
-        CK(ctx->pk[dir].ensure((n / 32 + 4) * sizeof(uint64_t)));
+        CK(need(ctx, ctx->pk[dir], (n / 32 + 4) * sizeof(uint64_t)));
         CK(pq::pack_text(ctx->reads.as<uint8_t>(), n, idx_t(ctx->L), dir, ctx->pk[dir].as<uint64_t>(), ctx->st));
         ctx->pk_ok[dir] = true;
     }
     DevBuf s, z, d, tmp;
-    CK(s.ensure(nr * sizeof(idx_t)));
-    CK(z.ensure(nr * sizeof(idx_t)));
-    CK(d.ensure(nr * sizeof(uint16_t)));
+    CK(need(ctx, s, nr * sizeof(idx_t)));
+    CK(need(ctx, z, nr * sizeof(idx_t)));
+    CK(need(ctx, d, nr * sizeof(uint16_t)));
     const size_t tb = pq::sort_seeds_tmp_bytes(n, nr);
-    CK(tmp.ensure(tb));
+    CK(need(ctx, tmp, tb));
     CK(pq::seed_init(ctx->reads.as<uint8_t>(), ctx->num_reads, idx_t(ctx->L), dir, ctx->C, d.as<uint16_t>(),
                      s.as<idx_t>(), z.as<idx_t>(), ctx->st));
     CK(pq::sort_seeds(ctx->sa[dir].as<idx_t>(), ctx->pk[dir].as<uint64_t>(), ctx->num_reads, idx_t(ctx->L), ctx->t, 0, n,
@@ -669,8 +709,6 @@ static int search_prepare(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
         f.sb = ctx->sb[d].as<idx_t>();
         f.reads_index = ctx->ri[d].as<idx_t>();
         f.kt = ctx->kt[d].as<idx_t>();
-        f.kx_bases = ctx->kx_bases[d];
-        f.kx = f.kx_bases ? ctx->kx[d].as<uint16_t>() : nullptr;
         f.sa = ctx->sa[d].as<idx_t>();
         f.pk = ctx->pk[d].as<uint64_t>();
         const idx_t* fix = d == 0 ? ctx->sfx : ctx->pfx;
@@ -700,7 +738,12 @@ static int search_prepare(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
             }
             if (ctx->lx_segs[0] && ctx->lx_segs[1]) A.sa_seed = 2;
         }
-        for (int d = 0; d < 2; ++d) A.fm[d].lx = lx_view(ctx, d);
+        for (int d = 0; d < 2; ++d) {
+            FmView& f = A.fm[d];
+            f.lx = lx_view(ctx, d);
+            f.kx_bases = ctx->kx_bases[d];          // after the learned index's allocations, which may take it
+            f.kx = f.kx_bases ? ctx->kx[d].as<uint16_t>() : nullptr;
+        }
     }
     ctx->lx_queries = A.sa_seed == 2 ? 4 * uint64_t(nr) : 0;
     // seed mode 0 is the reference's method throughout (walk + FM-index DFS); 1 and 2 reduce by
@@ -964,8 +1007,7 @@ static int search_end(pq_ctx* ctx) {
     return PQ_OK;
 }
 
-int pq_overlaps(pq_ctx* ctx) {
-    if (!ctx) return PQ_ERR_ARG;
+static int overlaps_once(pq_ctx* ctx) {
     pq::SearchArgs A{};
     pq::SearchOut O{};
     int rc = search_prepare(ctx, A, O);
@@ -997,6 +1039,12 @@ int pq_overlaps(pq_ctx* ctx) {
     if (rc == PQ_OK) rc = search_end(ctx);
     if (rc == PQ_OK) cudaEventElapsedTime(&ctx->ms_fast, ctx->evk0, ctx->evk1);
     return rc;
+}
+
+int pq_overlaps(pq_ctx* ctx) {
+    if (!ctx) return PQ_ERR_ARG;
+    const int rc = overlaps_once(ctx);
+    return rc == PQ_ERR_NOMEM && give_back(ctx) ? overlaps_once(ctx) : rc;
 }
 
 int pq_get_graph_sizes(pq_ctx* ctx, uint64_t* num_edges, uint64_t* probes, uint64_t* wide_reads) {
@@ -1099,7 +1147,7 @@ int pq_learned_build(pq_ctx* ctx, int dir, int steps) {
         ctx->lx_ok[dir] = true;
         return PQ_OK;
     }
-    CK(ctx->lx_tmp.ensure(pq::lx_tmp_bytes(n)));
+    CK(need(ctx, ctx->lx_tmp, pq::lx_tmp_bytes(n)));
     const pq::LxTmp T = pq::lx_tmp_layout(ctx->lx_tmp.p, n);
     unsigned long long m = 0;
     CK(cudaEventRecord(ctx->ev0, ctx->st));
@@ -1108,12 +1156,12 @@ int pq_learned_build(pq_ctx* ctx, int dir, int steps) {
     CK(cudaEventSynchronize(ctx->ev1));
     cudaEventElapsedTime(&info.keys_ms, ctx->ev0, ctx->ev1);
     const int S = int(std::min<unsigned long long>(pq::kLxMaxSegs, m));
-    CK(ctx->lx_bnd[dir].ensure(size_t(S) * 4 + 64));
-    CK(ctx->lx_base[dir].ensure(size_t(S + 1) * sizeof(idx_t) + 64));
-    CK(ctx->lx_par[dir].ensure(size_t(S) * pq::kLxStride * sizeof(float) + 64));
-    CK(ctx->lx_err[dir].ensure(size_t(S) * 8 + 64));
-    CK(ctx->lx_err_root[dir].ensure(size_t(S) * 8 + 64));
-    CK(ctx->lx_segof[dir].ensure(65537 * 2 + 64));
+    CK(need(ctx, ctx->lx_bnd[dir], size_t(S) * 4 + 64));
+    CK(need(ctx, ctx->lx_base[dir], size_t(S + 1) * sizeof(idx_t) + 64));
+    CK(need(ctx, ctx->lx_par[dir], size_t(S) * pq::kLxStride * sizeof(float) + 64));
+    CK(need(ctx, ctx->lx_err[dir], size_t(S) * 8 + 64));
+    CK(need(ctx, ctx->lx_err_root[dir], size_t(S) * 8 + 64));
+    CK(need(ctx, ctx->lx_segof[dir], 65537 * 2 + 64));
     CK(pq::lx_root(T, m, n, S, ctx->lx_bnd[dir].as<uint32_t>(), ctx->lx_base[dir].as<idx_t>(),
                    ctx->lx_segof[dir].as<uint16_t>(), ctx->st));
     CK(cudaEventRecord(ctx->ev0, ctx->st));
@@ -1205,7 +1253,7 @@ int pq_learned_keys(pq_ctx* ctx, int dir, uint32_t* keys, pq_idx* first_row, uin
     const size_t n = n_rows(ctx);
     *num_keys = 0;
     if (!n) return PQ_OK;
-    CK(ctx->lx_tmp.ensure(pq::lx_tmp_bytes(n)));
+    CK(need(ctx, ctx->lx_tmp, pq::lx_tmp_bytes(n)));
     const pq::LxTmp T = pq::lx_tmp_layout(ctx->lx_tmp.p, n);
     unsigned long long m = 0;
     CK(pq::lx_distinct_keys(ctx->sa[dir].as<idx_t>(), ctx->pk[dir].as<uint64_t>(), n, idx_t(ctx->L), T, &m, ctx->st));
@@ -1415,8 +1463,7 @@ static int queue_launch(pq_ctx* lead, const std::vector<pq::SearchBatch>& hb, co
     return PQ_OK;
 }
 
-int pq_overlaps_batched(pq_ctx** ctxs, int count, int flags) {
-    if (!ctxs || count <= 0) return PQ_ERR_ARG;
+static int batched_once(pq_ctx** ctxs, int count, int flags) {
     pq_ctx* lead = ctxs[0];
     if (!lead) return PQ_ERR_ARG;
     for (int b = 0; b < count; ++b) {
@@ -1476,6 +1523,15 @@ int pq_overlaps_batched(pq_ctx** ctxs, int count, int flags) {
         ctxs[b]->ms_fast = lead->q_kernel_ms;
     }
     return rc;
+}
+
+int pq_overlaps_batched(pq_ctx** ctxs, int count, int flags) {
+    if (!ctxs || count <= 0) return PQ_ERR_ARG;
+    const int rc = batched_once(ctxs, count, flags);
+    bool any = false;
+    if (rc == PQ_ERR_NOMEM)
+        for (int b = 0; b < count; ++b) any = give_back(ctxs[b]) || any;
+    return any ? batched_once(ctxs, count, flags) : rc;
 }
 
 int pq_set_batch_plan(pq_ctx* lead, int ctas_per_sm, int groups_per_item, int edge_slots) {
