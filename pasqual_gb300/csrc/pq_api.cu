@@ -750,7 +750,7 @@ static int search_prepare(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
     // sorted continuations wherever those fit in 256 bases
     A.sorted_reduce = (ctx->seed_mode != 0 && ctx->L - ctx->t <= 256) ? 1 : 0;
 
-    // [0] e_count [1] probes [2] ovf (u32) [3] learned misses [5] heavy ovf [6] sectors
+    // [0] e_count [1] probes [2] ovf (u32) [3] learned misses [4] lean misses (u32) [5] heavy ovf [6] sectors
     unsigned long long* ctr = ctx->ctrs.as<unsigned long long>();
     O.num_B = ctx->nB.as<uint16_t>();
     O.num_F = ctx->nF.as<uint16_t>();
@@ -769,6 +769,11 @@ static int search_prepare(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O) {
     O.probes = ctr + 1;
     O.sectors = ctr + 6;
     A.lx_misses = ctr + 3;
+    if (A.sorted_reduce && pq::lean_misses_by_chance(n_rows(ctx), ctx->t)) {
+        CK(ctx->ovf3.ensure(nrp * sizeof(idx_t)));
+        A.miss_list = ctx->ovf3.as<idx_t>();
+        A.miss_count = reinterpret_cast<unsigned*>(ctr + 4);
+    }
 
     CK(cudaMemsetAsync(ctr, 0, 64, ctx->st));
     return PQ_OK;
@@ -803,8 +808,26 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool 
     std::memcpy(hc, ctx->h_ctr, sizeof hc);
     ctx->lx_misses = hc[3];
     unsigned ovf = unsigned(hc[2] & 0xffffffffu);
-    const bool more = ovf != 0;
-    ctx->deferred_reads = lean ? ovf : 0;
+    const unsigned missed = unsigned(hc[4] & 0xffffffffu);
+    const bool more = ovf != 0 || missed != 0;
+    ctx->deferred_reads = lean ? ovf + missed : 0;
+    if (missed && missed < pq::kFastMisses) {
+        CK(cudaMemcpyAsync(ctx->ovf_list.as<idx_t>() + ovf, A.miss_list, missed * sizeof(idx_t), cudaMemcpyDeviceToDevice, ctx->st));
+        ovf += missed;
+    } else if (missed) {
+        // the fast tier over the reads whose scan the lean tier gave up; its own leftovers join the others
+        const int ebcap = 64;
+        int sms = 152;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+        const int blocks = int(std::min<size_t>((size_t(missed) + 127) / 128, size_t(pq::search_fast_blocks(ctx->L, ctx->L - ctx->t, sms))));
+        const size_t wsb = pq::warp_scratch_bytes(ctx->L, ctx->t, size_t(blocks) * 4, ebcap);
+        CK(ctx->warp_scratch.ensure(wsb));
+        CK(pq::search_fast(A, O, blocks, ctx->warp_scratch.p, wsb, ebcap, ctx->st, A.miss_list, A.miss_count));
+        CK(cudaMemcpyAsync(hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, ctx->st));
+        CK(cudaStreamSynchronize(ctx->st));
+        ovf = unsigned(hc[2] & 0xffffffffu);
+        if (hc[0] > O.e_cap) CK(grow_pool(ctx, O, size_t(2 * hc[0] + 4096), O.e_cap));
+    }
     const idx_t* ovf_src = ctx->ovf_list.as<idx_t>();
     const unsigned* ovf_cnt = reinterpret_cast<const unsigned*>(ctr + 2);     // device count of ovf_src
     ctx->heavy_reads = 0;

@@ -78,6 +78,8 @@ struct SearchArgs {
                                 // 2: the same with learned windows (needs fm[].lx)
     unsigned long long* lx_misses;  // learned windows that missed (those chains walk)
     int sorted_reduce;          // 1: edges from sorted continuations (L - t <= 256)
+    idx_t* miss_list;           // lean tier: the reads its scan does not serve go here, not to ovf_list
+    unsigned* miss_count;       //   (nullptr: there with the others)
 };
 
 // Global scratch of the fast kernel, per warp of 32 reads: level-0 candidates (4 kinds x (L - t)
@@ -130,10 +132,13 @@ struct SearchQueue {
 };
 size_t warp_scratch_bytes(int L, int t, size_t nwarps, int ebcap);
 int search_fast_blocks(int L, int M, int num_sms);   // resident blocks of the fast kernel (M = L - t)
-// blocks of 128 threads (4 warps); reads that outgrow the shared-memory stack, ebcap edges or
-// the frame count are listed for the wide kernel.
+// blocks of 128 threads (4 warps) over every read, or over list[0, *count); reads that outgrow the
+// warps' stacks (in global scratch), ebcap edges or the frame count are listed in o.ovf_list.
 cudaError_t search_fast(const SearchArgs& a, const SearchOut& o, int blocks, void* scratch, size_t scratch_bytes,
-                        int ebcap, cudaStream_t st);
+                        int ebcap, cudaStream_t st, const idx_t* list = nullptr, const unsigned* count = nullptr);
+// The fast tier takes the lean tier's misses where they come by chance and are enough of them.
+bool lean_misses_by_chance(size_t rows, int t);
+constexpr unsigned kFastMisses = 16384;
 // Lean tier (sorted reduction) over every read; the ones it does not serve (more than 64 candidates
 // on a side, a missed window, a full edge pool) are listed in o.ovf_list; needs a.sorted_reduce.
 int search_lean_blocks(int L, int M, int num_sms);

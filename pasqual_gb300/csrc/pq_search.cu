@@ -1374,8 +1374,8 @@ __global__ void __launch_bounds__(128, 5) k_search_fast(SearchArgs A0, SearchOut
                         const int st = reduce_sorted<W>(A, S, self, side, pbase_w + src, n0, rbase_w + lane, eb, ne, sc, probes);
                         if (st != OVF_NONE) status = st;
                         active = false;
-                    } else if (active && n0 > CAP) {
-                        status = OVF_STACK;
+                    } else if (active && (n0 > CAP || (CAP == kTaskCap && A.sorted_reduce && Q.read_list))) {
+                        status = OVF_STACK;             // of a listed read (the lean tier's misses): the block tier's
                         active = false;
                     }
                     fresh = active;
@@ -1711,7 +1711,7 @@ __global__ void __launch_bounds__(128, 5) k_search_fast(SearchArgs A0, SearchOut
 // was slower for every kind of such reads, whether it could hold them or not (1.5 M bases of 100-base
 // reads with 2 % dinucleotide runs, 2,165 such reads, 431 of which it could: 36 ms with it, 1.6
 // without; with half the genome in repeats, 565 and 555: 3.4 and 1.9; 400x coverage, 38 thousand and
-// 6 thousand: 8.6 and 5.3).
+// 6 thousand: 8.6 and 5.3) but one: where depth-t intervals are large by chance (lean_misses_by_chance).
 //
 // Bound by DRAM at random sectors (4.1 TB/s, of which every second sector of a 64-byte fetch goes
 // unused): k-mer table, kx, suffix array, text.  5.4 M reads of 100 bases, 566 M suffixes, 64-bit
@@ -1719,6 +1719,7 @@ __global__ void __launch_bounds__(128, 5) k_search_fast(SearchArgs A0, SearchOut
 // found by bisection; 1.2 M reads, 123 M suffixes: 1.5 against 2.4.  Eight CTAs of 64 registers per
 // SM; six or ten were 3 to 10 % slower.
 constexpr int kLeanThreads = 128;
+constexpr int kMissed = OVF_LEVELS;         // the scan does not serve the read
 
 template <int W>
 __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, SearchOut O0, WarpScratch S,
@@ -1795,7 +1796,10 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                     for (int w = 0; w < kScanWords; ++w) P1[w] = ~P0[w];
                 }
                 if (A.sa_seed == 2) {
-                    if (ok) ok = learned_rows(A, f0, f1, P0, P1, first, end, probes);
+                    if (ok && !learned_rows(A, f0, f1, P0, P1, first, end, probes)) {
+                        ok = false;
+                        status = kMissed;
+                    }
                     __syncwarp();
                 } else {
                     const int k = A.seed_k;
@@ -1811,7 +1815,10 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                     if (ok && (end[0] - first[0] > idx_t(kScanDirect) || end[1] - first[1] > idx_t(kScanDirect))) {
                         const idx_t lo[2] = {first[0], first[1]}, hi[2] = {end[0], end[1]};
                         sa_bounds2(f0, f1, A.dl, P0, P1, t < 32 * kScanWords ? t : 32 * kScanWords, lo, hi, first, end, probes);
-                        ok = end[0] - first[0] <= idx_t(kScanMax) && end[1] - first[1] <= idx_t(kScanMax);
+                        if (end[0] - first[0] > idx_t(kScanMax) || end[1] - first[1] > idx_t(kScanMax)) {
+                            ok = false;
+                            status = kMissed;
+                        }
                     }
                 }
                 slots[lane] = 0;
@@ -1901,10 +1908,10 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                 }
                 __syncwarp();
             }
-            if (have && (!ok || status != OVF_NONE)) {   // the block tier redoes this read
+            if (have && (!ok || status != OVF_NONE)) {   // the fast or the block tier redoes this read
                 if (ok) O.status[r] = uint8_t(status);
-                const unsigned k = atomicAdd(O.ovf_count, 1u);
-                O.ovf_list[k] = self;
+                if (status == kMissed && A.miss_list) A.miss_list[atomicAdd(A.miss_count, 1u)] = self;
+                else O.ovf_list[atomicAdd(O.ovf_count, 1u)] = self;
             }
             // one reservation of edge slots for the warp's reads
             const int mine = have && ok && status == OVF_NONE ? ne : 0;
@@ -1939,6 +1946,18 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
     }
     if (Q.count == 0 || cur >= 0) add_probes(O, probes);
 }
+
+// Reads the scan does not serve have a depth-t interval of more than kScanMax rows.  With long overlaps
+// those are repeats and low complexity, whose walks and DFS are long: the block tier's.  With short ones
+// an ordinary read's interval is that large by chance, rows / 4^t (several times that where bases are
+// skewed).  Such a read has few candidates: the fast tier, 32 reads a warp, takes 25 ns a read, the
+// block tier, a CTA a read, 90.  But its slowest warp takes 0.8 ms, which 9 thousand reads of the block
+// tier do not: kFastMisses.  Whole searches in ms, misses to the fast tier (and on where a side has more than
+// kRedMax candidates) and to the block tier, reads of 100 bases at 20x, GC 41 %:
+//   rows 54 M, t = 10 (51 rows by chance, 5 thousand misses): 6.1 and 5.4;  78 M (74, 46 thousand): 9.6 and 12.1;
+//   108 M (103, 198 thousand): 17.0 and 29.8;  431 M (411, 4.2 M): 210 and 415;  861 M, t = 11, 64-bit (205, 6.1
+//   M): 267 and 699;  t = 10 (821, 8.6 M, of which 3.1 M go on): 952 and 1006.
+bool lean_misses_by_chance(size_t rows, int t) { return t < 32 && (rows >> (2 * t)) >= size_t(kScanMax) / 8; }
 
 int search_lean_blocks(int L, int M, int num_sms) {
     (void)L;
@@ -2019,13 +2038,15 @@ size_t warp_scratch_bytes(int L, int t, size_t nwarps, int ebcap) {
 }
 
 cudaError_t search_fast(const SearchArgs& a, const SearchOut& o, int blocks, void* scratch, size_t scratch_bytes,
-                        int ebcap, cudaStream_t st) {
+                        int ebcap, cudaStream_t st, const idx_t* list, const unsigned* count) {
     const size_t nwarps = size_t(blocks) * kWarpsPerCta;
     WarpScratch S;
     if (scratch_bytes < scratch_layout(a.L - a.t, nwarps, ebcap, scratch, &S)) return cudaErrorInvalidValue;
     const int words = (a.L + 15) / 16;
     size_t smem = size_t(words) * 32 * kWarpsPerCta * sizeof(uint32_t);
     SearchQueue Q{};
+    Q.read_list = list;
+    Q.list_count = count;
     if (lam_words(a.L - a.t) == 2) k_search_fast<2, kTaskCap, kTaskFrames, kPMax><<<blocks, 32 * kWarpsPerCta, smem, st>>>(a, o, S, Q);
     else k_search_fast<kLamWords, kTaskCap, kTaskFrames, kPMax><<<blocks, 32 * kWarpsPerCta, smem, st>>>(a, o, S, Q);
     note_launch();
