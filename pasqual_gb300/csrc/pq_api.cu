@@ -315,7 +315,13 @@ int pq_set_reads(pq_ctx* ctx, const uint8_t* reads, pq_idx num_reads, int read_l
         return fail(ctx, PQ_ERR_ARG, "num_reads * read_len does not fit the index width");
     if (num_reads && !reads) return fail(ctx, PQ_ERR_ARG, "reads is NULL");
     cudaSetDevice(ctx->device);
-    ctx->num_reads = num_reads;
+    // until they are in place: what fails on the way leaves neither these reads nor anything of others
+    ctx->have_reads = false;
+    ctx->num_reads = 0;
+    ctx->pk_ok[0] = ctx->pk_ok[1] = false;
+    ctx->sa_ok[0] = ctx->sa_ok[1] = false;
+    ctx->fm_ok[0] = ctx->fm_ok[1] = false;
+    ctx->graph_ok = false;
     ctx->L = read_len;
     ctx->t = min_overlap;
     // default seed depth by index size: a k-mer's rows number about n / 4^k, and each halving of
@@ -344,15 +350,8 @@ int pq_set_reads(pq_ctx* ctx, const uint8_t* reads, pq_idx num_reads, int read_l
     unsigned long long h[13];
     CK(cudaMemcpyAsync(h, ctx->counts.p, sizeof h, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    if (h[12]) {   // the reference's import drops reads with N and rejects any other symbol
-        ctx->have_reads = false;
-        ctx->num_reads = 0;
-        ctx->pk_ok[0] = ctx->pk_ok[1] = false;
-        ctx->sa_ok[0] = ctx->sa_ok[1] = false;
-        ctx->fm_ok[0] = ctx->fm_ok[1] = false;
-        ctx->graph_ok = false;
+    if (h[12])     // the reference's import drops reads with N and rejects any other symbol
         return fail(ctx, PQ_ERR_ARG, "reads must hold base codes 1..4 (A, C, G, T) only");
-    }
     ctx->C[0] = 0;
     ctx->C[1] = 0;
     ctx->C[2] = idx_t(h[0]);
@@ -363,11 +362,8 @@ int pq_set_reads(pq_ctx* ctx, const uint8_t* reads, pq_idx num_reads, int read_l
         ctx->sfx[c] = idx_t(h[4 + c]);
         ctx->pfx[c] = idx_t(h[8 + c]);
     }
+    ctx->num_reads = num_reads;
     ctx->have_reads = true;
-    ctx->pk_ok[0] = ctx->pk_ok[1] = false;
-    ctx->sa_ok[0] = ctx->sa_ok[1] = false;
-    ctx->fm_ok[0] = ctx->fm_ok[1] = false;
-    ctx->graph_ok = false;
     return PQ_OK;
 }
 
@@ -557,6 +553,7 @@ int pq_build_fm(pq_ctx* ctx, int dir) {
     if (!ctx->sa_ok[dir]) return fail(ctx, PQ_ERR_STATE, "no suffix array for this direction");
     cudaSetDevice(ctx->device);
     const size_t n = n_rows(ctx);
+    ctx->fm_ok[dir] = ctx->graph_ok = false;
     CK(need(ctx, ctx->blk[dir], n_blocks(ctx) * sizeof(OccBlock)));
     CK(need(ctx, ctx->sb[dir], n_supers(ctx) * 4 * sizeof(idx_t) + 64));
     CK(need(ctx, ctx->ri[dir], size_t(ctx->num_reads) * sizeof(idx_t) + 64));
@@ -582,7 +579,6 @@ int pq_build_fm(pq_ctx* ctx, int dir) {
     ctx->fm_ok[dir] = true;
     ctx->fm_k[dir] = k;
     ctx->lx_ok[dir] = false;
-    ctx->graph_ok = false;
     return PQ_OK;
 }
 
@@ -1040,6 +1036,7 @@ static int overlaps_once(pq_ctx* ctx) {
     int dev_sms = 152;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device);
     CK(cudaEventRecord(ctx->evk0, ctx->st));
+    ctx->graph_ok = false;
     if (nr && A.sorted_reduce) {
         // lean tier over every read; what it hands over is taken in search_finish
         const int ebcap = 64;
@@ -1519,7 +1516,10 @@ static int batched_once(pq_ctx** ctxs, int count, int flags) {
     CK(lead->q_batches.ensure(sizeof(pq::SearchBatch) * size_t(count)));
     CK(cudaMemcpyAsync(lead->q_batches.p, hb.data(), sizeof(pq::SearchBatch) * size_t(count), cudaMemcpyHostToDevice,
                        lead->st));
-    for (int b = 0; b < count; ++b) CK(cudaEventRecord(ctxs[b]->ev0, lead->st));
+    for (int b = 0; b < count; ++b) {
+        CK(cudaEventRecord(ctxs[b]->ev0, lead->st));
+        ctxs[b]->graph_ok = false;
+    }
     if (total_reads) {
         const int rc = queue_launch(lead, hb, order, (flags & PQ_BATCH_GRAPH) ? 1 : 0);
         if (rc != PQ_OK) return rc;

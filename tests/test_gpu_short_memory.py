@@ -83,3 +83,26 @@ def test_a_search_with_less_memory(batch, reads):
     for a, b in zip(*out):
         for f in FIELDS:
             assert np.array_equal(getattr(a, f), getattr(b, f)), f
+
+
+def test_reads_that_do_not_fit(reads):
+    """Refused reads leave a context without reads, not one whose sizes are theirs and whose buffers are not."""
+    few = reads[:5_000]
+    with context(few, 32) as P:
+        P.build_index()
+        want = P.construct_string_graph()
+        many = np.full((5_000_000, 100), 1, np.uint8)
+        hog = fill(many.size // 2)
+        with pytest.raises(pq.PQError) as refused:
+            P.set_reads(many, T)
+        assert refused.value.code == 3
+        for call in (lambda: P.sort(0), P.build_index, lambda: P.build_fm(1), P.overlaps, P.counts, P.graph):
+            with pytest.raises(pq.PQError) as state:
+                call()
+            assert state.value.code == 5
+        del hog
+        torch.cuda.empty_cache()
+        P.construct_index(few, T)
+        got = P.construct_string_graph()
+    for f in FIELDS:
+        assert np.array_equal(getattr(got, f), getattr(want, f)), f
