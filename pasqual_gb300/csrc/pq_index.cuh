@@ -129,6 +129,7 @@ struct SearchQueue {
     // without a queue: search only the reads read_list[0, *list_count) (nullptr: every read)
     const idx_t* read_list;
     const unsigned* list_count;
+    int dfs_max;                // level-0 intervals a (read, side) of the FM-index DFS may have
 };
 size_t warp_scratch_bytes(int L, int t, size_t nwarps, int ebcap);
 int search_fast_blocks(int L, int M, int num_sms);   // resident blocks of the fast kernel (M = L - t)

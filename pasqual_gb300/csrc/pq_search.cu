@@ -1374,8 +1374,8 @@ __global__ void __launch_bounds__(128, 5) k_search_fast(SearchArgs A0, SearchOut
                         const int st = reduce_sorted<W>(A, S, self, side, pbase_w + src, n0, rbase_w + lane, eb, ne, sc, probes);
                         if (st != OVF_NONE) status = st;
                         active = false;
-                    } else if (active && (n0 > CAP || (CAP == kTaskCap && A.sorted_reduce && Q.read_list))) {
-                        status = OVF_STACK;             // of a listed read (the lean tier's misses): the block tier's
+                    } else if (active && n0 > Q.dfs_max) {
+                        status = OVF_STACK;
                         active = false;
                     }
                     fresh = active;
@@ -1719,7 +1719,6 @@ __global__ void __launch_bounds__(128, 5) k_search_fast(SearchArgs A0, SearchOut
 // found by bisection; 1.2 M reads, 123 M suffixes: 1.5 against 2.4.  Eight CTAs of 64 registers per
 // SM; six or ten were 3 to 10 % slower.
 constexpr int kLeanThreads = 128;
-constexpr int kMissed = OVF_LEVELS;         // the scan does not serve the read
 
 template <int W>
 __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, SearchOut O0, WarpScratch S,
@@ -1796,10 +1795,7 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                     for (int w = 0; w < kScanWords; ++w) P1[w] = ~P0[w];
                 }
                 if (A.sa_seed == 2) {
-                    if (ok && !learned_rows(A, f0, f1, P0, P1, first, end, probes)) {
-                        ok = false;
-                        status = kMissed;
-                    }
+                    if (ok) ok = learned_rows(A, f0, f1, P0, P1, first, end, probes);
                     __syncwarp();
                 } else {
                     const int k = A.seed_k;
@@ -1815,10 +1811,7 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                     if (ok && (end[0] - first[0] > idx_t(kScanDirect) || end[1] - first[1] > idx_t(kScanDirect))) {
                         const idx_t lo[2] = {first[0], first[1]}, hi[2] = {end[0], end[1]};
                         sa_bounds2(f0, f1, A.dl, P0, P1, t < 32 * kScanWords ? t : 32 * kScanWords, lo, hi, first, end, probes);
-                        if (end[0] - first[0] > idx_t(kScanMax) || end[1] - first[1] > idx_t(kScanMax)) {
-                            ok = false;
-                            status = kMissed;
-                        }
+                        ok = end[0] - first[0] <= idx_t(kScanMax) && end[1] - first[1] <= idx_t(kScanMax);
                     }
                 }
                 slots[lane] = 0;
@@ -1895,7 +1888,10 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                 if (lane < waiting) check(lane, (1u << waiting) - 1u);
                 __syncwarp();
                 const int m = slots[lane];
-                if (m > kRedMax) ok = false;
+                if (m > kRedMax) {
+                    ok = false;
+                    status = OVF_STACK;
+                }
                 int count = 0;
                 if (ok && m && status == OVF_NONE)
                     status = reduce_gathered<W>(L, S, self, side, rbase + lane, m, ebase, 32, ne, count);
@@ -1910,7 +1906,7 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
             }
             if (have && (!ok || status != OVF_NONE)) {   // the fast or the block tier redoes this read
                 if (ok) O.status[r] = uint8_t(status);
-                if (status == kMissed && A.miss_list) A.miss_list[atomicAdd(A.miss_count, 1u)] = self;
+                if (!ok && status == OVF_NONE && A.miss_list) A.miss_list[atomicAdd(A.miss_count, 1u)] = self;
                 else O.ovf_list[atomicAdd(O.ovf_count, 1u)] = self;
             }
             // one reservation of edge slots for the warp's reads
@@ -2047,6 +2043,7 @@ cudaError_t search_fast(const SearchArgs& a, const SearchOut& o, int blocks, voi
     SearchQueue Q{};
     Q.read_list = list;
     Q.list_count = count;
+    Q.dfs_max = list ? 0 : kTaskCap;        // of listed reads (the lean tier's misses) the sorted reduction only
     if (lam_words(a.L - a.t) == 2) k_search_fast<2, kTaskCap, kTaskFrames, kPMax><<<blocks, 32 * kWarpsPerCta, smem, st>>>(a, o, S, Q);
     else k_search_fast<kLamWords, kTaskCap, kTaskFrames, kPMax><<<blocks, 32 * kWarpsPerCta, smem, st>>>(a, o, S, Q);
     note_launch();
@@ -3011,6 +3008,7 @@ cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* l
     SearchQueue Q{};
     Q.read_list = list;
     Q.list_count = count;
+    Q.dfs_max = kHeavyCap;
     // static shared memory (~46 KB) plus the reads: past the 48 KB a launch may take unasked
     constexpr size_t kReadSmem = 180 * 1024;            // reads of up to 5760 bases
     if (smem > kReadSmem) return cudaErrorInvalidValue;
@@ -3031,13 +3029,15 @@ size_t queue_scratch_bytes(int M_max, size_t nwarps, int ebcap, bool lean) {
     return lean ? lean_layout(M_max, nwarps, ebcap, nullptr, nullptr) : scratch_layout(M_max, nwarps, ebcap, nullptr, nullptr);
 }
 
-cudaError_t search_fast_queue(const SearchQueue& q, int L_max, int M_max, int blocks, void* scratch,
+cudaError_t search_fast_queue(const SearchQueue& queue, int L_max, int M_max, int blocks, void* scratch,
                               size_t scratch_bytes, int ebcap, cudaStream_t st) {
     const size_t nwarps = size_t(blocks) * kWarpsPerCta;
     WarpScratch S;
     if (scratch_bytes < scratch_layout(M_max, nwarps, ebcap, scratch, &S)) return cudaErrorInvalidValue;
     const int words = (L_max + 15) / 16;
     size_t smem = size_t(words) * 32 * kWarpsPerCta * sizeof(uint32_t);
+    SearchQueue q = queue;
+    q.dfs_max = kTaskCap;
     SearchArgs a{};
     SearchOut o{};
     if (lam_words(M_max) == 2) k_search_fast<2, kTaskCap, kTaskFrames, kPMax><<<blocks, 32 * kWarpsPerCta, smem, st>>>(a, o, S, q);
