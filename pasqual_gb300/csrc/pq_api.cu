@@ -63,6 +63,11 @@ struct DevBuf {
     }
     template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
+struct TmpBuf : DevBuf {        // for one call
+    TmpBuf() = default;
+    TmpBuf(const TmpBuf&) = delete;
+    ~TmpBuf() { release(); }
+};
 
 }  // namespace
 
@@ -88,7 +93,7 @@ struct pq_ctx {
     bool sa_ok[2] = {false, false}, fm_ok[2] = {false, false};
     int fm_k[2] = {0, 0};
     int kx_bases[2] = {0, 0};  // bases per row kx holds beyond the table's k (0: none)
-    DevBuf sort_tmp, counts;
+    DevBuf sort_tmp, counts, seeds;                         // seeds: of the calls that return them
     int kmer_from_sort[2] = {0, 0};                         // k of the k-mer table the last sort entered
     const uint8_t* bwt_hint[2] = {nullptr, nullptr};       // the last sort's BWT symbols, inside sort_tmp
     bool pk_ok[2] = {false, false};                        // pk[dir] holds this read set's packed text
@@ -139,11 +144,12 @@ static int fail(pq_ctx* c, int code, const std::string& msg) {
     } while (0)
 
 // Gives back the device memory that the context holds but can do without: the last sort's working
-// memory, and the rows' next bases (the search then compares texts).  Not while a kernel that uses either
+// memory, that of the seeds, and the rows' next bases (the search then compares texts).  Not while a kernel that uses either
 // is about to be launched.  False where there was none.
 static bool give_back(pq_ctx* c) {
-    bool any = c->sort_tmp.p != nullptr;
+    bool any = c->sort_tmp.p || c->seeds.p;
     c->sort_tmp.release();
+    c->seeds.release();
     c->bwt_hint[0] = c->bwt_hint[1] = nullptr;
     for (int d = 0; d < 2; ++d) {
         any = any || c->kx[d].p;
@@ -152,7 +158,7 @@ static bool give_back(pq_ctx* c) {
     }
     return any;
 }
-// b (neither of those two) with `bytes` bytes, if need be after giving them back
+// b (not one of those in use) with `bytes` bytes, if need be after giving them back
 static cudaError_t need(pq_ctx* c, DevBuf& b, size_t bytes) {
     const cudaError_t e = b.ensure(bytes);
     return e == cudaErrorMemoryAllocation && give_back(c) ? b.ensure(bytes) : e;
@@ -270,7 +276,8 @@ void pq_destroy(pq_ctx* ctx) {
                       &ctx->oF, &ctx->status, &ctx->esrc, &ctx->e_dest, &ctx->e_trans, &ctx->e_len,
                       &ctx->e_type, &ctx->ctrs, &ctx->ovf_list, &ctx->off, &ctx->g_dest, &ctx->g_len,
                       &ctx->g_type, &ctx->g_trans, &ctx->asm_tmp, &ctx->wide, &ctx->warp_scratch,
-                      &ctx->heavy_scratch, &ctx->ovf2, &ctx->ovf3, &ctx->ovf4, &ctx->block_scratch};
+                      &ctx->heavy_scratch, &ctx->ovf2, &ctx->ovf3, &ctx->ovf4, &ctx->block_scratch, &ctx->lx_tmp,
+                      &ctx->seeds};
     for (DevBuf* b : bufs) b->release();
     for (int d = 0; d < 2; ++d) {
         ctx->sa[d].release();
@@ -488,6 +495,26 @@ int pq_get_sa_rows(pq_ctx* ctx, int dir, uint64_t first, uint64_t count, pq_idx*
     return PQ_OK;
 }
 
+// Every read's seed (first row, size, depth) and the working memory of `rows` rows' records, kept from call to
+// call: four allocations and releases a call took index and seeds of 0.8 M reads from 10.0 to 10.5 ms.
+struct SeedBufs {
+    idx_t *start, *size;
+    uint16_t* depth;
+    void* tmp;
+    size_t tmp_bytes;
+};
+static cudaError_t seed_bufs(pq_ctx* ctx, size_t rows, SeedBufs* b) {
+    const size_t nr = ctx->num_reads, idx = (nr * sizeof(idx_t) + 255) & ~size_t(255), dep = (nr * sizeof(uint16_t) + 255) & ~size_t(255);
+    b->tmp_bytes = rows ? pq::sort_seeds_tmp_bytes(rows, nr) : 0;
+    const cudaError_t e = need(ctx, ctx->seeds, 2 * idx + dep + b->tmp_bytes);
+    char* p = ctx->seeds.as<char>();
+    b->start = reinterpret_cast<idx_t*>(p);
+    b->size = reinterpret_cast<idx_t*>(p + idx);
+    b->depth = reinterpret_cast<uint16_t*>(p + 2 * idx);
+    b->tmp = p + 2 * idx + dep;
+    return e;
+}
+
 // The seed records of the sort buckets in rows [r0, r1) of direction dir applied to the host arrays
 // start/size/depth (one entry per read): a record replaces a read's seed when it is deeper, as in
 // src/sufsort.c:182-189.  Not part of the public header.
@@ -504,20 +531,16 @@ int pq_apply_sort_seeds(pq_ctx* ctx, int dir, uint64_t r0, uint64_t r1, pq_idx* 
         CK(pq::pack_text(ctx->reads.as<uint8_t>(), n, idx_t(ctx->L), dir, ctx->pk[dir].as<uint64_t>(), ctx->st));
         ctx->pk_ok[dir] = true;
     }
-    DevBuf s, z, d, tmp;
-    CK(need(ctx, s, nr * sizeof(idx_t)));
-    CK(need(ctx, z, nr * sizeof(idx_t)));
-    CK(need(ctx, d, nr * sizeof(uint16_t)));
-    const size_t tb = pq::sort_seeds_tmp_bytes(size_t(r1 - r0), nr);
-    CK(need(ctx, tmp, tb));
-    CK(cudaMemcpyAsync(s.p, start, nr * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(z.p, size, nr * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(d.p, depth, nr * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->st));
+    SeedBufs b;
+    CK(seed_bufs(ctx, size_t(r1 - r0), &b));
+    CK(cudaMemcpyAsync(b.start, start, nr * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(b.size, size, nr * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(b.depth, depth, nr * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->st));
     CK(pq::sort_seeds(ctx->sa[dir].as<idx_t>(), ctx->pk[dir].as<uint64_t>(), ctx->num_reads, idx_t(ctx->L), ctx->t, size_t(r0),
-                      size_t(r1), d.as<uint16_t>(), s.as<idx_t>(), z.as<idx_t>(), tmp.p, tb, ctx->st));
-    CK(cudaMemcpyAsync(start, s.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(size, z.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(depth, d.p, nr * sizeof(uint16_t), cudaMemcpyDeviceToHost, ctx->st));
+                      size_t(r1), b.depth, b.start, b.size, b.tmp, b.tmp_bytes, ctx->st));
+    CK(cudaMemcpyAsync(start, b.start, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(size, b.size, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(depth, b.depth, nr * sizeof(uint16_t), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return PQ_OK;
 }
@@ -612,7 +635,7 @@ int pq_get_index_ref(pq_ctx* ctx, int dir, uint64_t* bitmap, pq_idx* sample, pq_
     cudaSetDevice(ctx->device);
     const size_t nblk = n_blocks(ctx);
     if (bitmap || sample) {
-        DevBuf bm, smp;
+        TmpBuf bm, smp;
         CK(need(ctx, bm, nblk * 5 * sizeof(uint64_t)));
         CK(need(ctx, smp, nblk * 5 * sizeof(idx_t)));
         const idx_t* fix = dir == 0 ? ctx->sfx : ctx->pfx;
@@ -621,8 +644,6 @@ int pq_get_index_ref(pq_ctx* ctx, int dir, uint64_t* bitmap, pq_idx* sample, pq_
         if (bitmap) CK(cudaMemcpyAsync(bitmap, bm.p, nblk * 5 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->st));
         if (sample) CK(cudaMemcpyAsync(sample, smp.p, nblk * 5 * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
-        bm.release();
-        smp.release();
     }
     if (reads_index && ctx->num_reads)
         CK(cudaMemcpyAsync(reads_index, ctx->ri[dir].p, size_t(ctx->num_reads) * sizeof(idx_t),
@@ -637,13 +658,12 @@ int pq_get_seeds(pq_ctx* ctx, int dir, pq_idx* start, pq_idx* size, uint16_t* de
     cudaSetDevice(ctx->device);
     const size_t nr = ctx->num_reads;
     if (!nr) return PQ_OK;
-    DevBuf s, z;
-    CK(need(ctx, s, nr * sizeof(idx_t)));
-    CK(need(ctx, z, nr * sizeof(idx_t)));
+    SeedBufs b;
+    CK(seed_bufs(ctx, 0, &b));
     CK(pq::read_seeds(ctx->reads.as<uint8_t>(), ctx->num_reads, ctx->L, dir, ctx->fm_k[dir],
-                      ctx->kt[dir].as<idx_t>(), s.as<idx_t>(), z.as<idx_t>(), ctx->st));
-    if (start) CK(cudaMemcpyAsync(start, s.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
-    if (size) CK(cudaMemcpyAsync(size, z.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
+                      ctx->kt[dir].as<idx_t>(), b.start, b.size, ctx->st));
+    if (start) CK(cudaMemcpyAsync(start, b.start, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
+    if (size) CK(cudaMemcpyAsync(size, b.size, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     if (depth)
         for (size_t i = 0; i < nr; ++i) depth[i] = uint16_t(ctx->fm_k[dir]);
@@ -661,19 +681,14 @@ int pq_get_sort_seeds(pq_ctx* ctx, int dir, pq_idx* start, pq_idx* size, uint16_
         CK(pq::pack_text(ctx->reads.as<uint8_t>(), n, idx_t(ctx->L), dir, ctx->pk[dir].as<uint64_t>(), ctx->st));
         ctx->pk_ok[dir] = true;
     }
-    DevBuf s, z, d, tmp;
-    CK(need(ctx, s, nr * sizeof(idx_t)));
-    CK(need(ctx, z, nr * sizeof(idx_t)));
-    CK(need(ctx, d, nr * sizeof(uint16_t)));
-    const size_t tb = pq::sort_seeds_tmp_bytes(n, nr);
-    CK(need(ctx, tmp, tb));
-    CK(pq::seed_init(ctx->reads.as<uint8_t>(), ctx->num_reads, idx_t(ctx->L), dir, ctx->C, d.as<uint16_t>(),
-                     s.as<idx_t>(), z.as<idx_t>(), ctx->st));
+    SeedBufs b;
+    CK(seed_bufs(ctx, n, &b));
+    CK(pq::seed_init(ctx->reads.as<uint8_t>(), ctx->num_reads, idx_t(ctx->L), dir, ctx->C, b.depth, b.start, b.size, ctx->st));
     CK(pq::sort_seeds(ctx->sa[dir].as<idx_t>(), ctx->pk[dir].as<uint64_t>(), ctx->num_reads, idx_t(ctx->L), ctx->t, 0, n,
-                      d.as<uint16_t>(), s.as<idx_t>(), z.as<idx_t>(), tmp.p, tb, ctx->st));
-    if (start) CK(cudaMemcpyAsync(start, s.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
-    if (size) CK(cudaMemcpyAsync(size, z.p, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
-    if (depth) CK(cudaMemcpyAsync(depth, d.p, nr * sizeof(uint16_t), cudaMemcpyDeviceToHost, ctx->st));
+                      b.depth, b.start, b.size, b.tmp, b.tmp_bytes, ctx->st));
+    if (start) CK(cudaMemcpyAsync(start, b.start, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
+    if (size) CK(cudaMemcpyAsync(size, b.size, nr * sizeof(idx_t), cudaMemcpyDeviceToHost, ctx->st));
+    if (depth) CK(cudaMemcpyAsync(depth, b.depth, nr * sizeof(uint16_t), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return PQ_OK;
 }
@@ -956,7 +971,7 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool 
         W.stack = ctx->wide.p;
         W.frames = static_cast<char*>(ctx->wide.p) + ((st_bytes + 255) & ~size_t(255));
         W.edges = static_cast<char*>(W.frames) + ((fr_bytes + 255) & ~size_t(255));
-        DevBuf dlist;
+        TmpBuf dlist;
         for (int attempt = 0; attempt < 8 && !list.empty(); ++attempt) {
             CK(dlist.ensure(list.size() * sizeof(idx_t)));
             CK(cudaMemcpyAsync(dlist.p, list.data(), list.size() * sizeof(idx_t), cudaMemcpyHostToDevice, ctx->st));
@@ -969,17 +984,14 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool 
             for (idx_t r : list) {
                 uint8_t s = stv[r];
                 if (s == ERR_TOO_MANY) {
-                    dlist.release();
                     return fail(ctx, PQ_ERR_TOO_MANY_EDGES, "assembly failed. Try a larger min overlap length.");
                 }
                 if (s == ERR_CAP) {
-                    dlist.release();
                     return fail(ctx, PQ_ERR_CAPACITY, "interval table exceeded (2L)^2 entries for read " +
                                                           std::to_string((unsigned long long)r));
                 }
                 if (s == OVF_POOL) again.push_back(r);
                 else if (s != OVF_NONE) {
-                    dlist.release();
                     return fail(ctx, PQ_ERR_INTERNAL, "wide search left read unfinished");
                 }
             }
@@ -990,7 +1002,6 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool 
             CK(grow_pool(ctx, O, need, keep));
             list.swap(again);
         }
-        dlist.release();
         if (!list.empty()) return fail(ctx, PQ_ERR_INTERNAL, "edge pool retries exhausted");
     }
     if (ctx->wide_reads) ctx->ms_wide = wall_ms() - tw0;
@@ -1251,7 +1262,7 @@ int pq_learned_predict(pq_ctx* ctx, int dir, const uint32_t* keys, uint64_t n, i
     if (!ctx->lx_ok[dir] || !ctx->lx_segs[dir]) return fail(ctx, PQ_ERR_STATE, "no learned index for this direction");
     if (!n) return PQ_OK;
     cudaSetDevice(ctx->device);
-    DevBuf dk, dp, ds;
+    TmpBuf dk, dp, ds;
     CK(dk.ensure(n * 4));
     CK(dp.ensure(n * 8));
     CK(ds.ensure(n * 4));
@@ -1260,9 +1271,6 @@ int pq_learned_predict(pq_ctx* ctx, int dir, const uint32_t* keys, uint64_t n, i
     CK(cudaMemcpyAsync(pred, dp.p, n * 8, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(seg, ds.p, n * 4, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    dk.release();
-    dp.release();
-    ds.release();
     return PQ_OK;
 }
 
@@ -1287,7 +1295,7 @@ int pq_learned_keys(pq_ctx* ctx, int dir, uint32_t* keys, pq_idx* first_row, uin
 
 int pq_mlp_forward(const float* params, const float* x, int n, float* y) {
     if (!params || n < 0 || (n && (!x || !y))) return PQ_ERR_ARG;
-    DevBuf dp, dx, dy;
+    TmpBuf dp, dx, dy;
     if (dp.ensure(pq::kLxStride * 4) || dx.ensure(size_t(n) * 4 + 4) || dy.ensure(size_t(n) * 4 + 4)) return PQ_ERR_NOMEM;
     int rc = PQ_OK;
     if (cudaMemcpy(dp.p, params, pq::kLxStride * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -1295,15 +1303,12 @@ int pq_mlp_forward(const float* params, const float* x, int n, float* y) {
         pq::mlp_forward(dp.as<float>(), dx.as<float>(), n, dy.as<float>(), 0) != cudaSuccess ||
         (n && cudaMemcpy(y, dy.p, size_t(n) * 4, cudaMemcpyDeviceToHost) != cudaSuccess))
         rc = PQ_ERR_CUDA;
-    dp.release();
-    dx.release();
-    dy.release();
     return rc;
 }
 
 int pq_mlp_backward(const float* params, const float* x, const float* dy, int n, float* grad) {
     if (!params || !grad || n < 0 || (n && (!x || !dy))) return PQ_ERR_ARG;
-    DevBuf dp, dx, dg, dd;
+    TmpBuf dp, dx, dg, dd;
     if (dp.ensure(pq::kLxStride * 4) || dx.ensure(size_t(n) * 4 + 4) || dd.ensure(size_t(n) * 4 + 4) ||
         dg.ensure(pq::kLxParams * 4))
         return PQ_ERR_NOMEM;
@@ -1314,17 +1319,13 @@ int pq_mlp_backward(const float* params, const float* x, const float* dy, int n,
         pq::mlp_backward(dp.as<float>(), dx.as<float>(), dd.as<float>(), n, dg.as<float>(), 0) != cudaSuccess ||
         cudaMemcpy(grad, dg.p, pq::kLxParams * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = PQ_ERR_CUDA;
-    dp.release();
-    dx.release();
-    dd.release();
-    dg.release();
     return rc;
 }
 
 int pq_mlp_adam_step(float* params, float* m1, float* m2, const float* x, const float* target, int n, int step,
                      float lr) {
     if (!params || !m1 || !m2 || n <= 0 || !x || !target || step < 1) return PQ_ERR_ARG;
-    DevBuf dp, dm1, dm2, dx, dt;
+    TmpBuf dp, dm1, dm2, dx, dt;
     if (dp.ensure(pq::kLxStride * 4) || dm1.ensure(pq::kLxParams * 4) || dm2.ensure(pq::kLxParams * 4) ||
         dx.ensure(size_t(n) * 4) || dt.ensure(size_t(n) * 4))
         return PQ_ERR_NOMEM;
@@ -1340,11 +1341,6 @@ int pq_mlp_adam_step(float* params, float* m1, float* m2, const float* x, const 
         cudaMemcpy(m1, dm1.p, pq::kLxParams * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
         cudaMemcpy(m2, dm2.p, pq::kLxParams * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = PQ_ERR_CUDA;
-    dp.release();
-    dm1.release();
-    dm2.release();
-    dx.release();
-    dt.release();
     return rc;
 }
 
