@@ -102,7 +102,8 @@ PQ_API int pq_sort (pq_ctx * ctx, int dir);
  * working memory: one pass over everything is taken while it needs no more than chunks of this size
  * may (20 bytes and two positions a suffix of a chunk, 3 1/4 bytes a suffix of the index), else the
  * chunks are sorted one after the other into their place.  A bucket larger than a chunk makes
- * pq_sort return PQ_ERR_CAPACITY.  Without a limit, chunks are taken where the working memory of one
+ * pq_sort return PQ_ERR_CAPACITY, and so do reads of more than 268 bases with a limit below their
+ * suffixes.  Without a limit, chunks are taken where the working memory of one
  * pass does not fit the device.  Same suffix array either way. */
 PQ_API int pq_set_sort_chunk (pq_ctx * ctx, uint64_t max_suffixes);
 

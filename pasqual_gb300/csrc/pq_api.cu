@@ -410,7 +410,7 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
         want_kx = false;
         room = ctx->sort_tmp.ensure(tmp_bytes);
     }
-    bool too_small = false;             // chunks by the memory, not by the caller
+    bool too_small = false;             // the memory is: chunks that the caller did not ask for
     for (size_t c = std::min(n / 2, size_t(1) << 30); room == cudaErrorMemoryAllocation && !ctx->sort_chunk && c > n / 512; c /= 2) {
         const size_t b = pq::suffix_sort_tmp_bytes(n, ctx->num_reads, ctx->L, c);
         if (b >= tmp_bytes) continue;
@@ -433,6 +433,9 @@ static int sort_dir(pq_ctx* ctx, int dir, bool side_outputs) {
     if (rc == int(cudaErrorNotSupported)) {
         ctx->sa_ok[dir] = had_sa;       // a refusal leaves the rows as they were
         if (too_small) return fail(ctx, PQ_ERR_NOMEM, "suffix sort: no room for its working memory");
+        if (ctx->L > pq::kChunkMaxLen)
+            return fail(ctx, PQ_ERR_CAPACITY, cap && cap < n ? "suffix sort: reads of more than 268 bases are not sorted in chunks"
+                                                             : "suffix sort: reads this long are sorted up to 2^31 - 1 suffixes");
         return fail(ctx, PQ_ERR_CAPACITY, "suffix sort: a 6-base bucket holds more suffixes than a sort chunk");
     }
     if (rc != 0) {

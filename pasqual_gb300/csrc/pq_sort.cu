@@ -586,7 +586,6 @@ constexpr int kSplitTile = 8192;            // elements per tile of the partitio
 constexpr int kSplitThreads = 512;
 constexpr int kMaxDigit = 11;               // bits of one partition pass
 constexpr int kMaxWords = 9;                // 64-bit words of a suffix the networks compare
-constexpr int kChunkMaxLen = 268;           // longest reads sorted in chunks
 #ifdef PQ_IDX64
 using kmer_int = unsigned long long;
 #else

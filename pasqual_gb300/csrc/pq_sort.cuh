@@ -8,13 +8,15 @@ namespace pq {
 // then text position).  Returns 0 or a cudaError_t value.  cap (0: none) is the largest number of
 // suffixes the caller wants sorted at a time: the sort then takes no more working memory than chunks
 // of that size would (in chunks when one pass needs more), and returns cudaErrorNotSupported when a
-// 6-base bucket exceeds it.  When bwt_out is given it receives the BWT symbol (0 = `$`, 1..4) of
+// 6-base bucket exceeds it or the reads are longer than kChunkMaxLen (so do more than 2^31 - 1 suffixes of
+// reads too long for the networks, with or without it).  When bwt_out is given it receives the BWT symbol (0 = `$`, 1..4) of
 // every row, inside tmp (valid until tmp is reused), or nullptr when the sort went by prefix
 // doubling.  pk_out (n/32 + 4 words), when given, receives the packed text of the direction (see
 // pack_text) instead of tmp.  kt, when given, receives the table of kmer_k-mers (FmView::kt) and kx
 // (n entries), when given beside it, every row's next bases (FmView::kx); *kmer_done tells whether
 // the table is complete (else the caller builds it) and *kx_bases how many bases kx holds (0: none).
 constexpr int kSortKeyBases = 14;           // longest k-mers of the table
+constexpr int kChunkMaxLen = 268;           // longest reads sorted in chunks
 size_t suffix_sort_tmp_bytes(size_t n, size_t num_reads, int L, size_t cap = 0);
 int suffix_sort(const uint8_t* reads, idx_t num_reads, int L, int dir, idx_t* sa, size_t cap, void* tmp,
                 size_t tmp_bytes, cudaStream_t st, const uint8_t** bwt_out = nullptr, uint64_t* pk_out = nullptr,

@@ -36,3 +36,15 @@ def test_a_refused_rebuild_is_no_index(genome, width):
         got = P.construct_string_graph()
     for f in FIELDS:
         assert np.array_equal(getattr(got, f), getattr(want, f)), f
+
+
+@pytest.mark.parametrize("L,reason", [(300, "268 bases"), (100, "6-base bucket")])
+def test_a_refused_sort_names_its_reason(L, reason):
+    gen = synth.genome(length=40_000, gc=0.42, seed=43)
+    rd = synth.dedup(synth.reads_for_coverage(gen, L, 15, 0.003, seed=44))
+    with pq.Pasqual(32) as P:
+        P.set_reads(rd, 63)
+        P.set_sort_chunk(rd.size // 2 if L > 268 else max(2, rd.size // 2000))
+        with pytest.raises(pq.PQError, match=reason) as refused:
+            P.sort(0)
+        assert refused.value.code == 6
