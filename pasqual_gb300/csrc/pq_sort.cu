@@ -855,7 +855,7 @@ struct MsdRanges {
     const unsigned long long* start;
     const unsigned long long* end;
     const unsigned* tile0;
-    const int* shift;                   // a range's digit is (element >> shift) & (2^bits - 1),
+    const int* shift;                   // a range's digit is (element >> (shift & 63)) & (2^bits - 1),
     int ushift;                         // with one shift for all when `shift` is null
     int count, bits;
     unsigned long long base;            // of starts and ends: element 0 of the array is theirs of `base`
@@ -907,7 +907,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_msd_count(const uint64_t* __r
             q = range_of(r, t);
             __syncthreads();
         }
-        const int shift = r.shift ? r.shift[q] : r.ushift;
+        const int shift = r.shift ? r.shift[q] & 63 : r.ushift;
         const size_t b = r.start[q] - r.base + size_t(t - r.tile0[q]) * kSplitTile;
         const size_t e = zmin(r.end[q] - r.base, b + kSplitTile);
         #pragma unroll 4
@@ -954,7 +954,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_msd_split(const uint64_t* 
     constexpr int kPer = kSplitTile / kSplitThreads;
     for (unsigned t = blockIdx.x; t < tiles; t += gridDim.x) {
         const int q = range_of(r, t);
-        const int shift = r.shift ? r.shift[q] : r.ushift;
+        const int shift = r.shift ? r.shift[q] & 63 : r.ushift;
         const size_t b = r.start[q] - r.base + size_t(t - __ldg(r.tile0 + q)) * kSplitTile;
         const int m = int(zmin(size_t(kSplitTile), r.end[q] - r.base - b));
         uint64_t v[kPer];
@@ -1944,9 +1944,10 @@ __global__ void k_refine_cta(const unsigned long long* __restrict__ list, const 
 // strings, position -- and one whose suffixes all go on past equal heads first gets new elements
 // of its next bases, until every part fits the local kernel.
 
-constexpr int kMoreRanges = 4096;           // ranges described at a time,
-constexpr int kMoreSplits = 64;             // and split at a time
+constexpr int kMoreRanges = 4096;           // ranges described at a time
 constexpr int kMoreMerge = 2048;            // children put together for the local kernel
+// ranges split at a time (16 KB each: a quarter byte a suffix)
+static size_t more_splits_at(size_t m) { return std::min<size_t>(1024, std::max<size_t>(64, m >> 16)); }
 
 // new elements for ranges whose suffixes are equal in their first off[range] bases: the next
 // more_bits / 2 of them, left-aligned in the key
@@ -1993,6 +1994,89 @@ __global__ void __launch_bounds__(kSplitThreads) k_more_diff(const uint64_t* __r
     }
 }
 
+// The children of range blockIdx.x from their counts: their places (cursor, which the split advances) and,
+// from large[listed] on, their buckets.  Neighbours are one where they start in the same kMoreMerge elements
+// of the range (ten thousand equal strings split by position would else be a thousand buckets: 10 K equal
+// reads of 100 bases 5.3 ms, 2.3 together); children of more than kLocalLarge go to `again`, the first of
+// them also to r.first.  Listed here, their counts stay on the device: at 20 % GC half of 143 M suffixes come
+// in 3.4 thousand buckets that have to be split.  With 8 KB of counts of each read by the host, and two
+// launches for the k-mers of each, an index of both directions took 107 ms (radix passes and refinement
+// 26), now 18.8.
+struct MoreLists {
+    unsigned long long large, more;         // listed in `large` and in `again`
+    MsdBucket first[256];
+};
+__global__ void __launch_bounds__(kScanThreads) k_more_list(const unsigned long long* __restrict__ cnt, MsdRanges r,
+                                                            const int* __restrict__ off, unsigned long long* __restrict__ cursor,
+                                                            unsigned listed, MsdBucket* __restrict__ large, unsigned cap_large,
+                                                            MsdBucket* __restrict__ again, unsigned cap_again,
+                                                            MoreLists* __restrict__ c) {
+    constexpr int kBins = 1 << kMoreBits, kPer = kBins / kScanThreads, kWords = kBins / 32;
+    __shared__ unsigned pref[kBins], wsum[kScanThreads / 32], some[kWords], begin[kWords];
+    __shared__ unsigned long long wtot;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned long long* const n = cnt + (size_t(blockIdx.x) << kMoreBits);
+    const unsigned long long start = r.start[blockIdx.x];
+    const unsigned id_off = (unsigned(off[blockIdx.x]) << kIdBits) | (unsigned(r.shift[blockIdx.x]) >> 6);
+    if (tid < kWords) some[tid] = begin[tid] = 0;
+    unsigned v[kPer], mine = 0;                 // (a range has fewer than 2^32 elements)
+    #pragma unroll
+    for (int i = 0; i < kPer; ++i) mine += v[i] = unsigned(n[tid * kPer + i]);
+    unsigned x = mine;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    unsigned run = x - mine;
+    for (int w = 0; w < warp; ++w) run += wsum[w];
+    #pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int b = tid * kPer + i;
+        pref[b] = run;
+        cursor[(size_t(blockIdx.x) << kMoreBits) + b] = start + run;
+        if (v[i]) atomicOr(&some[b >> 5], 1u << (b & 31));
+        run += v[i];
+    }
+    if (tid == kScanThreads - 1) wtot = run;
+    __syncthreads();
+    // the first child from b + 1 on in a mask, or kBins
+    auto next = [](const unsigned* mask, int b) {
+        for (int w = (b + 1) >> 5; w < kWords; ++w) {
+            const unsigned y = w == (b + 1) >> 5 ? mask[w] & (~0u << ((b + 1) & 31)) : mask[w];
+            if (y) return 32 * w + __ffs(y) - 1;
+        }
+        return kBins;
+    };
+    // where a bucket begins: at a child too large for company, after one, and where another kMoreMerge begins
+    #pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int b = tid * kPer + i;
+        if (!v[i]) continue;
+        const bool alone = v[i] > unsigned(kLocalLarge - kMoreMerge);
+        if (alone || pref[b] == 0) atomicOr(&begin[b >> 5], 1u << (b & 31));
+        if (alone || pref[b] / kMoreMerge != (pref[b] + v[i]) / kMoreMerge) {
+            const int e = next(some, b);
+            if (e < kBins) atomicOr(&begin[e >> 5], 1u << (e & 31));
+        }
+    }
+    __syncthreads();
+    #pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int b = tid * kPer + i;
+        if (!((begin[b >> 5] >> (b & 31)) & 1u)) continue;
+        const int e = next(begin, b);
+        const unsigned size = (e < kBins ? pref[e] : unsigned(wtot)) - pref[b];
+        const bool fits = size <= unsigned(kLocalLarge);
+        const MsdBucket bucket{start + pref[b], size, id_off};
+        const unsigned long long at = fits ? listed + atomicAdd(&c->large, 1ull) : atomicAdd(&c->more, 1ull);
+        if (at < (fits ? cap_large : cap_again)) (fits ? large : again)[at] = bucket;
+        if (!fits && at < sizeof c->first / sizeof c->first[0]) c->first[at] = bucket;
+    }
+}
+
 __global__ void __launch_bounds__(kSplitThreads) k_more_copy(const uint64_t* __restrict__ from, MsdRanges r,
                                                              uint64_t* __restrict__ to) {
     const unsigned tiles = r.tile0[r.count];
@@ -2006,10 +2090,12 @@ __global__ void __launch_bounds__(kSplitThreads) k_more_copy(const uint64_t* __r
 
 // A k-mer table whose k-mers span buckets is entered by minimum and maximum: prepared so (mode 0;
 // mode 2 only where a k-mer is still absent), then absent ones set as everywhere else (mode 1:
-// last < first)
-__global__ void k_kmer_span(idx_t* __restrict__ kt, size_t c0, size_t c1, int mode) {
+// last < first).  Of all k-mers, or of those of `count` listed buckets, 2^shift each.
+__global__ void k_kmer_span(idx_t* __restrict__ kt, size_t count, int mode, const MsdBucket* __restrict__ list, int shift) {
     const size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t i = c0 + size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < c1; i += stride) {
+    for (size_t j = size_t(blockIdx.x) * blockDim.x + threadIdx.x; j < count << shift; j += stride) {
+        size_t i = j;
+        if (list) i = (size_t(list[j >> shift].id_off & ((1u << kIdBits) - 1)) << shift) | (j & ((size_t(1) << shift) - 1));
         idx_t* const k = kt + 2 * i;
         if (mode == 0 || (mode == 2 && k[1] < k[0])) {
             k[0] = ~idx_t(0);
@@ -2054,6 +2140,9 @@ struct MsdScratch {
     size_t rtmp_bytes;
     unsigned char* r_desc;                          // further splits: a RangeBlock,
     unsigned long long *r_diff, *r_cnt, *r_cursor;  // r_diff: differences, then first elements
+    MoreLists* r_lists;                             // before r_cnt, cleared with it
+    MsdBucket* again;
+    size_t splits;
     uint64_t* pk;
     uint8_t* bwt;
     unsigned long long* hist6;
@@ -2106,8 +2195,11 @@ MsdScratch msd_layout(void* base, const MsdPlan& p, size_t m, size_t nr) {
     s.rtmp = take(s.rtmp_bytes);
     s.r_desc = reinterpret_cast<unsigned char*>(take(RangeBlock{size_t(kMoreRanges)}.bytes()));
     s.r_diff = reinterpret_cast<U*>(take(2 * kMoreRanges * 8));
-    s.r_cnt = reinterpret_cast<U*>(take((size_t(kMoreSplits) << kMoreBits) * 8));
-    s.r_cursor = reinterpret_cast<U*>(take((size_t(kMoreSplits) << kMoreBits) * 8));
+    s.splits = more_splits_at(m);
+    s.r_lists = reinterpret_cast<MoreLists*>(take(sizeof(MoreLists)));
+    s.r_cnt = reinterpret_cast<U*>(take((s.splits << kMoreBits) * 8));
+    s.r_cursor = reinterpret_cast<U*>(take((s.splits << kMoreBits) * 8));
+    s.again = reinterpret_cast<MsdBucket*>(take(s.cap_more * sizeof(MsdBucket)));
     s.pk = reinterpret_cast<uint64_t*>(take((p.n / 32 + 4) * 8));
     s.bwt = reinterpret_cast<uint8_t*>(take(p.n));
     s.hist6 = reinterpret_cast<U*>(take(size_t(kBuckets) * 8));
@@ -2211,7 +2303,6 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
     const MsdPlan& P = a.plan;
     const int k = a.kmer_k, bits = P.d1 + P.d2;
     const bool own_span = a.kt && !a.kmer_spans;        // a listed bucket's k-mers span its parts
-    std::vector<unsigned> split_ids;
     auto wait_stream = [st] { return cudaStreamSynchronize(st); };
     HeldBlocks<decltype(wait_stream)> held(wait_stream);        // the sources of copies to the device
     auto h2d = [&](void* d, const void* h, size_t b) {
@@ -2239,16 +2330,30 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
             if (b.size == 0xffffffffu) return int(cudaErrorInvalidValue);       // 2^32 and more in one bucket
             const unsigned id = b.id_off & ((1u << kIdBits) - 1);
             work.push_back({b.start, b.start + b.size, 0, id, false});
-            if (own_span) {
-                const size_t per = size_t(1) << (2 * k - bits);
-                k_kmer_span<<<grid_for(per, 256), 256, 0, st>>>(a.kt, id * per, (id + 1) * per, 2);
-                note_launch();
-                split_ids.push_back(id);
-            }
         }
-        if (own_span) a.kmer_spans = 1;
     }
-    std::vector<SortRange> local;
+    const int per = 2 * k - bits;                       // s.more keeps the listed buckets, whose k-mers are 2^per each
+    auto span = [&](int mode) {
+        k_kmer_span<<<grid_for(size_t(c0.more) << per, 256), 256, 0, st>>>(a.kt, size_t(c0.more), mode, s.more, per);
+        note_launch();
+    };
+    if (own_span && c0.more) span(2);
+    if (own_span) a.kmer_spans = 1;
+    // the buckets of s.large finished; their groups of more than 1024 come back
+    size_t listed = 0;
+    auto finish = [&]() -> int {
+        MsdCounters c{};
+        c.large = listed;
+        h2d(s.counters, &c, sizeof c);
+        MsdKernels<W>::local(true, a, s, listed, sms, st);
+        MsdKernels<W>::groups(a, s, sms, st);
+        d2h(&c, s.counters, sizeof c);
+        const cudaError_t e = held.wait();
+        if (e != cudaSuccess) return int(e);
+        listed = 0;
+        if (c.mid > s.cap_mid || c.big > s.cap_big) return int(cudaErrorUnknown);
+        return take_huge(c.huge);
+    };
     // describes ranges v[i0, i1) (at most kMoreRanges) and their shifts on the device, one copy for all
     unsigned tiles = 0;
     const int* r_off = nullptr;
@@ -2267,141 +2372,126 @@ int more_splits(const MsdCounters& c0, MsdLocal a, const MsdScratch& s, uint64_t
         return r;
     };
     auto grid = [&] { return std::min(tiles, unsigned(sms * 4)); };
-    while (!work.empty() || !local.empty()) {
-        while (!work.empty()) {
-            // new elements where a range's are used up
-            std::vector<SortRange> v;
-            for (SortRange& r : work)
-                if (r.rebuild) v.push_back(r);
-            for (size_t i = 0; i < v.size(); i += kMoreRanges) {
-                const MsdRanges r = describe(v, i, std::min(v.size(), i + kMoreRanges), nullptr);
-                k_more_rebuild<<<grid(), kSplitThreads, 0, st>>>(a.pk, P, a.more_bits, r, r_off, a.buf);
-                note_launch();
-            }
-            v.clear();
-            for (SortRange& r : work) {
-                r.rebuild = false;
-                (r.end - r.start <= size_t(kLocalLarge) ? local : v).push_back(r);
-            }
-            work.clear();
-            // where the others' elements differ
-            std::vector<SortRange> split;
-            std::vector<int> shift;
-            for (size_t i = 0; i < v.size(); i += kMoreRanges) {
-                const size_t i1 = std::min(v.size(), i + kMoreRanges);
-                const MsdRanges r = describe(v, i, i1, nullptr);
-                cudaMemsetAsync(s.r_diff, 0, r.count * 8, st);
-                k_more_diff<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_diff, s.r_diff + r.count);
-                note_launch();
-                std::vector<unsigned long long> d(2 * size_t(r.count));
-                d2h(d.data(), s.r_diff, d.size() * 8);
-                const unsigned long long* const e0 = d.data() + r.count;
-                const cudaError_t e = held.wait();
-                if (e != cudaSuccess) return int(e);
-                for (int q = 0; q < r.count; ++q) {
-                    SortRange x = v[i + q];
-                    int hb = 63;
-                    while (hb > 0 && !((d[q] >> hb) & 1)) --hb;
-                    const int full = x.off ? a.more_bits / 2 : P.head;
-                    if (hb < P.len_shift && int((e0[q] >> P.len_shift) & 31) == full) {
-                        if (a.kt && !x.off) {                // one k-mer throughout
-                            const int top = 2 * k - P.d1;
-                            const uint64_t id1 = x.id >> P.d2, key = e0[q] >> P.key_shift;
-                            const uint64_t c = top >= 0 ? (id1 << top) | (key >> (P.kbits - top)) : id1 >> (-top);
-                            k_kmer_rows<<<1, 1, 0, st>>>(a.kt, size_t(c), a.row0 + x.start, a.row0 + x.end);
-                            note_launch();
-                            if (a.kx) {
-                                const size_t m = size_t(x.end - x.start);
-                                k_kx_rows<<<grid_for(m, 256), 256, 0, st>>>(
-                                    a.kx + x.start, m, uint16_t((e0[q] >> a.kx_shift) & ((1u << a.kx_bits) - 1u)));
-                                note_launch();
-                            }
-                        }
-                        x.off += full;
-                        x.rebuild = true;
-                        work.push_back(x);
-                        continue;
-                    }
-                    int sh = hb - (kMoreBits - 1);
-                    if (hb >= P.key_shift) sh = std::max(sh, P.key_shift);
-                    else if (hb >= P.len_shift) sh = P.len_shift;
-                    split.push_back(x);
-                    shift.push_back(std::max(sh, 0));
-                }
-            }
-            // split, the children's places from the counts on the device; the host learns the counts of
-            // kSplitBatch ranges (8 KB each) at a time
-            constexpr size_t kSplitBatch = 16 * kMoreSplits;
-            for (size_t z = 0; z < split.size(); z += kSplitBatch) {
-                const size_t z1 = std::min(split.size(), z + kSplitBatch);
-                std::vector<unsigned long long> cnt((z1 - z) << kMoreBits);
-                for (size_t i = z; i < z1; i += kMoreSplits) {
-                    const size_t i1 = std::min(z1, i + kMoreSplits);
-                    MsdRanges r = describe(split, i, i1, shift.data() + i);
-                    r.bits = kMoreBits;
-                    const size_t nc = (i1 - i) << kMoreBits;
-                    cudaMemsetAsync(s.r_cnt, 0, nc * 8, st);
-                    k_msd_count<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_cnt);
-                    k_msd_children<<<unsigned(i1 - i), kScanThreads, 0, st>>>(s.r_cnt, nullptr, kMoreBits, 0, r.start,
-                                                                             s.r_cursor, s.r_cursor, 0, a.G);
-                    k_msd_split<<<grid(), kSplitThreads, MsdSmem::bytes(kMoreBits, false), st>>>(a.buf, r, s.r_cursor, tmp);
-                    const cudaError_t e = cudaGetLastError();
-                    if (e != cudaSuccess) {
-                        held.wait();
-                        return int(e);
-                    }
-                    k_more_copy<<<grid(), kSplitThreads, 0, st>>>(tmp, r, a.buf);
-                    for (int q = 0; q < 4; ++q) note_launch();
-                    d2h(cnt.data() + ((i - z) << kMoreBits), s.r_cnt, nc * 8);
-                }
-                const cudaError_t e = held.wait();
-                if (e != cudaSuccess) return int(e);
-                // Children in a row of up to kMoreMerge together are one bucket of the local kernel: ten
-                // thousand equal strings split by position would else be a thousand (10 K equal reads of 100
-                // bases were 95 thousand buckets in 24 launches and 5.3 ms, now 2.3; larger buckets leave
-                // SMs idle where a chunk has few).
-                for (size_t q = z; q < z1; ++q) {
-                    const SortRange& p = split[q];
-                    SortRange run{p.start, p.start, p.off, p.id, false};
-                    auto list = [&] {
-                        if (run.end > run.start) (run.end - run.start <= size_t(kLocalLarge) ? local : work).push_back(run);
-                        run.start = run.end;
-                    };
-                    for (size_t c = (q - z) << kMoreBits; c < (q - z + 1) << kMoreBits; ++c) {
-                        if (run.end - run.start + cnt[c] > size_t(kMoreMerge)) list();
-                        run.end += cnt[c];
-                    }
-                    list();
-                }
-            }
+    while (!work.empty() || listed) {
+        if (work.empty()) {
+            if (const int rc = finish()) return rc;
+            continue;
         }
-        // every part fits the local kernel; its groups of more than 1024 come back
-        std::vector<SortRange> now;
-        now.swap(local);
-        for (size_t i = 0; i < now.size(); i += s.cap_list) {
-            const size_t i1 = std::min(now.size(), i + s.cap_list);
+        // new elements where a range's are used up
+        std::vector<SortRange> v, fits;
+        for (SortRange& r : work)
+            if (r.rebuild) v.push_back(r);
+        for (size_t i = 0; i < v.size(); i += kMoreRanges) {
+            const MsdRanges r = describe(v, i, std::min(v.size(), i + kMoreRanges), nullptr);
+            k_more_rebuild<<<grid(), kSplitThreads, 0, st>>>(a.pk, P, a.more_bits, r, r_off, a.buf);
+            note_launch();
+        }
+        v.clear();
+        for (SortRange& r : work) {
+            r.rebuild = false;
+            (r.end - r.start <= size_t(kLocalLarge) ? fits : v).push_back(r);
+        }
+        work.clear();
+        for (size_t i = 0, i1; i < fits.size(); i = i1) {
+            if (listed == s.cap_list)
+                if (const int rc = finish()) return rc;
+            i1 = std::min(fits.size(), i + s.cap_list - listed);
             std::vector<MsdBucket> b;
-            for (size_t q = i; q < i1; ++q)
-                b.push_back({now[q].start, unsigned(now[q].end - now[q].start), (unsigned(now[q].off) << kIdBits) | (now[q].off ? 0u : now[q].id)});
-            MsdCounters c{};
-            c.large = b.size();
-            h2d(s.counters, &c, sizeof c);
-            h2d(s.large, b.data(), b.size() * sizeof(MsdBucket));
-            MsdKernels<W>::local(true, a, s, b.size(), sms, st);
-            MsdKernels<W>::groups(a, s, sms, st);
-            d2h(&c, s.counters, sizeof c);
+            for (size_t q = i; q < i1; ++q) b.push_back({fits[q].start, unsigned(fits[q].end - fits[q].start), (unsigned(fits[q].off) << kIdBits) | (fits[q].off ? 0u : fits[q].id)});
+            h2d(s.large + listed, b.data(), b.size() * sizeof(MsdBucket));
+            listed += b.size();
+        }
+        // where the others' elements differ
+        std::vector<SortRange> split;
+        std::vector<int> shift;
+        for (size_t i = 0; i < v.size(); i += kMoreRanges) {
+            const size_t i1 = std::min(v.size(), i + kMoreRanges);
+            const MsdRanges r = describe(v, i, i1, nullptr);
+            cudaMemsetAsync(s.r_diff, 0, r.count * 8, st);
+            k_more_diff<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_diff, s.r_diff + r.count);
+            note_launch();
+            std::vector<unsigned long long> d(2 * size_t(r.count));
+            d2h(d.data(), s.r_diff, d.size() * 8);
+            const unsigned long long* const e0 = d.data() + r.count;
             const cudaError_t e = held.wait();
             if (e != cudaSuccess) return int(e);
-            if (c.mid > s.cap_mid || c.big > s.cap_big) return int(cudaErrorUnknown);
-            const int rc = take_huge(c.huge);
-            if (rc) return rc;
+            for (int q = 0; q < r.count; ++q) {
+                SortRange x = v[i + q];
+                int hb = 63;
+                while (hb > 0 && !((d[q] >> hb) & 1)) --hb;
+                const int full = x.off ? a.more_bits / 2 : P.head;
+                if (hb < P.len_shift && int((e0[q] >> P.len_shift) & 31) == full) {
+                    if (a.kt && !x.off) {                // one k-mer throughout
+                        const int top = 2 * k - P.d1;
+                        const uint64_t id1 = x.id >> P.d2, key = e0[q] >> P.key_shift;
+                        const uint64_t c = top >= 0 ? (id1 << top) | (key >> (P.kbits - top)) : id1 >> (-top);
+                        k_kmer_rows<<<1, 1, 0, st>>>(a.kt, size_t(c), a.row0 + x.start, a.row0 + x.end);
+                        note_launch();
+                        if (a.kx) {
+                            const size_t m = size_t(x.end - x.start);
+                            k_kx_rows<<<grid_for(m, 256), 256, 0, st>>>(
+                                a.kx + x.start, m, uint16_t((e0[q] >> a.kx_shift) & ((1u << a.kx_bits) - 1u)));
+                            note_launch();
+                        }
+                    }
+                    x.off += full;
+                    x.rebuild = true;
+                    work.push_back(x);
+                    continue;
+                }
+                int sh = hb - (kMoreBits - 1);
+                if (hb >= P.key_shift) sh = std::max(sh, P.key_shift);
+                else if (hb >= P.len_shift) sh = P.len_shift;
+                split.push_back(x);
+                shift.push_back(std::max(sh, 0) | int((x.off ? 0u : x.id) << 6));
+            }
+        }
+        // split, their children's places and buckets from the counts on the device: as many ranges at a
+        // time as there is room for their counts and, at most, for their buckets
+        for (size_t i = 0, i1; i < split.size(); i = i1) {
+            size_t most = listed;
+            for (i1 = i; i1 < split.size() && i1 - i < s.splits; ++i1) {
+                const size_t n = size_t(split[i1].end - split[i1].start);
+                const size_t b = std::min(size_t(1) << kMoreBits, n / kMoreMerge + 2 * (n / (kLocalLarge - kMoreMerge)) + 2);
+                if (most + b > s.cap_list) break;
+                most += b;
+            }
+            if (i1 == i) {
+                if (const int rc = finish()) return rc;
+                continue;
+            }
+            MsdRanges r = describe(split, i, i1, shift.data() + i);
+            r.bits = kMoreBits;
+            cudaMemsetAsync(s.r_lists, 0, al(sizeof(MoreLists)) + ((i1 - i) << kMoreBits) * 8, st);
+            k_msd_count<<<grid(), kSplitThreads, 0, st>>>(a.buf, r, s.r_cnt);
+            k_more_list<<<unsigned(i1 - i), kScanThreads, 0, st>>>(s.r_cnt, r, r_off, s.r_cursor, unsigned(listed), s.large,
+                                                                  unsigned(s.cap_list), s.again, unsigned(s.cap_more), s.r_lists);
+            k_msd_split<<<grid(), kSplitThreads, MsdSmem::bytes(kMoreBits, false), st>>>(a.buf, r, s.r_cursor, tmp);
+            cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) {
+                held.wait();
+                return int(e);
+            }
+            k_more_copy<<<grid(), kSplitThreads, 0, st>>>(tmp, r, a.buf);
+            for (int q = 0; q < 4; ++q) note_launch();
+            MoreLists c;
+            d2h(&c, s.r_lists, sizeof c);
+            e = held.wait();
+            if (e != cudaSuccess) return int(e);
+            if (listed + c.large > s.cap_list || c.more > s.cap_more) return int(cudaErrorUnknown);
+            listed += size_t(c.large);
+            std::vector<MsdBucket> again(c.first, c.first + std::min<size_t>(c.more, 256));
+            if (c.more > again.size()) {
+                again.resize(c.more);
+                d2h(again.data(), s.again, c.more * sizeof(MsdBucket));
+                e = held.wait();
+                if (e != cudaSuccess) return int(e);
+            }
+            for (const MsdBucket& b : again)
+                work.push_back({b.start, b.start + b.size, int(b.id_off >> kIdBits), b.id_off & ((1u << kIdBits) - 1), false});
         }
     }
-    for (unsigned id : split_ids) {
-        const size_t per = size_t(1) << (2 * k - bits);
-        k_kmer_span<<<grid_for(per, 256), 256, 0, st>>>(a.kt, id * per, (id + 1) * per, 1);
-        note_launch();
-    }
+    if (own_span && c0.more) span(1);
     return int(cudaGetLastError());
 }
 
@@ -2697,7 +2787,7 @@ static int sort_msd(const SortShape& sh, size_t nr, const MsdScratch& s, SortOut
     if (!o.kx_bases) o.kx = nullptr;
     const bool spans = o.kmer_spans = o.kmer_k <= P.S || 2 * o.kmer_k < std::max(P.d1 + P.d2, sh.chunked ? 2 * kBucketBases : 0);
     const size_t nk = size_t(1) << (2 * o.kmer_k);
-    if (o.kt && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kt, 0, nk, 0); note_launch(); }
+    if (o.kt && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kt, nk, 0, nullptr, 0); note_launch(); }
     if (o.kt && !spans) {
         const cudaError_t e = kmer_table_clear(o.kmer_k, o.kt, st);
         if (e != cudaSuccess) return int(e);
@@ -2739,7 +2829,7 @@ static int sort_msd(const SortShape& sh, size_t nr, const MsdScratch& s, SortOut
             lo = hi;
         }
     }
-    if (o.kt && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kt, 0, nk, 1); note_launch(); }
+    if (o.kt && spans) { k_kmer_span<<<grid_for(nk, 256), 256, 0, st>>>(o.kt, nk, 1, nullptr, 0); note_launch(); }
     o.kmer_done = o.kt != nullptr;
     return int(cudaGetLastError());
 }
