@@ -284,7 +284,11 @@ __device__ __forceinline__ int meta_type(uint32_t m) { return int(m >> 16); }
 
 constexpr int kScanWords = 2;       // bases of P_t searched by bisection: the first 64 at most
 constexpr int kScanMax = 256;       // larger depth-t intervals walk instead
-constexpr int kScanDirect = 48;     // rows checked without narrowing them to I_t first
+constexpr int kScanDirect = 48;     // rows checked without narrowing them to I_t first,
+constexpr int kScanBare = 8;        // where no next bases have narrowed them and every warp has 32 reads: a row
+                                    // of a k-mer is then of I_t by chance only (0.4 M reads of 76 random bases, 20 %
+                                    // GC: 0.41 ms with 48, 0.23; 30x of a genome 0.39 and 0.34), while fewer reads
+                                    // a warp wait for the bisection (20 thousand reads: 0.10 with 48, 0.12)
 
 // 64 bases of packed text starting at base p (first base in the top bits)
 __device__ __forceinline__ uint64_t text_window(const uint64_t* __restrict__ pk, size_t p) {
@@ -1808,7 +1812,9 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                     }
                     narrow_rows(*f0, k, t, P0[0], first[0], end[0], probes);
                     narrow_rows(*f1, k, t, P1[0], first[1], end[1], probes);
-                    if (ok && (end[0] - first[0] > idx_t(kScanDirect) || end[1] - first[1] > idx_t(kScanDirect))) {
+                    const int bare = per < 32 || t == k ? kScanDirect : kScanBare;
+                    if (ok && (end[0] - first[0] > idx_t(f0->kx_bases ? kScanDirect : bare) ||
+                               end[1] - first[1] > idx_t(f1->kx_bases ? kScanDirect : bare))) {
                         const idx_t lo[2] = {first[0], first[1]}, hi[2] = {end[0], end[1]};
                         sa_bounds2(f0, f1, A.dl, P0, P1, t < 32 * kScanWords ? t : 32 * kScanWords, lo, hi, first, end, probes);
                         ok = end[0] - first[0] <= idx_t(kScanMax) && end[1] - first[1] <= idx_t(kScanMax);
