@@ -1493,7 +1493,6 @@ static int batched_once(pq_ctx** ctxs, int count, int flags) {
     }
     cudaSetDevice(lead->device);
     std::vector<pq::SearchBatch> hb(count);
-    int L_max = 1, M_max = 1;
     for (int b = 0; b < count; ++b) {
         const int rc = search_prepare(ctxs[b], hb[b].a, hb[b].o);
         if (rc != PQ_OK) {
@@ -1502,8 +1501,6 @@ static int batched_once(pq_ctx** ctxs, int count, int flags) {
         }
         if (ctxs[b]->st != lead->st && cudaStreamSynchronize(ctxs[b]->st) != cudaSuccess)
             return fail(lead, PQ_ERR_CUDA, "batch stream synchronisation failed");
-        L_max = std::max(L_max, ctxs[b]->L);
-        M_max = std::max(M_max, ctxs[b]->L - ctxs[b]->t);
     }
     // batches longest reads first (they take longest); items are built per class in queue_launch
     std::vector<int> order(count);

@@ -108,15 +108,6 @@ __device__ __forceinline__ uint32_t rel_cnt(uint32_t c01, uint32_t c23, int c) {
     return ((c & 1) ? w : (w >> 16)) & 0xffff;
 }
 
-// rank of base c (1..4) in BWT[0, pos), without the fix offset
-__device__ __forceinline__ idx_t rank_c(const FmView& f, int c, idx_t pos) {
-    uint64_t lo, hi, dol;
-    uint32_t c01, c23;
-    ld_block(f.blk + (pos >> kBlockShift), lo, hi, dol, c01, c23);
-    idx_t s = __ldg(f.sb + size_t(pos >> kSuperShift) * 4 + (c - 1));
-    return s + rel_cnt(c01, c23, c) + idx_t(__popcll(match(lo, hi, dol, c) & below(pos)));
-}
-
 // ranks of all four bases in BWT[0, pos)
 __device__ __forceinline__ void rank_all(const FmView& f, idx_t pos, idx_t r[4]) {
     uint64_t lo, hi, dol;
@@ -144,43 +135,6 @@ __device__ __forceinline__ idx_t rank_dollar(const FmView& f, idx_t pos) {
     idx_t r[4];
     rank_all(f, pos, r);
     return pos - (r[0] + r[1] + r[2] + r[3]);
-}
-
-// search_1: LF-map the closed interval [l, u] by base c
-__device__ __forceinline__ void lf_step(const FmView& f, int c, idx_t& l, idx_t& u, Tally& probes) {
-    idx_t ol = rank_c(f, c, l);
-    idx_t ou = rank_c(f, c, u + 1);
-    probes += 2;
-    l = f.Cf[c] + ol;
-    u = f.Cf[c] + ou - 1;
-}
-
-// search_2: step on this index by c, keep the other index's interval [ll, uu] in sync.
-// #symbols < c in [l, u] ($ included) = (pos - sum_{k>=c} rank_k) differences; fixes cancel.
-__device__ __forceinline__ void bi_step(const FmView& f, int c, idx_t& l, idx_t& u, idx_t& ll, idx_t& uu,
-                                        Tally& probes) {
-    idx_t vl = l, vu = u + 1;
-    idx_t rl[4], ru[4];
-    rank_all(f, vl, rl);
-    rank_all(f, vu, ru);
-    probes += 2;
-    idx_t gel = 0, geu = 0;
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (k + 1 >= c) { gel += rl[k]; geu += ru[k]; }
-    }
-    idx_t less_l = vl - gel, less_u = vu - geu;
-    ll = ll + (less_u - less_l);
-    idx_t ol = rl[c - 1], ou = ru[c - 1];
-    l = f.Cf[c] + ol;
-    u = f.Cf[c] + ou - 1;
-    uu = ll + ou - ol - 1;
-}
-
-// search_3: (#$ in [l, u]) - 1, wrapping to all-ones at zero
-__device__ __forceinline__ idx_t dollars_m1(const FmView& f, idx_t l, idx_t u, Tally& probes) {
-    probes += 2;
-    return rank_dollar(f, u + 1) - rank_dollar(f, l) - 1;
 }
 
 // ------------------------------------------------------------------------------ per-read search
