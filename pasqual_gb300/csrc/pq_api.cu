@@ -932,7 +932,7 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool 
         // heavy tier (the fast kernel's DFS with larger capacities) over the reads the fast tier
         // could not hold; what it cannot hold either goes on to the wide tier
         const int hebcap = 4096;
-        const int hblocks = int(std::min<size_t>((size_t(ovf) + 127) / 128, size_t(152) * 2));
+        const int hblocks = pq::heavy_blocks(ovf);
         const size_t hbytes = pq::heavy_scratch_bytes(ctx->L, ctx->t, hblocks, hebcap);
         CK(ctx->heavy_scratch.ensure(hbytes));
         CK(ctx->ovf2.ensure(nrp * sizeof(idx_t)));
@@ -941,7 +941,7 @@ static int search_finish(pq_ctx* ctx, pq::SearchArgs& A, pq::SearchOut& O, bool 
         O2.ovf_count = reinterpret_cast<unsigned int*>(ctr + 5);
         CK(cudaMemsetAsync(ctr + 5, 0, sizeof(unsigned long long), ctx->st));
         // the heavy tier's list: the block tiers' leftovers, or the fast tier's own
-        CK(pq::search_heavy(A, O2, ovf_src, ovf_cnt, hblocks, ctx->heavy_scratch.p, hbytes, hebcap, ctx->st));
+        CK(pq::search_heavy(A, O2, ovf_src, ovf_cnt, ovf, hblocks, ctx->heavy_scratch.p, hbytes, hebcap, ctx->st));
         unsigned long long h5 = 0;
         CK(cudaMemcpyAsync(&h5, ctr + 5, sizeof h5, cudaMemcpyDeviceToHost, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));

@@ -129,6 +129,7 @@ struct SearchQueue {
     // without a queue: search only the reads read_list[0, *list_count) (nullptr: every read)
     const idx_t* read_list;
     const unsigned* list_count;
+    unsigned per;               // reads of a warp's group (32, less where there are few for the fast kernels)
     int dfs_max;                // level-0 intervals a (read, side) of the FM-index DFS may have
 };
 size_t warp_scratch_bytes(int L, int t, size_t nwarps, int ebcap);
@@ -160,8 +161,9 @@ cudaError_t search_block_global(const SearchArgs& a, const SearchOut& o, const i
                                 idx_t* next_list, unsigned* next_count, cudaStream_t st);
 // Heavy tier over reads[0, *count) with a wider DFS (reads the fast or block tiers could not hold).
 size_t heavy_scratch_bytes(int L, int t, int blocks, int ebcap);
-cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* list, const unsigned* count, int blocks,
-                         void* scratch, size_t scratch_bytes, int ebcap, cudaStream_t st);
+int heavy_blocks(unsigned count);
+cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* list, const unsigned* count, unsigned count_host,
+                         int blocks, void* scratch, size_t scratch_bytes, int ebcap, cudaStream_t st);
 // One persistent lean launch over a queue of batches (M_max: the largest L - t).
 cudaError_t search_lean_queue(const SearchQueue& q, int M_max, int blocks, void* scratch, size_t scratch_bytes, int ebcap,
                               cudaStream_t st);

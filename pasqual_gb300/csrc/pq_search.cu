@@ -1219,7 +1219,7 @@ __global__ void __launch_bounds__(128, 5) k_search_fast(SearchArgs A0, SearchOut
             }
         }
         const size_t n_items = Q.read_list ? list_n : size_t(A.num_reads);
-        const size_t groups = (n_items + 31) / 32;
+        const size_t groups = (n_items + Q.per - 1) / Q.per;
         if (!Q.count || gend > groups) gend = groups;
         const int M = A.L - A.t;
         const int L = A.L;
@@ -1232,8 +1232,8 @@ __global__ void __launch_bounds__(128, 5) k_search_fast(SearchArgs A0, SearchOut
         while (true) {
             if (!__any_sync(0xffffffffu, pend)) {
                 if (group >= gend || nq + 32 > kFastQueue) break;
-                const size_t item = group * 32 + lane;
-                pend = item < n_items;
+                const size_t item = group * Q.per + lane;
+                pend = unsigned(lane) < Q.per && item < n_items;
                 group += step;
                 if (pend) {
                     pr = Q.read_list ? Q.read_list[item] : idx_t(item);
@@ -2003,6 +2003,7 @@ cudaError_t search_fast(const SearchArgs& a, const SearchOut& o, int blocks, voi
     SearchQueue Q{};
     Q.read_list = list;
     Q.list_count = count;
+    Q.per = 32;
     Q.dfs_max = list ? 0 : kTaskCap;        // of listed reads (the lean tier's misses) the sorted reduction only
     if (lam_words(a.L - a.t) == 2) k_search_fast<2, kTaskCap, kTaskFrames, kPMax><<<blocks, 32 * kWarpsPerCta, smem, st>>>(a, o, S, Q);
     else k_search_fast<kLamWords, kTaskCap, kTaskFrames, kPMax><<<blocks, 32 * kWarpsPerCta, smem, st>>>(a, o, S, Q);
@@ -2957,7 +2958,16 @@ size_t heavy_scratch_bytes(int L, int t, int blocks, int ebcap) {
                           kHeavyPMax);
 }
 
-cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* list, const unsigned* count, int blocks,
+// A step of a warp takes as long as the intervals of all its reads, so few reads are spread over up to 512
+// warps (8 MB of scratch each), 4 reads a warp or more: 3.8 thousand run reads of 320 bases at t = 30 took
+// 600 ms with 32 a warp, now 288.
+static int heavy_reads(unsigned count) { return int(std::min(32u, std::max(4u, (count + 511) / 512))); }
+int heavy_blocks(unsigned count) {
+    const unsigned per = unsigned(heavy_reads(count)), warps = (count + per - 1) / per;
+    return int(std::min((warps + kWarpsPerCta - 1) / kWarpsPerCta, 152u * 2));
+}
+
+cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* list, const unsigned* count, unsigned count_host, int blocks,
                          void* scratch, size_t scratch_bytes, int ebcap, cudaStream_t st) {
     WarpScratch S;
     if (scratch_bytes < scratch_layout(a.L - a.t, size_t(blocks) * kWarpsPerCta, ebcap, scratch, &S, kHeavyCap,
@@ -2968,6 +2978,7 @@ cudaError_t search_heavy(const SearchArgs& a, const SearchOut& o, const idx_t* l
     SearchQueue Q{};
     Q.read_list = list;
     Q.list_count = count;
+    Q.per = unsigned(heavy_reads(count_host));
     Q.dfs_max = kHeavyCap;
     // static shared memory (~46 KB) plus the reads: past the 48 KB a launch may take unasked
     constexpr size_t kReadSmem = 180 * 1024;            // reads of up to 5760 bases
@@ -2997,6 +3008,7 @@ cudaError_t search_fast_queue(const SearchQueue& queue, int L_max, int M_max, in
     const int words = (L_max + 15) / 16;
     size_t smem = size_t(words) * 32 * kWarpsPerCta * sizeof(uint32_t);
     SearchQueue q = queue;
+    q.per = 32;
     q.dfs_max = kTaskCap;
     SearchArgs a{};
     SearchOut o{};
@@ -3006,16 +3018,19 @@ cudaError_t search_fast_queue(const SearchQueue& queue, int L_max, int M_max, in
     return cudaGetLastError();
 }
 
-// Wide tier: the reference's own capacity bounds, scratch in global memory, one slot per thread.
+// Wide tier: the reference's own capacity bounds, scratch in global memory, one slot per thread, `lanes`
+// of them a warp.  Threads of one warp go through their reads' DFS one after the other (they seldom stand at
+// the same instruction), so a warp takes one read while there are warps: 13 run reads of 306 bases took
+// 1.3 s in one warp, now 0.22.
 __global__ void __launch_bounds__(64) k_search_wide(SearchArgs A, SearchOut O, const idx_t* list, unsigned count,
-                                                    WideScratch W) {
+                                                    WideScratch W, int lanes) {
     extern __shared__ uint32_t s_reads[];
     __shared__ FmView s_fm[2];
     if (threadIdx.x < 2) s_fm[threadIdx.x] = A.fm[threadIdx.x];
     __syncthreads();
-    const unsigned slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned slot = (blockIdx.x * blockDim.x + threadIdx.x) / 32 * unsigned(lanes) + (threadIdx.x & 31u);
     Tally probes;
-    if (slot < unsigned(W.slots)) {
+    if (int(threadIdx.x & 31u) < lanes && slot < unsigned(W.slots)) {
         Cand* stk = reinterpret_cast<Cand*>(W.stack) + size_t(slot) * W.stack_cap;
         Frame* fr = reinterpret_cast<Frame*>(W.frames) + size_t(slot) * W.frame_cap;
         EdgeRec* eb = reinterpret_cast<EdgeRec*>(W.edges) + size_t(slot) * W.edge_cap;
@@ -3065,8 +3080,12 @@ cudaError_t search_wide(const SearchArgs& a, const SearchOut& o, const idx_t* li
     const int tpb = 64;
     const int words = (a.L + 15) / 16;
     size_t smem = size_t(words) * tpb * sizeof(uint32_t);
-    int blocks = (ws.slots + tpb - 1) / tpb;
-    { k_search_wide<<<blocks, tpb, smem, st>>>(a, o, list, count, ws); note_launch(); }
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int lanes = std::min(32, (ws.slots + 16 * sms - 1) / (16 * sms));
+    const int warps = (ws.slots + lanes - 1) / lanes;
+    { k_search_wide<<<(warps + 1) / 2, tpb, smem, st>>>(a, o, list, count, ws, lanes); note_launch(); }
     return cudaGetLastError();
 }
 
