@@ -7,13 +7,14 @@
 // with the rank primitives OCCx/search_1/search_2/search_3 (src/string_graph.c:11-159) on the
 // one-sector occ blocks of pq_common.cuh.
 //
-// One thread searches one read.  The reference's recursion becomes an explicit stack: candidate
-// intervals of every open level live in a per-thread array laid out exactly as the reference's
-// I_fw/I_bw (a level's children directly after it), and one frame per level remembers which
-// extension base comes next.  The fast kernel keeps stack, frames and edge buffer in local
-// memory with fixed capacities; a read that outgrows any of them is recorded and redone by the
-// wide kernel, whose per-slot scratch has the reference's own bounds ((2L)^2 candidates,
-// 65535 edges per side), so every read completes with the reference's result.
+// Tiers, each of which lists the reads it cannot hold for a later one, so that every read completes
+// with the reference's result: the lean tier (a warp takes up to 32 reads' rows of the suffix array and
+// reduces their candidates by sorted continuations), the block tier (a CTA a read, the same by sorting in
+// shared or global memory), the fast and the heavy tier (the reference's walk and DFS, a read a lane,
+// intervals spread over the warp), and the wide tier, one thread a read: candidate intervals of every open
+// level in an array laid out as the reference's I_fw/I_bw (a level's children directly after it), one frame per
+// level for the extension base that comes next, and the reference's own bounds ((2L)^2 candidates, 65535
+// edges per side).
 #include "pq_index.cuh"
 #include "pq_learned.cuh"
 
@@ -48,7 +49,7 @@ struct EdgeRec {
 
 // Per-thread counters of a search: rank probes (one occurrence block each, the unit of the
 // reference's OCCx/search_* calls) and the 32-byte sectors of every global load of index data the
-// method issues -- occurrence blocks, k-mer table entries, suffix-array and inverse-SA entries,
+// method issues -- occurrence blocks, k-mer table entries and next bases, suffix-array entries,
 // packed-text words, reads_index entries and read bytes.  Tables that stay resident in L2 (the
 // superblock counts, learned models) and the search's own scratch are not counted.  `+= n` is n
 // rank probes, one sector each (an occurrence block is one aligned sector).
@@ -239,12 +240,13 @@ __device__ __forceinline__ int meta_type(uint32_t m) { return int(m >> 16); }
 constexpr int kScanWords = 2;       // bases of P_t searched by bisection: the first 64 at most
 constexpr int kScanMax = 256;       // larger depth-t intervals walk instead
 constexpr int kScanDirect = 48;     // rows checked without narrowing them to I_t first,
-constexpr int kScanBare = 8;        // where no next bases have narrowed them and every warp has 32 reads: a row
-                                    // of a k-mer is then of I_t by chance only (0.4 M reads of 76 random bases, 20 %
-                                    // GC: 0.41 ms with 48, 0.23; 30x of a genome 0.39 and 0.34), while fewer reads
-                                    // a warp wait for the bisection (20 thousand reads: 0.10 with 48, 0.12)
+constexpr int kScanBare = 8;        // where no next bases have narrowed them: a row of a k-mer may be of I_t by
+                                    // chance only (0.4 M reads of 76 random bases, 20 % GC: 0.41 ms with 48, 0.23; 30x
+                                    // of a genome, 100 bases, 0.38 and 0.33).  Not where a warp has fewer than 32 reads,
+                                    // which wait for the bisection (20 thousand reads: 0.10 with 48, 0.12), nor for reads
+                                    // of up to 64 bases, whose k-mers have few rows (61 bases at 20x: 0.28 and 0.30)
 
-// 64 bases of packed text starting at base p (first base in the top bits)
+// 32 bases of packed text starting at base p (first base in the top bits)
 __device__ __forceinline__ uint64_t text_window(const uint64_t* __restrict__ pk, size_t p) {
     const size_t w = p >> 5;
     const int s = int(p & 31) * 2;
@@ -1766,7 +1768,7 @@ __global__ void __launch_bounds__(kLeanThreads, 8) k_search_lean(SearchArgs A0, 
                     }
                     narrow_rows(*f0, k, t, P0[0], first[0], end[0], probes);
                     narrow_rows(*f1, k, t, P1[0], first[1], end[1], probes);
-                    const int bare = per < 32 || t == k ? kScanDirect : kScanBare;
+                    const int bare = per < 32 || L <= 64 || t == k ? kScanDirect : kScanBare;
                     if (ok && (end[0] - first[0] > idx_t(f0->kx_bases ? kScanDirect : bare) ||
                                end[1] - first[1] > idx_t(f1->kx_bases ? kScanDirect : bare))) {
                         const idx_t lo[2] = {first[0], first[1]}, hi[2] = {end[0], end[1]};

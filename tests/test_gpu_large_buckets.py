@@ -33,14 +33,14 @@ def suffix_words(rd, backward):
     return w[0, :, :L].ravel(), w[1, :, :L].ravel(), length.ravel()
 
 
-# 28 kinds of 50 bases: 1,400 buckets of 12 thousand suffixes, of which 257 and more at a time have a part that is
-# too large once more
+# 32 kinds of 50 bases: 1,600 buckets of 12 thousand suffixes, 293 of which are split at a time, each with a part that
+# is too large once more
 @pytest.mark.parametrize("name", ["gc05", "gc25", "copies", "copies_few"])
 @pytest.mark.parametrize("width", [32, 64])
 def test_large_buckets(name, width):
     rng = np.random.default_rng(17)
     rd = {"gc05": lambda: skewed(250_000, 40, 0.05, rng), "gc25": lambda: skewed(600_000, 40, 0.25, rng),
-          "copies": lambda: copies(28, 12_000, 50, 0.004, rng), "copies_few": lambda: copies(3, 30_000, 33, 0.002, rng)}[name]()
+          "copies": lambda: copies(32, 12_000, 50, 0.004, rng), "copies_few": lambda: copies(3, 30_000, 33, 0.002, rng)}[name]()
     with pq.Pasqual(width) as P:
         P.set_reads(rd, 20)
         P.set_seed_k(11)
