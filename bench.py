@@ -472,10 +472,10 @@ def run_ours(args):
     kms = statistics.median(kern_ms)
     alg_bytes = 32.0 * sec + outb
     achieved = alg_bytes / (kms * 1e-3) / 1e9
-    dram_per_read = profile_figure("k_search_lean_250Mbp_L100.md", "dram_bytes_per_read")
+    dram_per_read = profile_figure("search_kernels.md", "dram_bytes_per_read")
     # the committed capture describes this launch only if its kernel did the same work per read
     # (same algorithmic bytes, within 5 %): otherwise no traffic figure is claimed
-    cap_alg = profile_figure("k_search_lean_250Mbp_L100.md", "algorithmic_bytes_per_read")
+    cap_alg = profile_figure("search_kernels.md", "algorithmic_bytes_per_read")
     traffic_applies = bool(dram_per_read and cap_alg and args.seed_mode == 1 and
                            abs(alg_bytes / nr - cap_alg) <= 0.05 * cap_alg)
 
@@ -536,8 +536,7 @@ def run_ours(args):
     cb = None
     if world == 1 and not args.no_cpu_baseline:
         cb = cpu_baseline(args.workload, args.cpu_scale, args.cpu_seconds)
-    ref_ppr = cb["probes_per_read"] if cb else profile_figure("k_search_lean_250Mbp_L100.md",
-                                                               "reference_probes_per_read")
+    ref_ppr = cb["probes_per_read"] if cb else profile_figure("search_kernels.md", "reference_probes_per_read")
     out = {
         "metric": METRIC, "value": r4(replica_throughput(nr, world, step_ms)), "unit": "reads/s",
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": r4(step_ms),
@@ -581,8 +580,8 @@ def run_ours(args):
     out["sort_msuffix_per_s"] = r4(2 * n / (sort_ms_med * 1e-3) / 1e6)
     # the sort against its algorithmic bytes: per suffix, the 2-bit text of the prefix that tells
     # it apart from its neighbours plus one suffix-array entry (measured on the oracle's suffix
-    # arrays of a sample of this workload, recorded with the launch list)
-    sbytes = (profile_figure("launches_250Mbp_L100_full.md", "sort_bytes_per_suffix")
+    # arrays of a sample of this workload, recorded with its counters)
+    sbytes = (profile_figure("sort_and_block_kernels.md", "sort_bytes_per_suffix")
               if args.workload == "250Mbp_L100_20x_t55" else None)
     if sbytes:
         sach = sbytes * 2 * n / (sort_ms_med * 1e-3) / 1e9

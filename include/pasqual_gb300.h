@@ -171,8 +171,8 @@ PQ_API int pq_get_graph_sizes (pq_ctx * ctx, uint64_t * num_edges, uint64_t * pr
                         uint64_t * wide_reads);
 
 /* Memory traffic of the last pq_overlaps, as the method in use defines it: load_sectors = the
- * 32-byte sectors of index data its kernels loaded (occurrence blocks, k-mer table, suffix-array
- * and inverse-SA entries, packed-text words, reads_index entries, read bytes; every load counted
+ * 32-byte sectors of index data its kernels loaded (occurrence blocks, k-mer table and next bases,
+ * suffix-array entries, packed-text words, reads_index entries, read bytes; every load counted
  * where it is issued, so a sector loaded twice counts twice; tables that stay in L2 -- superblock
  * counts, learned models -- and the kernels' own scratch are not counted); store_bytes = the
  * bytes of per-read results and edges the search kernels write.  32 * load_sectors + store_bytes

@@ -297,7 +297,7 @@ class Pasqual:
         self._ck(self.lib.pq_set_seed_mode(self.h, int(mode)), "pq_set_seed_mode")
 
     def set_sort_chunk(self, max_suffixes: int) -> None:
-        """Sort in chunks of at most this many suffixes (0: one pass up to 2^31 - 1)."""
+        """Sort at most this many suffixes at a time where more would take more memory (0: as it allows)."""
         self._ck(self.lib.pq_set_sort_chunk(self.h, int(max_suffixes)), "pq_set_sort_chunk")
 
     def sort(self, direction: int) -> None:

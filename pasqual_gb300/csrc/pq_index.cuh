@@ -6,7 +6,7 @@ namespace pq {
 
 // FM-index build from a suffix array (pq_index.cu)
 // pk: the packed text of direction dir (preferred for the BWT gathers), or nullptr; hint: the
-// sort's per-row BWT symbols (0xff = none), or nullptr
+// sort's BWT symbols, one of 0..4 for every row, or nullptr
 cudaError_t build_occ(const idx_t* sa, const uint8_t* reads, idx_t num_reads, idx_t L, int dir,
                       OccBlock* blk, idx_t* sb, idx_t* reads_index, cudaStream_t st, const uint64_t* pk = nullptr,
                       const uint8_t* hint = nullptr);
@@ -52,7 +52,7 @@ struct SearchOut {
     int32_t* olp_B;
     int32_t* olp_F;
     uint8_t* status;            // OVF_* / ERR_* per read (0 = done)
-    unsigned long long* edge_src;  // per read: offset into pool 1, or (1<<63 | offset) into pool 2
+    unsigned long long* edge_src;  // per read: its first edge in the pool
     // edge pool (struct of arrays)
     idx_t* e_dest;
     int32_t* e_trans;
@@ -60,7 +60,7 @@ struct SearchOut {
     uint8_t* e_type;
     unsigned long long* e_count;   // atomic bump counter
     unsigned long long e_cap;
-    idx_t* ovf_list;               // reads handed to the wide kernel
+    idx_t* ovf_list;               // reads handed to the next tier
     unsigned int* ovf_count;
     unsigned long long* probes;    // total rank probes (one 32-byte sector each)
     unsigned long long* sectors;   // total 32-byte sectors of index data loaded (see Tally)
@@ -76,7 +76,7 @@ struct SearchArgs {
     int seed_k;                 // k-mer seed depth (0 = start at depth 1 from C[])
     int sa_seed;                // 1: candidates by depth-t interval scan (needs fm[].sa/pk),
                                 // 2: the same with learned windows (needs fm[].lx)
-    unsigned long long* lx_misses;  // learned windows that missed (those chains walk)
+    unsigned long long* lx_misses;  // learned windows that missed (those reads walk)
     int sorted_reduce;          // 1: edges from sorted continuations (L - t <= 256)
     idx_t* miss_list;           // lean tier: the reads its scan does not serve go here, not to ovf_list
     unsigned* miss_count;       //   (nullptr: there with the others)
